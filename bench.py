@@ -328,18 +328,19 @@ class Job:
         self.stream = torch.cuda.Stream(device=device)
         self.fwd.stream = self.stream.cuda_stream
         self.graph = None
-        self.launches_per_step = 0
+        self.launches_per_step = self.kernels_per_step = 0
 
     def step(self):
         """One token: every layer's append + attention, recorded by one library call."""
         self.fwd.decode_token(self.q, self.k, self.v, self.out, None, self.pos, self.batch, self.max_len)
 
     def count_launches(self):
-        n0 = self.ctx.launch_count()
+        n0, k0 = self.ctx.launch_count(), self.ctx.kernel_count()
         with self.torch.cuda.stream(self.stream):
             self.step()
         self.torch.cuda.synchronize()
-        self.launches_per_step = self.ctx.launch_count() - n0       # kernels of libvfkv.so per token
+        self.launches_per_step = self.ctx.launch_count() - n0       # per token, one per layer that a kernel carries
+        self.kernels_per_step = self.ctx.kernel_count() - k0        # kernels of libvfkv.so per token
         return self.launches_per_step
 
     def capture(self):
@@ -903,7 +904,7 @@ def run_ours(args, w, rank, world, local_rank):
     run = job.graph.replay if job.graph is not None else job.step
     ms, blocks, total_ms = timed_blocks(run, job.stream, args.steps, args.warmup, dist)
     clocks = sampler.finish()
-    launches = job.launches_per_step * args.steps * blocks
+    launches = job.kernels_per_step * args.steps * blocks
     ms_stream = ms
     if job.graph is not None:                                  # same steps, one launch call per kernel
         ms_stream, _, _ = timed_blocks(job.step, job.stream, args.steps, 3, dist, 100.0)
@@ -951,15 +952,16 @@ def run_ours(args, w, rank, world, local_rank):
         split = prof.get("fa_split")
         roofline = None
         if split:
-            # The timed region launches one kernel per layer-step and nothing else (append and merge
-            # are fused into it), so its mean launch duration inside the region is region time /
-            # launches; consecutive launches overlap under dependent launch, which per-launch event
-            # pairs (kept in "kernels", measured in a separate pass) cannot show.
+            # The timed region launches the fused kernel (append and merge are in it) and nothing else,
+            # one launch for all layers with the same window, so the time of a layer-step inside the
+            # region is region time / layers; per-launch event pairs are kept in "kernels".
             fused = job.launches_per_step == w["n_layers"]
             mean_us = ms * 1e3 / (args.steps * w["n_layers"]) if fused else split["mean_us"]
             roofline = roofline_of(w, job.lens, mean_us, peak, peak_kind, NCU_TRAFFIC_BYTES.get(args.workload))
             roofline["kernel"] = "attn_split_mma_kernel (fa_split: append + attention + merge)" if fused else "fa_split"
             roofline["mean_launch_us_isolated_events"] = split["mean_us"]
+            # "launch" in this object's keys is one layer-step; this many of them share a kernel
+            roofline["layers_per_kernel"] = job.launches_per_step / max(job.kernels_per_step, 1)
         step_bytes = sum(algorithmic_bytes(w, job.lens, l) for l in range(w["n_layers"]))
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": False,

@@ -310,7 +310,8 @@ int32_t vfkv_decode_step(vfkv_cache *cache, vfkv_workspace *ws, uint32_t layer,
 /* The decode step for every layer of one token, device buffers: d_q, d_out
  * [n_layers][n_seqs][n_q_heads][D]; d_k, d_v [n_layers][n_seqs][kv_heads][D].  One call records
  * what record_decode_dispatches (src/backend/vulkan/forward/decode.rs:43-82) records for this
- * path: per layer, KvWrite then Attention.  windows: NULL, or n_layers host entries (0 = global
+ * path: per layer, KvWrite then Attention.  Since every layer's inputs are given, layers with the
+ * same window share one launch.  windows: NULL, or n_layers host entries (0 = global
  * layer).  Uniform-shape caches only.  Nothing in it synchronises or allocates, so a caller may
  * capture it in a CUDA graph (after one warm-up call) and replay it per token: positions and
  * slot ids are read from device memory at run time. */
@@ -563,8 +564,11 @@ int32_t vfkv_ctx_set_trace_buffer(vfkv_ctx *ctx, void *d_buffer);
  * that launch's grid: the phases of consecutive layers of one token side by side, on the GPU's
  * common nanosecond clock.  The blocks of one ring must belong to launches with equal grids. */
 int32_t vfkv_ctx_set_trace_ring(vfkv_ctx *ctx, uint32_t n_blocks);
-/* Kernels this context has launched since creation (for launch accounting). */
+/* Kernels this context has launched since creation (for launch accounting); one that carries several
+ * layers of a token (vfkv_decode_token) counts once for each layer, so that the count of a step does
+ * not depend on how its layers are grouped.  vfkv_ctx_kernel_count counts it once. */
 uint64_t vfkv_ctx_launch_count(const vfkv_ctx *ctx);
+uint64_t vfkv_ctx_kernel_count(const vfkv_ctx *ctx);
 
 /* Per-kernel GPU timing with the reference's profiler labels
  * (executor/attention.rs:560-573, runs.rs:1527,1561,1127; enabled there by

@@ -156,6 +156,7 @@ extern "C" {
     pub fn vfkv_ctx_set_trace_buffer(ctx: *mut vfkv_ctx, d_buffer: *mut c_void) -> i32;
     pub fn vfkv_ctx_set_trace_ring(ctx: *mut vfkv_ctx, n_blocks: u32) -> i32;
     pub fn vfkv_ctx_launch_count(ctx: *const vfkv_ctx) -> u64;
+    pub fn vfkv_ctx_kernel_count(ctx: *const vfkv_ctx) -> u64;
     pub fn vfkv_profile_enable(ctx: *mut vfkv_ctx, on: i32) -> i32;
     pub fn vfkv_profile_collect(ctx: *mut vfkv_ctx, label: u32, count: *mut u64, total_ms: *mut f64, min_ms: *mut f64, reset: i32) -> i32;
     pub fn vfkv_flash_attn(cache: *mut vfkv_cache, layer: u32, kv_layer: u32, d_q: *const f32, d_out: *mut f32, n_q_heads: u32, slot: u32, seq_len: u32, kv_start: u32, scale: f32, softcap: f32, stream: *mut c_void) -> i32;

@@ -73,11 +73,23 @@ KvView make_view(vfkv_cache *c, uint32_t kv_layer)
         c->tm_v.resize(kv.config.n_layers);
     }
     if (c->tm_state[kv_layer] == 0)
-        c->tm_state[kv_layer] = encode_layer_maps(c->ctx, v, c->tm_k[kv_layer].b, c->tm_v[kv_layer].b) ? 1 : 2;
+        c->tm_state[kv_layer] = encode_layer_maps(c->ctx, v, 1, c->tm_k[kv_layer].b, c->tm_v[kv_layer].b) ? 1 : 2;
     if (c->tm_state[kv_layer] == 1) {
         v.tm_k = c->tm_k[kv_layer].b;
         v.tm_v = c->tm_v[kv_layer].b;
     }
+    return v;
+}
+
+// View of layer 0 with tensor maps over every layer: for launches that carry several layers of a
+// uniform cache (slot index = layer * n_slots + slot).
+KvView make_view_all(vfkv_cache *c)
+{
+    KvView v = make_view(c, 0);
+    if (c->tm_all_state == 0)
+        c->tm_all_state = encode_layer_maps(c->ctx, v, c->kv.config.n_layers, c->tm_all_k.b, c->tm_all_v.b) ? 1 : 2;
+    v.tm_k = c->tm_all_state == 1 ? c->tm_all_k.b : nullptr;
+    v.tm_v = c->tm_all_state == 1 ? c->tm_all_v.b : nullptr;
     return v;
 }
 
@@ -231,6 +243,7 @@ int32_t vfkv_ctx_set_trace_ring(vfkv_ctx *ctx, uint32_t n_blocks)
 }
 
 uint64_t vfkv_ctx_launch_count(const vfkv_ctx *ctx) { return ctx ? ctx->launches : 0; }
+uint64_t vfkv_ctx_kernel_count(const vfkv_ctx *ctx) { return ctx ? ctx->kernels : 0; }
 
 int32_t vfkv_profile_enable(vfkv_ctx *ctx, int32_t on)
 {
@@ -475,28 +488,37 @@ int32_t vfkv_workspace_create(vfkv_ctx *ctx, uint32_t max_seqs, uint32_t n_q_hea
     ws->ctx = ctx; ws->max_seqs = max_seqs; ws->n_q_heads = n_q_heads; ws->head_dim = head_dim;
     ws->max_splits = max_splits;
     DeviceGuard g(ctx->device);
-    const uint64_t u32_bytes = uint64_t(max_seqs) * 4 * 4;
-    cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&ws->part_o), ofl);
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ws->part_m), parts * 4);
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ws->part_l), parts * 4);
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ws->d_u32), u32_bytes);
-    ws->n_counters = rows;
+    // A launch that carries several layers has a group for every (layer, sequence, kv-head); it is cut
+    // into splits only while the groups are fewer than about two per SM, or very long.
+    ws->n_counters = rows > 1024 ? rows : 1024;
     // per (q-head row, split): the o words, and room for the {m, l} words and padding of up to sixteen
-    // slices of the output (one per merging CTA; a launch takes fewer slices if that is not enough)
+    // slices of the output (one per merging CTA; a launch takes fewer slices if that is not enough);
+    // at least two CTAs per SM with eight q-heads a group, whatever the sequences of one layer would need
     ws->tag_words = parts * (uint64_t(head_dim) + 68);
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ws->tickets), rows * 256 * 8);
-    if (e == cudaSuccess) e = cudaMemset(ws->tickets, 0, rows * 256 * 8);
-    // tag 0 is never used by a launch, so zeroed words read as "not there yet"
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ws->tag_part), ws->tag_words * 8);
-    if (e == cudaSuccess) e = cudaMemset(ws->tag_part, 0, ws->tag_words * 8);
+    const uint64_t least = uint64_t(ctx->sm_count) * 2 * (uint64_t(n_q_heads < 8 ? n_q_heads : 8) * (uint64_t(head_dim) + 2) + 2);
+    if (ws->tag_words < least) ws->tag_words = least;
+    // one allocation for all of it; the part that starts at zero (tickets; tag 0 is never used by a
+    // launch, so zeroed words read as "not there yet") comes first
+    auto up = [](uint64_t n) { return (n + 255) / 256 * 256; };
+    const uint64_t tickets_at = 0, tags_at = tickets_at + up(ws->n_counters * 256 * 8), zeroed = tags_at + up(ws->tag_words * 8);
+    const uint64_t o_at = zeroed, m_at = o_at + up(ofl), l_at = m_at + up(parts * 4), u32_at = l_at + up(parts * 4);
+    ws->bytes = u32_at + up(uint64_t(max_seqs) * 4 * 4);
+    uint8_t *base = nullptr;
+    cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&base), ws->bytes);
+    if (e == cudaSuccess) e = cudaMemset(base, 0, zeroed);
     if (e != cudaSuccess) {
-        cudaFree(ws->part_o); cudaFree(ws->part_m); cudaFree(ws->part_l); cudaFree(ws->d_u32); cudaFree(ws->tickets);
-        cudaFree(ws->tag_part);
+        cudaFree(base);
         cudaGetLastError();
         delete ws;
         return check_cuda(ctx, e, "vfkv_workspace_create: cudaMalloc");
     }
-    ws->bytes = ofl + parts * 8 + u32_bytes + rows * 256 * 8 + ws->tag_words * 8;
+    ws->block = base;
+    ws->tickets = reinterpret_cast<unsigned long long *>(base + tickets_at);
+    ws->tag_part = reinterpret_cast<uint64_t *>(base + tags_at);
+    ws->part_o = reinterpret_cast<float *>(base + o_at);
+    ws->part_m = reinterpret_cast<float *>(base + m_at);
+    ws->part_l = reinterpret_cast<float *>(base + l_at);
+    ws->d_u32 = reinterpret_cast<uint32_t *>(base + u32_at);
     *out = ws;
     return VFKV_OK;
 }
@@ -505,8 +527,7 @@ int32_t vfkv_workspace_destroy(vfkv_workspace *ws)
 {
     if (!ws) return VFKV_OK;
     DeviceGuard g(ws->ctx->device);
-    cudaFree(ws->part_o); cudaFree(ws->part_m); cudaFree(ws->part_l); cudaFree(ws->d_u32); cudaFree(ws->tickets);
-    cudaFree(ws->tag_part);
+    cudaFree(ws->block);
     cudaFree(ws->stage_in); cudaFree(ws->stage_out);
     for (auto gexec : ws->tok_graphs)
         if (gexec) cudaGraphExecDestroy(gexec);
@@ -724,6 +745,83 @@ int32_t vfkv_decode_step(vfkv_cache *cache, vfkv_workspace *ws, uint32_t layer, 
     return launch_attention(ctx, ws, a, as_stream(stream));
 }
 
+// Append + attention of layers [l0, l1) of a uniform cache for one token per sequence; Q, new rows
+// and outputs are indexed by the absolute layer.  Every layer's inputs are there, so nothing orders
+// the layers among each other: layers with the same window go into one launch, as if they were
+// further sequences.  One layer of one sequence is a chain of latencies that leaves HBM idle
+// (8192 positions, FP8, 32 q / 8 kv / 128: 7.9 us for 17 MB); 36 of them in one launch stream at the
+// rate of a batch.  Windows differ -> separate launches, because one split count serves a launch.
+static int32_t decode_layers(vfkv_cache *cache, vfkv_workspace *ws, uint32_t l0, uint32_t l1, const float *d_q,
+                             const float *d_k, const float *d_v, float *d_out, uint32_t n_q_heads,
+                             const uint32_t *d_slot_ids, const uint32_t *d_positions, uint32_t n_seqs,
+                             uint32_t max_seq_len_hint, const uint32_t *windows, float scale, float softcap,
+                             uint32_t n_splits, void *stream)
+{
+    vfkv_ctx *ctx = cache->ctx;
+    KvCache &kv = cache->kv;
+    const uint32_t D = kv.config.head_dim, Hkv = kv.config.n_kv_heads;
+    if (l0 >= l1 || n_seqs == 0) return VFKV_OK;
+    int32_t rc = attend_common(cache, l0, l0, n_q_heads, "vfkv_decode_token");
+    if (rc) return rc;
+    if (!d_q || !d_k || !d_v || !d_out || !d_positions)
+        return set_error(ctx, VFKV_ERR_INVALID, "vfkv_decode_token: null argument");
+    if ((reinterpret_cast<uintptr_t>(d_k) | reinterpret_cast<uintptr_t>(d_v)) % 16 != 0)
+        return set_error(ctx, VFKV_ERR_INVALID, "vfkv_decode_token: K and V inputs must be 16-byte aligned");
+    DeviceGuard g(ctx->device);
+    AttnArgs a;
+    a.kv = make_view_all(cache);
+    a.seq.n_seqs = n_seqs; a.seq.slot_ids = d_slot_ids; a.seq.positions = d_positions;
+    a.seq.max_len_hint = max_seq_len_hint;
+    a.q = d_q; a.out = d_out; a.n_q_heads = n_q_heads; a.scale = scale; a.softcap = softcap; a.n_splits = n_splits;
+    const bool fused = ctx->attn_impl != 1 && attn_mma_supported(a);
+    // a grid holds at most 65535 units, and the row coordinate of a tensor map is a signed 32-bit number
+    uint32_t most = 65535u / n_seqs;
+    if (most > kMaxLaunchLayers) most = kMaxLaunchLayers;
+    if (most < 2 || (fused && cache->tm_all_state != 1)) {
+        const uint64_t q_stride = uint64_t(n_seqs) * n_q_heads * D, kv_stride = uint64_t(n_seqs) * Hkv * D;
+        for (uint32_t l = l0; l < l1; ++l) {
+            rc = vfkv_decode_step(cache, ws, l, d_q + l * q_stride, d_k + l * kv_stride, d_v + l * kv_stride,
+                                  d_out + l * q_stride, n_q_heads, d_slot_ids, d_positions, n_seqs, max_seq_len_hint,
+                                  windows ? windows[l] : 0, scale, softcap, n_splits, stream);
+            if (rc) return rc;
+        }
+        return VFKV_OK;
+    }
+    uint16_t ids[kMaxLaunchLayers];
+    auto launch = [&](uint32_t n) -> int32_t {
+        a.seq.n_layers = n; a.seq.layer_ids = ids;
+        if (fused) {
+            a.k_new = d_k;
+            a.v_new = d_v;
+        } else {
+            AppendArgs ap = make_append(cache, 0, d_k, d_v);
+            ap.n_rows = n_seqs; ap.slot_ids = d_slot_ids; ap.positions = d_positions;
+            ap.n_layers = n; ap.layer_ids = ids;
+            if (int32_t arc = launch_append(ctx, ap, as_stream(stream))) return arc;
+        }
+        return launch_attention(ctx, ws, a, as_stream(stream));
+    };
+    auto window_of = [&](uint32_t l) { return windows ? windows[l] : 0u; };
+    for (uint32_t first = l0; first < l1; ++first) {
+        const uint32_t w = window_of(first);
+        bool seen = false;                         // a window that an earlier layer had is done already
+        for (uint32_t l = l0; l < first && !seen; ++l) seen = window_of(l) == w;
+        if (seen) continue;
+        a.seq.window = w;
+        uint32_t n = 0;
+        for (uint32_t l = first; l < l1; ++l) {
+            if (window_of(l) != w) continue;
+            ids[n++] = uint16_t(l);
+            if (n == most) {
+                if ((rc = launch(n))) return rc;
+                n = 0;
+            }
+        }
+        if (n && (rc = launch(n))) return rc;
+    }
+    return VFKV_OK;
+}
+
 int32_t vfkv_decode_token(vfkv_cache *cache, vfkv_workspace *ws, const float *d_q, const float *d_k, const float *d_v,
                           float *d_out, uint32_t n_q_heads, const uint32_t *d_slot_ids, const uint32_t *d_positions,
                           uint32_t n_seqs, uint32_t max_seq_len_hint, const uint32_t *windows, float scale,
@@ -733,15 +831,8 @@ int32_t vfkv_decode_token(vfkv_cache *cache, vfkv_workspace *ws, const float *d_
     vfkv_ctx *ctx = cache->ctx;
     KvCache &kv = cache->kv;
     if (kv.layer_byte_offsets) return set_error(ctx, VFKV_ERR_UNSUPPORTED, "vfkv_decode_token: uniform-shape caches only");
-    const uint32_t L = kv.config.n_layers, D = kv.config.head_dim, Hkv = kv.config.n_kv_heads;
-    const uint64_t q_stride = uint64_t(n_seqs) * n_q_heads * D, kv_stride = uint64_t(n_seqs) * Hkv * D;
-    for (uint32_t l = 0; l < L; ++l) {
-        int32_t rc = vfkv_decode_step(cache, ws, l, d_q + l * q_stride, d_k + l * kv_stride, d_v + l * kv_stride,
-                                      d_out + l * q_stride, n_q_heads, d_slot_ids, d_positions, n_seqs,
-                                      max_seq_len_hint, windows ? windows[l] : 0, scale, softcap, n_splits, stream);
-        if (rc) return rc;
-    }
-    return VFKV_OK;
+    return decode_layers(cache, ws, 0, kv.config.n_layers, d_q, d_k, d_v, d_out, n_q_heads, d_slot_ids, d_positions,
+                         n_seqs, max_seq_len_hint, windows, scale, softcap, n_splits, stream);
 }
 
 int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const float *h_q, const float *h_k,
@@ -820,14 +911,8 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
     const uint32_t n_chunks = L < vfkv_workspace::kTokChunks ? L : vfkv_workspace::kTokChunks;
     auto chunk_begin = [&](uint32_t c) { return uint32_t(uint64_t(L) * c / n_chunks); };
     auto run_layers = [&](uint32_t l0, uint32_t l1, uint32_t len_hint) -> int32_t {
-        for (uint32_t l = l0; l < l1; ++l) {
-            int32_t rc = vfkv_decode_step(cache, ws, l, dq + l * q_stride, dk + l * kv_stride, dv + l * kv_stride,
-                                          ws->stage_out + l * q_stride, n_q_heads, h_slot_ids ? d_slots : nullptr,
-                                          d_pos, n_seqs, len_hint, windows ? windows[l] : 0, scale, softcap,
-                                          n_splits, stream);
-            if (rc) return rc;
-        }
-        return VFKV_OK;
+        return decode_layers(cache, ws, l0, l1, dq, dk, dv, ws->stage_out, n_q_heads, h_slot_ids ? d_slots : nullptr,
+                             d_pos, n_seqs, len_hint, windows, scale, softcap, n_splits, stream);
     };
     if (graphable && !ws->copy_stream) {
         bool ok = cudaStreamCreateWithFlags(&ws->copy_stream, cudaStreamNonBlocking) == cudaSuccess;
@@ -841,10 +926,12 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
         for (uint32_t c = 0; c < n_chunks; ++c) {
             cudaGraph_t graph = nullptr;
             if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); break; }
-            const uint64_t launches = ctx->launches;
+            const uint64_t launches = ctx->launches, kernels = ctx->kernels;
             int32_t rc = run_layers(chunk_begin(c), chunk_begin(c + 1), hint);
             cudaError_t ce = cudaStreamEndCapture(st, &graph);
-            ctx->launches = launches;                           // recorded, not run
+            ws->tok_launches[c] = uint32_t(ctx->launches - launches);
+            ws->tok_kernels[c] = uint32_t(ctx->kernels - kernels);
+            ctx->launches = launches; ctx->kernels = kernels;   // recorded, not run
             const bool ok = rc == VFKV_OK && ce == cudaSuccess && graph &&
                             cudaGraphInstantiate(&ws->tok_graphs[c], graph, 0) == cudaSuccess;
             if (graph) cudaGraphDestroy(graph);
@@ -882,7 +969,7 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
             e = cudaStreamWaitEvent(st, ev_in[c], 0);
             if (e == cudaSuccess) e = cudaGraphLaunch(ws->tok_graphs[c], st);
             if (e == cudaSuccess) e = cudaEventRecord(ev_done[c], st);
-            if (e == cudaSuccess) ctx->launches += nl;
+            if (e == cudaSuccess) { ctx->launches += ws->tok_launches[c]; ctx->kernels += ws->tok_kernels[c]; }
             if (e == cudaSuccess && c + 1 < n_chunks) e = copy_in(c + 1);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(cs, ev_done[c], 0);
             if (e == cudaSuccess) e = cudaMemcpyAsync(h_out + l0 * q_stride, ws->stage_out + l0 * q_stride, nl * q_stride * 4, cudaMemcpyDeviceToHost, cs);
@@ -969,7 +1056,6 @@ int32_t vfkv_decode_token_host_submit(vfkv_cache *cache, vfkv_workspace *ws, con
     }
     float *dq = hs->in, *dk = dq + q_elems, *dv = dk + kv_elems;
     uint32_t *d_pos = hs->u32, *d_slots = hs->u32 + ws->max_seqs;
-    const uint64_t q_stride = uint64_t(n_seqs) * n_q_heads * D, kv_stride = uint64_t(n_seqs) * Hkv * D;
     uint32_t hint = (max_pos + 1 + 1023u) / 1024u * 1024u;
     if (hint > kv.config.max_seq_len) hint = kv.config.max_seq_len;
     uint64_t wh = 1469598103934665603ull;
@@ -991,14 +1077,12 @@ int32_t vfkv_decode_token_host_submit(vfkv_cache *cache, vfkv_workspace *ws, con
         cudaGraph_t graph = nullptr;
         e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return check_cuda(ctx, e, "vfkv_decode_token_host_submit: capture");
-        const uint64_t launches = ctx->launches;
-        int32_t rc = VFKV_OK;
-        for (uint32_t l = 0; l < L && rc == VFKV_OK; ++l)
-            rc = vfkv_decode_step(cache, ws, l, dq + l * q_stride, dk + l * kv_stride, dv + l * kv_stride,
-                                  hs->out + l * q_stride, n_q_heads, h_slot_ids ? d_slots : nullptr, d_pos, n_seqs, hint,
-                                  windows ? windows[l] : 0, scale, softcap, n_splits, stream);
+        const uint64_t launches = ctx->launches, kernels = ctx->kernels;
+        const int32_t rc = decode_layers(cache, ws, 0, L, dq, dk, dv, hs->out, n_q_heads, h_slot_ids ? d_slots : nullptr,
+                                         d_pos, n_seqs, hint, windows, scale, softcap, n_splits, stream);
         hs->launches = uint32_t(ctx->launches - launches);
-        ctx->launches = launches;                               // recorded, not run
+        hs->kernels = uint32_t(ctx->kernels - kernels);
+        ctx->launches = launches; ctx->kernels = kernels;       // recorded, not run
         cudaError_t ce = cudaStreamEndCapture(st, &graph);
         if (rc == VFKV_OK && ce == cudaSuccess && graph) ce = cudaGraphInstantiate(&hs->graph, graph, 0);
         if (graph) cudaGraphDestroy(graph);
@@ -1026,6 +1110,7 @@ int32_t vfkv_decode_token_host_submit(vfkv_cache *cache, vfkv_workspace *ws, con
         return check_cuda(ctx, e, "vfkv_decode_token_host_submit");
     }
     ctx->launches += hs->launches;
+    ctx->kernels += hs->kernels;
     hs->ticket = ws->next_ticket++;
     *ticket = hs->ticket;
     return VFKV_OK;

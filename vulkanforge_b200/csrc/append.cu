@@ -96,7 +96,7 @@ static int32_t launch_store_t(vfkv_ctx *ctx, const float *src, void *dst, uint64
         if (blocks > cap) blocks = cap;
         ProfScope ps(ctx, VFKV_PROF_KV_STORE, st);
         store_vec_kernel<DT><<<unsigned(blocks), 256, 0, st>>>(src, static_cast<uint8_t *>(dst), n);
-        ctx->launches++;
+        ctx->count_launch();
         done = n_vec * E;
     }
     if (done < n) {
@@ -104,9 +104,9 @@ static int32_t launch_store_t(vfkv_ctx *ctx, const float *src, void *dst, uint64
         ProfScope ps(ctx, VFKV_PROF_KV_STORE, st);
         store_word_kernel<DT><<<unsigned((words + 255) / 256), 256, 0, st>>>(
             src, static_cast<uint32_t *>(dst), done, n);
-        ctx->launches++;
+        ctx->count_launch();
     }
-    ctx->last_written_slab = vfkv::kAnySlab;        // a raw destination may lie in any layer
+    ctx->set_written_any();
     return check_cuda(ctx, cudaGetLastError(), "store kernel launch");
 }
 
@@ -133,12 +133,26 @@ struct AppendParams {
     uint32_t row_elems, head_dim, n_kv_heads, max_seq, n_slots, n_rows, slot, base_pos;
     uint32_t shard_world, shard_rank, shard_page;   // world > 1: base_pos + row is a global position dealt out in pages
     uint32_t *status;
+    uint32_t total_rows;
 };
+// Layers of a launch that carries several: its rows are [layer of the launch][sequence], n_rows of each.
+// (A kernel for one layer has no such argument: 128 bytes more cost a launch 0.7 us.)
+template <bool LAYERED> struct AppendLayers { uint16_t id[kMaxLaunchLayers]; };
+template <> struct AppendLayers<false> {};
 
-__device__ __forceinline__ bool row_target(const AppendParams &p, uint32_t row, uint32_t *slot,
-                                           uint32_t *pos)
+// Slot and position of a row of the launch; a row of a launch of several layers becomes its row in the sources.
+template <bool LAYERED>
+__device__ __forceinline__ bool row_target(const AppendParams &p, const AppendLayers<LAYERED> &layers, uint32_t &row,
+                                           uint32_t *slot, uint32_t *pos)
 {
-    if (p.positions) {
+    uint32_t slot_base = 0;
+    if constexpr (LAYERED) {
+        const uint32_t i = row / p.n_rows, layer = layers.id[i], s = row - i * p.n_rows;
+        *slot = p.slot_ids ? p.slot_ids[s] : s;
+        *pos = p.positions[s];
+        slot_base = layer * p.n_slots;
+        row = layer * p.n_rows + s;
+    } else if (p.positions) {
         *slot = p.slot_ids ? p.slot_ids[row] : row;
         *pos = p.positions[row];
     } else {
@@ -154,23 +168,24 @@ __device__ __forceinline__ bool row_target(const AppendParams &p, uint32_t row, 
         atomicOr(p.status, 2u);   // out-of-range row: skipped, reported through vfkv_ctx_poll
         return false;
     }
+    *slot += slot_base;
     return true;
 }
 
 // grid.y selects K (0) or V (1); each thread emits one 16-byte piece of a row.
-template <int DT>
-__global__ void __launch_bounds__(256) append_kernel(const AppendParams p)
+template <int DT, bool LAYERED>
+__global__ void __launch_bounds__(256) append_kernel(const AppendParams p, const __grid_constant__ AppendLayers<LAYERED> layers)
 {
     constexpr int E = Enc<DT>::kElems;
     const uint32_t which = blockIdx.y;
     const uint32_t chunks_per_row = p.row_elems / E;
-    const uint64_t total = uint64_t(p.n_rows) * chunks_per_row;
+    const uint64_t total = uint64_t(p.total_rows) * chunks_per_row;
     const uint64_t row_bytes = uint64_t(p.row_elems) * (DT == VFKV_F8 ? 1 : DT == VFKV_F16 ? 2 : 4);
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < total;
          i += uint64_t(gridDim.x) * blockDim.x) {
         uint32_t row = uint32_t(i / chunks_per_row), c = uint32_t(i % chunks_per_row);
         uint32_t slot, pos;
-        if (!row_target(p, row, &slot, &pos)) continue;
+        if (!row_target<LAYERED>(p, layers, row, &slot, &pos)) continue;
         const float4 *s = reinterpret_cast<const float4 *>(p.src[which] + uint64_t(row) * p.row_elems +
                                                            uint64_t(c) * E);
         uint4 r = Enc<DT>::run(s);
@@ -182,17 +197,18 @@ __global__ void __launch_bounds__(256) append_kernel(const AppendParams p)
 // Extension: per-(token, kv-head) absmax scale.  One warp per (row, head, K|V).
 // scale = max(absmax * (1/448), 1e-12); inv = 1/scale; code = e4m3(clamp(x*inv, +-448)):
 // the recipe of vk_shaders/mul_coopmat_fp8_native_bn32.comp:149-152,214.
-__global__ void __launch_bounds__(256) append_scaled_kernel(const AppendParams p)
+template <bool LAYERED>
+__global__ void __launch_bounds__(256) append_scaled_kernel(const AppendParams p, const __grid_constant__ AppendLayers<LAYERED> layers)
 {
     const uint32_t warps_per_block = blockDim.x / 32;
     const uint32_t which = blockIdx.y;
     const uint32_t lane = threadIdx.x & 31;
-    const uint64_t total = uint64_t(p.n_rows) * p.n_kv_heads;
+    const uint64_t total = uint64_t(p.total_rows) * p.n_kv_heads;
     for (uint64_t w = blockIdx.x * uint64_t(warps_per_block) + threadIdx.x / 32; w < total;
          w += uint64_t(gridDim.x) * warps_per_block) {
         uint32_t row = uint32_t(w / p.n_kv_heads), head = uint32_t(w % p.n_kv_heads);
         uint32_t slot, pos;
-        if (!row_target(p, row, &slot, &pos)) continue;
+        if (!row_target<LAYERED>(p, layers, row, &slot, &pos)) continue;
         const float *x = p.src[which] + uint64_t(row) * p.row_elems + uint64_t(head) * p.head_dim;
         float amax = 0.f;
         for (uint32_t d = lane * 4; d < p.head_dim; d += 128) {
@@ -232,36 +248,48 @@ int32_t launch_append(vfkv_ctx *ctx, const AppendArgs &a, cudaStream_t st)
     p.row_elems = a.row_elems; p.head_dim = a.head_dim; p.n_kv_heads = a.n_kv_heads;
     p.max_seq = a.max_seq; p.n_slots = a.n_slots; p.n_rows = a.n_rows; p.slot = a.slot;
     p.base_pos = a.base_pos; p.status = ctx->d_status;
+    p.total_rows = a.n_rows * a.n_layers;
+    const bool layered = a.layer_ids != nullptr;
+    AppendLayers<true> layers{};
+    const AppendLayers<false> none{};
+    for (uint32_t i = 0; layered && i < a.n_layers; ++i) layers.id[i] = a.layer_ids[i];
+    const uint64_t last_layer = layered ? a.layer_ids[a.n_layers - 1] : 0u;      // the list ascends
+    const uint64_t written = (last_layer + 1) * a.n_slots * a.slot_stride_bytes;
     p.shard_world = a.shard_world; p.shard_rank = a.shard_rank; p.shard_page = a.shard_page ? a.shard_page : 1u;
 
     if (a.k_scales) {
         if (a.head_dim % 4 != 0) return set_error(ctx, VFKV_ERR_UNSUPPORTED, "scaled append needs head_dim % 4 == 0");
-        uint64_t warps = uint64_t(a.n_rows) * a.n_kv_heads;
+        uint64_t warps = uint64_t(p.total_rows) * a.n_kv_heads;
         uint64_t blocks = (warps + 7) / 8, cap = uint64_t(ctx->sm_count) * 8;
         if (blocks > cap) blocks = cap;
         {
             ProfScope ps(ctx, VFKV_PROF_KV_STORE, st);
-            append_scaled_kernel<<<dim3(unsigned(blocks), 2), 256, 0, st>>>(p);
+            if (layered) append_scaled_kernel<true><<<dim3(unsigned(blocks), 2), 256, 0, st>>>(p, layers);
+            else append_scaled_kernel<false><<<dim3(unsigned(blocks), 2), 256, 0, st>>>(p, none);
         }
-        ctx->launches++;
-        ctx->last_written_slab = a.k_dst;
+        ctx->count_launch(a.n_layers);
+        ctx->set_written(a.k_dst, written);
         return check_cuda(ctx, cudaGetLastError(), "append_scaled launch");
     }
     const int E = a.dtype == VFKV_F8 ? 16 : a.dtype == VFKV_F16 ? 8 : 4;
-    uint64_t chunks = uint64_t(a.n_rows) * (a.row_elems / E);
+    uint64_t chunks = uint64_t(p.total_rows) * (a.row_elems / E);
     uint64_t blocks = (chunks + 255) / 256, cap = uint64_t(ctx->sm_count) * 8;
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
     dim3 grid(unsigned(blocks), 2);
     ProfScope ps(ctx, VFKV_PROF_KV_STORE, st);
+    auto launch = [&](auto plain, auto several) {
+        if (layered) several<<<grid, 256, 0, st>>>(p, layers);
+        else plain<<<grid, 256, 0, st>>>(p, none);
+    };
     switch (a.dtype) {
-    case VFKV_F8: append_kernel<VFKV_F8><<<grid, 256, 0, st>>>(p); break;
-    case VFKV_F16: append_kernel<VFKV_F16><<<grid, 256, 0, st>>>(p); break;
-    case VFKV_F32: append_kernel<VFKV_F32><<<grid, 256, 0, st>>>(p); break;
+    case VFKV_F8: launch(append_kernel<VFKV_F8, false>, append_kernel<VFKV_F8, true>); break;
+    case VFKV_F16: launch(append_kernel<VFKV_F16, false>, append_kernel<VFKV_F16, true>); break;
+    case VFKV_F32: launch(append_kernel<VFKV_F32, false>, append_kernel<VFKV_F32, true>); break;
     default: return set_error(ctx, VFKV_ERR_INVALID, "unknown dtype");
     }
-    ctx->launches++;
-    ctx->last_written_slab = a.k_dst;
+    ctx->count_launch(a.n_layers);
+    ctx->set_written(a.k_dst, written);
     return check_cuda(ctx, cudaGetLastError(), "append launch");
 }
 
@@ -306,7 +334,7 @@ int32_t launch_fp8_to_f16(vfkv_ctx *ctx, const void *src, void *dst, uint64_t n,
         ProfScope ps(ctx, VFKV_PROF_FP8_TO_F16, st);
         fp8_to_f16_vec_kernel<<<unsigned(blocks), 256, 0, st>>>(
             static_cast<const uint4 *>(src), static_cast<uint4 *>(dst), n_vec);
-        ctx->launches++;
+        ctx->count_launch();
         done = n_vec * 16;
     }
     if (done < n) {
@@ -314,7 +342,7 @@ int32_t launch_fp8_to_f16(vfkv_ctx *ctx, const void *src, void *dst, uint64_t n,
         ProfScope ps(ctx, VFKV_PROF_FP8_TO_F16, st);
         fp8_to_f16_scalar_kernel<<<unsigned((rem + 255) / 256), 256, 0, st>>>(
             static_cast<const uint8_t *>(src), static_cast<__half *>(dst), done, n);
-        ctx->launches++;
+        ctx->count_launch();
     }
     return check_cuda(ctx, cudaGetLastError(), "fp8_to_f16 launch");
 }

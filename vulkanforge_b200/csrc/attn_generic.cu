@@ -80,14 +80,15 @@ attn_split_generic_kernel(const AttnParams p)
     const uint32_t split = blockIdx.x;
     const uint32_t head_blocks = (p.group + GB - 1) / GB;
     const uint32_t kvh = blockIdx.y / head_blocks, hb = blockIdx.y % head_blocks;
-    const uint32_t s = blockIdx.z;
+    const UnitOf unit = unit_of(p, blockIdx.z);
+    const uint32_t s = unit.row;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t D = p.head_dim;
     const uint32_t h0 = kvh * p.group + hb * GB;
     const uint32_t nh = min(uint32_t(GB), p.group - hb * GB);
 
     uint32_t slot, start, len, begin, end;
-    seq_range(p, s, &slot, &start, &len);
+    seq_range(p, unit, &slot, &start, &len);
     split_range(start, len, p.n_splits, split, 32, &begin, &end);
 
     // this lane's slice of each of the CTA's q rows
@@ -213,7 +214,7 @@ attn_split_generic_kernel(const AttnParams p)
                 if (d == 0) { p.out_m[row] = M; p.out_l[row] = L; }
             }
         } else {
-            const uint64_t pi = row * p.n_splits + split;
+            const uint64_t pi = ((uint64_t(blockIdx.z) * p.n_q_heads + h0 + j) * p.n_splits) + split;
             p.part_o[pi * D + d] = O;
             if (d == 0) { p.part_m[pi] = M; p.part_l[pi] = L; }
         }
@@ -224,7 +225,7 @@ template <int DT, int VEC, int GB>
 static int32_t launch_one(vfkv_ctx *ctx, const AttnParams &p, cudaStream_t st)
 {
     const uint32_t head_blocks = (p.group + GB - 1) / GB;
-    dim3 grid(p.n_splits, p.n_kv_heads * head_blocks, p.n_seqs);
+    dim3 grid(p.n_splits, p.n_kv_heads * head_blocks, p.n_seqs * p.n_layers);
     size_t smem = sizeof(float) * size_t(kGenericWarps) * GB * (p.head_dim + 2);
     auto kern = attn_split_generic_kernel<DT, VEC, GB>;
     if (smem > 48 * 1024) {
@@ -235,7 +236,7 @@ static int32_t launch_one(vfkv_ctx *ctx, const AttnParams &p, cudaStream_t st)
         ProfScope ps(ctx, VFKV_PROF_FA_SPLIT, st);
         kern<<<grid, kGenericWarps * 32, smem, st>>>(p);
     }
-    ctx->launches++;
+    ctx->count_launch(p.n_layers);
     return check_cuda(ctx, cudaGetLastError(), "generic attention launch");
 }
 

@@ -10,13 +10,21 @@ namespace vfkv {
 // maximum of the partial maxima; the final multiply by 1/sum is skipped when
 // the caller wants the unnormalised triple (sequence-dimension sharding).
 // Partial i of row r: m and l at i*ml_part + r*ml_row, o at i*o_part + r*o_row (+ dim), all in floats.
+// Output row of partial row r when a launch carries several layers (see SeqArgs); the identity otherwise.
+struct LayerRows { uint32_t per_layer; uint16_t layer_ids[kMaxLaunchLayers]; };
+
 __global__ void __launch_bounds__(128)
 merge_kernel(const float *__restrict__ pm, const float *__restrict__ pl, const float *__restrict__ po,
              uint32_t n_parts, uint64_t ml_part, uint64_t ml_row, uint64_t o_part, uint64_t o_row, uint32_t head_dim,
              float *__restrict__ out, float *__restrict__ out_m, float *__restrict__ out_l,
-             float *__restrict__ out_o)
+             float *__restrict__ out_o, const LayerRows lr)
 {
     const uint64_t row = blockIdx.x;
+    uint64_t orow = row;
+    if (lr.per_layer != 0u) {
+        const uint32_t i = blockIdx.x / lr.per_layer;
+        orow = uint64_t(lr.layer_ids[i]) * lr.per_layer + (blockIdx.x - i * lr.per_layer);
+    }
     constexpr int kMaxDims = 4;                      // 128 threads x 4 = head_dim 512
     __shared__ float s_red[4], s_sum[4];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -69,22 +77,27 @@ merge_kernel(const float *__restrict__ pm, const float *__restrict__ pl, const f
     for (int j = 0; j < kMaxDims; ++j) {
         uint32_t d = threadIdx.x + j * 128;
         if (d < head_dim) {
-            if (out) out[row * head_dim + d] = acc[j] * inv;
-            if (out_o) out_o[row * head_dim + d] = acc[j];
+            if (out) out[orow * head_dim + d] = acc[j] * inv;
+            if (out_o) out_o[orow * head_dim + d] = acc[j];
         }
     }
-    if (out_o && threadIdx.x == 0) { out_m[row] = gmax; out_l[row] = gsum; }
+    if (out_o && threadIdx.x == 0) { out_m[orow] = gmax; out_l[orow] = gsum; }
 }
 
 int32_t launch_merge_ws(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits,
                         cudaStream_t st)
 {
-    const uint32_t rows = a.seq.n_seqs * a.n_q_heads;
+    const uint32_t rows = a.seq.units() * a.n_q_heads;
+    LayerRows lr{};
+    if (a.seq.layer_ids) {
+        lr.per_layer = a.seq.n_seqs * a.n_q_heads;
+        for (uint32_t i = 0; i < a.seq.n_layers; ++i) lr.layer_ids[i] = a.seq.layer_ids[i];
+    }
     ProfScope ps(ctx, VFKV_PROF_FA_REDUCE, st);
     const uint64_t D = a.kv.head_dim;
     merge_kernel<<<rows, 128, 0, st>>>(ws->part_m, ws->part_l, ws->part_o, n_splits, 1, n_splits, D, n_splits * D,
-                                      a.kv.head_dim, a.out, a.out_m, a.out_l, a.out_o);
-    ctx->launches++;
+                                      a.kv.head_dim, a.out, a.out_m, a.out_l, a.out_o, lr);
+    ctx->count_launch(a.seq.n_layers);
     return check_cuda(ctx, cudaGetLastError(), "merge launch");
 }
 
@@ -95,8 +108,8 @@ int32_t launch_merge_partials(vfkv_ctx *ctx, const float *m, const float *l, con
     if (n_rows == 0) return VFKV_OK;
     ProfScope ps(ctx, VFKV_PROF_FA_REDUCE, st);
     merge_kernel<<<n_rows, 128, 0, st>>>(m, l, o, n_parts, n_rows, 1, uint64_t(n_rows) * head_dim, head_dim,
-                                        head_dim, out, nullptr, nullptr, nullptr);
-    ctx->launches++;
+                                        head_dim, out, nullptr, nullptr, nullptr, LayerRows{});
+    ctx->count_launch();
     return check_cuda(ctx, cudaGetLastError(), "merge_partials launch");
 }
 
@@ -109,8 +122,8 @@ int32_t launch_merge_partials_packed(vfkv_ctx *ctx, const float *packed, uint32_
     const uint64_t block = uint64_t(n_rows) * (head_dim + 2);
     ProfScope ps(ctx, VFKV_PROF_FA_REDUCE, st);
     merge_kernel<<<n_rows, 128, 0, st>>>(packed, packed + n_rows, packed + 2 * uint64_t(n_rows), n_parts, block, 1,
-                                        block, head_dim, head_dim, out, nullptr, nullptr, nullptr);
-    ctx->launches++;
+                                        block, head_dim, head_dim, out, nullptr, nullptr, nullptr, LayerRows{});
+    ctx->count_launch();
     return check_cuda(ctx, cudaGetLastError(), "merge_partials_packed launch");
 }
 
@@ -127,7 +140,7 @@ uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile)
     // HBM-bound, so a ragged last wave costs little, while every extra split costs a partial
     // write, a ticket and a merge.  Smaller grids are cut until about two CTAs per SM exist, but
     // never below 256 positions per split.
-    const uint64_t base = uint64_t(a.seq.n_seqs) * a.kv.n_kv_heads;
+    const uint64_t base = uint64_t(a.seq.units()) * a.kv.n_kv_heads;
     const uint64_t slots = uint64_t(ctx->sm_count) * 2;
     // (an 8-warp CTA of the tensor-core kernel takes 8 tiles at a time: 256 positions of an FP8
     // cache, 128 of an F16 cache, where 16 splits of 128 measured 6.2 us against 6.6 us with 8 of 256
@@ -206,6 +219,13 @@ int32_t launch_attention(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, c
         if (n_splits > ws->max_splits) n_splits = ws->max_splits;
         if (a.seq.n_seqs > ws->max_seqs || a.n_q_heads > ws->n_q_heads || a.kv.head_dim > ws->head_dim)
             return set_error(ctx, VFKV_ERR_INVALID, "workspace too small for this call");
+        // the workspace is sized for max_splits of each sequence of one layer; a launch of several layers shares it out
+        if (a.seq.n_layers > 1) {
+            const uint64_t g = a.n_q_heads / a.kv.n_kv_heads, groups = uint64_t(a.seq.units()) * a.kv.n_kv_heads;
+            const uint64_t most = use_mma ? (groups <= ws->n_counters ? ws->tag_words / (groups * (g * (a.kv.head_dim + 2) + 2)) : 1)
+                                          : uint64_t(ws->max_seqs) * ws->max_splits / a.seq.units();
+            if (n_splits > most) n_splits = most > 1 ? uint32_t(most) : 1u;
+        }
     }
     int32_t rc = use_mma ? launch_attn_mma(ctx, ws, a, n_splits, st)
                          : launch_attn_generic(ctx, ws, a, n_splits, st);

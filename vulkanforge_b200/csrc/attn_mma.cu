@@ -428,7 +428,9 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     __shared__ uint32_t s_flag, s_epoch, s_tag, s_merger, s_late;
     __shared__ PeerFanout s_fan;          // the group's fan-out table (position-sharded calls only)
 
-    const uint32_t split = blockIdx.x, kvh = blockIdx.y, s = blockIdx.z;
+    const uint32_t split = blockIdx.x, kvh = blockIdx.y, s = blockIdx.z;     // s: unit of the launch (tickets, partials)
+    const UnitOf unit = unit_of(p, s);
+    const uint32_t sr = unit.row;                                           // its row in Q, new tokens and outputs
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t gid = lane >> 2, tig = lane & 3;
     const uint32_t g = p.group;
@@ -456,7 +458,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     if constexpr (TR) {
         const uint32_t hcol = gid >> 1;
         const bool hv = hcol < g;
-        const float *qp = p.q + (uint64_t(s) * p.n_q_heads + kvh * g + (hv ? hcol : 0)) * D;
+        const float *qp = p.q + (uint64_t(sr) * p.n_q_heads + kvh * g + (hv ? hcol : 0)) * D;
 #pragma unroll
         for (int u = 0; u < NQB; ++u) {
             if constexpr (FP8) {
@@ -473,7 +475,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     for (int r = 0; r < RS; ++r) {
         const uint32_t hrow = gid + 8 * r;
         const bool hv = hrow < g;
-        const float *qp = p.q + (uint64_t(s) * p.n_q_heads + kvh * g + (hv ? hrow : 0)) * D;
+        const float *qp = p.q + (uint64_t(sr) * p.n_q_heads + kvh * g + (hv ? hrow : 0)) * D;
 #pragma unroll
         for (int ks = 0; ks < KSTEPS; ++ks) {
             if constexpr (FP8) {
@@ -516,7 +518,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 
     VFKV_TRACE(0);
     uint32_t slot, start, len, begin, end;
-    seq_range(p, s, &slot, &start, &len);
+    seq_range(p, unit, &slot, &start, &len);
     split_range(start, len, p.n_splits, split, 32, &begin, &end);
     const uint32_t n_tiles = (end - begin + TP - 1) / TP;
     VFKV_TRACE(1);
@@ -578,7 +580,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             const uint32_t u = lane + 32 * i;
             newu[i] = make_uint4(0, 0, 0, 0);
             if (u < 2 * UPT) {
-                const float *src = (u < UPT ? mp.k_new : mp.v_new) + (uint64_t(s) * p.n_kv_heads + kvh) * D +
+                const float *src = (u < UPT ? mp.k_new : mp.v_new) + (uint64_t(sr) * p.n_kv_heads + kvh) * D +
                                    (u % UPT) * (16 / S::ES);
                 const float4 *s4 = reinterpret_cast<const float4 *>(src);
                 if constexpr (FP8) {
@@ -1075,7 +1077,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                 gsum = fmaf(ll[i], kn, gsum);
                 a = fmaf(oo[i], kn, a);
             }
-            const uint64_t row = uint64_t(s) * p.n_q_heads + kvh * g + j;
+            const uint64_t row = uint64_t(sr) * p.n_q_heads + kvh * g + j;
             if (p.out) p.out[row * D + d] = gsum > 0.f ? a * (1.0f / gsum) : 0.f;
             if (p.out_o) {
                 p.out_o[row * D + d] = a;
@@ -1122,7 +1124,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // GPU's exchange buffer.
     auto emit = [&](uint32_t idx, float a0, float a1, float gmax, float gsum) {
         const uint32_t j = idx / HD2, d = 2 * (idx % HD2);
-        const uint64_t row = uint64_t(s) * p.n_q_heads + kvh * g + j;
+        const uint64_t row = uint64_t(sr) * p.n_q_heads + kvh * g + j;
         if (p.out && mp.fan_merge == 0u) {
             const float inv = gsum > 0.f ? 1.0f / gsum : 0.f;
             *reinterpret_cast<float2 *>(p.out + row * D + d) = make_float2(a0 * inv, a1 * inv);
@@ -1385,7 +1387,7 @@ int32_t launch_k(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
         // A merging CTA stages its slice of every split's partial in the ring, and the group's partials
         // ([slice][split][span] words, see the kernel) have to fit the workspace: fewer splits where the
         // ring is too small, fewer merging CTAs where the workspace is.
-        const uint64_t n_pairs = uint64_t(mp.a.group) * (D / 2), groups = uint64_t(mp.a.n_kv_heads) * mp.a.n_seqs;
+        const uint64_t n_pairs = uint64_t(mp.a.group) * (D / 2), groups = uint64_t(mp.a.n_kv_heads) * mp.a.n_seqs * mp.a.n_layers;
         auto span_of = [&](uint32_t n_mrg) {
             const uint64_t per = (n_pairs + n_mrg - 1) / n_mrg;
             return 2 * (per + mp.a.group) + (((per + mp.a.group) & 1) ? 0 : 2);
@@ -1415,7 +1417,7 @@ int32_t launch_k(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
         }
         if (lp.fan_merge && 8ull * (uint64_t(mp.a.group) * D * 8 + 2ull * mp.a.group * 4) > uint64_t(S::RING_BYTES))
             return set_error(ctx, VFKV_ERR_UNSUPPORTED, "one-launch exchange does not fit this kernel shape");
-        dim3 grid(lp.a.n_splits, mp.a.n_kv_heads, mp.a.n_seqs);
+        dim3 grid(lp.a.n_splits, mp.a.n_kv_heads, mp.a.n_seqs * mp.a.n_layers);
         {
             ProfScope ps(ctx, VFKV_PROF_FA_SPLIT, st);
             cudaLaunchConfig_t cfg = {};
@@ -1455,14 +1457,14 @@ int32_t launch_k(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
                     cudaGetLastError();
                     slot_known.store(known, std::memory_order_release);
                 }
-                const uint64_t clusters = uint64_t(mp.a.n_kv_heads) * mp.a.n_seqs;
+                const uint64_t clusters = uint64_t(mp.a.n_kv_heads) * mp.a.n_seqs * mp.a.n_layers;
                 if (known > 0 && clusters <= uint64_t(known)) lp.cluster = 1;
                 else cfg.numAttrs = n_attr;
             }
             cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tk, tv, lp);
             if (e != cudaSuccess) return check_cuda(ctx, e, "tensor-core attention launch");
         }
-        ctx->launches++;
+        ctx->count_launch(mp.a.n_layers);
         return check_cuda(ctx, cudaGetLastError(), "tensor-core attention launch");
     }
 }
@@ -1474,7 +1476,7 @@ int32_t launch_c(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
     // Everything else: 4 warps x 3 stages, two CTAs per SM at 8 KB stages (measured faster than
     // three CTAs of 4 x 2, whose 168-register cap costs more than the extra warps give).
     constexpr bool kWide = Shape<DT, D, 8, 3>::SMEM_BYTES <= 200 * 1024;
-    const uint64_t ctas = uint64_t(mp.a.n_splits) * mp.a.n_kv_heads * mp.a.n_seqs;
+    const uint64_t ctas = uint64_t(mp.a.n_splits) * mp.a.n_kv_heads * mp.a.n_seqs * mp.a.n_layers;
     uint32_t w = ctx->tune_warps, ns = ctx->tune_stages;
     if (w == 0) w = (kWide && ctas <= uint64_t(ctx->sm_count)) ? 8 : 4;
     // 4 warps: as many stages (up to 3) as still let two CTAs share an SM.  At head_dim 256 a stage
@@ -1533,6 +1535,8 @@ int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, ui
         return set_error(ctx, VFKV_ERR_INVALID, "slots must be contiguous slabs");
     const uint32_t box_rows = a.kv.dtype == VFKV_F8 ? 32 : 16;
     CUtensorMap tk, tv;
+    if (a.seq.layer_ids && (!a.kv.tm_k || !a.kv.tm_v))
+        return set_error(ctx, VFKV_ERR_UNSUPPORTED, "several layers in one launch need the tensor maps of the whole cache");
     if (a.kv.tm_k && a.kv.tm_v) {
         tk = *static_cast<const CUtensorMap *>(a.kv.tm_k);
         tv = *static_cast<const CUtensorMap *>(a.kv.tm_v);
@@ -1551,7 +1555,7 @@ int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, ui
     // groups have the GPU to themselves and are cut into many splits -- as long as all the CTAs that
     // may be waiting at one time stay a small part of the SMs (a waiting CTA holds its SM).
     {
-        const uint64_t groups = uint64_t(a.seq.n_seqs) * a.kv.n_kv_heads;
+        const uint64_t groups = uint64_t(a.seq.units()) * a.kv.n_kv_heads;
         const uint64_t room = uint64_t(ctx->sm_count) / 4 / (groups ? groups : 1);
         const uint64_t most = n_splits > 16 ? (n_splits + 7) / 8 : 4;      // a merger for every eight splits
         mp.n_mergers = uint32_t(room < 1 ? 1 : room > most ? most : room);
@@ -1559,14 +1563,16 @@ int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, ui
     }
     mp.trace = ctx->d_trace;
     if (ctx->d_trace && ctx->trace_ring > 1) {      // successive launches write successive blocks of the buffer
-        const uint64_t ctas = uint64_t(n_splits) * a.kv.n_kv_heads * a.seq.n_seqs;
+        const uint64_t ctas = uint64_t(n_splits) * a.kv.n_kv_heads * a.seq.units();
         mp.trace = ctx->d_trace + (ctx->trace_seq++ % ctx->trace_ring) * ctas * 16;
     }
     // Mode 2 prefetches K/V before it waits for the kernel in front of it.  When that kernel was
     // launched through this context and wrote rows of the very slab this call reads (the same layer
     // twice in a row, or a layer that reads its publisher's slab right after the publisher's
     // append), the prefetch has to wait as well.
-    mp.pdl = (ctx->pdl == 2u && (ctx->last_written_slab == a.kv.k || ctx->last_written_slab == kAnySlab)) ? 1u : ctx->pdl;
+    const uint64_t last_layer = a.seq.layer_ids ? a.seq.layer_ids[a.seq.n_layers - 1] : 0u;      // the list ascends
+    const uint64_t slab_bytes = (last_layer + 1) * rows * row_bytes;
+    mp.pdl = (ctx->pdl == 2u && ctx->reads_written(a.kv.k, slab_bytes)) ? 1u : ctx->pdl;
     mp.cluster = 0;
     mp.fan_merge = (a.fan && a.fan_merge) ? 1u : 0u;
     mp.fail_split = ctx->debug_fail_split;
@@ -1576,7 +1582,7 @@ int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, ui
         return set_error(ctx, VFKV_ERR_INVALID, "new K/V rows must be 16-byte aligned");
     if (n_splits > 1 && (!mp.tickets || !mp.tag_part)) return set_error(ctx, VFKV_ERR_INVALID, "workspace has no split-merge storage");
     if (n_splits > 255) return set_error(ctx, VFKV_ERR_UNSUPPORTED, "the tensor-core attention kernel merges at most 255 splits");
-    if (n_splits > 1 && uint64_t(a.seq.n_seqs) * a.kv.n_kv_heads > ws->n_counters)
+    if (n_splits > 1 && uint64_t(a.seq.units()) * a.kv.n_kv_heads > ws->n_counters)
         return set_error(ctx, VFKV_ERR_INVALID, "workspace too small for this call");
     const uint32_t g = a.n_q_heads / a.kv.n_kv_heads;
     auto run = [&]() -> int32_t {
@@ -1592,18 +1598,20 @@ int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, ui
         return set_error(ctx, VFKV_ERR_UNSUPPORTED, "shape outside the tensor-core attention kernel");
     };
     const int32_t rc = run();
-    if (rc == VFKV_OK) ctx->last_written_slab = a.k_new ? a.kv.k : nullptr;
+    if (rc == VFKV_OK) ctx->set_written(a.kv.k, a.k_new ? slab_bytes : 0u);
     return rc;
 }
 
-// Pre-encodes the two tensor maps of one layer of a cache (host memory; reused by every call).
-bool encode_layer_maps(vfkv_ctx *ctx, const KvView &v, void *tm_k_out, void *tm_v_out)
+// Pre-encodes the two tensor maps of n_layers layers of a cache from the one that v views on (host
+// memory; reused by every call).
+bool encode_layer_maps(vfkv_ctx *ctx, const KvView &v, uint32_t n_layers, void *tm_k_out, void *tm_v_out)
 {
     if (v.dtype == VFKV_F32) return false;
     const uint32_t es = v.dtype == VFKV_F8 ? 1 : 2;
     const uint64_t row_bytes = uint64_t(v.n_kv_heads) * v.head_dim * es;
     if (row_bytes < 128 || (uint64_t(v.head_dim) * es) % 128 != 0) return false;
-    const uint64_t rows = uint64_t(v.n_slots) * v.max_seq;
+    const uint64_t rows = uint64_t(n_layers) * v.n_slots * v.max_seq;
+    if (rows >= (1ull << 31)) return false;
     const uint32_t box_rows = v.dtype == VFKV_F8 ? 32 : 16;
     return encode_map(ctx, static_cast<CUtensorMap *>(tm_k_out), v.k, row_bytes, rows, box_rows) &&
            encode_map(ctx, static_cast<CUtensorMap *>(tm_v_out), v.v, row_bytes, rows, box_rows);

@@ -19,6 +19,9 @@ struct AttnParams {
     float scale, softcap;
     uint32_t *status;
     const PeerFanout *fan;             // device memory, or null
+    uint32_t n_layers;                 // > 1 or layered: see SeqArgs
+    uint32_t layered;
+    uint16_t layer_ids[kMaxLaunchLayers];
 };
 
 inline AttnParams make_params(const vfkv_ctx *ctx, const vfkv_workspace *ws, const AttnArgs &a,
@@ -47,16 +50,30 @@ inline AttnParams make_params(const vfkv_ctx *ctx, const vfkv_workspace *ws, con
     p.scale = a.scale; p.softcap = a.softcap;
     p.status = ctx->d_status;
     p.fan = a.fan;
+    p.n_layers = a.seq.n_layers;
+    p.layered = a.seq.layer_ids != nullptr;
+    for (uint32_t i = 0; p.layered && i < a.seq.n_layers; ++i) p.layer_ids[i] = a.seq.layer_ids[i];
     return p;
 }
 
 #ifdef __CUDACC__
-// Visible range [start, len) of sequence s and its slot.  Out-of-range
+// What unit u of a launch works on: its sequence, its row in Q / outputs / new tokens (in sequences),
+// and the slots in front of its layer's.
+struct UnitOf { uint32_t seq, row, slot_base; };
+__device__ __forceinline__ UnitOf unit_of(const AttnParams &p, uint32_t u)
+{
+    if (!p.layered) return {u, u, 0u};
+    const uint32_t i = u / p.n_seqs, s = u - i * p.n_seqs, layer = p.layer_ids[i];
+    return {s, layer * p.n_seqs + s, layer * p.n_slots};
+}
+
+// Visible range [start, len) of a unit's sequence and its slot.  Out-of-range
 // arguments from device arrays are clamped and reported through the status
 // word instead of being dereferenced.
-__device__ __forceinline__ void seq_range(const AttnParams &p, uint32_t s, uint32_t *slot,
+__device__ __forceinline__ void seq_range(const AttnParams &p, const UnitOf &unit, uint32_t *slot,
                                           uint32_t *start, uint32_t *len)
 {
+    const uint32_t s = unit.seq;
     uint32_t sl = p.slot_ids ? p.slot_ids[s] : p.slot0 + s;
     uint32_t n, st;
     if (p.positions) {
@@ -73,7 +90,7 @@ __device__ __forceinline__ void seq_range(const AttnParams &p, uint32_t s, uint3
         if (n > p.max_seq) n = p.max_seq;
     }
     if (st > n) st = n;
-    *slot = sl; *start = st; *len = n;
+    *slot = sl + unit.slot_base; *start = st; *len = n;
 }
 
 // Positions [*begin, *end) of split `split`; chunks are multiples of `align`.

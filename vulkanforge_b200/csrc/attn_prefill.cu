@@ -462,7 +462,7 @@ int32_t launch_mma_t(vfkv_ctx *ctx, const PrefillParams &p, cudaStream_t st)
     }
     const uint32_t row_blocks = (p.m * p.group + BM - 1) / BM;
     kern<<<dim3(row_blocks, p.n_kv_heads), 128, kSmem, st>>>(p);
-    ctx->launches++;
+    ctx->count_launch();
     return check_cuda(ctx, cudaGetLastError(), "prefill attention launch");
 }
 
@@ -557,6 +557,6 @@ extern "C" int32_t vfkv_attend_prefill(vfkv_cache *cache, uint32_t layer, uint32
         return launch_mma_d<VFKV_F16, 256>(ctx, p, st);
     }
     prefill_simple_kernel<<<dim3(m, n_q_heads), 128, 0, st>>>(p, dt);
-    ctx->launches++;
+    ctx->count_launch();
     return check_cuda(ctx, cudaGetLastError(), "prefill attention launch");
 }

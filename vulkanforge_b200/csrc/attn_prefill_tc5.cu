@@ -1713,14 +1713,14 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
             cfg.attrs = attr;
             cfg.numAttrs = 1;
             if (cudaLaunchKernelEx(&cfg, kern, p, tm_k, tm_v) == cudaSuccess) {
-                ctx->launches++;
+                ctx->count_launch();
                 return check_cuda(ctx, cudaGetLastError(), "tcgen05 prefill attention launch");
             }
             (void)cudaGetLastError();          // not all resident: the pieces go to the merge kernel instead
             p.inline_merge = 0u;
         }
         kern<<<grid_h, 384, kSmemBytes, st>>>(p, tm_k, tm_v);
-        ctx->launches++;
+        ctx->count_launch();
         if (spread) {
             // launched as a programmatic dependent: it is resident, its table built, when the last CTA
             // of the attention kernel ends
@@ -1735,7 +1735,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
             cfg.numAttrs = 1;
             cudaError_t e = cudaLaunchKernelEx(&cfg, prefill_tc5_merge_kernel, p);
             if (e != cudaSuccess) return check_cuda(ctx, e, "tcgen05 prefill merge launch");
-            ctx->launches++;
+            ctx->count_launch();
         }
         return check_cuda(ctx, cudaGetLastError(), "tcgen05 prefill attention launch");
     }
@@ -1759,7 +1759,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
             if (cap) prefill_tc5p_kernel<VFKV_F16, true><<<grid, 256, kSmemBytes, st>>>(p);
             else prefill_tc5p_kernel<VFKV_F16, false><<<grid, 256, kSmemBytes, st>>>(p);
         }
-        ctx->launches++;
+        ctx->count_launch();
         return check_cuda(ctx, cudaGetLastError(), "tcgen05 prefill attention launch");
     }
     if (dtype == VFKV_F8) {
@@ -1769,7 +1769,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
         if (cap) prefill_tc5_kernel<VFKV_F16, true><<<grid, 256, kSmemBytes, st>>>(p);
         else prefill_tc5_kernel<VFKV_F16, false><<<grid, 256, kSmemBytes, st>>>(p);
     }
-    ctx->launches++;
+    ctx->count_launch();
     return check_cuda(ctx, cudaGetLastError(), "tcgen05 prefill attention launch");
 }
 

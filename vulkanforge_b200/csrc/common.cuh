@@ -23,13 +23,26 @@ struct vfkv_ctx {
     uint32_t prefill_scratch_ctas = 0;
     uint32_t prefill_epoch = 0;                 // value the flags of the current spread prefill launch take
     uint32_t pdl = 0;                  // programmatic dependent launch mode of the attention kernel (0 / 1 / 2)
-    // Layer slab (K base address) that the last launch on this context wrote cache rows into, or
-    // null: a mode-2 launch that reads the same slab next waits before its K/V prefetch (mode 1).
-    const void *last_written_slab = nullptr;
+    // K addresses that the last launch on this context wrote cache rows into, or an empty range: a
+    // mode-2 launch that reads any of them next waits before its K/V prefetch (mode 1).
+    uintptr_t written_lo = 0, written_hi = 0;
+    void set_written(const void *lo, uint64_t bytes)
+    {
+        written_lo = bytes ? uintptr_t(lo) : 0;
+        written_hi = written_lo + bytes;
+    }
+    void set_written_any() { written_lo = 0; written_hi = ~uintptr_t(0); }      // a raw destination may lie in any layer
+    bool reads_written(const void *lo, uint64_t bytes) const
+    {
+        return uintptr_t(lo) < written_hi && uintptr_t(lo) + bytes > written_lo;
+    }
     uint64_t merge_wait_ns = 1000000000ull;   // limit of the merging CTA's wait for the other splits' partials
     uint32_t debug_fail_split = 0xFFFFFFFFu;  // failure injection for tests (vfkv_ctx_debug_fail_split)
     uint32_t cluster_merge = 0;        // 1: merge the splits inside a thread-block cluster where the device allows it
-    uint64_t launches = 0;
+    // kernels enqueued, and the same count with a kernel that carries several layers of a token
+    // counted once for each of them (so that it does not depend on how layers are grouped)
+    uint64_t kernels = 0, launches = 0;
+    void count_launch(uint32_t layers = 1) { ++kernels; launches += layers; }
     unsigned long long *d_trace = nullptr;   // caller-owned device buffer for kernel phase timestamps, or null
     uint32_t trace_ring = 1;                 // blocks in d_trace; launch k of the decode kernel writes block k % trace_ring
     uint64_t trace_seq = 0;
@@ -48,11 +61,14 @@ struct vfkv_cache {
     struct alignas(64) TmapBytes { unsigned char b[128]; };
     std::vector<TmapBytes> tm_k, tm_v;
     std::vector<unsigned char> tm_state;   // 0 = not tried, 1 = ready, 2 = not encodable
+    TmapBytes tm_all_k, tm_all_v;          // the same over all layers of a uniform cache, for calls that take several at once
+    unsigned char tm_all_state = 0;
 };
 
 struct vfkv_workspace {
     vfkv_ctx *ctx = nullptr;
     uint32_t max_seqs = 0, n_q_heads = 0, head_dim = 0, max_splits = 0;
+    void *block = nullptr;      // the one allocation that the pointers below lie in
     float *part_o = nullptr;    // [seq][q_head][split][head_dim]
     float *part_m = nullptr;    // [seq][q_head][split]
     float *part_l = nullptr;    // [seq][q_head][split]
@@ -77,6 +93,7 @@ struct vfkv_workspace {
     // next group's inputs and the previous group's outputs while a group computes.
     static constexpr uint32_t kTokChunks = 4;
     cudaGraphExec_t tok_graphs[kTokChunks] = {nullptr, nullptr, nullptr, nullptr};
+    uint32_t tok_launches[kTokChunks] = {}, tok_kernels[kTokChunks] = {};   // what one replay adds to the context's counts
     uint64_t tok_key[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t tok_events[2 * kTokChunks] = {};         // inputs there / group done, per group
@@ -91,7 +108,7 @@ struct vfkv_workspace {
         uint64_t key[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         cudaEvent_t ev_in = nullptr, ev_done = nullptr, ev_out = nullptr;
         uint64_t ticket = 0;                             // ticket in flight on this slot, 0 = free
-        uint32_t launches = 0;
+        uint32_t launches = 0, kernels = 0;              // what one replay adds to the context's counts
     };
     HostSlot host_slot[2];
     cudaStream_t h2d_stream = nullptr, d2h_stream = nullptr;
@@ -102,6 +119,8 @@ namespace vfkv {
 
 int32_t set_error(vfkv_ctx *ctx, int32_t status, const std::string &msg);
 int32_t check_cuda(vfkv_ctx *ctx, cudaError_t e, const char *what);
+
+constexpr uint32_t kMaxLaunchLayers = 64;   // layers one launch can carry (their indexes travel as a kernel argument)
 
 // One layer's slab(s) as seen by the attention kernels.
 struct KvView {
@@ -130,8 +149,14 @@ struct SeqArgs {
     uint32_t seq_len_scalar = 0;
     uint32_t kv_start_scalar = 0;
     uint32_t window = 0;                  // with positions: kv_start = max(0, pos+1-window)
-    uint32_t n_seqs = 1;
+    uint32_t n_seqs = 1;                  // sequences of one layer
     uint32_t max_len_hint = 0;
+    // Several layers of a uniform cache in one launch: kv is then the view of layer 0, unit u of the
+    // launch is sequence u % n_seqs of layer layer_ids[u / n_seqs], and Q, outputs and new rows are
+    // indexed [layer][sequence].  n_layers 1 with a null list: the one layer that kv views.
+    uint32_t n_layers = 1;
+    const uint16_t *layer_ids = nullptr;  // host memory, n_layers <= kMaxLaunchLayers entries
+    uint32_t units() const { return n_seqs * n_layers; }
 };
 
 // Fan-out of the (m, l, o) partial to every GPU of a position-sharded group, written by the
@@ -206,6 +231,9 @@ struct AppendArgs {
     const uint32_t *positions = nullptr;
     // consecutive mode on a position-sharded cache: base_pos is global, only this rank's rows are stored
     uint32_t shard_world = 0, shard_rank = 0, shard_page = 0;
+    // batch mode over several layers (see SeqArgs): n_rows is per layer, k_dst / v_dst are layer 0's
+    uint32_t n_layers = 1;
+    const uint16_t *layer_ids = nullptr;
 };
 int32_t launch_append(vfkv_ctx *ctx, const AppendArgs &a, cudaStream_t st);
 
@@ -237,15 +265,12 @@ uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile);
 int32_t launch_attn_generic(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits,
                             cudaStream_t st);
 bool attn_mma_supported(const AttnArgs &a);
-bool encode_layer_maps(vfkv_ctx *ctx, const KvView &v, void *tm_k_out, void *tm_v_out);
+bool encode_layer_maps(vfkv_ctx *ctx, const KvView &v, uint32_t n_layers, void *tm_k_out, void *tm_v_out);
 int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits,
                         cudaStream_t st);
 // merges ws partials [seq][head][split] into a.out (normalised) or a.out_{m,l,o}
 int32_t launch_merge_ws(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits,
                         cudaStream_t st);
-
-// vfkv_ctx::last_written_slab after a store whose destination is a raw pointer.
-static const void *const kAnySlab = reinterpret_cast<const void *>(~uintptr_t(0));
 
 // Sentinel of vk_shaders/flash_attn_split.comp:104 for masked scores.
 constexpr float kMaskedScore = -1e30f;

@@ -145,7 +145,7 @@ int32_t launch_fanout_push(vfkv_ctx *ctx, const PeerFanout &fan, const float *st
 {
     const uint64_t n = fanout_block_words(fan.n_rows, head_dim);
     fanout_push_kernel<<<uint32_t((n + 255) / 256), 256, 0, st>>>(fan, staging, head_dim);
-    ctx->launches++;
+    ctx->count_launch();
     return check_cuda(ctx, cudaGetLastError(), "fanout_push launch");
 }
 
@@ -303,7 +303,7 @@ int32_t vfkv_exchange_merge(vfkv_exchange *ex, float *d_out, void *stream)
     cudaError_t le = cudaLaunchKernelEx(&cfg, exchange_merge_kernel, ex->fan, static_cast<const uint64_t *>(ex->local),
                                         ex->ctl, ex->head_dim, ex->wait_ns, d_out, ctx->d_status);
     if (le != cudaSuccess) return check_cuda(ctx, le, "exchange_merge launch");
-    ctx->launches++;
+    ctx->count_launch();
     return check_cuda(ctx, cudaGetLastError(), "exchange_merge launch");
 }
 

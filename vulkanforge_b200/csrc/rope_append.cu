@@ -169,8 +169,8 @@ static int32_t launch_rope_append_t(vfkv_ctx *ctx, const RopeAppendParams &p, cu
     if (blocks > cap) blocks = cap;
     ProfScope ps(ctx, VFKV_PROF_KV_STORE, st);
     rope_append_kernel<DT><<<dim3(unsigned(blocks), 2), 256, 0, st>>>(p);
-    ctx->launches++;
-    ctx->last_written_slab = p.k_dst;
+    ctx->count_launch();
+    ctx->set_written(p.k_dst, uint64_t(p.n_slots) * p.slot_stride_bytes);
     return check_cuda(ctx, cudaGetLastError(), "rope_append launch");
 }
 
@@ -289,7 +289,7 @@ int32_t vfkv_rope_neox(vfkv_ctx *ctx, const float *d_x, float *d_out, uint32_t n
     rope_neox_kernel<<<unsigned(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         d_x, d_out, n_rows, n_heads, head_dim, d_positions, base_pos, rope->n_dims, theta_scale_of(*rope),
         rope->freq_scale);
-    ctx->launches++;
+    ctx->count_launch();
     return check_cuda(ctx, cudaGetLastError(), "rope_neox launch");
 }
 

@@ -142,6 +142,10 @@ class Context:
     def launch_count(self) -> int:
         return int(self._lib.vfkv_ctx_launch_count(self.handle))
 
+    def kernel_count(self) -> int:
+        """launch_count with a kernel that carries several layers of a token counted once."""
+        return int(self._lib.vfkv_ctx_kernel_count(self.handle))
+
     def destroy(self) -> None:
         if self.handle:
             self._lib.vfkv_ctx_destroy(self.handle)

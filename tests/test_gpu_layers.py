@@ -1,0 +1,78 @@
+"""vfkv_decode_token with several layers in a launch: the same rows and outputs as a decode step per layer."""
+import numpy as np
+import pytest
+
+import vulkanforge_b200 as vf
+from util import kv_values, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype,scaled,hq,hkv,d,n_layers,lens,windows,n_splits", [
+    ("F8", False, 32, 8, 128, 1, [300], None, 0),
+    ("F8", False, 8, 1, 128, 70, [130], None, 0),                       # more layers than one launch carries
+    ("F8", False, 16, 8, 128, 7, [257, 1, 64], [64, 0, 64, 100, 0, 64, 0], 0),   # windows: a launch for each
+    ("F16", False, 16, 8, 256, 5, [500, 33], [128, 128, 128, 128, 0], 3),
+    ("F16", False, 4, 2, 64, 3, [2000], None, 64),                      # more splits than the workspace has room for
+    ("F32", False, 8, 2, 128, 6, [700, 65], [0, 50, 0, 50, 0, 50], 0),  # CUDA-core kernels: append, split, merge
+    ("F32", False, 16, 2, 512, 4, [300, 20], None, 5),
+    ("F8", True, 32, 8, 128, 5, [400, 31, 129], None, 0),
+])
+@pytest.mark.parametrize("slots", [False, True])
+def test_layers_of_a_token_share_launches(ctx, dtype, scaled, hq, hkv, d, n_layers, lens, windows, n_splits, slots):
+    import torch
+    n, longest = len(lens), max(lens)
+    rng = np.random.default_rng(n_layers * 100 + longest)
+    gen = torch.Generator(device="cuda").manual_seed(longest)
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(n_layers, hkv, d, longest + 3, n_slots=n + 1, scale_mode=int(scaled)),
+                       vf.KvDtype[dtype])
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq, max_batch=n, n_splits=n_splits)
+    ids = list(range(n, 0, -1)) if slots else list(range(n))
+    try:
+        for layer in range(n_layers):
+            for i, length in enumerate(lens):
+                kv = torch.randn(2, length, hkv, d, device="cuda", generator=gen)
+                fwd.b_step_kv_write(layer, kv[0], kv[1], length, 0, ids[i])
+        q = torch.randn(n_layers, n, hq, d, device="cuda", generator=gen)
+        k = to_dev(kv_values(rng, (n_layers, n, hkv, d)))
+        v = to_dev(kv_values(rng, (n_layers, n, hkv, d)))
+        pos = to_dev(np.array([x - 1 for x in lens], np.uint32))
+        d_ids = to_dev(np.array(ids, np.uint32)) if slots else None
+        row = cache.row_bytes(0)
+
+        def state():
+            torch.cuda.synchronize()
+            L, out = ctx._lib, np.empty((2, cache.bytes_per_buffer()), np.uint8)
+            for o, a in zip(out, (cache.k_buffer, cache.v_buffer)):
+                ctx.check(L.vfkv_memcpy_d2h(ctx.handle, o.ctypes.data, a, o.nbytes, None))
+            ctx.check(L.vfkv_stream_synchronize(ctx.handle, None))
+            return [out[:, cache.slot_offset_bytes(l, s) + (x - 1) * row:][:, :row].copy()
+                    for l in range(n_layers) for s, x in zip(ids, lens)]
+
+        per_layer, together = torch.zeros_like(q), torch.zeros_like(q)
+        w_of = lambda l: windows[l] if windows else 0
+        for layer in range(n_layers):
+            fwd.sliding_layers, fwd.sliding_window = ({layer}, w_of(layer)) if w_of(layer) else (set(), 0)
+            fwd.decode_step(layer, q[layer], k[layer], v[layer], per_layer[layer], d_ids, pos, n, longest)
+        want = state()
+        for layer in range(n_layers):                      # other rows in the token's place, to be overwritten again
+            for i, length in enumerate(lens):
+                z = torch.zeros(2, 1, hkv, d, device="cuda")
+                fwd.b_step_kv_write(layer, z[0], z[1], 1, length - 1, ids[i])
+        kernels = ctx.kernel_count()
+        import ctypes as C
+        arr = (C.c_uint32 * n_layers)(*windows) if windows else None
+        ctx.check(ctx._lib.vfkv_decode_token(cache.handle, fwd.workspace.handle, q.data_ptr(), k.data_ptr(), v.data_ptr(),
+                                             together.data_ptr(), hq, None if d_ids is None else d_ids.data_ptr(),
+                                             pos.data_ptr(), n, longest, C.cast(arr, C.c_void_p) if windows else None,
+                                             fwd.attn_scale, 0.0, n_splits, None))
+        got = state()
+        ctx.poll()
+        launches = len(set(windows)) if windows else -(-n_layers // 64)
+        assert ctx.kernel_count() - kernels <= 3 * launches
+        assert all(np.array_equal(a, b) for a, b in zip(want, got))
+        scale = float(per_layer.abs().max())
+        assert float((together - per_layer).abs().max()) < 2e-5 * max(1.0, scale)
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

@@ -7,39 +7,18 @@
 // query and head; here one CTA owns 64 rows = (64 / g) consecutive queries x the g q-heads of
 // one kv-head, so a K/V tile is fetched once per 64 rows, widened to half precision once
 // (FP8 caches; the kv_fp8_to_f16.comp step) and consumed by m16n8k16 tensor-core MMAs with the
-// usual online softmax.  Shapes outside that kernel use a CUDA-core kernel with the reference's
-// work split (one CTA per (query, head)).
+// usual online softmax.  Shapes outside that kernel take the f32 tiles of attn_prefill_f32.cu, or for
+// other head_dims and unaligned buffers a kernel with the reference's work split (one CTA per (query, head)).
 #include <cmath>
 
 #include "../../include/vfkv_next.h"
-#include "common.cuh"
 #include "fp8_codec.cuh"
+#include "prefill_params.cuh"
 
 namespace vfkv {
 namespace {
 
 constexpr float kLog2e = 1.4426950408889634f;
-
-struct PrefillParams {
-    const uint8_t *k, *v;              // rows of the slot: [pos][kv_head][dim]
-    const float *k_scales, *v_scales;  // [pos][kv_head] or null
-    const float *q;                    // [m][n_q_heads][dim]
-    float *out;                        // [m][n_q_heads][dim]
-    uint64_t row_bytes;
-    uint32_t n_q_heads, n_kv_heads, group, head_dim, m, q_start, n_kv, kv_start, window;
-    float scale, softcap;
-};
-
-// Visible range [lo, hi) of query i (flash_attn_batch.comp:116-119,141-144; window: per-query bound).
-__device__ __forceinline__ void query_range(const PrefillParams &p, uint32_t i, uint32_t *lo, uint32_t *hi)
-{
-    uint32_t c = p.q_start + i + 1u;
-    if (c > p.n_kv) c = p.n_kv;
-    uint32_t l = p.kv_start;
-    if (p.window != 0u && c > p.window && c - p.window > l) l = c - p.window;
-    if (l > c) l = c;
-    *lo = l; *hi = c;
-}
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
@@ -556,6 +535,7 @@ extern "C" int32_t vfkv_attend_prefill(vfkv_cache *cache, uint32_t layer, uint32
         if (D == 128) return launch_mma_d<VFKV_F16, 128>(ctx, p, st);
         return launch_mma_d<VFKV_F16, 256>(ctx, p, st);
     }
+    if (aligned && prefill_f32_supported(D)) return launch_prefill_f32(ctx, dt, p, st);
     prefill_simple_kernel<<<dim3(m, n_q_heads), 128, 0, st>>>(p, dt);
     ctx->count_launch();
     return check_cuda(ctx, cudaGetLastError(), "prefill attention launch");

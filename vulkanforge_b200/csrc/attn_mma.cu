@@ -402,7 +402,13 @@ __device__ __forceinline__ void pv_t_f16(const uint32_t (&vb)[4], const uint32_t
 // leave SMs idle run 8 warps x 3 stages, spreading a CTA's short stream over more warps.
 // CAP compiles the score soft-cap in or out.
 // TR selects the transposed products (heads on the N side; the host picks it for groups of at most 4).
-template <int DT, int D, bool ROWS2, int W, int NS, bool CAP, bool TR>
+// SC: an FP8 cache with a scale per (position, kv-head).  The codes go through the products as they
+// are; a score is multiplied by its position's K scale and a p by its V scale in f32.  p * V scale has
+// no bound that half precision would hold, so it is fed relative to the largest power of two seen
+// among the warp's V scales (exact), which the accumulators follow like they follow the maximum.
+// A lane holds the two scales of position `lane` of the next tile in registers: one 4-byte load each,
+// issued a tile ahead (the CUDA-core kernel took 67 us for 8 x 4099 positions, 32 q / 8 kv / 128).
+template <int DT, int D, bool ROWS2, int W, int NS, bool CAP, bool TR, bool SC>
 __global__ void __launch_bounds__(W * 32, (W == 4 && NS == 2 && Shape<DT, D, W, NS>::STAGE_BYTES <= 8192) ? 3 : 1)
 attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                       const MmaParams mp)
@@ -413,6 +419,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     constexpr int TP = S::TP, NB = S::NB, NC = S::NC, KSTEPS = S::KSTEPS, NDB = S::NDB;
     constexpr bool FP8 = DT == VFKV_F8;
     static_assert(!(TR && ROWS2), "the transposed products hold at most 4 heads");
+    static_assert(!SC || FP8, "scales belong to FP8 caches");
     constexpr int RS = (!FP8 && ROWS2) ? 2 : 1;          // logical score rows per thread
     constexpr int MB = TP / 16;                          // transposed form: 16-position M blocks per tile
     constexpr int NQB = D / 16;                          // transposed form: 16-dim k steps of Q K^T / M blocks of O^T
@@ -557,6 +564,18 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         for (uint32_t n = 0; n < pre; ++n) issue(n);
     }
 
+    // scales of position `lane` of this warp's n-th tile
+    const float *const ksc = SC ? p.k_scales + uint64_t(slot) * p.slot_stride_scales + kvh : nullptr;
+    const float *const vsc = SC ? p.v_scales + uint64_t(slot) * p.slot_stride_scales + kvh : nullptr;
+    float ks_next = 1.f, vs_next = 1.f;
+    auto load_scales = [&](uint32_t n) {
+        const uint32_t pos = begin + (warp + n * kWarps) * TP + lane;
+        const bool ok = n < my_tiles && pos < end;
+        ks_next = ok ? ksc[uint64_t(pos) * p.n_kv_heads] : 1.f;
+        vs_next = ok ? vsc[uint64_t(pos) * p.n_kv_heads] : 0.f;
+    };
+    if constexpr (SC) load_scales(0);
+
     if (mp.pdl == 2u) {       // the prefetch is in flight; now wait for the predecessor, then read Q
         asm volatile("griddepcontrol.wait;" ::: "memory");
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -574,7 +593,39 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     const uint32_t new_tile = has_new ? (len - 1 - begin) / TP : 0;
     const bool new_owner = has_new && (new_tile % kWarps) == warp;
     uint4 newu[NEWU];
+    float new_ks = 1.f, new_vs = 1.f;
     if (new_owner) {
+        if constexpr (SC) {
+            // scale = max(absmax / 448, 1e-12), code = e4m3(clamp(x / scale)), as in append_scaled_kernel;
+            // lanes 0 .. UPT-1 hold K's units, the next UPT lanes V's
+            static_assert(2 * UPT <= 32 && (UPT & (UPT - 1)) == 0, "a unit per lane");
+            float x[16];
+            const bool mine = lane < 2 * UPT, is_k = lane < UPT;
+            const float4 *s4 = reinterpret_cast<const float4 *>((is_k ? mp.k_new : mp.v_new) +
+                                                                (uint64_t(sr) * p.n_kv_heads + kvh) * D + (lane % UPT) * 16);
+            float amax = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 a = mine ? s4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[4 * i] = a.x; x[4 * i + 1] = a.y; x[4 * i + 2] = a.z; x[4 * i + 3] = a.w;
+                amax = fmaxf(amax, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))));
+            }
+#pragma unroll
+            for (uint32_t o = 1; o < UPT; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            const float sc = fmaxf(__fmul_rn(amax, 1.0f / 448.0f), 1e-12f), inv = __fdiv_rn(1.0f, sc);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) x[i] = x[i] != x[i] ? x[i] : fminf(fmaxf(__fmul_rn(x[i], inv), -448.f), 448.f);
+            newu[0] = make_uint4(f32x4_to_e4m3x4(x[0], x[1], x[2], x[3]), f32x4_to_e4m3x4(x[4], x[5], x[6], x[7]),
+                                 f32x4_to_e4m3x4(x[8], x[9], x[10], x[11]), f32x4_to_e4m3x4(x[12], x[13], x[14], x[15]));
+            if (mine) {
+                uint8_t *dst = const_cast<uint8_t *>(is_k ? p.k : p.v) + uint64_t(slot) * p.slot_stride_bytes +
+                               uint64_t(len - 1) * p.n_kv_heads * D + uint64_t(kvh) * D + (lane % UPT) * 16;
+                *reinterpret_cast<uint4 *>(dst) = newu[0];
+                if (lane % UPT == 0u) const_cast<float *>(is_k ? ksc : vsc)[uint64_t(len - 1) * p.n_kv_heads] = sc;
+            }
+            new_ks = __shfl_sync(0xffffffffu, sc, 0);
+            new_vs = __shfl_sync(0xffffffffu, sc, UPT);
+        } else {
 #pragma unroll
         for (uint32_t i = 0; i < NEWU; ++i) {
             const uint32_t u = lane + 32 * i;
@@ -596,6 +647,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                                uint64_t(len - 1) * p.n_kv_heads * D * S::ES + uint64_t(kvh) * D * S::ES + (u % UPT) * 16;
                 *reinterpret_cast<uint4 *>(dst) = newu[i];
             }
+        }
         }
     }
 
@@ -677,6 +729,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 #pragma unroll
     for (int nb = 0; nb < NACC; ++nb) { acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.f; }
     bool timed_out = false;
+    uint32_t vs_ref = 0u;                // SC: exponent bits of the largest V scale so far; acc is relative to it
     // ---- split ticket -----------------------------------------------------------------------------
     // Every CTA of a (sequence, kv-head) draws one ticket from a 64-bit word that only ever counts
     // up; there is one word per split count, so ticket / n_splits is the number of the launch among
@@ -758,6 +811,19 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         }
 
         const bool full = n_valid == uint32_t(TP);
+        float ks_cur = 1.f, vs_cur = 1.f, vs_corr = 1.f;      // vs_cur: V scale x kPScale, relative to vs_ref
+        if constexpr (SC) {
+            ks_cur = ks_next; vs_cur = vs_next;
+            if (new_owner && n == new_tile / kWarps && t0 + lane == len - 1) { ks_cur = new_ks; vs_cur = new_vs; }
+            load_scales(n + 1);
+            const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(vs_cur)) & 0x7f800000u;
+            if (top > vs_ref) {          // at least 1e-12 and at most 2^119, so every power of two below is a normal number
+                vs_corr = vs_ref != 0u ? __uint_as_float((127u << 23) - (top - vs_ref)) : 0.f;
+                if (vs_ref != 0u && top - vs_ref >= (127u << 23)) vs_corr = 0.f;
+                vs_ref = top;
+            }
+            vs_cur *= __uint_as_float((254u << 23) - vs_ref) * kPScale;
+        }
         if constexpr (TR) {
         // ---- S^T = K Q^T : M = 16 positions per block, N = the heads' high / low columns ----------
         float sc[MB][4];
@@ -775,6 +841,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 float v = (sc[mb][2 * i] + sc[mb][2 * i + 1]) * mult[0];
+                if constexpr (SC) v *= __shfl_sync(0xffffffffu, ks_cur, 16 * mb + 8 * i + gid);
                 if constexpr (CAP) v = p.softcap * tanhf(v / p.softcap) * kLog2e;
                 if (!full) v = uint32_t(16 * mb + 8 * i) + gid < n_valid ? v : kMaskedScore;
                 x[mb][i] = v;
@@ -785,12 +852,13 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 16));
         const float mn = fmaxf(m[0], tmax);
         const float corr = fast_exp2(m[0] - mn);
-        const bool changed = mn != m[0];
+        const bool changed = mn != m[0] || (SC && vs_corr != 1.f);
         m[0] = mn;
         l[0] *= corr;
         if (__any_sync(0xffffffffu, changed)) {
+            const float f = SC ? corr * vs_corr : corr;
 #pragma unroll
-            for (int nb = 0; nb < NACC; ++nb) { acc[nb][0] *= corr; acc[nb][1] *= corr; acc[nb][2] *= corr; acc[nb][3] *= corr; }
+            for (int nb = 0; nb < NACC; ++nb) { acc[nb][0] *= f; acc[nb][1] *= f; acc[nb][2] *= f; acc[nb][3] *= f; }
         }
         // p = 2^(x - m) as {high, low} half pairs = this thread's two columns of a position row;
         // the 8x8 transpose turns them into the B fragment (k = positions, n = columns) of O^T += V^T P^T
@@ -801,7 +869,8 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             for (int i = 0; i < 2; ++i) {
                 const float pv = fast_exp2(x[mb][i] - mn);
                 l[0] += pv;
-                pb[mb][i] = movmatrix_trans(hi_lo_f16x2(pv * kPScale));
+                if constexpr (SC) pb[mb][i] = movmatrix_trans(hi_lo_f16x2(pv * __shfl_sync(0xffffffffu, vs_cur, 16 * mb + 8 * i + gid)));
+                else pb[mb][i] = movmatrix_trans(hi_lo_f16x2(pv * kPScale));
             }
         if constexpr (FP8) {
             uint32_t vb[8];
@@ -836,9 +905,11 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                     float v = SPLIT ? (sc[j][i] + sc[j][i + 2]) : sc[j][2 * r + i];
                     if constexpr (CAP) {
                         v *= mult[r];
+                        if constexpr (SC) v *= __shfl_sync(0xffffffffu, ks_cur, 8 * j + 2 * tig + i);
                         v = p.softcap * tanhf(v / p.softcap) * kLog2e;
                     } else {
                         v *= mult[r];                      // scale * log2(e) / q_scale
+                        if constexpr (SC) v *= __shfl_sync(0xffffffffu, ks_cur, 8 * j + 2 * tig + i);
                     }
                     x[r][j][i] = v;
                 }
@@ -860,9 +931,10 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         for (int r = 0; r < RS; ++r) {
             const float mn = fmaxf(m[r], tmax[r]);
             corr[r] = fast_exp2(m[r] - mn);
-            changed |= mn != m[r];
+            changed |= mn != m[r] || (SC && vs_corr != 1.f);
             m[r] = mn;
             l[r] *= corr[r];
+            if constexpr (SC) corr[r] *= vs_corr;
         }
         if (__any_sync(0xffffffffu, changed)) {
 #pragma unroll
@@ -881,7 +953,8 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const float pv = fast_exp2(x[r][j][i] - mo);
-                    x[r][j][i] = pv * kPScale;
+                    if constexpr (SC) x[r][j][i] = pv * __shfl_sync(0xffffffffu, vs_cur, 8 * j + 2 * tig + i);
+                    else x[r][j][i] = pv * kPScale;
                     l[r] += pv;
                 }
         }
@@ -955,6 +1028,8 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 
     // ---- merge the warps' partials in shared memory ---------------------------------------------
     constexpr int NH = (FP8 || !ROWS2) ? 8 : 16;              // head rows this CTA can hold
+    // accumulators back to units of V
+    const float acc_unit = SC ? kInvPScale * __uint_as_float(vs_ref) : kInvPScale;
     constexpr int DP = D + 1;                                 // odd row pitch: the 32 lanes hit 32 banks
     float *sm_o = reinterpret_cast<float *>(ring_ptr);        // [kWarps][NH][DP]
     float *sm_m = sm_o + kWarps * NH * DP;                    // [kWarps][NH]
@@ -971,11 +1046,11 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             for (int db = 0; db < NACC; ++db) {
                 if constexpr (FP8) {
                     const uint32_t d0 = 32 * (db / 2) + 4 * gid + 2 * (db % 2);
-                    o[d0] = (acc[db][0] + acc[db][1]) * kInvPScale;
-                    o[d0 + 1] = (acc[db][2] + acc[db][3]) * kInvPScale;
+                    o[d0] = (acc[db][0] + acc[db][1]) * acc_unit;
+                    o[d0 + 1] = (acc[db][2] + acc[db][3]) * acc_unit;
                 } else {
-                    o[16 * db + gid] = (acc[db][0] + acc[db][1]) * kInvPScale;
-                    o[16 * db + 8 + gid] = (acc[db][2] + acc[db][3]) * kInvPScale;
+                    o[16 * db + gid] = (acc[db][0] + acc[db][1]) * acc_unit;
+                    o[16 * db + 8 + gid] = (acc[db][2] + acc[db][3]) * acc_unit;
                 }
             }
         }
@@ -995,16 +1070,16 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             // column n of block nb is dim 32*(nb/4) + 4n + nb%4 (see the V transpose above)
             const uint32_t d0 = 32 * (nb / 4) + 4 * (2 * tig) + (nb % 4);
             float *o = sm_o + (warp * NH + gid) * DP;
-            o[d0] = (acc[nb][0] + acc[nb][2]) * kInvPScale;
-            o[d0 + 4] = (acc[nb][1] + acc[nb][3]) * kInvPScale;
+            o[d0] = (acc[nb][0] + acc[nb][2]) * acc_unit;
+            o[d0 + 4] = (acc[nb][1] + acc[nb][3]) * acc_unit;
         } else {
             const uint32_t d0 = 8 * nb + 2 * tig;
             float *o = sm_o + (warp * NH + gid) * DP;
             if constexpr (SPLIT) {
-                o[d0] = (acc[nb][0] + acc[nb][2]) * kInvPScale; o[d0 + 1] = (acc[nb][1] + acc[nb][3]) * kInvPScale;
+                o[d0] = (acc[nb][0] + acc[nb][2]) * acc_unit; o[d0 + 1] = (acc[nb][1] + acc[nb][3]) * acc_unit;
             } else {
-                o[d0] = acc[nb][0] * kInvPScale; o[d0 + 1] = acc[nb][1] * kInvPScale;
-                o[8 * DP + d0] = acc[nb][2] * kInvPScale; o[8 * DP + d0 + 1] = acc[nb][3] * kInvPScale;
+                o[d0] = acc[nb][0] * acc_unit; o[d0 + 1] = acc[nb][1] * acc_unit;
+                o[8 * DP + d0] = acc[nb][2] * acc_unit; o[8 * DP + d0 + 1] = acc[nb][3] * acc_unit;
             }
         }
     }
@@ -1364,7 +1439,7 @@ bool encode_map(vfkv_ctx *ctx, CUtensorMap *out, const void *base, uint64_t row_
     return r == CUDA_SUCCESS;
 }
 
-template <int DT, int D, bool ROWS2, int W, int NS, bool CAP, bool TR>
+template <int DT, int D, bool ROWS2, int W, int NS, bool CAP, bool TR, bool SC>
 int32_t launch_k(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, const MmaParams &mp, cudaStream_t st)
 {
     using S = Shape<DT, D, W, NS>;
@@ -1374,7 +1449,7 @@ int32_t launch_k(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
     if constexpr (S::SMEM_BYTES > 227 * 1024 || !kMergeFits) {
         return set_error(ctx, VFKV_ERR_UNSUPPORTED, "tuning does not fit in shared memory for this shape");
     } else {
-        auto kern = attn_split_mma_kernel<DT, D, ROWS2, W, NS, CAP, TR>;
+        auto kern = attn_split_mma_kernel<DT, D, ROWS2, W, NS, CAP, TR, SC>;
         // per device, shared by every context and thread: setting the attribute twice is harmless,
         // the flag only saves the call
         static std::atomic<bool> configured[64];
@@ -1469,7 +1544,7 @@ int32_t launch_k(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
     }
 }
 
-template <int DT, int D, bool ROWS2, bool CAP, bool TR>
+template <int DT, int D, bool ROWS2, bool CAP, bool TR, bool SC>
 int32_t launch_c(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, const MmaParams &mp, cudaStream_t st)
 {
     // Small grids (at most one CTA per SM): 8 warps x 3 stages where that fits in shared memory.
@@ -1488,32 +1563,32 @@ int32_t launch_c(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
     constexpr bool kOk2 = Shape<DT, D, 4, 2>::SMEM_BYTES <= kTwoPerSm && kMergeBytes <= Shape<DT, D, 4, 2>::RING_BYTES;
     constexpr bool kOk1 = Shape<DT, D, 4, 1>::SMEM_BYTES <= kTwoPerSm && kMergeBytes <= Shape<DT, D, 4, 1>::RING_BYTES;
     if (ns == 0) ns = (w == 8 || Shape<DT, D, 4, 3>::SMEM_BYTES <= kTwoPerSm) ? 3 : kOk2 ? 2 : kOk1 ? 1 : 3;
-    if (w == 8 && ns == 3) return launch_k<DT, D, ROWS2, 8, 3, CAP, TR>(ctx, tk, tv, mp, st);
-    if (w == 4 && ns == 3) return launch_k<DT, D, ROWS2, 4, 3, CAP, TR>(ctx, tk, tv, mp, st);
-    if (w == 4 && ns == 2) return launch_k<DT, D, ROWS2, 4, 2, CAP, TR>(ctx, tk, tv, mp, st);
-    if (w == 4 && ns == 1) return launch_k<DT, D, ROWS2, 4, 1, CAP, TR>(ctx, tk, tv, mp, st);
-    if (w == 8 && ns == 1) return launch_k<DT, D, ROWS2, 8, 1, CAP, TR>(ctx, tk, tv, mp, st);
+    if (w == 8 && ns == 3) return launch_k<DT, D, ROWS2, 8, 3, CAP, TR, SC>(ctx, tk, tv, mp, st);
+    if (w == 4 && ns == 3) return launch_k<DT, D, ROWS2, 4, 3, CAP, TR, SC>(ctx, tk, tv, mp, st);
+    if (w == 4 && ns == 2) return launch_k<DT, D, ROWS2, 4, 2, CAP, TR, SC>(ctx, tk, tv, mp, st);
+    if (w == 4 && ns == 1) return launch_k<DT, D, ROWS2, 4, 1, CAP, TR, SC>(ctx, tk, tv, mp, st);
+    if (w == 8 && ns == 1) return launch_k<DT, D, ROWS2, 8, 1, CAP, TR, SC>(ctx, tk, tv, mp, st);
     return set_error(ctx, VFKV_ERR_INVALID, "attention tuning must be 4x1, 4x2, 4x3, 8x1 or 8x3 (warps x stages)");
 }
 
-template <int DT, int D, bool ROWS2>
+template <int DT, int D, bool ROWS2, bool SC = false>
 int32_t launch_t(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, const MmaParams &mp, cudaStream_t st)
 {
     // groups of at most 4 q-heads: the transposed products (heads on the N side of the MMAs)
     if constexpr (!ROWS2) {
         if (mp.a.group <= 4u)
-            return mp.a.softcap > 0.f ? launch_c<DT, D, ROWS2, true, true>(ctx, tk, tv, mp, st)
-                                      : launch_c<DT, D, ROWS2, false, true>(ctx, tk, tv, mp, st);
+            return mp.a.softcap > 0.f ? launch_c<DT, D, ROWS2, true, true, SC>(ctx, tk, tv, mp, st)
+                                      : launch_c<DT, D, ROWS2, false, true, SC>(ctx, tk, tv, mp, st);
     }
-    return mp.a.softcap > 0.f ? launch_c<DT, D, ROWS2, true, false>(ctx, tk, tv, mp, st)
-                              : launch_c<DT, D, ROWS2, false, false>(ctx, tk, tv, mp, st);
+    return mp.a.softcap > 0.f ? launch_c<DT, D, ROWS2, true, false, SC>(ctx, tk, tv, mp, st)
+                              : launch_c<DT, D, ROWS2, false, false, SC>(ctx, tk, tv, mp, st);
 }
 
 }  // namespace
 
 bool attn_mma_supported(const AttnArgs &a)
 {
-    if (a.kv.k_scales || a.kv.v_scales) return false;
+    if ((a.kv.k_scales || a.kv.v_scales) && a.kv.dtype != VFKV_F8) return false;
     if (a.kv.n_kv_heads == 0 || a.n_q_heads % a.kv.n_kv_heads != 0) return false;
     const uint32_t g = a.n_q_heads / a.kv.n_kv_heads, D = a.kv.head_dim;
     if (uint64_t(a.kv.n_slots) * a.kv.max_seq >= (1ull << 31)) return false;
@@ -1587,6 +1662,10 @@ int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, ui
     const uint32_t g = a.n_q_heads / a.kv.n_kv_heads;
     auto run = [&]() -> int32_t {
         if (a.kv.dtype == VFKV_F8) {
+            if (a.kv.k_scales) {
+                if (D == 128) return launch_t<VFKV_F8, 128, false, true>(ctx, tk, tv, mp, st);
+                if (D == 256) return launch_t<VFKV_F8, 256, false, true>(ctx, tk, tv, mp, st);
+            }
             if (D == 128) return launch_t<VFKV_F8, 128, false>(ctx, tk, tv, mp, st);
             if (D == 256) return launch_t<VFKV_F8, 256, false>(ctx, tk, tv, mp, st);
         } else {

@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(256) store_vec_kernel(const float *__restrict_
 {
     constexpr int E = Enc<DT>::kElems;
     const uint64_t n_vec = n / E;
+    pdl_wait();
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n_vec;
          i += uint64_t(gridDim.x) * blockDim.x) {
         uint4 r = Enc<DT>::run(reinterpret_cast<const float4 *>(src + i * E));
@@ -68,6 +69,7 @@ __global__ void __launch_bounds__(256) store_word_kernel(const float *__restrict
                                                          uint64_t first, uint64_t n)
 {
     constexpr int W = DT == VFKV_F8 ? 4 : DT == VFKV_F16 ? 2 : 1;
+    pdl_wait();
     uint64_t w = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
     uint64_t e = first + w * W;
     if (e >= n) return;
@@ -95,15 +97,18 @@ static int32_t launch_store_t(vfkv_ctx *ctx, const float *src, void *dst, uint64
         uint64_t cap = uint64_t(ctx->sm_count) * 16;
         if (blocks > cap) blocks = cap;
         ProfScope ps(ctx, VFKV_PROF_KV_STORE, st);
-        store_vec_kernel<DT><<<unsigned(blocks), 256, 0, st>>>(src, static_cast<uint8_t *>(dst), n);
+        if (cudaError_t e = launch_dependent(ctx, store_vec_kernel<DT>, dim3(unsigned(blocks)), dim3(256), 0, st, src,
+                                             static_cast<uint8_t *>(dst), n))
+            return check_cuda(ctx, e, "store kernel launch");
         ctx->count_launch();
         done = n_vec * E;
     }
     if (done < n) {
         uint64_t words = (n - done + W - 1) / W;
         ProfScope ps(ctx, VFKV_PROF_KV_STORE, st);
-        store_word_kernel<DT><<<unsigned((words + 255) / 256), 256, 0, st>>>(
-            src, static_cast<uint32_t *>(dst), done, n);
+        if (cudaError_t e = launch_dependent(ctx, store_word_kernel<DT>, dim3(unsigned((words + 255) / 256)), dim3(256), 0, st, src,
+                                             static_cast<uint32_t *>(dst), done, n))
+            return check_cuda(ctx, e, "store kernel launch");
         ctx->count_launch();
     }
     ctx->set_written_any();
@@ -178,6 +183,7 @@ __global__ void __launch_bounds__(256) append_kernel(const AppendParams p, const
 {
     constexpr int E = Enc<DT>::kElems;
     const uint32_t which = blockIdx.y;
+    pdl_wait();
     const uint32_t chunks_per_row = p.row_elems / E;
     const uint64_t total = uint64_t(p.total_rows) * chunks_per_row;
     const uint64_t row_bytes = uint64_t(p.row_elems) * (DT == VFKV_F8 ? 1 : DT == VFKV_F16 ? 2 : 4);
@@ -200,6 +206,7 @@ __global__ void __launch_bounds__(256) append_kernel(const AppendParams p, const
 template <bool LAYERED>
 __global__ void __launch_bounds__(256) append_scaled_kernel(const AppendParams p, const __grid_constant__ AppendLayers<LAYERED> layers)
 {
+    pdl_wait();
     const uint32_t warps_per_block = blockDim.x / 32;
     const uint32_t which = blockIdx.y;
     const uint32_t lane = threadIdx.x & 31;
@@ -264,8 +271,9 @@ int32_t launch_append(vfkv_ctx *ctx, const AppendArgs &a, cudaStream_t st)
         if (blocks > cap) blocks = cap;
         {
             ProfScope ps(ctx, VFKV_PROF_KV_STORE, st);
-            if (layered) append_scaled_kernel<true><<<dim3(unsigned(blocks), 2), 256, 0, st>>>(p, layers);
-            else append_scaled_kernel<false><<<dim3(unsigned(blocks), 2), 256, 0, st>>>(p, none);
+            const cudaError_t e = layered ? launch_dependent(ctx, append_scaled_kernel<true>, dim3(unsigned(blocks), 2), dim3(256), 0, st, p, layers)
+                                          : launch_dependent(ctx, append_scaled_kernel<false>, dim3(unsigned(blocks), 2), dim3(256), 0, st, p, none);
+            if (e != cudaSuccess) return check_cuda(ctx, e, "append_scaled launch");
         }
         ctx->count_launch(a.n_layers);
         ctx->set_written(a.k_dst, written);
@@ -278,9 +286,10 @@ int32_t launch_append(vfkv_ctx *ctx, const AppendArgs &a, cudaStream_t st)
     if (blocks == 0) blocks = 1;
     dim3 grid(unsigned(blocks), 2);
     ProfScope ps(ctx, VFKV_PROF_KV_STORE, st);
+    cudaError_t le = cudaSuccess;
     auto launch = [&](auto plain, auto several) {
-        if (layered) several<<<grid, 256, 0, st>>>(p, layers);
-        else plain<<<grid, 256, 0, st>>>(p, none);
+        le = layered ? launch_dependent(ctx, several, grid, dim3(256), 0, st, p, layers)
+                     : launch_dependent(ctx, plain, grid, dim3(256), 0, st, p, none);
     };
     switch (a.dtype) {
     case VFKV_F8: launch(append_kernel<VFKV_F8, false>, append_kernel<VFKV_F8, true>); break;
@@ -290,17 +299,27 @@ int32_t launch_append(vfkv_ctx *ctx, const AppendArgs &a, cudaStream_t st)
     }
     ctx->count_launch(a.n_layers);
     ctx->set_written(a.k_dst, written);
-    return check_cuda(ctx, cudaGetLastError(), "append launch");
+    return check_cuda(ctx, le, "append launch");
 }
 
 // ---- E4M3 -> binary16 (vk_shaders/kv_fp8_to_f16.comp:28-34) ----------------
+// HBM-bound: 3 bytes an element.  A thread has four 16-byte loads in flight, and stores 32 bytes, a
+// whole sector, at a time (two 16-byte stores 32 bytes apart write every sector twice by halves).
+constexpr int kCvtUnroll = 4;
 __global__ void __launch_bounds__(256) fp8_to_f16_vec_kernel(const uint4 *__restrict__ src,
-                                                             uint4 *__restrict__ dst, uint64_t n_vec)
+                                                             uint4 *__restrict__ dst, uint64_t n_vec, bool wide)
 {
-    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n_vec;
-         i += uint64_t(gridDim.x) * blockDim.x) {
-        uint4 s = src[i];
-        uint32_t w[4] = {s.x, s.y, s.z, s.w};
+    pdl_wait();
+    const uint64_t first = blockIdx.x * uint64_t(256 * kCvtUnroll) + threadIdx.x;
+    uint4 s[kCvtUnroll];
+#pragma unroll
+    for (int k = 0; k < kCvtUnroll; ++k)
+        if (first + k * 256 < n_vec) s[k] = src[first + k * 256];
+#pragma unroll
+    for (int k = 0; k < kCvtUnroll; ++k) {
+        const uint64_t i = first + k * 256;
+        if (i >= n_vec) break;
+        const uint32_t w[4] = {s[k].x, s[k].y, s[k].z, s[k].w};
         uint32_t o[8];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -308,8 +327,13 @@ __global__ void __launch_bounds__(256) fp8_to_f16_vec_kernel(const uint4 *__rest
             o[2 * j] = *reinterpret_cast<uint32_t *>(&lo);
             o[2 * j + 1] = *reinterpret_cast<uint32_t *>(&hi);
         }
-        dst[2 * i] = make_uint4(o[0], o[1], o[2], o[3]);
-        dst[2 * i + 1] = make_uint4(o[4], o[5], o[6], o[7]);
+        if (wide) {
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + 2 * i), "r"(o[0]), "r"(o[1]), "r"(o[2]),
+                         "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
+        } else {
+            dst[2 * i] = make_uint4(o[0], o[1], o[2], o[3]);
+            dst[2 * i + 1] = make_uint4(o[4], o[5], o[6], o[7]);
+        }
     }
 }
 
@@ -317,6 +341,7 @@ __global__ void __launch_bounds__(256) fp8_to_f16_scalar_kernel(const uint8_t *_
                                                                 __half *__restrict__ dst,
                                                                 uint64_t first, uint64_t n)
 {
+    pdl_wait();
     uint64_t i = first + blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
     if (i >= n) return;
     dst[i] = __low2half(e4m3x2_to_half2(src[i]));
@@ -329,19 +354,21 @@ int32_t launch_fp8_to_f16(vfkv_ctx *ctx, const void *src, void *dst, uint64_t n,
                          (reinterpret_cast<uintptr_t>(dst) % 16 == 0);
     uint64_t done = 0;
     if (aligned && n >= 16) {
-        uint64_t n_vec = n / 16, blocks = (n_vec + 255) / 256, cap = uint64_t(ctx->sm_count) * 16;
-        if (blocks > cap) blocks = cap;
+        const uint64_t n_vec = n / 16, per = 256 * kCvtUnroll;
         ProfScope ps(ctx, VFKV_PROF_FP8_TO_F16, st);
-        fp8_to_f16_vec_kernel<<<unsigned(blocks), 256, 0, st>>>(
-            static_cast<const uint4 *>(src), static_cast<uint4 *>(dst), n_vec);
+        const bool wide = reinterpret_cast<uintptr_t>(dst) % 32 == 0;
+        if (cudaError_t e = launch_dependent(ctx, fp8_to_f16_vec_kernel, dim3(unsigned((n_vec + per - 1) / per)), dim3(256), 0, st,
+                                             static_cast<const uint4 *>(src), static_cast<uint4 *>(dst), n_vec, wide))
+            return check_cuda(ctx, e, "fp8_to_f16 launch");
         ctx->count_launch();
         done = n_vec * 16;
     }
     if (done < n) {
         uint64_t rem = n - done;
         ProfScope ps(ctx, VFKV_PROF_FP8_TO_F16, st);
-        fp8_to_f16_scalar_kernel<<<unsigned((rem + 255) / 256), 256, 0, st>>>(
-            static_cast<const uint8_t *>(src), static_cast<__half *>(dst), done, n);
+        if (cudaError_t e = launch_dependent(ctx, fp8_to_f16_scalar_kernel, dim3(unsigned((rem + 255) / 256)), dim3(256), 0, st,
+                                             static_cast<const uint8_t *>(src), static_cast<__half *>(dst), done, n))
+            return check_cuda(ctx, e, "fp8_to_f16 launch");
         ctx->count_launch();
     }
     return check_cuda(ctx, cudaGetLastError(), "fp8_to_f16 launch");

@@ -87,6 +87,7 @@ attn_split_generic_kernel(const AttnParams p)
     const uint32_t h0 = kvh * p.group + hb * GB;
     const uint32_t nh = min(uint32_t(GB), p.group - hb * GB);
 
+    pdl_wait();
     uint32_t slot, start, len, begin, end;
     seq_range(p, unit, &slot, &start, &len);
     split_range(start, len, p.n_splits, split, 32, &begin, &end);
@@ -234,7 +235,8 @@ static int32_t launch_one(vfkv_ctx *ctx, const AttnParams &p, cudaStream_t st)
     }
     {
         ProfScope ps(ctx, VFKV_PROF_FA_SPLIT, st);
-        kern<<<grid, kGenericWarps * 32, smem, st>>>(p);
+        if (cudaError_t e = launch_dependent(ctx, kern, grid, dim3(kGenericWarps * 32), smem, st, p))
+            return check_cuda(ctx, e, "generic attention launch");
     }
     ctx->count_launch(p.n_layers);
     return check_cuda(ctx, cudaGetLastError(), "generic attention launch");

@@ -25,6 +25,7 @@ merge_kernel(const float *__restrict__ pm, const float *__restrict__ pl, const f
         const uint32_t i = blockIdx.x / lr.per_layer;
         orow = uint64_t(lr.layer_ids[i]) * lr.per_layer + (blockIdx.x - i * lr.per_layer);
     }
+    pdl_wait();
     constexpr int kMaxDims = 4;                      // 128 threads x 4 = head_dim 512
     __shared__ float s_red[4], s_sum[4];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -95,10 +96,11 @@ int32_t launch_merge_ws(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, ui
     }
     ProfScope ps(ctx, VFKV_PROF_FA_REDUCE, st);
     const uint64_t D = a.kv.head_dim;
-    merge_kernel<<<rows, 128, 0, st>>>(ws->part_m, ws->part_l, ws->part_o, n_splits, 1, n_splits, D, n_splits * D,
-                                      a.kv.head_dim, a.out, a.out_m, a.out_l, a.out_o, lr);
+    const cudaError_t e = launch_dependent(ctx, merge_kernel, dim3(rows), dim3(128), 0, st, ws->part_m, ws->part_l, ws->part_o,
+                                           n_splits, uint64_t(1), uint64_t(n_splits), D, n_splits * D, a.kv.head_dim, a.out,
+                                           a.out_m, a.out_l, a.out_o, lr);
     ctx->count_launch(a.seq.n_layers);
-    return check_cuda(ctx, cudaGetLastError(), "merge launch");
+    return check_cuda(ctx, e, "merge launch");
 }
 
 int32_t launch_merge_partials(vfkv_ctx *ctx, const float *m, const float *l, const float *o,

@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(128) prefill_mma_kernel(const PrefillParams p)
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
     const uint32_t kvh = blockIdx.y, g = p.group;
     const uint32_t n_rows = p.m * g;
+    pdl_wait();
     // heaviest row blocks (latest queries) first
     const uint32_t rb = gridDim.x - 1u - blockIdx.x;
     const uint32_t row0 = rb * BM;
@@ -440,9 +441,9 @@ int32_t launch_mma_t(vfkv_ctx *ctx, const PrefillParams &p, cudaStream_t st)
         configured[ctx->device & 63] = true;
     }
     const uint32_t row_blocks = (p.m * p.group + BM - 1) / BM;
-    kern<<<dim3(row_blocks, p.n_kv_heads), 128, kSmem, st>>>(p);
+    const cudaError_t e = launch_dependent(ctx, kern, dim3(row_blocks, p.n_kv_heads), dim3(128), kSmem, st, p);
     ctx->count_launch();
-    return check_cuda(ctx, cudaGetLastError(), "prefill attention launch");
+    return check_cuda(ctx, e, "prefill attention launch");
 }
 
 template <int DT, int D>

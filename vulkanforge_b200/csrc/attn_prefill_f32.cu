@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
         t_begin = first + uint32_t(uint64_t(n) * split / n_splits);
         t_end = first + uint32_t(uint64_t(n) * (split + 1) / n_splits);
     }
+    pdl_wait();
     // Q rows, scaled into the log2 domain (with a soft-cap the factor is applied after it)
     const float q_mult = p.scale * (p.softcap > 0.f ? 1.0f : kLog2e);
     for (uint32_t i = threadIdx.x; i < uint32_t(BM * D / 4); i += kThreads) {
@@ -390,11 +391,18 @@ int32_t launch_t(vfkv_ctx *ctx, const PrefillParams &p, cudaStream_t st)
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = S::SMEM;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = n_splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    unsigned n_attr = 0;
+    if (ctx->pdl) {
+        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n_attr++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (n_splits > 1) {
+        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+        attr[n_attr].val.clusterDim.x = n_splits; attr[n_attr].val.clusterDim.y = 1; attr[n_attr++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = n_splits > 1 ? 1 : 0;
+    cfg.numAttrs = n_attr;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
     ctx->count_launch();
     return check_cuda(ctx, e == cudaSuccess ? cudaGetLastError() : e, "f32 prefill attention launch");

@@ -955,6 +955,7 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
         }
         __syncthreads();
     }
+    pdl_wait();
     // K/V tiles this CTA has been through: every barrier completes once per tile (K/V ready and
     // free: once per two), so all phase parities follow from this count, across segments
     uint32_t gt = 0u;
@@ -1719,7 +1720,8 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
             (void)cudaGetLastError();          // not all resident: the pieces go to the merge kernel instead
             p.inline_merge = 0u;
         }
-        kern<<<grid_h, 384, kSmemBytes, st>>>(p, tm_k, tm_v);
+        if (cudaError_t le = launch_dependent(ctx, kern, grid_h, dim3(384), kSmemBytes, st, p, tm_k, tm_v))
+            return check_cuda(ctx, le, "tcgen05 prefill attention launch");
         ctx->count_launch();
         if (spread) {
             // launched as a programmatic dependent: it is resident, its table built, when the last CTA

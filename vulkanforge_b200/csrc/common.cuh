@@ -22,7 +22,7 @@ struct vfkv_ctx {
     float *d_prefill_scratch = nullptr;         // pieces of prefill items cut between CTAs; allocated at first use
     uint32_t prefill_scratch_ctas = 0;
     uint32_t prefill_epoch = 0;                 // value the flags of the current spread prefill launch take
-    uint32_t pdl = 0;                  // programmatic dependent launch mode of the attention kernel (0 / 1 / 2)
+    uint32_t pdl = 0;                  // programmatic dependent launch mode (0 / 1 / 2)
     // K addresses that the last launch on this context wrote cache rows into, or an empty range: a
     // mode-2 launch that reads any of them next waits before its K/V prefetch (mode 1).
     uintptr_t written_lo = 0, written_hi = 0;
@@ -212,6 +212,34 @@ struct ProfScope {
     }
     ~ProfScope() { if (e1) cudaEventRecord(e1, st); }
 };
+
+// Launch of a kernel that begins with pdl_wait(): with dependent launch on (vfkv_ctx_set_dependent_launch)
+// it may be scheduled while its predecessor drains, which hides most of a launch's latency.
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(const vfkv_ctx *ctx, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t st, A &&...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctx->pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
+#ifdef __CUDACC__
+// Waits for everything in front of this kernel on its stream, then lets the next kernel be scheduled.
+// Nothing that the predecessor may have written, and nothing that it may still read, is touched before.
+// (The release comes after the wait, so a kernel that reads ahead of its own wait only ever overlaps
+// its direct predecessor.)  Both do nothing in a launch without the attribute.
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
 
 // Launchers (each returns a vfkv_status).
 int32_t launch_store(vfkv_ctx *ctx, uint32_t dtype, const float *src, void *dst, uint64_t n,

@@ -162,3 +162,14 @@ def load() -> C.CDLL:
         fn.restype, fn.argtypes = res, args
     _lib = lib
     return lib
+
+
+def native():
+    """The compiled bindings of the per-layer calls (csrc/py_calls.cpp); raises if they are not built."""
+    load()
+    try:
+        from . import _native
+    except ImportError as e:
+        raise RuntimeError(f"the compiled bindings beside {LIB_PATH} cannot be loaded ({e}): build them with "
+                           "`python -m vulkanforge_b200.build`") from e
+    return _native

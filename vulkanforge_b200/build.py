@@ -10,10 +10,12 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libvfkv.so")
+CALLS = os.path.join(HERE, "_native.so")        # Python bindings of the per-layer calls (csrc/py_calls.cpp), linked to OUT
 SOURCES = ["api.cu", "append.cu", "attn_generic.cu", "attn_mma.cu", "attn_merge.cu", "exchange.cu", "attn_prefill.cu", "attn_prefill_f32.cu", "attn_prefill_tc5.cu", "rope_append.cu", "routes.cpp", "noalloc.cu", "kv_cache.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -26,9 +28,9 @@ def _nvcc() -> str:
 
 
 def _stale() -> bool:
-    if not os.path.exists(OUT):
+    if not (os.path.exists(OUT) and os.path.exists(CALLS)):
         return True
-    t = os.path.getmtime(OUT)
+    t = min(os.path.getmtime(OUT), os.path.getmtime(CALLS))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
     deps.append(os.path.join(HERE, "..", "include", "vfkv.h"))
     deps.append(os.path.join(HERE, "..", "include", "vfkv_next.h"))
@@ -61,7 +63,14 @@ def build(force: bool = False, verbose: bool = False) -> str:
         raise RuntimeError("nvcc failed; see messages above")
     link = [_nvcc(), "-shared", "-o", OUT] + objs + ARCH + ["-ccbin", "/usr/bin/g++"]
     subprocess.run(link, check=True)
+    build_calls()
     return OUT
+
+
+def build_calls() -> str:
+    subprocess.run(["/usr/bin/g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"],
+                    os.path.join(CSRC, "py_calls.cpp"), "-o", CALLS, OUT, "-Wl,-rpath,$ORIGIN"], check=True)
+    return CALLS
 
 
 if __name__ == "__main__":

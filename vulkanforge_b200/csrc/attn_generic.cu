@@ -16,6 +16,7 @@
 //   - the partial count is a parameter instead of ceil(seq_len / 64).
 #include "attn_params.cuh"
 #include "fp8_codec.cuh"
+#include "softcap.cuh"
 
 namespace vfkv {
 
@@ -107,6 +108,7 @@ attn_split_generic_kernel(const AttnParams p)
     const float *ksc = p.k_scales ? p.k_scales + uint64_t(slot) * p.slot_stride_scales + kvh : nullptr;
     const float *vsc = p.v_scales ? p.v_scales + uint64_t(slot) * p.slot_stride_scales + kvh : nullptr;
 
+    const float inv_cap = p.softcap > 0.f ? 1.0f / p.softcap : 0.f;
     float m[GB], l[GB], acc[GB][VEC];
 #pragma unroll
     for (int j = 0; j < GB; ++j) {
@@ -154,7 +156,8 @@ attn_split_generic_kernel(const AttnParams p)
             const bool valid = (t0 + u) < end;
 #pragma unroll
             for (int j = 0; j < GB; ++j) {
-                float x = apply_softcap(sc[u][j] * kscale[u] * p.scale, p.softcap);
+                float x = sc[u][j] * kscale[u] * p.scale;
+                if (p.softcap > 0.f) x = softcap_any(x, p.softcap, inv_cap);
                 x = valid ? x : kMaskedScore;
                 sc[u][j] = x;
                 mnew[j] = fmaxf(mnew[j], x);

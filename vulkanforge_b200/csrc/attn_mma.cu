@@ -41,6 +41,7 @@
 
 #include "attn_params.cuh"
 #include "fp8_codec.cuh"
+#include "softcap.cuh"
 
 namespace vfkv {
 
@@ -724,6 +725,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     float m[RS], l[RS];
 #pragma unroll
     for (int r = 0; r < RS; ++r) { m[r] = kMaskedScore; l[r] = 0.f; }
+    const float inv_cap = CAP ? 1.0f / p.softcap : 0.f;
     constexpr int NACC = TR ? NQB : NDB;
     float acc[NACC][4];
 #pragma unroll
@@ -842,7 +844,14 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             for (int i = 0; i < 2; ++i) {
                 float v = (sc[mb][2 * i] + sc[mb][2 * i + 1]) * mult[0];
                 if constexpr (SC) v *= __shfl_sync(0xffffffffu, ks_cur, 16 * mb + 8 * i + gid);
-                if constexpr (CAP) v = p.softcap * tanhf(v / p.softcap) * kLog2e;
+                x[mb][i] = v;
+            }
+        if constexpr (CAP) softcap_all(reinterpret_cast<float (&)[2 * MB]>(x), p.softcap, inv_cap);
+#pragma unroll
+        for (int mb = 0; mb < MB; ++mb)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                float v = CAP ? x[mb][i] * kLog2e : x[mb][i];
                 if (!full) v = uint32_t(16 * mb + 8 * i) + gid < n_valid ? v : kMaskedScore;
                 x[mb][i] = v;
                 tmax = fmaxf(tmax, v);
@@ -906,13 +915,17 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                     if constexpr (CAP) {
                         v *= mult[r];
                         if constexpr (SC) v *= __shfl_sync(0xffffffffu, ks_cur, 8 * j + 2 * tig + i);
-                        v = p.softcap * tanhf(v / p.softcap) * kLog2e;
                     } else {
                         v *= mult[r];                      // scale * log2(e) / q_scale
                         if constexpr (SC) v *= __shfl_sync(0xffffffffu, ks_cur, 8 * j + 2 * tig + i);
                     }
                     x[r][j][i] = v;
                 }
+            if constexpr (CAP) {
+                softcap_all(reinterpret_cast<float (&)[2 * NB]>(x[r]), p.softcap, inv_cap);
+#pragma unroll
+                for (int j = 0; j < NB; ++j) { x[r][j][0] *= kLog2e; x[r][j][1] *= kLog2e; }
+            }
             if (!full) {                                   // a split's last tile: mask the tail
 #pragma unroll
                 for (int j = 0; j < NB; ++j)

@@ -177,12 +177,6 @@ __device__ __forceinline__ bool tags_are(ulonglong2 w, uint32_t tag)
 }
 __device__ __forceinline__ float tagged_value(uint64_t w) { return __uint_as_float(uint32_t(w)); }
 
-__device__ __forceinline__ float apply_softcap(float s, float cap)
-{
-    // extension: cap * tanh(s / cap), the formula the reference applies to final
-    // logits (src/backend/vulkan/forward/arch/gemma4.rs:85-94)
-    return cap > 0.f ? cap * tanhf(s / cap) : s;
-}
 #endif
 
 }  // namespace vfkv

@@ -14,6 +14,7 @@
 #include "../../include/vfkv_next.h"
 #include "fp8_codec.cuh"
 #include "prefill_params.cuh"
+#include "softcap.cuh"
 
 namespace vfkv {
 namespace {
@@ -275,6 +276,7 @@ __global__ void __launch_bounds__(128) prefill_mma_kernel(const PrefillParams p)
         const uint32_t c_max_lo = __reduce_max_sync(0xffffffffu, max(r_lo[0], r_lo[1]));
         const bool all_ok = __all_sync(0xffffffffu, r_ok[0] && r_ok[1]);
         const bool full = all_ok && t0 + BN <= c_min_hi && t0 >= c_max_lo;   // no masking needed in this tile
+        if constexpr (CAP) softcap_all(reinterpret_cast<float (&)[NB * 4]>(sc), p.softcap, 1.0f / p.softcap);
         float alpha[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -284,7 +286,6 @@ __global__ void __launch_bounds__(128) prefill_mma_kernel(const PrefillParams p)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     float s = sc[nb][2 * h + e];
-                    if constexpr (CAP) s = p.softcap * tanhf(s / p.softcap);
                     s *= kLog2e;
                     if (!full) {
                         const uint32_t pos = t0 + 8 * nb + 2 * tig + e;
@@ -395,7 +396,7 @@ __global__ void __launch_bounds__(128) prefill_simple_kernel(const PrefillParams
         for (int x = 16; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
         if (p.k_scales) s *= p.k_scales[uint64_t(pos) * p.n_kv_heads + kvh];
         s *= p.scale;
-        if (p.softcap > 0.f) s = p.softcap * tanhf(s / p.softcap);
+        if (p.softcap > 0.f) s = softcap_any(s, p.softcap, 1.0f / p.softcap);
         const float mn = fmaxf(m, s);
         const float ko = __expf(m - mn), pn = __expf(s - mn);
         const float vs = p.v_scales ? p.v_scales[uint64_t(pos) * p.n_kv_heads + kvh] : 1.0f;

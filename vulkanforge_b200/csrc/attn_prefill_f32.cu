@@ -16,6 +16,7 @@
 // distributed shared memory: no scratch, no second launch.
 #include "fp8_codec.cuh"
 #include "prefill_params.cuh"
+#include "softcap.cuh"
 
 #include <atomic>
 
@@ -216,10 +217,14 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 float mx = kMaskedScore;
+                if (p.softcap > 0.f) {
+                    softcap_all(s[h], p.softcap, 1.0f / p.softcap);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) s[h][j] *= kLog2e;
+                }
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     float x = s[h][j];
-                    if (p.softcap > 0.f) x = p.softcap * tanhf(x / p.softcap) * kLog2e;
                     const uint32_t pos = t0 + cl + 8 * j;
                     if (!full && (pos < r_lo[h] || pos >= r_hi[h])) x = kMaskedScore;
                     s[h][j] = x;

@@ -22,6 +22,7 @@
 #include "../../include/vfkv_next.h"
 #include "common.cuh"
 #include "fp8_codec.cuh"
+#include "softcap.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -279,6 +280,7 @@ __global__ void __launch_bounds__(256) prefill_tc5_kernel(const Tc5Params p)
     // Q: f32 -> scaled half precision, two K-major swizzled tiles.  Without a soft-cap the factor
     // log2(e) of the exponentials is folded into the scale, so S arrives in log2 units.
     const float qs = CAP ? p.scale : p.scale * kLog2e;
+    const float inv_cap = CAP ? 1.0f / p.softcap : 0.f;
     for (uint32_t i = tid; i < uint32_t(CTA_ROWS * 16); i += 256) {
         const uint32_t row = i >> 4, c = i & 15u;
         const uint32_t rr = row0 + row;
@@ -425,6 +427,7 @@ __global__ void __launch_bounds__(256) prefill_tc5_kernel(const Tc5Params p)
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         // tiles inside every row's range (all but the diagonal and window edges) need no mask
         const bool warp_full = __all_sync(0xffffffffu, full);
+        if constexpr (CAP) softcap_all(s, p.softcap, inv_cap);
         float mx = kMaskedScore;
         if (warp_full && !CAP) {
 #pragma unroll
@@ -433,7 +436,7 @@ __global__ void __launch_bounds__(256) prefill_tc5_kernel(const Tc5Params p)
 #pragma unroll
             for (int j = 0; j < BN; ++j) {
                 float x = s[j];
-                if constexpr (CAP) x = p.softcap * tanhf(x / p.softcap) * kLog2e;
+                if constexpr (CAP) x *= kLog2e;
                 if (!full) {
                     const uint32_t pos = t0 + j;
                     if (pos < r_lo || pos >= r_hi) x = kMaskedScore;
@@ -618,6 +621,7 @@ __global__ void __launch_bounds__(256, 1) prefill_tc5p_kernel(const Tc5Params p)
     const uint32_t n_tiles = c_hi > c_lo ? (c_hi - c_lo + BN - 1) / BN : 0u;
 
     const float qs = CAP ? p.scale : p.scale * kLog2e;
+    const float inv_cap = CAP ? 1.0f / p.softcap : 0.f;
     for (uint32_t i = tid; i < uint32_t(CTA_ROWS * 16); i += 256) {
         const uint32_t row = i >> 4, c = i & 15u;
         const uint32_t rr = row0 + row;
@@ -732,6 +736,7 @@ __global__ void __launch_bounds__(256, 1) prefill_tc5p_kernel(const Tc5Params p)
         for (int c = 0; c < 4; ++c) tmem_ld32_nowait(tm_s + t_lane + 32 * c, &s[32 * c]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         const bool warp_full = __all_sync(0xffffffffu, full);
+        if constexpr (CAP) softcap_all(s, p.softcap, inv_cap);
         float mx = kMaskedScore;
         if (warp_full && !CAP) {
 #pragma unroll
@@ -740,7 +745,7 @@ __global__ void __launch_bounds__(256, 1) prefill_tc5p_kernel(const Tc5Params p)
 #pragma unroll
             for (int j = 0; j < BN; ++j) {
                 float x = s[j];
-                if constexpr (CAP) x = p.softcap * tanhf(x / p.softcap) * kLog2e;
+                if constexpr (CAP) x *= kLog2e;
                 if (!full) {
                     const uint32_t pos = t0 + j;
                     if (pos < r_lo || pos >= r_hi) x = kMaskedScore;
@@ -937,6 +942,7 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     const float qs = CAP ? p.scale : p.scale * kLog2e;
+    const float inv_cap = CAP ? 1.0f / p.softcap : 0.f;
     volatile uint32_t *abort_flag = &s_abort;
     uint32_t cur = 0u, t_end = 0u;                       // this CTA's tiles on the line of all tiles
     if (p.n_cta != 0u) {
@@ -1066,15 +1072,19 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
                     tmem_ld64(tm_s + t_lane + 64u * h, s);
                     const bool full = t0 >= r_lo && t0 + 64u <= r_hi;
                     const bool warp_full = __all_sync(0xffffffffu, full);
+                    if constexpr (CAP) softcap_all(s, p.softcap, inv_cap);
                     float mx = kMaskedScore;
                     if (warp_full && !CAP) {
 #pragma unroll
                         for (int j = 0; j < 64; j += 2) mx = fmaxf(mx, fmaxf(s[j], s[j + 1]));
+                    } else if (warp_full) {
+#pragma unroll
+                        for (int j = 0; j < 64; ++j) { s[j] *= kLog2e; mx = fmaxf(mx, s[j]); }
                     } else {
 #pragma unroll
                         for (int j = 0; j < 64; ++j) {
                             float x = s[j];
-                            if constexpr (CAP) x = p.softcap * tanhf(x / p.softcap) * kLog2e;
+                            if constexpr (CAP) x *= kLog2e;
                             if (!full) {
                                 const uint32_t pos = t0 + j;
                                 if (pos < r_lo || pos >= r_hi) x = kMaskedScore;

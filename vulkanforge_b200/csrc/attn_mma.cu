@@ -183,6 +183,7 @@ struct MmaParams {
     uint32_t fail_split;          // test hook: this split of (sequence 0, kv-head 0) acts as if a TMA wait ran out
     uint32_t per_recip;           // ceil(2^32 / output pairs per merging CTA): idx / per == umulhi(idx, per_recip) for idx < 65536
     uint64_t tag_words;           // host side only: size of tag_part in words
+    uint32_t longest;             // host side only: positions of the longest sequence, as far as the caller says
 };
 
 // Phase timestamps for latency analysis; costs one predicated branch when tracing is off.
@@ -1562,7 +1563,10 @@ int32_t launch_c(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
 {
     // Small grids (at most one CTA per SM): 8 warps x 3 stages where that fits in shared memory.
     // Everything else: 4 warps x 3 stages, two CTAs per SM at 8 KB stages (measured faster than
-    // three CTAs of 4 x 2, whose 168-register cap costs more than the extra warps give).
+    // three CTAs of 4 x 2, whose 168-register cap costs more than the extra warps give), except where a
+    // warp has at most eight tiles: there a CTA is mostly latencies, and the third one an SM hides them
+    // (16 layers x 29 sequences of 133 positions, F16: 87 -> 70 us; 16 x 16 of 600, FP8: 71 -> 61;
+    // 16 x 8 of 2000: 88 either way).
     constexpr bool kWide = Shape<DT, D, 8, 3>::SMEM_BYTES <= 200 * 1024;
     const uint64_t ctas = uint64_t(mp.a.n_splits) * mp.a.n_kv_heads * mp.a.n_seqs * mp.a.n_layers;
     uint32_t w = ctx->tune_warps, ns = ctx->tune_stages;
@@ -1575,6 +1579,9 @@ int32_t launch_c(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
     constexpr int kMergeBytes = (4 * kNH * (D + 1) + 2 * 4 * kNH) * 4;       // cross-warp merge scratch, 4 warps
     constexpr bool kOk2 = Shape<DT, D, 4, 2>::SMEM_BYTES <= kTwoPerSm && kMergeBytes <= Shape<DT, D, 4, 2>::RING_BYTES;
     constexpr bool kOk1 = Shape<DT, D, 4, 1>::SMEM_BYTES <= kTwoPerSm && kMergeBytes <= Shape<DT, D, 4, 1>::RING_BYTES;
+    const uint32_t longest = mp.a.window && mp.a.window < mp.longest ? mp.a.window : mp.longest;
+    const bool few_tiles = (longest + mp.a.n_splits - 1) / mp.a.n_splits <= 8u * 4u * uint32_t(Shape<DT, D, 4, 2>::TP);
+    if (ns == 0 && w == 4 && kOk2 && Shape<DT, D, 4, 2>::STAGE_BYTES <= 8192 && few_tiles && ctas > uint64_t(ctx->sm_count) * 2) ns = 2;
     if (ns == 0) ns = (w == 8 || Shape<DT, D, 4, 3>::SMEM_BYTES <= kTwoPerSm) ? 3 : kOk2 ? 2 : kOk1 ? 1 : 3;
     if (w == 8 && ns == 3) return launch_k<DT, D, ROWS2, 8, 3, CAP, TR, SC>(ctx, tk, tv, mp, st);
     if (w == 4 && ns == 3) return launch_k<DT, D, ROWS2, 4, 3, CAP, TR, SC>(ctx, tk, tv, mp, st);
@@ -1637,6 +1644,8 @@ int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, ui
     mp.tickets = ws ? ws->tickets : nullptr;
     mp.tag_part = ws ? ws->tag_part : nullptr;
     mp.tag_words = ws ? ws->tag_words : 0;
+    mp.longest = !a.seq.seq_lens && !a.seq.positions ? a.seq.seq_len_scalar - a.seq.kv_start_scalar
+                                                     : a.seq.max_len_hint ? a.seq.max_len_hint : a.kv.max_seq;
     mp.merge_wait_ns = ctx->merge_wait_ns;
     mp.launch_seq = (ws && n_splits > 1) ? ws->launch_seq++ : 0u;
     // Several CTAs per (sequence, kv-head) share the merge -- four, or up to sixteen when a few

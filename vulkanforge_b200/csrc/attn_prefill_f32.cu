@@ -391,26 +391,9 @@ int32_t launch_t(vfkv_ctx *ctx, const PrefillParams &p, cudaStream_t st)
     const uint32_t tiles = (visible + BN - 1) / BN;
     uint32_t n_splits = 1;
     while (n_splits < 8 && blocks * n_splits * 2 <= slots + slots / 4 && tiles >= n_splits * 4) n_splits *= 2;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(n_splits, row_blocks, p.n_kv_heads);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = S::SMEM;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    unsigned n_attr = 0;
-    if (ctx->pdl) {
-        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n_attr++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    if (n_splits > 1) {
-        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-        attr[n_attr].val.clusterDim.x = n_splits; attr[n_attr].val.clusterDim.y = 1; attr[n_attr++].val.clusterDim.z = 1;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = n_attr;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
+    const cudaError_t e = launch_clusters(ctx, kern, dim3(n_splits, row_blocks, p.n_kv_heads), dim3(kThreads), S::SMEM, st, n_splits, p);
     ctx->count_launch();
-    return check_cuda(ctx, e == cudaSuccess ? cudaGetLastError() : e, "f32 prefill attention launch");
+    return check_cuda(ctx, e, "f32 prefill attention launch");
 }
 
 template <int DT>

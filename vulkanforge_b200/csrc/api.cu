@@ -529,11 +529,13 @@ int32_t vfkv_workspace_destroy(vfkv_workspace *ws)
     DeviceGuard g(ws->ctx->device);
     cudaFree(ws->block);
     cudaFree(ws->stage_in); cudaFree(ws->stage_out);
-    for (auto gexec : ws->tok_graphs)
-        if (gexec) cudaGraphExecDestroy(gexec);
+    for (auto &tg : ws->tok)
+        if (tg.exec) cudaGraphExecDestroy(tg.exec);
+    cudaFreeHost(ws->tok_u32);
     for (auto ev : ws->tok_events)
         if (ev) cudaEventDestroy(ev);
-    if (ws->copy_stream) cudaStreamDestroy(ws->copy_stream);
+    if (ws->tok_in) cudaStreamDestroy(ws->tok_in);
+    if (ws->tok_out) cudaStreamDestroy(ws->tok_out);
     for (auto &hs : ws->host_slot) {
         cudaFree(hs.in); cudaFree(hs.out); cudaFree(hs.u32);
         if (hs.graph) cudaGraphExecDestroy(hs.graph);
@@ -877,120 +879,155 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
     }
     float *dq = ws->stage_in, *dk = dq + q_elems, *dv = dk + kv_elems;
     uint32_t *d_pos = ws->d_u32, *d_slots = ws->d_u32 + ws->max_seqs;
-    cudaError_t e = cudaMemcpyAsync(d_pos, h_positions, n_seqs * 4, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && h_slot_ids) e = cudaMemcpyAsync(d_slots, h_slot_ids, n_seqs * 4, cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return check_cuda(ctx, e, "vfkv_decode_token_host: H2D");
     const uint64_t q_stride = uint64_t(n_seqs) * n_q_heads * D, kv_stride = uint64_t(n_seqs) * Hkv * D;
-    // The launches of one token depend on the host only through the configuration below
-    // (positions and slots are device-side inputs; the length hint is rounded up so that it
-    // changes rarely): capture them once, replay afterwards.
+    auto run_layers = [&](uint32_t l0, uint32_t l1, uint32_t len_hint) -> int32_t {
+        return decode_layers(cache, ws, l0, l1, dq, dk, dv, ws->stage_out, n_q_heads, h_slot_ids ? d_slots : nullptr,
+                             d_pos, n_seqs, len_hint, windows, scale, softcap, n_splits, stream);
+    };
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(st, &cap);
+    bool pipelined = cap == cudaStreamCaptureStatusNone && !ctx->profiling && !ctx->d_trace && st != nullptr;
+    cudaError_t e = cudaSuccess;
+    if (pipelined && !ws->tok_out) {
+        bool ok = cudaHostAlloc(reinterpret_cast<void **>(&ws->tok_u32), uint64_t(ws->max_seqs) * 2 * 4, cudaHostAllocDefault) == cudaSuccess &&
+                  cudaStreamCreateWithFlags(&ws->tok_in, cudaStreamNonBlocking) == cudaSuccess;
+        for (uint32_t i = 0; ok && i < 2 * vfkv_workspace::kTokChunks + 2; ++i)
+            ok = cudaEventCreateWithFlags(&ws->tok_events[i], cudaEventDisableTiming) == cudaSuccess;
+        ok = ok && cudaStreamCreateWithFlags(&ws->tok_out, cudaStreamNonBlocking) == cudaSuccess;
+        if (!ok) {
+            cudaGetLastError();
+            return set_error(ctx, VFKV_ERR_CUDA, "vfkv_decode_token_host: streams and events");
+        }
+    }
+    if (!pipelined) {      // stream order only: on the default stream, inside a capture, under the profiler or the phase trace
+        e = cudaMemcpyAsync(d_pos, h_positions, n_seqs * 4, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess && h_slot_ids) e = cudaMemcpyAsync(d_slots, h_slot_ids, n_seqs * 4, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dq, h_q, q_elems * 4, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dk, h_k, kv_elems * 4, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dv, h_v, kv_elems * 4, cudaMemcpyHostToDevice, st);
+        if (e != cudaSuccess) return check_cuda(ctx, e, "vfkv_decode_token_host: H2D");
+        if (int32_t rc = run_layers(0, L, max_pos + 1)) return rc;
+        e = cudaMemcpyAsync(h_out, ws->stage_out, out_bytes, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        return check_cuda(ctx, e, "vfkv_decode_token_host: D2H");
+    }
+    // Groups of about 300 KB of inputs, eight at most: a group has to be worth its copies and its launch
+    // (36 layers of one sequence, 0.88 MB: three groups), and only the first group's inputs and the last
+    // one's outputs are exposed.
+    const uint64_t by_bytes = (in_bytes + 150000) / 300000;
+    uint32_t n_chunks = by_bytes < 1 ? 1 : by_bytes > vfkv_workspace::kTokChunks ? vfkv_workspace::kTokChunks : uint32_t(by_bytes);
+    if (n_chunks > L) n_chunks = L;
+    auto chunk_begin = [&](uint32_t c) { return uint32_t(uint64_t(L) * c / n_chunks); };
+    // the length hint steers the split count only; it is rounded up so that recordings stay valid for long
     uint32_t hint = (max_pos + 1 + 1023u) / 1024u * 1024u;
     if (hint > kv.config.max_seq_len) hint = kv.config.max_seq_len;
+    memcpy(ws->tok_u32, h_positions, n_seqs * 4);
+    if (h_slot_ids) memcpy(ws->tok_u32 + ws->max_seqs, h_slot_ids, n_seqs * 4);
+    cudaEvent_t *ev_in = ws->tok_events, *ev_done = ev_in + vfkv_workspace::kTokChunks;
+    cudaEvent_t ev_begin = ws->tok_events[2 * vfkv_workspace::kTokChunks], ev_end = ws->tok_events[2 * vfkv_workspace::kTokChunks + 1];
+    // The token's copies and launches on three streams that fork from `st` and join it again.  The order
+    // of the calls is that of the work, so that a call that blocks (pageable buffers) holds up nothing
+    // that could already run.
+    auto enqueue = [&]() -> int32_t {
+        cudaError_t ce = cudaEventRecord(ev_begin, st);
+        if (ce == cudaSuccess) ce = cudaStreamWaitEvent(ws->tok_in, ev_begin, 0);
+        if (ce == cudaSuccess) ce = cudaMemcpyAsync(d_pos, ws->tok_u32, n_seqs * 4, cudaMemcpyHostToDevice, ws->tok_in);
+        if (ce == cudaSuccess && h_slot_ids) ce = cudaMemcpyAsync(d_slots, ws->tok_u32 + ws->max_seqs, n_seqs * 4, cudaMemcpyHostToDevice, ws->tok_in);
+        auto copy_in = [&](uint32_t c) {
+            const uint32_t l0 = chunk_begin(c), nl = chunk_begin(c + 1) - l0;
+            if (ce == cudaSuccess) ce = cudaMemcpyAsync(dq + l0 * q_stride, h_q + l0 * q_stride, nl * q_stride * 4, cudaMemcpyHostToDevice, ws->tok_in);
+            if (ce == cudaSuccess) ce = cudaMemcpyAsync(dk + l0 * kv_stride, h_k + l0 * kv_stride, nl * kv_stride * 4, cudaMemcpyHostToDevice, ws->tok_in);
+            if (ce == cudaSuccess) ce = cudaMemcpyAsync(dv + l0 * kv_stride, h_v + l0 * kv_stride, nl * kv_stride * 4, cudaMemcpyHostToDevice, ws->tok_in);
+            if (ce == cudaSuccess) ce = cudaEventRecord(ev_in[c], ws->tok_in);
+        };
+        auto copy_out = [&](uint32_t c) {
+            const uint32_t l0 = chunk_begin(c), nl = chunk_begin(c + 1) - l0;
+            if (ce == cudaSuccess) ce = cudaStreamWaitEvent(ws->tok_out, ev_done[c], 0);
+            if (ce == cudaSuccess) ce = cudaMemcpyAsync(h_out + l0 * q_stride, ws->stage_out + l0 * q_stride, nl * q_stride * 4, cudaMemcpyDeviceToHost, ws->tok_out);
+        };
+        copy_in(0);
+        for (uint32_t c = 0; c < n_chunks; ++c) {
+            if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st, ev_in[c], 0);
+            if (ce != cudaSuccess) break;
+            if (int32_t rc = run_layers(chunk_begin(c), chunk_begin(c + 1), hint)) return rc;
+            ce = cudaEventRecord(ev_done[c], st);
+            if (c + 1 < n_chunks) copy_in(c + 1);
+            if (c > 0) copy_out(c - 1);
+        }
+        copy_out(n_chunks - 1);
+        if (ce == cudaSuccess) ce = cudaEventRecord(ev_end, ws->tok_out);
+        if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st, ev_end, 0);
+        return check_cuda(ctx, ce, "vfkv_decode_token_host: pipelined step");
+    };
+    // What a recording depends on: the configuration, the caller's buffers and the context's settings
+    // (positions and slots travel through buffers of the workspace).
     uint64_t wh = 1469598103934665603ull;
     auto mix = [&](uint64_t x) { wh = (wh ^ x) * 1099511628211ull; };
     for (uint32_t l = 0; windows && l < L; ++l) mix(windows[l]);
     // a cache object re-created at the same address must not find the old graphs
     mix(reinterpret_cast<uint64_t>(kv.k_buffer)); mix(reinterpret_cast<uint64_t>(kv.v_buffer));
     mix(L); mix(D); mix(Hkv); mix(uint64_t(kv.kv_dtype)); mix(kv.config.max_seq_len); mix(kv.config.n_slots);
-    mix(reinterpret_cast<uint64_t>(ws->part_o)); mix(reinterpret_cast<uint64_t>(dk));
+    mix(kv.config.scale_mode); mix(ctx->merge_wait_ns); mix(ctx->debug_fail_split);
     uint32_t fs, fc;
     memcpy(&fs, &scale, 4); memcpy(&fc, &softcap, 4);
-    const uint64_t key[8] = {reinterpret_cast<uint64_t>(cache), reinterpret_cast<uint64_t>(dq),
-                             reinterpret_cast<uint64_t>(ws->stage_out),
-                             uint64_t(n_q_heads) << 32 | n_seqs, uint64_t(hint) << 32 | n_splits,
-                             uint64_t(fs) << 32 | fc, wh ^ (h_slot_ids ? 1u : 0u),
-                             uint64_t(ctx->pdl) | uint64_t(ctx->tune_warps) << 8 | uint64_t(ctx->tune_stages) << 16 |
-                                 uint64_t(ctx->attn_impl) << 24 | uint64_t(ctx->cluster_merge) << 32 |
-                                 uint64_t(reinterpret_cast<uintptr_t>(st) & 0xffffffu) << 40};
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(st, &cap);
-    bool graphable = cap == cudaStreamCaptureStatusNone && !ctx->profiling && !ctx->d_trace && st != nullptr;
-    // The layers are cut into up to four groups, one graph each: the inputs of group c + 1 cross
-    // the bus on a second stream while group c computes, and the outputs of group c go back while
-    // group c + 1 computes.  Only the first group's inputs and the last group's outputs are exposed.
-    const uint32_t n_chunks = L < vfkv_workspace::kTokChunks ? L : vfkv_workspace::kTokChunks;
-    auto chunk_begin = [&](uint32_t c) { return uint32_t(uint64_t(L) * c / n_chunks); };
-    auto run_layers = [&](uint32_t l0, uint32_t l1, uint32_t len_hint) -> int32_t {
-        return decode_layers(cache, ws, l0, l1, dq, dk, dv, ws->stage_out, n_q_heads, h_slot_ids ? d_slots : nullptr,
-                             d_pos, n_seqs, len_hint, windows, scale, softcap, n_splits, stream);
+    const uint64_t key[14] = {reinterpret_cast<uint64_t>(cache), reinterpret_cast<uint64_t>(dq),
+                              reinterpret_cast<uint64_t>(ws->stage_out), uint64_t(n_q_heads) << 32 | n_seqs,
+                              uint64_t(hint) << 32 | n_splits, uint64_t(fs) << 32 | fc, wh ^ (h_slot_ids ? 1u : 0u),
+                              uint64_t(ctx->pdl) | uint64_t(ctx->tune_warps) << 8 | uint64_t(ctx->tune_stages) << 16 |
+                                  uint64_t(ctx->attn_impl) << 24 | uint64_t(ctx->cluster_merge) << 32,
+                              reinterpret_cast<uint64_t>(st), reinterpret_cast<uint64_t>(h_q), reinterpret_cast<uint64_t>(h_k),
+                              reinterpret_cast<uint64_t>(h_v), reinterpret_cast<uint64_t>(h_out), 0};
+    vfkv_workspace::TokGraph *tg = nullptr;
+    for (auto &cand : ws->tok)
+        if (cand.known && memcmp(cand.key, key, sizeof(key)) == 0) tg = &cand;
+    // pageable buffers are copied by the host as the calls are made, which no recording can do
+    auto pinned = [](const void *p) {
+        cudaPointerAttributes at;
+        const bool ok = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost;
+        cudaGetLastError();
+        return ok;
     };
-    if (graphable && !ws->copy_stream) {
-        bool ok = cudaStreamCreateWithFlags(&ws->copy_stream, cudaStreamNonBlocking) == cudaSuccess;
-        for (uint32_t i = 0; ok && i < 2 * vfkv_workspace::kTokChunks; ++i)
-            ok = cudaEventCreateWithFlags(&ws->tok_events[i], cudaEventDisableTiming) == cudaSuccess;
-        if (!ok) { cudaGetLastError(); graphable = false; }
-    }
-    if (graphable && (!ws->tok_graphs[0] || memcmp(key, ws->tok_key, sizeof(key)) != 0)) {
-        for (auto &gexec : ws->tok_graphs)
-            if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
-        for (uint32_t c = 0; c < n_chunks; ++c) {
-            cudaGraph_t graph = nullptr;
-            if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); break; }
+    const bool recordable = tg && pinned(h_q) && pinned(h_k) && pinned(h_v) && pinned(h_out);
+    if (recordable && !tg->exec) {
+        cudaGraph_t graph = nullptr;
+        if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
             const uint64_t launches = ctx->launches, kernels = ctx->kernels;
-            int32_t rc = run_layers(chunk_begin(c), chunk_begin(c + 1), hint);
-            cudaError_t ce = cudaStreamEndCapture(st, &graph);
-            ws->tok_launches[c] = uint32_t(ctx->launches - launches);
-            ws->tok_kernels[c] = uint32_t(ctx->kernels - kernels);
-            ctx->launches = launches; ctx->kernels = kernels;   // recorded, not run
-            const bool ok = rc == VFKV_OK && ce == cudaSuccess && graph &&
-                            cudaGraphInstantiate(&ws->tok_graphs[c], graph, 0) == cudaSuccess;
+            const int32_t rc = enqueue();
+            const cudaError_t ce = cudaStreamEndCapture(st, &graph);
+            tg->launches = uint32_t(ctx->launches - launches);
+            tg->kernels = uint32_t(ctx->kernels - kernels);
+            ctx->launches = launches; ctx->kernels = kernels;       // recorded, not run
+            if (rc != VFKV_OK || ce != cudaSuccess || !graph || cudaGraphInstantiate(&tg->exec, graph, 0) != cudaSuccess)
+                tg->exec = nullptr;
             if (graph) cudaGraphDestroy(graph);
-            cudaGetLastError();
-            if (rc) return rc;
-            if (!ok) { ws->tok_graphs[c] = nullptr; break; }
         }
-        bool all = true;
-        for (uint32_t c = 0; c < n_chunks; ++c) all = all && ws->tok_graphs[c];
-        if (all) memcpy(ws->tok_key, key, sizeof(key));
-        else {
-            for (auto &gexec : ws->tok_graphs)
-                if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
-        }
+        cudaGetLastError();
     }
-    if (graphable && ws->tok_graphs[0]) {
-        cudaStream_t cs = ws->copy_stream;
-        cudaEvent_t *ev_in = ws->tok_events, *ev_done = ws->tok_events + vfkv_workspace::kTokChunks;
-        // The staging buffers belong to the workspace and every earlier call drained both streams,
-        // so the first copies need not wait for the caller's stream.  Each group's launch is issued
-        // as soon as its own copies are queued: the host calls for the later groups then run while
-        // the first group computes.  On the copy stream the order is in(0) in(1) out(0) in(2) out(1)
-        // ..., so an input copy never waits for a group that has not started.
-        auto copy_in = [&](uint32_t c) {
-            const uint32_t l0 = chunk_begin(c), nl = chunk_begin(c + 1) - l0;
-            cudaError_t ce = cudaMemcpyAsync(dq + l0 * q_stride, h_q + l0 * q_stride, nl * q_stride * 4, cudaMemcpyHostToDevice, cs);
-            if (ce == cudaSuccess) ce = cudaMemcpyAsync(dk + l0 * kv_stride, h_k + l0 * kv_stride, nl * kv_stride * 4, cudaMemcpyHostToDevice, cs);
-            if (ce == cudaSuccess) ce = cudaMemcpyAsync(dv + l0 * kv_stride, h_v + l0 * kv_stride, nl * kv_stride * 4, cudaMemcpyHostToDevice, cs);
-            if (ce == cudaSuccess) ce = cudaEventRecord(ev_in[c], cs);
-            return ce;
-        };
-        e = copy_in(0);
-        for (uint32_t c = 0; c < n_chunks && e == cudaSuccess; ++c) {
-            const uint32_t l0 = chunk_begin(c), nl = chunk_begin(c + 1) - l0;
-            e = cudaStreamWaitEvent(st, ev_in[c], 0);
-            if (e == cudaSuccess) e = cudaGraphLaunch(ws->tok_graphs[c], st);
-            if (e == cudaSuccess) e = cudaEventRecord(ev_done[c], st);
-            if (e == cudaSuccess) { ctx->launches += ws->tok_launches[c]; ctx->kernels += ws->tok_kernels[c]; }
-            if (e == cudaSuccess && c + 1 < n_chunks) e = copy_in(c + 1);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(cs, ev_done[c], 0);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(h_out + l0 * q_stride, ws->stage_out + l0 * q_stride, nl * q_stride * 4, cudaMemcpyDeviceToHost, cs);
-        }
-        // The last output copy follows the last group, so the copy stream finishing means the step
-        // is complete; the caller's stream is drained as well, also after an error, so that
-        // nothing of this call is left in flight.
-        cudaError_t e2 = cudaStreamSynchronize(cs);
-        cudaError_t e3 = cudaStreamSynchronize(st);
-        if (e == cudaSuccess) e = e2 != cudaSuccess ? e2 : e3;
-        return check_cuda(ctx, e, "vfkv_decode_token_host: pipelined step");
+    if (!tg) {             // a first call with these buffers: remembered in the older one's place
+        tg = &ws->tok[ws->tok_oldest];
+        ws->tok_oldest ^= 1u;
+        if (tg->exec) cudaGraphExecDestroy(tg->exec);
+        tg->exec = nullptr;
+        memcpy(tg->key, key, sizeof(key));
+        tg->known = true;
     }
-    // stream order only (inside a capture, under the profiler or with the phase trace on)
-    e = cudaMemcpyAsync(dq, h_q, q_elems * 4, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dk, h_k, kv_elems * 4, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dv, h_v, kv_elems * 4, cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return check_cuda(ctx, e, "vfkv_decode_token_host: H2D");
-    if (int32_t rc = run_layers(0, L, max_pos + 1)) return rc;
-    e = cudaMemcpyAsync(h_out, ws->stage_out, out_bytes, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    return check_cuda(ctx, e, "vfkv_decode_token_host: D2H");
+    int32_t rc = VFKV_OK;
+    if (recordable && tg->exec) {
+        e = cudaGraphLaunch(tg->exec, st);
+        if (e == cudaSuccess) { ctx->launches += tg->launches; ctx->kernels += tg->kernels; }
+        rc = check_cuda(ctx, e, "vfkv_decode_token_host: graph launch");
+    } else {
+        rc = enqueue();
+    }
+    // the other streams have joined `st`; after an error they are drained as well, so that nothing of
+    // this call is left in flight
+    const cudaError_t done = cudaStreamSynchronize(st);
+    if (rc != VFKV_OK) {
+        cudaStreamSynchronize(ws->tok_in);
+        cudaStreamSynchronize(ws->tok_out);
+        return rc;
+    }
+    return check_cuda(ctx, done, "vfkv_decode_token_host: pipelined step");
 }
 
 /* ---- the same step without waiting: two tokens in flight ------------------------------------- */

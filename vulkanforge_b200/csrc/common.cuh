@@ -87,16 +87,23 @@ struct vfkv_workspace {
     float *stage_in = nullptr;
     float *stage_out = nullptr;
     uint64_t stage_in_bytes = 0, stage_out_bytes = 0;
-    // vfkv_decode_token_host: the kernel sequence of one token, captured once per configuration and
-    // replayed (the analogue of the reference's pre-recorded command buffers, forward/decode.rs:169-259)
-    // The layers form up to kTokChunks groups with one graph each, so that a second stream moves the
-    // next group's inputs and the previous group's outputs while a group computes.
-    static constexpr uint32_t kTokChunks = 4;
-    cudaGraphExec_t tok_graphs[kTokChunks] = {nullptr, nullptr, nullptr, nullptr};
-    uint32_t tok_launches[kTokChunks] = {}, tok_kernels[kTokChunks] = {};   // what one replay adds to the context's counts
-    uint64_t tok_key[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    cudaStream_t copy_stream = nullptr;
-    cudaEvent_t tok_events[2 * kTokChunks] = {};         // inputs there / group done, per group
+    // vfkv_decode_token_host: copies and kernels of one token, in up to kTokChunks groups of layers, so
+    // that the next group's inputs and the previous group's outputs cross the bus while one computes.  The
+    // whole sequence is recorded as a graph when a call with the same buffers comes a second time and
+    // replayed from then on (the analogue of the reference's pre-recorded command buffers,
+    // forward/decode.rs:169-259); two recordings, for hosts that alternate between two sets of buffers.
+    static constexpr uint32_t kTokChunks = 8;
+    struct TokGraph {
+        uint64_t key[14] = {};
+        bool known = false;                              // the key is that of a call that was made
+        cudaGraphExec_t exec = nullptr;
+        uint32_t launches = 0, kernels = 0;              // what one replay adds to the context's counts
+    };
+    TokGraph tok[2];
+    uint32_t tok_oldest = 0;
+    cudaStream_t tok_in = nullptr, tok_out = nullptr;
+    cudaEvent_t tok_events[2 * kTokChunks + 2] = {};     // inputs there / group done, per group; begin, end
+    uint32_t *tok_u32 = nullptr;                         // pinned: positions, then slot ids
     // vfkv_decode_token_host_submit / _wait: two tokens in flight, each with its own staging set and
     // its own recorded graph (the analogue of the reference's two command-buffer / fence pairs and
     // per-slot scratch, forward/decode.rs:169-259, forward/setup.rs:203-230).

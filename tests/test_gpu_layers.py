@@ -76,3 +76,44 @@ def test_layers_of_a_token_share_launches(ctx, dtype, scaled, hq, hkv, d, n_laye
     finally:
         fwd.workspace.destroy()
         cache.destroy()
+
+
+@pytest.mark.parametrize("n_layers,n,pinned", [(3, 2, "all"), (40, 8, "all"), (3, 2, "none"), (40, 8, "inputs"), (3, 2, "output")])
+def test_host_token_pinned_buffers_and_replays(ctx, n_layers, n, pinned):
+    """vfkv_decode_token_host by every way its buffers can travel (one kernel, groups of layers, pageable),
+    called again with the same buffers (a recording) and alternating between two sets of them."""
+    import torch
+    hq, hkv, d, length = 32, 8, 128, 200
+    gen = torch.Generator().manual_seed(n_layers)
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(n_layers, hkv, d, 256, n_slots=n), vf.KvDtype.F16)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq, max_batch=n)
+    ref = vf.CudaForward(ctx, cache, n_heads=hq, max_batch=n)
+    stream = torch.cuda.Stream()
+    try:
+        cache.zero_fill()
+        for layer in range(n_layers):
+            for slot in range(n):
+                kv = torch.randn(2, length, hkv, d, generator=gen).cuda()
+                fwd.b_step_kv_write(layer, kv[0], kv[1], length, 0, slot)
+        torch.cuda.synchronize()
+        fwd.stream = stream.cuda_stream
+        host = lambda x, when: x.pin_memory() if pinned in ("all", when) else x
+        sets = [[host(torch.randn(n_layers, n, h, d, generator=gen), "inputs") for h in (hq, hkv, hkv)] +
+                [host(torch.zeros(n_layers, n, hq, d), "output")] for _ in range(2)]
+        for step, which in enumerate((0, 0, 0, 1, 1, 0, 1)):
+            q, k, v, out = sets[which]
+            q.normal_(generator=gen)
+            out.fill_(7.0)
+            pos = np.array([length + step - 3 * i for i in range(n)], np.uint32)
+            ids = np.arange(n, dtype=np.uint32)[::-1].copy() if step % 2 else None
+            fwd.decode_token_host(q, k, v, out, pos, n, ids)
+            want = torch.zeros(n_layers, n, hq, d, device="cuda")
+            ref.decode_token(q.cuda(), k.cuda(), v.cuda(), want, None if ids is None else to_dev(ids), to_dev(pos), n, 256)
+            torch.cuda.synchronize()
+            assert float((want.cpu() - out).abs().max()) < 1e-5
+        ctx.poll()
+    finally:
+        fwd.stream = None
+        fwd.workspace.destroy()
+        ref.workspace.destroy()
+        cache.destroy()

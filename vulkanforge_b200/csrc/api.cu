@@ -869,7 +869,34 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
         if (e != cudaSuccess) return check_cuda(ctx, e, "vfkv_decode_token_host: staging");
         ws->stage_in_bytes = in_bytes;
     }
-    if (ws->stage_out_bytes < out_bytes) {
+    float *dq = ws->stage_in, *dk = dq + q_elems, *dv = dk + kv_elems;
+    uint32_t *d_pos = ws->d_u32, *d_slots = ws->d_u32 + ws->max_seqs;
+    const uint64_t q_stride = uint64_t(n_seqs) * n_q_heads * D, kv_stride = uint64_t(n_seqs) * Hkv * D;
+    float *d_out = nullptr;
+    auto run_layers = [&](uint32_t l0, uint32_t l1, uint32_t len_hint) -> int32_t {
+        return decode_layers(cache, ws, l0, l1, dq, dk, dv, d_out, n_q_heads, h_slot_ids ? d_slots : nullptr,
+                             d_pos, n_seqs, len_hint, windows, scale, softcap, n_splits, stream);
+    };
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(st, &cap);
+    bool pipelined = cap == cudaStreamCaptureStatusNone && !ctx->profiling && !ctx->d_trace && st != nullptr;
+    cudaError_t e = cudaSuccess;
+    // Buffers in pinned memory are on the device's own bus: the attention kernel writes its rows straight
+    // into h_out, and the inputs of a small token come by one kernel.
+    auto pinned_at = [](uintptr_t p) {
+        cudaPointerAttributes at;
+        const bool ok = cudaPointerGetAttributes(&at, reinterpret_cast<void *>(p)) == cudaSuccess &&
+                        at.type == cudaMemoryTypeHost && reinterpret_cast<uintptr_t>(at.devicePointer) == p;
+        cudaGetLastError();
+        return ok;
+    };
+    auto pinned = [&](const float *p, uint64_t n) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+        return a % 16 == 0 && pinned_at(a) && pinned_at(a + n * 4 - 4);
+    };
+    const bool out_direct = pipelined && pinned(h_out, q_elems);
+    const bool in_pinned = pinned(h_q, q_elems) && pinned(h_k, kv_elems) && pinned(h_v, kv_elems);
+    if (!out_direct && ws->stage_out_bytes < out_bytes) {
         cudaStreamSynchronize(st);
         cudaFree(ws->stage_out);
         ws->stage_out = nullptr; ws->stage_out_bytes = 0;
@@ -877,28 +904,7 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
         if (e != cudaSuccess) return check_cuda(ctx, e, "vfkv_decode_token_host: staging");
         ws->stage_out_bytes = out_bytes;
     }
-    float *dq = ws->stage_in, *dk = dq + q_elems, *dv = dk + kv_elems;
-    uint32_t *d_pos = ws->d_u32, *d_slots = ws->d_u32 + ws->max_seqs;
-    const uint64_t q_stride = uint64_t(n_seqs) * n_q_heads * D, kv_stride = uint64_t(n_seqs) * Hkv * D;
-    auto run_layers = [&](uint32_t l0, uint32_t l1, uint32_t len_hint) -> int32_t {
-        return decode_layers(cache, ws, l0, l1, dq, dk, dv, ws->stage_out, n_q_heads, h_slot_ids ? d_slots : nullptr,
-                             d_pos, n_seqs, len_hint, windows, scale, softcap, n_splits, stream);
-    };
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(st, &cap);
-    bool pipelined = cap == cudaStreamCaptureStatusNone && !ctx->profiling && !ctx->d_trace && st != nullptr;
-    cudaError_t e = cudaSuccess;
-    if (pipelined && !ws->tok_out) {
-        bool ok = cudaHostAlloc(reinterpret_cast<void **>(&ws->tok_u32), uint64_t(ws->max_seqs) * 2 * 4, cudaHostAllocDefault) == cudaSuccess &&
-                  cudaStreamCreateWithFlags(&ws->tok_in, cudaStreamNonBlocking) == cudaSuccess;
-        for (uint32_t i = 0; ok && i < 2 * vfkv_workspace::kTokChunks + 2; ++i)
-            ok = cudaEventCreateWithFlags(&ws->tok_events[i], cudaEventDisableTiming) == cudaSuccess;
-        ok = ok && cudaStreamCreateWithFlags(&ws->tok_out, cudaStreamNonBlocking) == cudaSuccess;
-        if (!ok) {
-            cudaGetLastError();
-            return set_error(ctx, VFKV_ERR_CUDA, "vfkv_decode_token_host: streams and events");
-        }
-    }
+    d_out = out_direct ? h_out : ws->stage_out;
     if (!pipelined) {      // stream order only: on the default stream, inside a capture, under the profiler or the phase trace
         e = cudaMemcpyAsync(d_pos, h_positions, n_seqs * 4, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess && h_slot_ids) e = cudaMemcpyAsync(d_slots, h_slot_ids, n_seqs * 4, cudaMemcpyHostToDevice, st);
@@ -911,13 +917,28 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         return check_cuda(ctx, e, "vfkv_decode_token_host: D2H");
     }
-    // Groups of about 300 KB of inputs, eight at most: a group has to be worth its copies and its launch
-    // (36 layers of one sequence, 0.88 MB: three groups), and only the first group's inputs and the last
-    // one's outputs are exposed.
-    const uint64_t by_bytes = (in_bytes + 150000) / 300000;
+    // Large tokens cross the bus in groups of layers, so that a group computes while the next one's inputs
+    // arrive.  A group costs some 12 us of dependencies between streams and launches (36 layers of one
+    // sequence, 0.9 MB in, 0.6 MB out: 157 us as one group, 167 as two, 182 as four; 32 layers of 16, 20 MB:
+    // 575 as one, 474 as four), so it has to be worth them: about 1.5 MB each, four at most.
+    const uint64_t by_bytes = (in_bytes + out_bytes) / 1500000;
     uint32_t n_chunks = by_bytes < 1 ? 1 : by_bytes > vfkv_workspace::kTokChunks ? vfkv_workspace::kTokChunks : uint32_t(by_bytes);
     if (n_chunks > L) n_chunks = L;
     auto chunk_begin = [&](uint32_t c) { return uint32_t(uint64_t(L) * c / n_chunks); };
+    const bool one_kernel_in = n_chunks == 1 && in_pinned && out_direct;
+    if (!ws->tok_u32) {
+        e = cudaHostAlloc(reinterpret_cast<void **>(&ws->tok_u32), uint64_t(ws->max_seqs) * 2 * 4, cudaHostAllocDefault);
+        if (e != cudaSuccess) return check_cuda(ctx, e, "vfkv_decode_token_host: positions");
+    }
+    if (!one_kernel_in && !ws->tok_out) {
+        bool ok = ws->tok_in || cudaStreamCreateWithFlags(&ws->tok_in, cudaStreamNonBlocking) == cudaSuccess;
+        for (auto &ev : ws->tok_events) ok = ok && (ev || cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess);
+        ok = ok && cudaStreamCreateWithFlags(&ws->tok_out, cudaStreamNonBlocking) == cudaSuccess;
+        if (!ok) {
+            cudaGetLastError();
+            return set_error(ctx, VFKV_ERR_CUDA, "vfkv_decode_token_host: streams and events");
+        }
+    }
     // the length hint steers the split count only; it is rounded up so that recordings stay valid for long
     uint32_t hint = (max_pos + 1 + 1023u) / 1024u * 1024u;
     if (hint > kv.config.max_seq_len) hint = kv.config.max_seq_len;
@@ -929,6 +950,19 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
     // of the calls is that of the work, so that a call that blocks (pageable buffers) holds up nothing
     // that could already run.
     auto enqueue = [&]() -> int32_t {
+        if (one_kernel_in) {
+            StageArgs a;
+            const float *src[3] = {h_q, h_k, h_v};
+            float *dst[3] = {dq, dk, dv};
+            for (int i = 0; i < 3; ++i) {
+                a.src[i] = reinterpret_cast<const uint4 *>(src[i]);
+                a.dst[i] = reinterpret_cast<uint4 *>(dst[i]);
+                a.units[i] = (i == 0 ? q_elems : kv_elems) / 4;      // cache rows are whole 16-byte units, so these are too
+            }
+            a.words_src = ws->tok_u32; a.words_dst = d_pos; a.n_words = h_slot_ids ? ws->max_seqs + n_seqs : n_seqs;
+            if (int32_t rc = launch_stage_in(ctx, a, st)) return rc;
+            return run_layers(0, L, hint);
+        }
         cudaError_t ce = cudaEventRecord(ev_begin, st);
         if (ce == cudaSuccess) ce = cudaStreamWaitEvent(ws->tok_in, ev_begin, 0);
         if (ce == cudaSuccess) ce = cudaMemcpyAsync(d_pos, ws->tok_u32, n_seqs * 4, cudaMemcpyHostToDevice, ws->tok_in);
@@ -941,6 +975,7 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
             if (ce == cudaSuccess) ce = cudaEventRecord(ev_in[c], ws->tok_in);
         };
         auto copy_out = [&](uint32_t c) {
+            if (out_direct) return;
             const uint32_t l0 = chunk_begin(c), nl = chunk_begin(c + 1) - l0;
             if (ce == cudaSuccess) ce = cudaStreamWaitEvent(ws->tok_out, ev_done[c], 0);
             if (ce == cudaSuccess) ce = cudaMemcpyAsync(h_out + l0 * q_stride, ws->stage_out + l0 * q_stride, nl * q_stride * 4, cudaMemcpyDeviceToHost, ws->tok_out);
@@ -955,8 +990,10 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
             if (c > 0) copy_out(c - 1);
         }
         copy_out(n_chunks - 1);
-        if (ce == cudaSuccess) ce = cudaEventRecord(ev_end, ws->tok_out);
-        if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st, ev_end, 0);
+        if (!out_direct) {
+            if (ce == cudaSuccess) ce = cudaEventRecord(ev_end, ws->tok_out);
+            if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st, ev_end, 0);
+        }
         return check_cuda(ctx, ce, "vfkv_decode_token_host: pipelined step");
     };
     // What a recording depends on: the configuration, the caller's buffers and the context's settings
@@ -981,13 +1018,7 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
     for (auto &cand : ws->tok)
         if (cand.known && memcmp(cand.key, key, sizeof(key)) == 0) tg = &cand;
     // pageable buffers are copied by the host as the calls are made, which no recording can do
-    auto pinned = [](const void *p) {
-        cudaPointerAttributes at;
-        const bool ok = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-        return ok;
-    };
-    const bool recordable = tg && pinned(h_q) && pinned(h_k) && pinned(h_v) && pinned(h_out);
+    const bool recordable = tg && in_pinned && out_direct;
     if (recordable && !tg->exec) {
         cudaGraph_t graph = nullptr;
         if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
@@ -1015,6 +1046,7 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
     if (recordable && tg->exec) {
         e = cudaGraphLaunch(tg->exec, st);
         if (e == cudaSuccess) { ctx->launches += tg->launches; ctx->kernels += tg->kernels; }
+        ctx->set_written_any();        // the replay ends with kernels that wrote rows of many layers
         rc = check_cuda(ctx, e, "vfkv_decode_token_host: graph launch");
     } else {
         rc = enqueue();
@@ -1023,8 +1055,8 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
     // this call is left in flight
     const cudaError_t done = cudaStreamSynchronize(st);
     if (rc != VFKV_OK) {
-        cudaStreamSynchronize(ws->tok_in);
-        cudaStreamSynchronize(ws->tok_out);
+        if (ws->tok_in) cudaStreamSynchronize(ws->tok_in);
+        if (ws->tok_out) cudaStreamSynchronize(ws->tok_out);
         return rc;
     }
     return check_cuda(ctx, done, "vfkv_decode_token_host: pipelined step");
@@ -1148,6 +1180,7 @@ int32_t vfkv_decode_token_host_submit(vfkv_cache *cache, vfkv_workspace *ws, con
     }
     ctx->launches += hs->launches;
     ctx->kernels += hs->kernels;
+    ctx->set_written_any();            // the replay ends with kernels that wrote rows of many layers
     hs->ticket = ws->next_ticket++;
     *ticket = hs->ticket;
     return VFKV_OK;

@@ -302,6 +302,33 @@ int32_t launch_append(vfkv_ctx *ctx, const AppendArgs &a, cudaStream_t st)
     return check_cuda(ctx, le, "append launch");
 }
 
+// ---- host rows -> device staging ---------------------------------------------------
+// A token's inputs read straight out of pinned host memory.  A few hundred KB are bound by latencies:
+// four copy-engine transfers and their dependencies take longer than this one kernel.
+__global__ void __launch_bounds__(256) stage_in_kernel(const StageArgs a)
+{
+    pdl_wait();
+    const uint64_t units = a.units[0] + a.units[1] + a.units[2];
+    for (uint64_t i = blockIdx.x * uint64_t(256) + threadIdx.x; i < units; i += uint64_t(gridDim.x) * 256) {
+        uint64_t k = i;
+        int s = 0;
+        while (k >= a.units[s]) k -= a.units[s++];
+        a.dst[s][k] = a.src[s][k];
+    }
+    if (blockIdx.x == 0)
+        for (uint32_t i = threadIdx.x; i < a.n_words; i += 256) a.words_dst[i] = a.words_src[i];
+}
+
+int32_t launch_stage_in(vfkv_ctx *ctx, const StageArgs &a, cudaStream_t st)
+{
+    const uint64_t units = a.units[0] + a.units[1] + a.units[2];
+    uint64_t blocks = (units + 255) / 256, cap = uint64_t(ctx->sm_count) * 4;
+    if (blocks > cap) blocks = cap;
+    const cudaError_t e = launch_dependent(ctx, stage_in_kernel, dim3(unsigned(blocks)), dim3(256), 0, st, a);
+    ctx->set_written_any();        // what follows reads its positions from here: no reading ahead
+    return check_cuda(ctx, e, "stage_in launch");
+}
+
 // ---- E4M3 -> binary16 (vk_shaders/kv_fp8_to_f16.comp:28-34) ----------------
 // HBM-bound: 3 bytes an element.  A thread has four 16-byte loads in flight, and stores 32 bytes, a
 // whole sector, at a time (two 16-byte stores 32 bytes apart write every sector twice by halves).

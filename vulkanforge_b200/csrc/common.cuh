@@ -92,7 +92,7 @@ struct vfkv_workspace {
     // whole sequence is recorded as a graph when a call with the same buffers comes a second time and
     // replayed from then on (the analogue of the reference's pre-recorded command buffers,
     // forward/decode.rs:169-259); two recordings, for hosts that alternate between two sets of buffers.
-    static constexpr uint32_t kTokChunks = 8;
+    static constexpr uint32_t kTokChunks = 4;
     struct TokGraph {
         uint64_t key[14] = {};
         bool known = false;                              // the key is that of a call that was made
@@ -103,7 +103,7 @@ struct vfkv_workspace {
     uint32_t tok_oldest = 0;
     cudaStream_t tok_in = nullptr, tok_out = nullptr;
     cudaEvent_t tok_events[2 * kTokChunks + 2] = {};     // inputs there / group done, per group; begin, end
-    uint32_t *tok_u32 = nullptr;                         // pinned: positions, then slot ids
+    uint32_t *tok_u32 = nullptr;                         // pinned: positions, then slot ids (the layout of d_u32)
     // vfkv_decode_token_host_submit / _wait: two tokens in flight, each with its own staging set and
     // its own recorded graph (the analogue of the reference's two command-buffer / fence pairs and
     // per-slot scratch, forward/decode.rs:169-259, forward/setup.rs:203-230).
@@ -292,6 +292,17 @@ struct AppendArgs {
     const uint16_t *layer_ids = nullptr;
 };
 int32_t launch_append(vfkv_ctx *ctx, const AppendArgs &a, cudaStream_t st);
+
+// Three runs of 16-byte units and one of words, from pinned host memory to the device.
+struct StageArgs {
+    const uint4 *src[3];
+    uint4 *dst[3];
+    uint64_t units[3];
+    const uint32_t *words_src;
+    uint32_t *words_dst;
+    uint32_t n_words;
+};
+int32_t launch_stage_in(vfkv_ctx *ctx, const StageArgs &a, cudaStream_t st);
 
 int32_t launch_attention(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, cudaStream_t st);
 int32_t launch_merge_partials(vfkv_ctx *ctx, const float *m, const float *l, const float *o,

@@ -1,0 +1,71 @@
+"""The tcgen05 prefill kernel with one Q tile of 128 rows a CTA: head_dim 64, 128 and 256, FP8 (plain and
+with scales) and F16 rows, at the edges of its tiles (128 rows, 64 positions), cut into pieces and whole,
+every mask, and the soft-cap on either side of its polynomial's range."""
+import numpy as np
+import pytest
+
+import oracle
+import vulkanforge_b200 as vf
+from util import dev_view_bytes, encode_cache, kv_values, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype,hq,hkv,d,m,q_start,kv_start,window,softcap,q_gain", [
+    ("F16", 16, 8, 256, 64, 64, 0, 0, 0.0, 1.0),         # exactly one block of rows, two tiles
+    ("F16", 16, 8, 256, 65, 130, 0, 0, 0.0, 1.0),        # one row block and one query
+    ("F16", 16, 8, 256, 200, 1500, 0, 1024, 50.0, 1.0),  # window and soft-cap
+    ("F16", 8, 8, 64, 300, 1000, 0, 0, 0.0, 1.0),
+    ("F16", 8, 8, 64, 40, 3000, 17, 0, 30.0, 1.0),       # pieces; kv_start inside a tile
+    ("F8", 16, 8, 256, 100, 2100, 0, 0, 0.0, 1.0),       # pieces
+    ("F8", 16, 8, 256, 900, 100, 0, 0, 50.0, 20.0),      # scores beyond the cap; 120 blocks
+    ("F8", 8, 8, 64, 130, 600, 0, 100, 0.0, 1.0),
+    ("F8s", 32, 8, 128, 100, 333, 0, 0, 0.0, 1.0),
+    ("F8s", 32, 8, 128, 33, 5000, 0, 0, 0.0, 30.0),      # pieces; peaked rows move the maximum and the scales' reference
+    ("F8s", 16, 8, 256, 70, 900, 0, 256, 50.0, 1.0),
+    ("F8s", 8, 8, 64, 200, 200, 0, 0, 0.0, 1.0),
+    ("F8s", 24, 8, 128, 50, 1200, 0, 0, 0.0, 1.0),       # g = 3: a query's heads in two row blocks
+    ("F8s", 64, 8, 128, 300, 700, 0, 0, 30.0, 1.0),
+    ("F8s", 32, 8, 128, 80, 0, 50, 0, 0.0, 1.0),         # early queries have an empty range -> zeros
+    ("F8s", 32, 8, 128, 1, 700, 0, 0, 0.0, 1.0),
+])
+def test_one_tile_kernel_matches_the_oracle(ctx, dtype, hq, hkv, d, m, q_start, kv_start, window, softcap, q_gain):
+    import torch
+    scaled, name = dtype == "F8s", dtype[:2] if dtype == "F8s" else dtype
+    L = q_start + m
+    rng = np.random.default_rng(L + d)
+    frac = 0.01 if name == "F8" else 0.0
+    k, v = kv_values(rng, (L, hkv, d), frac), kv_values(rng, (L, hkv, d), frac)
+    if scaled:                                           # V scales that grow along the sequence by many binary orders
+        v *= np.exp2(np.linspace(-6, 6, L, dtype=np.float32))[:, None, None]
+    q = rng.standard_normal((m, hq, d), dtype=np.float32) * np.float32(q_gain)
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(2, hkv, d, L + 5, n_slots=2, scale_mode=int(scaled)), vf.KvDtype[name])
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq, softcap=softcap)
+    try:
+        fwd.b_step_kv_write(1, to_dev(k), to_dev(v), L, 0, 1)
+        out = torch.full((m, hq, d), float("nan"), device="cuda")
+        for _ in range(2):
+            fwd.run_flash_attn_batch(1, to_dev(q), out, m, q_start, L, 1, kv_start, slot=1, window=window)
+        torch.cuda.synchronize()
+        ctx.poll()
+        if scaled:                                       # the reference reads the codes and scales that the append stored
+            def rows(buf, scales):
+                codes = dev_view_bytes(buf + cache.slot_offset_bytes(1, 1), L * hkv * d)
+                sc = dev_view_bytes(scales + 3 * (L + 5) * hkv * 4, L * hkv * 4).view(np.float32).reshape(L, hkv, 1)
+                return oracle.kv_fp8_to_f16(codes).view(np.float16).astype(np.float32).reshape(L, hkv, d) * sc
+            odt, kc, vc = oracle.F32, rows(cache.k_buffer, cache.k_scales), rows(cache.v_buffer, cache.v_scales)
+        else:
+            odt = oracle.F16 if name == "F16" else oracle.F8
+            kc, vc = encode_cache(k, odt), encode_cache(v, odt)
+        got = out.cpu().numpy()
+        assert np.isfinite(got).all()
+        for i in sorted({0, 1, m // 3, m // 2, max(m - 2, 0), m - 1} & set(range(m))):
+            causal = q_start + i + 1
+            lo = min(causal, max(kv_start, causal - window) if window and causal > window else kv_start)
+            want = oracle.attention_ref(q[i], kc, vc, odt, hq, hkv, d, causal, lo, None, softcap) if lo < causal \
+                else np.zeros((hq, d), np.float32)
+            top = max(1.0 if scaled else 1e-3, float(np.max(np.abs(want))))
+            assert float(np.max(np.abs(got[i] - want))) < (1e-5 * top if scaled else 5e-3 * top if name == "F8" else 1e-3)
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

@@ -527,6 +527,8 @@ extern "C" int32_t vfkv_attend_prefill(vfkv_cache *cache, uint32_t layer, uint32
         (ctx->attn_impl == 2 || prefill_tc5_pays(ctx, n_q_heads, hkv, m, q_start, n_kv, kv_start, window)))
         return launch_prefill_tc5(ctx, dt, p.k, p.v, d_q, d_out, p.row_bytes, n_q_heads, hkv, m, q_start, n_kv, kv_start,
                                   window, scale, softcap, st);
+    static const char *xone = getenv("XONE");
+    if (xone && aligned && ctx->attn_impl == 0 && prefill_one_tile_supported(ctx, dt, D)) return launch_prefill_one_tile(ctx, dt, !tc5_accurate, p, st);
     if (mma_ok) {
         if (dt == VFKV_F8) {
             if (D == 64) return launch_mma_d<VFKV_F8, 64>(ctx, p, st);

@@ -22,7 +22,9 @@
 #include "../../include/vfkv_next.h"
 #include "common.cuh"
 #include "fp8_codec.cuh"
+#include "prefill_params.cuh"
 #include "softcap.cuh"
+#include "tcgen05.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -66,139 +68,6 @@ struct Tc5Params {
     uint32_t n_split;
 };
 
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ uint64_t timer_ns()
-{
-    uint64_t t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
-}
-// One box of a byte-typed 2-D tensor map (x bytes into the row, row y) into 128-byte-swizzled shared memory.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t bar)
-{
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
-}
-// One look at the phase with the given parity.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity)
-{
-    uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    return done != 0u;
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(count) : "memory");
-}
-// Bounded wait for the phase with the given parity; false after one second.  The hint lets the
-// hardware park the thread for up to that long instead of returning for another look (a waiting
-// warp that spins takes issue slots from the warps of its scheduler that work).
-constexpr uint32_t kSuspendNs = 20000u;
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
-{
-    uint64_t t0 = 0;
-    for (uint32_t it = 0;; ++it) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done) : "r"(bar), "r"(parity), "r"(kSuspendNs) : "memory");
-        if (done) return true;
-        // the timer is slow to read: look at it only now and then
-        if ((it & 255u) == 255u) {
-            if (t0 == 0) t0 = timer_ns();
-            else if (timer_ns() - t0 > 1000000000ull) return false;
-        }
-    }
-}
-
-// Shared-memory matrix descriptor, 128-byte swizzle, version 1 (sm_100).
-// K-major: 8-row groups 1024 B apart (SBO), LBO unused.  MN-major: 64-element groups along
-// MN `lbo` bytes apart, 8-row groups along K 1024 B apart.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes)
-{
-    return uint64_t((addr >> 4) & 0x3fffu) | (uint64_t((lbo_bytes >> 4) & 0x3fffu) << 16) |
-           (uint64_t((sbo_bytes >> 4) & 0x3fffu) << 32) | (1ull << 46) | (2ull << 61);
-}
-// Instruction descriptor of kind::f16: F32 accumulate, F16 x F16, M 128, N 128; bit 16 = B is MN-major.
-__host__ __device__ constexpr uint32_t idesc_f16(bool b_mn_major)
-{
-    return (1u << 4) | (uint32_t(b_mn_major) << 16) | (uint32_t(128 >> 3) << 17) | (uint32_t(128 >> 4) << 24);
-}
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32])
-{
-    uint32_t r[32];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-// The same load without the wait, into 32 consecutive floats (wait once after a batch of loads).
-__device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, float *v)
-{
-    uint32_t r[32];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr) : "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float *v)
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-                 "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-                 "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-                 :: "r"(taddr),
-                    "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
-                    "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
-                    "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-                    "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15])),
-                    "r"(__float_as_uint(v[16])), "r"(__float_as_uint(v[17])), "r"(__float_as_uint(v[18])), "r"(__float_as_uint(v[19])),
-                    "r"(__float_as_uint(v[20])), "r"(__float_as_uint(v[21])), "r"(__float_as_uint(v[22])), "r"(__float_as_uint(v[23])),
-                    "r"(__float_as_uint(v[24])), "r"(__float_as_uint(v[25])), "r"(__float_as_uint(v[26])), "r"(__float_as_uint(v[27])),
-                    "r"(__float_as_uint(v[28])), "r"(__float_as_uint(v[29])), "r"(__float_as_uint(v[30])), "r"(__float_as_uint(v[31]))
-                 : "memory");
-}
-__device__ __forceinline__ float fast_exp2(float x)
-{
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ uint32_t pack_half2(float lo, float hi)
-{
-    __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t *>(&h);
-}
 // byte offset of 16-byte chunk c (0..15, 8 halves each) of row r in a [128][128] half tile
 __device__ __forceinline__ uint32_t tile_off(uint32_t r, uint32_t c)
 {
@@ -551,6 +420,7 @@ __global__ void __launch_bounds__(256) prefill_tc5_kernel(const Tc5Params p)
 
 constexpr int kSmemBytes = 6 * TILE + 1024;
 
+
 // ---- pipelined form ---------------------------------------------------------------------------------
 // Same tiles and the same arithmetic as prefill_tc5_kernel, with the two warpgroups running as two
 // independent pipelines over the shared K/V tiles:
@@ -563,17 +433,6 @@ constexpr int kSmemBytes = 6 * TILE + 1024;
 //   * each warpgroup's first thread issues that warpgroup's MMAs, so while one warpgroup computes
 //     its softmax the tensor pipe works for the other.
 // Barriers: 0,1 S complete (per Q tile)   2,3 P V complete   4,5 K/V buffer 0 / 1 ready.
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                 :: "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar)
-{
-    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" :: "r"(bar) : "memory");
-}
-
 template <int DT, bool CAP>
 __global__ void __launch_bounds__(256, 1) prefill_tc5p_kernel(const Tc5Params p)
 {
@@ -870,25 +729,6 @@ __global__ void __launch_bounds__(256, 1) prefill_tc5p_kernel(const Tc5Params p)
 // [tile][half] (1, commit)   K / V ready [buffer] (96)   K / V free [buffer] (1, commit).  Each
 // completes once per K/V tile (or once per two), so a wait on a phase parity is never more than
 // one phase away from the barrier's state.
-__host__ __device__ constexpr uint32_t idesc_f16_n(bool b_mn_major, uint32_t n)
-{
-    return (1u << 4) | (uint32_t(b_mn_major) << 16) | (uint32_t(n >> 3) << 17) | (uint32_t(128 >> 4) << 24);
-}
-
-// 64 columns of this thread's lane, loaded and waited for inside one statement: the compiler may
-// not touch the destination registers before the wait (it knows nothing of the load being
-// asynchronous).
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&v)[64])
-{
-    uint32_t r[64];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];\n\t"
-                 "tcgen05.wait::ld.sync.aligned;"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
-                 : "r"(taddr) : "memory");
-#pragma unroll
-    for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
-}
-
 // Bounded wait for a flag that another CTA of this (cooperative) launch sets; false after limit_ns.
 __device__ __forceinline__ bool flag_wait(const uint32_t *flag, uint32_t want, uint64_t limit_ns)
 {
@@ -1711,6 +1551,48 @@ bool spread_pays(const vfkv_ctx *ctx, const Tc5Params &p, uint64_t *total_out, u
 
 }  // namespace
 
+// Device scratch for pieces of row blocks: allocated at the first call outside a stream capture, owned by
+// the context; null where there is none (the caller then cuts nothing).
+float *prefill_scratch(vfkv_ctx *ctx, cudaStream_t st, uint64_t *floats)
+{
+    const uint32_t n_sm = uint32_t(ctx->sm_count);
+    const uint64_t n = uint64_t(n_sm) * 2 * CTA_ROWS * (HD + 2);
+    if (ctx->d_prefill_scratch == nullptr) {
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        cudaStreamIsCapturing(st, &capturing);
+        if (capturing != cudaStreamCaptureStatusNone) return nullptr;
+        void *d = nullptr;
+        // the pieces, then one flag per CTA
+        if (cudaMalloc(&d, n * sizeof(float) + n_sm * sizeof(uint32_t)) != cudaSuccess ||
+            cudaMemset(static_cast<float *>(d) + n, 0, n_sm * sizeof(uint32_t)) != cudaSuccess) {
+            (void)cudaGetLastError();
+            cudaFree(d);
+            return nullptr;
+        }
+        ctx->d_prefill_scratch = static_cast<float *>(d);
+        ctx->prefill_scratch_ctas = n_sm;
+    }
+    *floats = n;
+    return ctx->d_prefill_scratch;
+}
+
+// A byte-typed map of rows of row_bytes, boxes of 128 bytes x box_rows with the 128-byte swizzle.
+bool encode_rows_map(vfkv_ctx *ctx, CUtensorMap *out, const void *base, uint64_t row_bytes, uint32_t rows, uint32_t box_rows)
+{
+    typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                      const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                      CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    if (!ctx->encode_tiled) return false;
+    cuuint64_t dims[2] = {row_bytes, rows};
+    cuuint64_t strides[1] = {row_bytes};
+    cuuint32_t box[2] = {128, box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    return reinterpret_cast<EncodeTiledFn>(ctx->encode_tiled)(
+               out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool prefill_tc5_supported(uint32_t dtype, uint32_t head_dim, uint32_t group, bool has_scales)
 {
     return (dtype == VFKV_F8 || dtype == VFKV_F16) && head_dim == 128 && !has_scales && group != 0 && BM % group == 0;
@@ -1789,18 +1671,8 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
         uint32_t tj_max = 0;
         if (spread_pays(ctx, p, &total, &tj_max)) {
             cudaStreamIsCapturing(st, &capturing);
-            if (ctx->d_prefill_scratch == nullptr && capturing == cudaStreamCaptureStatusNone) {
-                const size_t bytes = size_t(n_sm) * 2 * CTA_ROWS * (HD + 2) * sizeof(float);
-                void *d = nullptr;
-                // the pieces, then one flag per CTA
-                if (cudaMalloc(&d, bytes + n_sm * sizeof(uint32_t)) == cudaSuccess &&
-                    cudaMemset(static_cast<uint8_t *>(d) + bytes, 0, n_sm * sizeof(uint32_t)) == cudaSuccess) {
-                    ctx->d_prefill_scratch = static_cast<float *>(d);
-                    ctx->prefill_scratch_ctas = n_sm;
-                } else {
-                    (void)cudaGetLastError();      // no room: one CTA per item
-                }
-            }
+            uint64_t floats = 0;
+            prefill_scratch(ctx, st, &floats);
             if (ctx->d_prefill_scratch != nullptr && ctx->prefill_scratch_ctas >= n_sm) {
                 spread = true;
                 p.total_tiles = uint32_t(total);
@@ -1857,22 +1729,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
         memset(&tm_k, 0, sizeof tm_k);
         memset(&tm_v, 0, sizeof tm_v);
         if (dtype == VFKV_F16 && ctx->encode_tiled != nullptr && n_kv != 0u) {
-            typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                              const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-            cuuint64_t dims[2] = {row_bytes, n_kv};
-            cuuint64_t strides[1] = {row_bytes};
-            cuuint32_t box[2] = {128, 128};
-            cuuint32_t estr[2] = {1, 1};
-            auto enc = reinterpret_cast<EncodeTiledFn>(ctx->encode_tiled);
-            const bool made =
-                enc(&tm_k, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(k), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS &&
-                enc(&tm_v, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(v), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-            p.use_tma = made ? 1u : 0u;
+            p.use_tma = encode_rows_map(ctx, &tm_k, k, row_bytes, n_kv, 128) && encode_rows_map(ctx, &tm_v, v, row_bytes, n_kv, 128) ? 1u : 0u;
         }
         typedef void (*Kernel)(const Tc5Params, const CUtensorMap, const CUtensorMap);
         const Kernel kerns[2][2][2] = {{{prefill_tc5h_kernel<VFKV_F8, false, false>, prefill_tc5h_kernel<VFKV_F8, false, true>},

@@ -19,9 +19,18 @@ struct PrefillParams {
 bool prefill_f32_supported(uint32_t head_dim);
 int32_t launch_prefill_f32(vfkv_ctx *ctx, uint32_t dtype, const PrefillParams &p, cudaStream_t st);
 
+// tcgen05 kernel with one Q tile of 128 rows a CTA (attn_prefill_tc5s.cu): F8 (scaled or not) and F16 rows of 64,
+// 128 or 256 dims, any group size.  split_q: F16 with Q as two half-precision terms (always for 64 and 256 dims)
+bool prefill_one_tile_supported(const vfkv_ctx *ctx, uint32_t dtype, uint32_t head_dim);
+int32_t launch_prefill_one_tile(vfkv_ctx *ctx, uint32_t dtype, bool split_q, const PrefillParams &p, cudaStream_t st);
+
+// shared by the tcgen05 kernels (attn_prefill_tc5.cu)
+float *prefill_scratch(vfkv_ctx *ctx, cudaStream_t st, uint64_t *floats);
+bool encode_rows_map(vfkv_ctx *ctx, CUtensorMap *out, const void *base, uint64_t row_bytes, uint32_t rows, uint32_t box_rows);
+
 #ifdef __CUDACC__
 // Visible range [lo, hi) of query i (flash_attn_batch.comp:116-119,141-144; window: per-query bound).
-__device__ __forceinline__ void query_range(const PrefillParams &p, uint32_t i, uint32_t *lo, uint32_t *hi)
+__host__ __device__ __forceinline__ void query_range(const PrefillParams &p, uint32_t i, uint32_t *lo, uint32_t *hi)
 {
     uint32_t c = p.q_start + i + 1u;
     if (c > p.n_kv) c = p.n_kv;

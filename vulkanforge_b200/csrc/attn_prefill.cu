@@ -7,8 +7,10 @@
 // query and head; here one CTA owns 64 rows = (64 / g) consecutive queries x the g q-heads of
 // one kv-head, so a K/V tile is fetched once per 64 rows, widened to half precision once
 // (FP8 caches; the kv_fp8_to_f16.comp step) and consumed by m16n8k16 tensor-core MMAs with the
-// usual online softmax.  Shapes outside that kernel take the f32 tiles of attn_prefill_f32.cu, or for
-// other head_dims and unaligned buffers a kernel with the reference's work split (one CTA per (query, head)).
+// usual online softmax.  Larger chunks take the tcgen05 kernels of attn_prefill_tc5.cu and
+// attn_prefill_tc5s.cu.  F32 caches, head_dim 512 and other odd shapes take the f32 tiles of
+// attn_prefill_f32.cu, or for other head_dims and unaligned buffers a kernel with the reference's work
+// split (one CTA per (query, head)).
 #include <cmath>
 
 #include "../../include/vfkv_next.h"
@@ -513,22 +515,36 @@ extern "C" int32_t vfkv_attend_prefill(vfkv_cache *cache, uint32_t layer, uint32
                         (dt == VFKV_F8 || dt == VFKV_F16) && (D == 64 || D == 128 || D == 256);
     if (ctx->attn_impl == 2 && !mma_ok)
         return set_error(ctx, VFKV_ERR_UNSUPPORTED, "vfkv_attend_prefill: shape outside the tensor-core kernel");
-    // The tcgen05 kernel works on 256-row blocks, one CTA per SM: it pays once those fill most of
-    // the GPU, or the context is long enough for it to cut the blocks' K/V tiles into even shares
-    // for all SMs (256 queries at position 60 000: 1955 us on the mma.sync kernel, 332 us), or
-    // for its faster tiles to outweigh its fixed cost; short chunks at short contexts keep the
-    // 64-row mma.sync kernel (four times the CTAs).  attn_impl 2 forces it.
     // F16 caches carry the error budget of the reference's f32 shader (2e-3 absolute): the tcgen05
     // kernel feeds Q as one half-precision value, which holds it (1e-4 .. 5e-4 measured) with the usual
     // 1/sqrt(head_dim) scale but not with scale 1.0 (1e-2: the Gemma-4 rule); those keep the
     // mma.sync kernel and its hi + lo split of Q.
     const bool tc5_accurate = dt == VFKV_F8 || scale * sqrtf(float(D)) <= 1.5f;
-    if (mma_ok && ctx->attn_impl != 3 && prefill_tc5_supported(dt, D, p.group, kv.k_scales != nullptr) && tc5_accurate &&
-        (ctx->attn_impl == 2 || prefill_tc5_pays(ctx, n_q_heads, hkv, m, q_start, n_kv, kv_start, window)))
+    const bool two_ok = mma_ok && ctx->attn_impl != 3 && prefill_tc5_supported(dt, D, p.group, false) && tc5_accurate;
+    // Three kernels do the same work in different portions, and the one whose model of the call is the
+    // shortest takes it: two Q tiles of 128 rows a CTA (attn_prefill_tc5.cu: large chunks; most work per K/V
+    // byte), one tile (attn_prefill_tc5s.cu: fewer rows, tiles cut over idle SMs, and the shapes the first
+    // does not hold), and 64 rows on mma.sync (a few positions: no tensor memory to set up).  Measured with
+    // the RoPE and append launches in front, 32 / 8 / 128 FP8, two tiles / one / mma.sync:
+    //   64 queries at 0: - / 11 / 9 us;  64 at 1936: 24 / 20 / 76;  16 at 30 000: 92 / 50 / -;
+    //   333 at 1000: 44 / 38 / -;  1000 at 3000: 133 / 139 / -;  2000 at 0: 94 / 107 / -
+    // attn_impl 2 and the tuning knob force the first where it holds the shape.
+    if (ctx->attn_impl == 0 && aligned && prefill_one_tile_supported(ctx, dt, D) && (kv.k_scales || mma_ok) &&
+        !(two_ok && ctx->tune_stages != 0)) {
+        const double one_us = prefill_one_tile_us(ctx, dt, !tc5_accurate, p);
+        const double two_us = two_ok ? prefill_tc5_us(ctx, n_q_heads, hkv, m, q_start, n_kv, kv_start, window) : 1e30;
+        const uint32_t last = q_start + m < n_kv ? q_start + m : n_kv;
+        const uint32_t seen = window && window + BM / p.group < last ? window + BM / p.group : last - (kv_start < last ? kv_start : last);
+        const double mma_us = mma_ok ? 3.0 + 2.2 * (D / 128.0) * ((seen + BN - 1) / BN) : 1e30;
+        if (one_us <= two_us && one_us < mma_us)
+            return launch_prefill_one_tile(ctx, dt, !tc5_accurate, p, st);
+        if (two_us < mma_us)
+            return launch_prefill_tc5(ctx, dt, p.k, p.v, d_q, d_out, p.row_bytes, n_q_heads, hkv, m, q_start, n_kv, kv_start,
+                                      window, scale, softcap, st);
+    } else if (two_ok && (ctx->attn_impl == 2 || ctx->attn_impl == 0)) {
         return launch_prefill_tc5(ctx, dt, p.k, p.v, d_q, d_out, p.row_bytes, n_q_heads, hkv, m, q_start, n_kv, kv_start,
                                   window, scale, softcap, st);
-    static const char *xone = getenv("XONE");
-    if (xone && aligned && ctx->attn_impl == 0 && prefill_one_tile_supported(ctx, dt, D)) return launch_prefill_one_tile(ctx, dt, !tc5_accurate, p, st);
+    }
     if (mma_ok) {
         if (dt == VFKV_F8) {
             if (D == 64) return launch_mma_d<VFKV_F8, 64>(ctx, p, st);

@@ -63,9 +63,6 @@ struct Tc5Params {
     uint32_t use_tma;                  // F16 rows, specialised form: K/V tiles by TMA through the two tensor maps
     uint64_t wait_ns;                  // time limit of the head CTA's wait for the other pieces
     uint32_t fail_cta;                 // failure injection (tests): this CTA never announces its piece
-    // specialised form, few items: the K/V tiles of an item are cut over a cluster of n_split CTAs, which
-    // put their O, reference maxima and sums together through distributed shared memory (n_cta == 0)
-    uint32_t n_split;
 };
 
 // byte offset of 16-byte chunk c (0..15, 8 halves each) of row r in a [128][128] half tile
@@ -744,23 +741,20 @@ __device__ __forceinline__ bool flag_wait(const uint32_t *flag, uint32_t want, u
     }
 }
 
-// CL: launched in clusters (n_split > 1); compiled apart because its code beside the other modes' made
-// those 7 % slower (2048 queries at 14 336: 725 -> 775 us).
-template <int DT, bool CAP, bool CL>
+template <int DT, bool CAP>
 __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p, const __grid_constant__ CUtensorMap tm_k,
                                                               const __grid_constant__ CUtensorMap tm_v)
 {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_bar[20];
     __shared__ uint32_t s_tmem, s_abort, s_seg[7];
-    __shared__ float s_ml[2 * CTA_ROWS];               // a cluster's piece: reference maxima and sums of the rows
     __shared__ uint32_t s_tj[kMaxRowBlocks], s_cl[kMaxRowBlocks];      // tiles and first position of every row block
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
     uint8_t *sm = smem_raw + (base - smem_addr(smem_raw));
     const uint32_t q_sm = base, k_sm = base + 2 * TILE, v_sm = base + 4 * TILE;
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
-    // One CTA per item (n_cta == 0): grid = (kv-heads x n_split, row blocks), the heaviest row blocks (latest
-    // queries) of every kv-head start first; n_split > 1: one cluster per item, a piece of it per CTA.  Work spread evenly (n_cta != 0): grid = n_cta, this CTA
+    // One CTA per item (n_cta == 0): grid = (kv-heads, row blocks), the heaviest row blocks (latest
+    // queries) of every kv-head start first.  Work spread evenly (n_cta != 0): grid = n_cta, this CTA
     // takes its share of the line of all items' tiles as a sequence of segments, each a run of
     // K/V tiles of one item; a segment that is a whole item writes the output rows, the first and
     // the last segment may be pieces of items and go to scratch for prefill_tc5_merge_kernel.
@@ -818,18 +812,7 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
             TC5H_STAMP(13);
             uint32_t live = 0u, kvh_ = 0u, row0_ = 0u, c_lo_ = 0u, nt_ = 0u, mode_ = 0u, more_ = 0u;
             if (p.n_cta == 0u) {
-                if (seg_i == 0u) {
-                    live = 1u;
-                    kvh_ = CL ? blockIdx.x / p.n_split : blockIdx.x;
-                    item_extent(p, blockIdx.y, &row0_, &c_lo_, &nt_);
-                    if constexpr (CL) {
-                        const uint32_t rank = blockIdx.x - kvh_ * p.n_split;
-                        const uint32_t a = nt_ * rank / p.n_split, e = nt_ * (rank + 1u) / p.n_split;
-                        c_lo_ += a * BN;
-                        nt_ = e - a;
-                        mode_ = 5u;
-                    }
-                }
+                if (seg_i == 0u) { live = 1u; kvh_ = blockIdx.x; item_extent(p, blockIdx.y, &row0_, &c_lo_, &nt_); }
             } else if (cur < t_end) {
                 uint32_t acc = 0u;
                 for (uint32_t rb = 0u; rb < p.n_rb; ++rb) {
@@ -842,7 +825,7 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
                         nt_ = min(tj - tin, t_end - cur);
                         row0_ = (p.n_rb - 1u - rb) * uint32_t(CTA_ROWS);
                         c_lo_ = s_cl[rb] + tin * BN;
-                        // (5: a cluster's piece)  0: a whole item; 1 / 2: a piece of one for the merge kernel, as this CTA's first / a
+                        // 0: a whole item; 1 / 2: a piece of one for the merge kernel, as this CTA's first / a
                         // later segment; 3: a piece that is not the item's head, for the CTA that holds the
                         // head; 4: the head, which waits for the more_ pieces of the next CTAs
                         if (tin == 0u && nt_ == tj) mode_ = 0u;
@@ -1017,7 +1000,7 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
             float *row_dst;
             float piece_scale[3] = {0.f, 0.f, 0.f};
             constexpr uint64_t PIECE = uint64_t(CTA_ROWS) * (HD + 2);
-            if (!CL && mode == 4u) {
+            if (mode == 4u) {
                 // the head of a cut item: the other pieces were the first work of the next CTAs
                 const uint32_t rl = wg * BM + t;
                 bool got = true;
@@ -1045,14 +1028,6 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
 #pragma unroll
                 for (uint32_t i = 0; i < 3u; ++i) piece_scale[i] *= inv;
                 row_dst = r_ok ? p.out + (uint64_t(q_idx) * p.n_q_heads + kvh * g + hj) * HD : nullptr;
-            } else if (CL) {
-                // a cluster's piece: O stays in shared memory as it is, with the reference maximum and the
-                // sum (negative: this CTA failed) beside it
-                const uint32_t rl = wg * BM + t;
-                s_ml[rl] = (ran && !failed) ? mref : kMaskedScore;
-                s_ml[CTA_ROWS + rl] = failed ? -1.f : ran ? lrow : 0.f;
-                row_scale = 1.0f;
-                row_dst = nullptr;
             } else if (mode != 0u) {
                 // a piece of an item: O as it stands, with the reference maximum (log2 units) and the sum
                 float *sc = p.scratch + (uint64_t(blockIdx.x) * 2u + (mode == 2u ? 1u : 0u)) * PIECE;
@@ -1083,7 +1058,6 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
                             make_float4(v[4 * j] * row_scale, v[4 * j + 1] * row_scale, v[4 * j + 2] * row_scale, v[4 * j + 3] * row_scale);
                 }
                 __syncwarp();
-                if (!CL) {
                 const unsigned long long mine = reinterpret_cast<unsigned long long>(row_dst);
 #pragma unroll 4
                 for (uint32_t r = 0; r < 32u; ++r) {
@@ -1101,7 +1075,6 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
                         }
                     }
                     if (dst != 0ull) *reinterpret_cast<float4 *>(reinterpret_cast<float *>(dst) + 4u * lane) = x;
-                }
                 }
                 __syncwarp();
             }
@@ -1304,79 +1277,6 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if constexpr (CL) {
-            // every CTA of the cluster has its piece in shared memory: CTA r merges the r-th rows (the
-            // reduce shader's update, flash_attn_reduce.comp:51-80, maximum first), a warp per row
-            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-            const uint32_t n = p.n_split, rank = blockIdx.x % n, lane = tid & 31u;
-            auto peer = [&](uint32_t addr, uint32_t i) {
-                uint32_t a;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(i));
-                return a;
-            };
-            const uint32_t r_end = min((rank + 1u) * uint32_t(CTA_ROWS) / n, n_rows > row0 ? n_rows - row0 : 0u);
-            constexpr uint32_t RU = 2u;         // rows of a warp in flight together; short code, for it runs once and is fetched cold
-            for (uint32_t r0 = rank * uint32_t(CTA_ROWS) / n + warp * RU; r0 < r_end; r0 += 12u * RU) {
-                float m[RU], l[RU], w[RU];                                // lane i: piece i
-#pragma unroll
-                for (uint32_t u = 0; u < RU; ++u) {
-                    m[u] = kMaskedScore; l[u] = 0.f;
-                    if (lane < n && r0 + u < r_end) {
-                        const uint32_t a = peer(smem_addr(s_ml + r0 + u), lane);
-                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(m[u]) : "r"(a) : "memory");
-                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l[u]) : "r"(a + 4u * uint32_t(CTA_ROWS)) : "memory");
-                    }
-                }
-#pragma unroll
-                for (uint32_t u = 0; u < RU; ++u) {
-                    float mx = m[u];
-#pragma unroll
-                    for (int d = 4; d >= 1; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));     // n <= 8
-                    mx = __shfl_sync(0xffffffffu, mx, 0);
-                    w[u] = fast_exp2(m[u] - mx);
-                    float sum = lane < n ? w[u] * l[u] : 0.f;
-#pragma unroll
-                    for (int d = 4; d >= 1; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-                    sum = __shfl_sync(0xffffffffu, sum, 0);
-                    w[u] *= (sum > 0.f && !__any_sync(0xffffffffu, l[u] < 0.f)) ? 1.0f / sum : 0.f;
-                }
-                // all pieces of both rows requested before the first is used: a remote access takes most of a
-                // microsecond here (one piece at a time, eight pieces: 8.5 us for the whole merge)
-                float4 x[RU][8];
-#pragma unroll
-                for (uint32_t i = 0; i < 8u; ++i)
-#pragma unroll
-                    for (uint32_t u = 0; u < RU; ++u) {
-                        const uint32_t rl = min(r0 + u, uint32_t(CTA_ROWS) - 1u);
-                        const uint32_t at = q_sm + (rl >> 5) * 16384u + (rl & 31u) * 512u + ((lane ^ rl) & 31u) * 16u;
-                        x[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (i < n)
-                            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                         : "=f"(x[u][i].x), "=f"(x[u][i].y), "=f"(x[u][i].z), "=f"(x[u][i].w) : "r"(peer(at, i)) : "memory");
-                    }
-                float4 o[RU];
-#pragma unroll
-                for (uint32_t u = 0; u < RU; ++u) {
-                    o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                    for (uint32_t i = 0; i < 8u; ++i) {
-                        const float wi = __shfl_sync(0xffffffffu, w[u], int(i));
-                        o[u].x = fmaf(wi, x[u][i].x, o[u].x); o[u].y = fmaf(wi, x[u][i].y, o[u].y);
-                        o[u].z = fmaf(wi, x[u][i].z, o[u].z); o[u].w = fmaf(wi, x[u][i].w, o[u].w);
-                    }
-                }
-#pragma unroll
-                for (uint32_t u = 0; u < RU; ++u) {
-                    const uint32_t rr = row0 + r0 + u;
-                    if (r0 + u < r_end)
-                        *reinterpret_cast<float4 *>(p.out + (uint64_t(rr / g) * p.n_q_heads + kvh * g + rr % g) * HD + 4u * lane) = o[u];
-                }
-            }
-            __syncwarp();
-            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // a peer may still be reading this CTA's memory
-            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-        }
         if (tid == 0) TC5H_STAMP(29);
         if (mode == 3u && tid == 0 && blockIdx.x != p.fail_cta) {
             // the piece is in scratch (every thread's stores are ordered before the barrier above)
@@ -1468,56 +1368,6 @@ __global__ void __launch_bounds__(256) prefill_tc5_merge_kernel(const Tc5Params 
     }
 }
 
-// Clusters of n CTAs of the specialised form that the device keeps resident at once (0: none).
-uint32_t max_clusters(const vfkv_ctx *ctx, uint32_t n)
-{
-    static std::atomic<int> known[64][9];       // per device; 0 = not asked yet, -1 = none
-    std::atomic<int> &k = known[ctx->device & 63][n];
-    int v = k.load(std::memory_order_acquire);
-    if (v == 0) {
-        v = -1;
-        auto kern = prefill_tc5h_kernel<VFKV_F8, false, true>;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(n);
-        cfg.blockDim = dim3(384);
-        cfg.dynamicSmemBytes = kSmemBytes;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = n; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int got = 0;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&got, kern, &cfg) == cudaSuccess && got > 0)
-            v = got;
-        (void)cudaGetLastError();
-        k.store(v, std::memory_order_release);
-    }
-    return v > 0 ? uint32_t(v) : 0u;
-}
-
-// CTAs of a cluster that an item's K/V tiles are cut over (1: not cut), by the model of a launch that
-// the measurements give: a CTA pays 8 us once and 3.5 us a tile, the merge in a cluster 4 us, and the
-// even shares over all SMs 45 us for their segments, pieces and second kernel and 2.8 us a tile -- they
-// only win where the items are long and clusters leave many SMs idle (8 items of 157 tiles: 64 CTAs of
-// 20 tiles against 148 of 8.5).  A cluster has to find its SMs in one GPC, so the device is asked how
-// many fit (74 of two CTAs, 45 of three, 33 of four, 15 of eight).  Measured: 333 F16 queries at 1000,
-// 48 items of 11 tiles in clusters of two, 47 -> 31 us; 36 at 7700, 8 of 61 in eights, 53 -> 41 with RoPE.
-uint32_t cluster_split(const vfkv_ctx *ctx, uint64_t items, uint32_t tj_max, uint64_t total)
-{
-    const uint32_t n_sm = uint32_t(ctx->sm_count);
-    if (items == 0 || items * 2 > n_sm || tj_max < 2) return 1;
-    auto cta_us = [](uint64_t tiles) { return 8.0 + 3.5 * double(tiles); };
-    double best = cta_us(tj_max);
-    uint32_t pick = 1;
-    for (uint32_t n = 2; n <= 8 && n <= tj_max && items * n <= n_sm; ++n) {
-        if (items > max_clusters(ctx, n)) continue;
-        const double us = cta_us((tj_max + n - 1) / n) + 4.0;
-        if (us < best) { best = us; pick = n; }
-    }
-    return 45.0 + 2.8 * double(total) / n_sm < best ? 1u : pick;
-}
-
 // Whether the even shares are allowed for this call and expected to pay; the sum of all items'
 // tiles and the longest item on the way.  p.n_rb is set.
 bool spread_pays(const vfkv_ctx *ctx, const Tc5Params &p, uint64_t *total_out, uint32_t *tj_max_out)
@@ -1538,8 +1388,6 @@ bool spread_pays(const vfkv_ctx *ctx, const Tc5Params &p, uint64_t *total_out, u
     *total_out = total;
     *tj_max_out = tj_max;
     const uint64_t waves = (items + n_sm - 1) / n_sm;
-    // Few items cut over clusters instead, where that is expected to be quicker
-    if (ctx->tune_stages == 0 && cluster_split(ctx, items, tj_max, total) > 1u) return false;
     // Items for at most half the SMs: shares of two tiles or more, if they shorten the longest CTA
     // by ten tiles (29 us) -- the shares' segments, the pieces and the merge kernel cost about half of
     // that (512 queries at 1024, 64 items of 12 tiles: 46 us one CTA an item, 56 us in shares of 5;
@@ -1598,31 +1446,30 @@ bool prefill_tc5_supported(uint32_t dtype, uint32_t head_dim, uint32_t group, bo
     return (dtype == VFKV_F8 || dtype == VFKV_F16) && head_dim == 128 && !has_scales && group != 0 && BM % group == 0;
 }
 
-bool prefill_tc5_pays(const vfkv_ctx *ctx, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m, uint32_t q_start,
+// Expected time (us): a CTA pays 8 us and 3.5 us a tile of 128 positions, the even shares 45 us (segments,
+// pieces, the merge) and 2.8 us a tile.  Measured: 1000 queries at 3000 (128 items of up to 32 tiles) 121 us;
+// 500 at 7500 (64 of 63, in shares) 131.
+double prefill_tc5_us(const vfkv_ctx *ctx, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m, uint32_t q_start,
                       uint32_t n_kv, uint32_t kv_start, uint32_t window)
 {
     Tc5Params p{};
     p.n_q_heads = n_q_heads; p.n_kv_heads = n_kv_heads; p.group = n_q_heads / n_kv_heads;
     p.m = m; p.q_start = q_start; p.n_kv = n_kv; p.kv_start = kv_start; p.window = window;
     p.n_rb = (m * p.group + CTA_ROWS - 1) / CTA_ROWS;
-    // 256-row blocks that fill most of the GPU
-    if (uint64_t(p.n_rb) * n_kv_heads * 4 >= uint64_t(ctx->sm_count) * 3) return true;
     uint64_t total = 0;
     uint32_t tj_max = 0;
-    if (p.n_rb > kMaxRowBlocks) return false;
-    if (spread_pays(ctx, p, &total, &tj_max)) return true;
-    if (cluster_split(ctx, uint64_t(p.n_rb) * n_kv_heads, tj_max, total) > 1u && tj_max >= 6) return true;
-    // Fewer blocks, one CTA each: a CTA pays about 12 us once and 2.9 us per 128 positions, the
-    // 64-row mma.sync kernel (four times the CTAs) 2.15 us per 64 positions -- measured on 64
-    // queries at 4096: 103 against 140 us, on 128 at 2048: 60 against 76 -- so from ten K/V tiles on
-    // the tcgen05 kernel is ahead even on a few SMs.
-    tj_max = 0;
     for (uint32_t rb = 0; rb < p.n_rb; ++rb) {
         uint32_t r0, cl, tj;
         item_extent(p, rb, &r0, &cl, &tj);
+        total += uint64_t(tj) * n_kv_heads;
         tj_max = std::max(tj_max, tj);
     }
-    return tj_max >= 10;
+    const double n_sm = double(ctx->sm_count), items = double(p.n_rb) * n_kv_heads;
+    double us = 8.0 + 3.5 * tj_max;
+    if (items > n_sm) us = std::max(us, 1.25 * (8.0 * items + 3.5 * double(total)) / n_sm);
+    uint64_t t2 = 0;
+    if (spread_pays(ctx, p, &t2, &tj_max)) us = std::min(us, 45.0 + 2.8 * double(total) / n_sm);
+    return us;
 }
 
 int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, const uint8_t *v, const float *q, float *out,
@@ -1697,33 +1544,17 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
     if ((ctx->tune_stages == 0 && (dtype == VFKV_F8 || f16_h)) || ctx->tune_stages == 3) {
         static bool configured_h[64] = {};
         if (!configured_h[ctx->device & 63]) {
-            const void *kernels[8] = {reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F8, false, false>),
-                                      reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F8, true, false>),
-                                      reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F16, false, false>),
-                                      reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F16, true, false>),
-                                      reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F8, false, true>),
-                                      reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F8, true, true>),
-                                      reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F16, false, true>),
-                                      reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F16, true, true>)};
+            const void *kernels[4] = {reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F8, false>),
+                                      reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F8, true>),
+                                      reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F16, false>),
+                                      reinterpret_cast<const void *>(prefill_tc5h_kernel<VFKV_F16, true>)};
             for (const void *kn : kernels) {
                 cudaError_t e = cudaFuncSetAttribute(kn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
                 if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(tcgen05 prefill attention)");
             }
             configured_h[ctx->device & 63] = true;
         }
-        p.n_split = 1;
-        if (!spread && ctx->tune_stages == 0) {
-            uint64_t total = 0;
-            uint32_t tj_max = 0;
-            for (uint32_t rb = 0; rb < p.n_rb; ++rb) {
-                uint32_t r0, cl, tj;
-                item_extent(p, rb, &r0, &cl, &tj);
-                total += uint64_t(tj) * n_kv_heads;
-                tj_max = std::max(tj_max, tj);
-            }
-            p.n_split = cluster_split(ctx, items, tj_max, total);
-        }
-        const dim3 grid_h = spread ? dim3(n_sm, 1, 1) : dim3(grid.y * p.n_split, grid.x);
+        const dim3 grid_h = spread ? dim3(n_sm, 1, 1) : dim3(grid.y, grid.x);
         // F16 rows by TMA: byte-typed maps of the slot's rows [0, n_kv), one row = one position
         CUtensorMap tm_k, tm_v;
         memset(&tm_k, 0, sizeof tm_k);
@@ -1731,12 +1562,8 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
         if (dtype == VFKV_F16 && ctx->encode_tiled != nullptr && n_kv != 0u) {
             p.use_tma = encode_rows_map(ctx, &tm_k, k, row_bytes, n_kv, 128) && encode_rows_map(ctx, &tm_v, v, row_bytes, n_kv, 128) ? 1u : 0u;
         }
-        typedef void (*Kernel)(const Tc5Params, const CUtensorMap, const CUtensorMap);
-        const Kernel kerns[2][2][2] = {{{prefill_tc5h_kernel<VFKV_F8, false, false>, prefill_tc5h_kernel<VFKV_F8, false, true>},
-                                        {prefill_tc5h_kernel<VFKV_F8, true, false>, prefill_tc5h_kernel<VFKV_F8, true, true>}},
-                                       {{prefill_tc5h_kernel<VFKV_F16, false, false>, prefill_tc5h_kernel<VFKV_F16, false, true>},
-                                        {prefill_tc5h_kernel<VFKV_F16, true, false>, prefill_tc5h_kernel<VFKV_F16, true, true>}}};
-        const Kernel kern = kerns[dtype == VFKV_F16][cap][p.n_split > 1u];
+        void (*kern)(const Tc5Params, const CUtensorMap, const CUtensorMap) = dtype == VFKV_F8 ? (cap ? prefill_tc5h_kernel<VFKV_F8, true> : prefill_tc5h_kernel<VFKV_F8, false>)
+                                                         : (cap ? prefill_tc5h_kernel<VFKV_F16, true> : prefill_tc5h_kernel<VFKV_F16, false>);
         if (spread && p.inline_merge != 0u) {
             // CTAs of this launch wait for one another's pieces: a cooperative launch, which the
             // driver accepts only if the whole grid is resident at once
@@ -1761,7 +1588,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
             (void)cudaGetLastError();          // not all resident: the pieces go to the merge kernel instead
             p.inline_merge = 0u;
         }
-        if (cudaError_t le = launch_clusters(ctx, kern, grid_h, dim3(384), kSmemBytes, st, p.n_split, p, tm_k, tm_v))
+        if (cudaError_t le = launch_dependent(ctx, kern, grid_h, dim3(384), kSmemBytes, st, p, tm_k, tm_v))
             return check_cuda(ctx, le, "tcgen05 prefill attention launch");
         ctx->count_launch();
         if (spread) {

@@ -54,7 +54,11 @@ template <int D, bool SPLITQ> struct OneTile {
     static constexpr uint32_t ROOM = 227 * 1024 - kSmall - Q, NST = ROOM / STAGE < 8 ? ROOM / STAGE : 8;
     static constexpr uint32_t NK = (NST + 1) / 2, NV = NST / 2;  // stages of K, stages of V behind them
     static constexpr uint32_t SMEM = Q + NST * STAGE + kSmall;
-    static constexpr uint32_t TMEM = D > 128 ? 512 : 256;       // S0, S1: 64 columns each; O: D columns from 128 on
+    // Columns of tensor memory: S of even and odd tiles, then O.  With 32 products a tile (256 dims, Q in two
+    // terms) those of S go to two accumulators in turn, which the softmax adds: MMAs into one wait for each
+    // other (1.85 -> 1.73 us a tile; with 16 products the addition costs as much as it saves).
+    static constexpr bool ACC2 = D > 128 && SPLITQ;
+    static constexpr uint32_t S_COLS = ACC2 ? 128 : 64, O_COL = 2 * S_COLS, TMEM = O_COL + D > 256 ? 512 : 256;
     static constexpr uint64_t PIECE = uint64_t(BM) * (D + 2);
 };
 
@@ -202,7 +206,7 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
         const bool r_ok = r < n_rows;
         uint32_t r_lo = 0u, r_hi = 0u;
         if (r_ok) query_range(p, r / g, &r_lo, &r_hi);
-        const uint32_t t_lane = (warp * 32u) << 16, tm_o = tmem + 128u + t_lane;
+        const uint32_t t_lane = (warp * 32u) << 16, tm_o = tmem + T::O_COL + t_lane;
         const float mult = SPLITQ ? s_mult[tid] : 1.0f, inv_cap = CAP ? 1.0f / p.softcap : 0.f;
         constexpr float GROW = SC ? 4.0f : 8.0f;
         float mref = kMaskedScore, lrow = 0.f;
@@ -237,11 +241,20 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
                 __syncwarp();
                 load_scales(it + 1);
             }
-            const uint32_t buf = it & 1u, tm_s = tmem + buf * 64u + t_lane, t0 = c_lo + it * BN;
+            const uint32_t buf = it & 1u, tm_s = tmem + buf * T::S_COLS + t_lane, t0 = c_lo + it * BN;
             if (!mbar_wait(bar(buf), (it >> 1) & 1u)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float s[64];
             tmem_ld64(tm_s, s);
+            if constexpr (T::ACC2) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float x[32];
+                    tmem_ld32(tm_s + 64u + 32u * h, x);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) s[32 * h + j] += x[j];
+                }
+            }
             if constexpr (SC) {
 #pragma unroll
                 for (int j = 0; j < 64; j += 4) {
@@ -369,25 +382,24 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
         // ================= the MMA thread ===================================================================
         if (lane == 0u && n_tiles > 0u) {
             auto issue_s = [&](uint32_t t) {
-                const uint32_t st = t % NK, b0 = ring + st * T::STAGE, d = tmem + (t & 1u) * 64u;
-#pragma unroll 1
+                const uint32_t st = t % NK, b0 = ring + st * T::STAGE, d = tmem + (t & 1u) * T::S_COLS;
                 for (uint32_t h = 0; h < (SPLITQ ? 2u : 1u); ++h) {
                     const uint32_t a0 = q_sm + h * T::QT;
 #pragma unroll
                     for (uint32_t ks = 0; ks < D / 16; ++ks)
-                        umma_f16(d, smem_desc(a0 + (ks >> 2) * SLAB_Q + (ks & 3u) * 32u, 16, 1024),
-                                 smem_desc(b0 + (ks >> 2) * SLAB_KV + (ks & 3u) * 32u, 16, 1024), idesc_f16(false, BN), h | ks);
+                        umma_f16(d + (T::ACC2 ? (ks & 1u) * 64u : 0u), smem_desc(a0 + (ks >> 2) * SLAB_Q + (ks & 3u) * 32u, 16, 1024),
+                                 smem_desc(b0 + (ks >> 2) * SLAB_KV + (ks & 3u) * 32u, 16, 1024), idesc_f16(false, BN), T::ACC2 ? h | (ks >> 1) : h | ks);
                 }
                 umma_commit(bar(t & 1u));
                 umma_commit(bar(free0 + st));
             };
             auto issue_pv = [&](uint32_t t) {
-                const uint32_t st = NK + t % NV, b0 = ring + st * T::STAGE, a0 = tmem + (t & 1u) * 64u;
+                const uint32_t st = NK + t % NV, b0 = ring + st * T::STAGE, a0 = tmem + (t & 1u) * T::S_COLS;
 #pragma unroll
                 for (uint32_t h = 0; h < (SC ? 2u : 1u); ++h)
 #pragma unroll
                     for (uint32_t kk = 0; kk < BN / 16; ++kk)
-                        umma_f16_ts(tmem + 128u, a0 + 32u * h + kk * 8u, smem_desc(b0 + kk * 2048u, SLAB_KV, 1024),
+                        umma_f16_ts(tmem + T::O_COL, a0 + 32u * h + kk * 8u, smem_desc(b0 + kk * 2048u, SLAB_KV, 1024),
                                     idesc_f16(true, D), t | h | kk);
                 umma_commit(bar(4u + (t & 1u)));
                 umma_commit(bar(free0 + st));
@@ -525,27 +537,36 @@ __global__ void __launch_bounds__(256) prefill_pieces_kernel(const OneTileParams
     }
 }
 
-// CTAs that the tiles of a row block are cut over, by a model of a launch: a CTA pays t0 once and t1 a
-// tile, pieces cost a second launch.
-uint32_t pieces_of(const vfkv_ctx *ctx, const PrefillParams &p, uint32_t n_rb, bool split_q, bool sc)
+// CTAs that the tiles of a row block are cut over, and the time of the launch (us), by a model of it: a CTA
+// pays t0 once and t1 a tile (measured, in us: 1.07 for FP8 and 0.87 for F16 rows of 128 dims, 1.31 and, with
+// Q in two terms, 1.75 for 256, 1.65 for scaled FP8 of 128), pieces cost a second launch and their traffic.
+struct Cut { uint32_t pieces; double us; };
+Cut best_cut(const vfkv_ctx *ctx, uint32_t dtype, bool split_q, const PrefillParams &p)
 {
-    static const char *env = getenv("XSPLIT"); if (env) return atoi(env);
+    const uint32_t D = p.head_dim, n_rb = uint32_t((uint64_t(p.m) * p.group + BM - 1) / BM);
     uint32_t longest = 0;
+    uint64_t total = 0;
     for (uint32_t rb = 0; rb < n_rb; ++rb) {
         uint32_t r0, cl, nt;
         block_extent(p, n_rb, rb, &r0, &cl, &nt);
         longest = std::max(longest, nt);
+        total += uint64_t(nt) * p.n_kv_heads;
     }
-    const double t0 = 9.0, t1 = (p.head_dim == 256 ? 1.3 : 1.0) + (split_q ? 0.4 : 0.0) * (p.head_dim / 128.0) + (sc ? 0.3 : 0.0), t_pieces = 6.0;
+    const bool sc = p.k_scales != nullptr;
+    const double t1 = (dtype == VFKV_F8 ? (D == 256 ? 1.31 : D == 128 ? 1.07 : 0.95) : 0.87) +
+                      (sc ? (D == 256 ? 0.9 : 0.6) : split_q ? (D == 256 ? 0.88 : D == 128 ? 0.2 : 0.0) : 0.0) + (p.softcap > 0.f ? 0.3 : 0.0);
+    const double t0 = D == 256 ? 9.0 : 7.0;
     const uint64_t items = uint64_t(n_rb) * p.n_kv_heads, n_sm = uint64_t(ctx->sm_count);
-    double best = 1e30;
-    uint32_t pick = 1;
+    Cut best{1, 1e30};
     for (uint32_t n = 1; n <= 64 && n <= std::max(longest, 1u); ++n) {
-        const double waves = double((items * n + n_sm - 1) / n_sm);
-        const double us = waves * (t0 + t1 * double((longest + n - 1) / n)) + (n > 1 ? t_pieces : 0.0);
-        if (us < best * 0.97) { best = us; pick = n; }
+        if (n > 1 && items * n > n_sm * 2) break;
+        const double one_cta = t0 + t1 * double((longest + n - 1) / n);
+        double us = one_cta;
+        if (items * n > n_sm) us = std::max(us, 1.25 * (t0 * double(items * n) + t1 * double(total)) / double(n_sm));
+        if (n > 1) us += 5.0 + 0.3 * n * D / 128.0;
+        if (us < best.us * 0.98) best = {n, us};
     }
-    return pick;
+    return best;
 }
 
 template <int DT, int D, bool SPLITQ, bool SC, bool CAP>
@@ -567,7 +588,7 @@ int32_t launch_one_tile_t(vfkv_ctx *ctx, OneTileParams op, cudaStream_t st)
         (!encode_rows_map(ctx, &tm_k, p.k, p.row_bytes, p.n_kv, BN) || !encode_rows_map(ctx, &tm_v, p.v, p.row_bytes, p.n_kv, BN)))
         return set_error(ctx, VFKV_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     op.n_rb = uint32_t((uint64_t(p.m) * p.group + BM - 1) / BM);
-    op.n_split = pieces_of(ctx, p, op.n_rb, SPLITQ, SC);
+    op.n_split = best_cut(ctx, DT, SPLITQ, p).pieces;
     if (op.n_split > 1) {
         uint64_t floats = 0;
         op.scratch = prefill_scratch(ctx, st, &floats);
@@ -606,6 +627,11 @@ int32_t launch_one_tile_d(vfkv_ctx *ctx, uint32_t dtype, bool split_q, const One
 bool prefill_one_tile_supported(const vfkv_ctx *ctx, uint32_t dtype, uint32_t D)
 {
     return (D == 64 || D == 128 || D == 256) && (dtype == VFKV_F8 || (dtype == VFKV_F16 && ctx->encode_tiled));
+}
+
+double prefill_one_tile_us(const vfkv_ctx *ctx, uint32_t dtype, bool split_q, const PrefillParams &p)
+{
+    return best_cut(ctx, dtype, split_q || (dtype == VFKV_F16 && p.head_dim != 128), p).us;
 }
 
 int32_t launch_prefill_one_tile(vfkv_ctx *ctx, uint32_t dtype, bool split_q, const PrefillParams &p, cudaStream_t st)

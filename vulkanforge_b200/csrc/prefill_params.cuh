@@ -24,6 +24,9 @@ int32_t launch_prefill_f32(vfkv_ctx *ctx, uint32_t dtype, const PrefillParams &p
 bool prefill_one_tile_supported(const vfkv_ctx *ctx, uint32_t dtype, uint32_t head_dim);
 int32_t launch_prefill_one_tile(vfkv_ctx *ctx, uint32_t dtype, bool split_q, const PrefillParams &p, cudaStream_t st);
 
+// expected time of the call, in us
+double prefill_one_tile_us(const vfkv_ctx *ctx, uint32_t dtype, bool split_q, const PrefillParams &p);
+
 // shared by the tcgen05 kernels (attn_prefill_tc5.cu)
 float *prefill_scratch(vfkv_ctx *ctx, cudaStream_t st, uint64_t *floats);
 bool encode_rows_map(vfkv_ctx *ctx, CUtensorMap *out, const void *base, uint64_t row_bytes, uint32_t rows, uint32_t box_rows);

@@ -742,11 +742,11 @@ __device__ __forceinline__ bool flag_wait(const uint32_t *flag, uint32_t want, u
 }
 
 template <int DT, bool CAP>
-__global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p, const __grid_constant__ CUtensorMap tm_k,
+__global__ void __launch_bounds__(416, 1) prefill_tc5h_kernel(const Tc5Params p, const __grid_constant__ CUtensorMap tm_k,
                                                               const __grid_constant__ CUtensorMap tm_v)
 {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t s_bar[20];
+    __shared__ __align__(8) uint64_t s_bar[22];
     __shared__ uint32_t s_tmem, s_abort, s_seg[7];
     __shared__ uint32_t s_tj[kMaxRowBlocks], s_cl[kMaxRowBlocks];      // tiles and first position of every row block
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
@@ -773,7 +773,8 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
         for (uint32_t i = 4; i < 8; ++i) mbar_init(bar(i), 128);
         for (uint32_t i = 8; i < 12; ++i) mbar_init(bar(i), 1);
         for (uint32_t i = 12; i < 16; ++i) mbar_init(bar(i), p.use_tma != 0u ? 1u : 96u);
-        for (uint32_t i = 16; i < 20; ++i) mbar_init(bar(i), 1);
+        for (uint32_t i = 16; i < 20; ++i) mbar_init(bar(i), 2);
+        for (uint32_t i = 20; i < 22; ++i) mbar_init(bar(i), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0u;
     }
@@ -794,7 +795,7 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
     if (p.n_cta != 0u) {
         // one thread walking the row blocks with item_extent (divisions, clamps) costs 0.8 us a row
         // block; all threads fill a table once, the walk then only adds
-        for (uint32_t rb = tid; rb < p.n_rb; rb += 384u) {
+        for (uint32_t rb = tid; rb < p.n_rb; rb += 416u) {
             uint32_t r0, cl, tj;
             item_extent(p, rb, &r0, &cl, &tj);
             s_tj[rb] = tj;
@@ -854,8 +855,8 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
         // Q tiles -> shared memory (half precision, scale folded in), all threads
         // by the nine warps that are not fetching K/V (those start on their first tiles meanwhile);
         // eight pieces a thread in flight at a time, two rounds.  g divides 128, so it is a power of two.
-        if (warp < 9u) {
-            constexpr uint32_t QT = 288u, QB = 8u;
+        if (warp < 10u) {
+            constexpr uint32_t QT = 320u, QB = 8u;
             const uint32_t g_shift = uint32_t(__ffs(int(g))) - 1u;
             for (uint32_t i0 = tid; i0 < uint32_t(CTA_ROWS * 16); i0 += QT * QB) {
                 float4 qa[QB], qb[QB];
@@ -877,7 +878,7 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
                 }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            asm volatile("bar.sync 1, 288;" ::: "memory");
+            asm volatile("bar.sync 1, 320;" ::: "memory");
         }
         if (tid == 0) TC5H_STAMP(14);
 #define TC5H_TRACE(slot)                                                                           \
@@ -902,12 +903,12 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
             for (uint32_t it = 0; it < n_tiles && ok; ++it) {
                 if (tid == 0) TC5H_TRACE(16);
                 const uint32_t gi = gt + it;
-                if (!mbar_wait(bar(wg), gi & 1u)) { ok = false; break; }
-                if (tid == 0 && it == 0u) TC5H_STAMP(15);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
                 for (uint32_t h = 0; h < 2u; ++h) {
                     const uint32_t t0 = c_lo + it * BN + h * 64u;
+                    if (!mbar_wait(bar(h * 20u + wg), gi & 1u)) { ok = false; break; }
+                    if (tid == 0 && it == 0u && h == 0u) TC5H_STAMP(15);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (tid == 0) TC5H_TRACE(17 + 4 * h);
                     float s[64];
                     tmem_ld64(tm_s + t_lane + 64u * h, s);
@@ -988,6 +989,7 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
             bool ran = n_tiles > 0 && ok;
             if (ran && !mbar_wait(bar(8u + wg * 2u + 1u), (gt + n_tiles - 1u) & 1u)) { *abort_flag = 1u; ran = false; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            asm volatile("bar.sync 2, 256;" ::: "memory");         // of the other Q tile as well: Q and K are free below
             const bool failed = *abort_flag != 0u;
             if (tid == 0) TC5H_STAMP(28);
             // The rows leave through shared memory so that a warp's store covers one row's 512 bytes (a
@@ -1078,116 +1080,52 @@ __global__ void __launch_bounds__(384, 1) prefill_tc5h_kernel(const Tc5Params p,
                 }
                 __syncwarp();
             }
-        } else if (warp == 8) {
-            // ================= the MMA thread ================================================================
+        } else if (warp < 10) {
+            // ================= the MMA threads, one per Q tile ==================================================
             if ((tid & 31u) == 0u && n_tiles > 0u) {
+                const uint32_t wg = warp - 8u;
                 bool ok = true;
-                // S of one Q tile in one piece (N = 128): two N = 64 products take twice the time
-                auto issue_s = [&](uint32_t wg, uint32_t b) {
+                // S of half h of a K/V tile (64 positions): its columns hold P of the tile before until the P V of
+                // that half, which is issued first (the MMAs of a thread run in order)
+                auto issue_s = [&](uint32_t gi, uint32_t h) {
+                    const uint32_t b = gi & 1u;
+                    if (h == 0u) {
+                        if (!mbar_wait(bar(12u + b), (gi >> 1) & 1u)) { ok = false; return; }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    }
 #pragma unroll
                     for (uint32_t ks = 0; ks < HD / 16; ++ks) {
                         const uint32_t o = (ks >> 2) * SLAB + (ks & 3u) * 32;
-                        umma_f16(tmem + wg * 128u, smem_desc(q_sm + wg * TILE + o, 16, 1024),
-                                 smem_desc(k_sm + b * TILE + o, 16, 1024), idesc_f16(false), ks);
+                        umma_f16(tmem + wg * 128u + 64u * h, smem_desc(q_sm + wg * TILE + o, 16, 1024),
+                                 smem_desc(k_sm + b * TILE + h * 8192u + o, 16, 1024), idesc_f16(false, 64), ks);
                     }
-                    umma_commit(bar(wg));
+                    umma_commit(bar(h * 20u + wg));
+                    if (h == 1u) umma_commit(bar(16u + b));
                 };
-                if (!mbar_wait(bar(12u + (gt & 1u)), (gt >> 1) & 1u)) ok = false;
-                if (ok) {
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    issue_s(0, gt & 1u); issue_s(1, gt & 1u);
-                    umma_commit(bar(16u + (gt & 1u)));
-                }
-                // Per K/V tile six groups of products: P V of (Q tile, half) x 4 and S of the next tile x 2.
-                // They are issued as their inputs arrive -- a look at the four P barriers in turn -- and
-                // not in a fixed order: in a fixed order (P V a0, a1, b0, then S0 alternating with P V
-                // b1, then S1) Q tile 0 waited for Q tile 1's softmax before its next S was issued
-                // (653 -> 643 us on 2048 queries at 14 336, 1258 -> 1234 at 30 000).  The S of the next
-                // tile for a Q tile goes right behind that Q tile's P V of half b (its S columns hold
-                // P until then; MMAs of one thread execute in order), alternating with a P V of the
-                // other Q tile when one is ready at that moment: consecutive MMAs into the same
-                // accumulator follow one another about every 60 ns, MMAs into different accumulators
-                // about every 40 ns (measured).  (Taking the ready groups of both Q tiles together whenever
-                // both are ready, their MMAs alternating, measured 627 -> 710 us: the two softmaxes then
-                // run in step and the tensor pipe idles while both compute; the stagger is what keeps it fed.)
+                issue_s(gt, 0u);
+                if (ok) issue_s(gt, 1u);
                 for (uint32_t it = 0; it < n_tiles && ok; ++it) {
                     const uint32_t gi = gt + it, b = gi & 1u;
-                    const bool more = it + 1u < n_tiles;
-                    auto pv_step = [&](uint32_t wg, uint32_t h, uint32_t kk) {
-                        umma_f16_ts(tmem + 256u + wg * 128u, tmem + wg * 128u + 64u * h + kk * 8u,
-                                    smem_desc(v_sm + b * TILE + (4u * h + kk) * 2048u, SLAB, 1024), idesc_f16(true),
-                                    (it | h | kk) != 0u ? 1u : 0u);
-                    };
-                    auto s_step = [&](uint32_t wg, uint32_t bb, uint32_t ks) {
-                        const uint32_t o = (ks >> 2) * SLAB + (ks & 3u) * 32;
-                        umma_f16(tmem + wg * 128u, smem_desc(q_sm + wg * TILE + o, 16, 1024),
-                                 smem_desc(k_sm + bb * TILE + o, 16, 1024), idesc_f16(false), ks);
-                    };
-                    TC5H_TRACE(0);
                     if (!mbar_wait(bar(14u + b), (gi >> 1) & 1u)) { ok = false; break; }
-                    bool k_next = !more;
-                    uint32_t todo = 0xFu;                  // bit h * 2 + wg: P V of (Q tile wg, half h) not issued yet
-                    uint64_t t_idle = 0;
-                    uint32_t idle = 0;
-                    while (todo != 0u && ok) {
-                        bool did = false;
 #pragma unroll 1
-                        for (uint32_t wg = 0; wg < 2u && ok; ++wg) {
-                            const uint32_t h = ((todo >> wg) & 1u) ? 0u : 1u;            // half a before half b
-                            if (((todo >> (h * 2u + wg)) & 1u) == 0u) continue;
-                            if (!mbar_test(bar(4u + wg * 2u + h), gi & 1u)) continue;
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            did = true;
+                    for (uint32_t h = 0; h < 2u && ok; ++h) {
+                        if (!mbar_wait(bar(4u + wg * 2u + h), gi & 1u)) { ok = false; break; }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                            for (uint32_t kk = 0; kk < 4u; ++kk) pv_step(wg, h, kk);
-                            umma_commit(bar(8u + wg * 2u + h));
-                            todo &= ~(1u << (h * 2u + wg));
-                            if (h == 0u || !more) continue;
-                            // S of the next K/V tile for this Q tile: its S columns are free behind the P V
-                            // just issued.  Alternating with a P V of the other Q tile if one is ready now.
-                            if (!k_next) {
-                                if (!mbar_wait(bar(12u + (b ^ 1u)), ((gi + 1u) >> 1) & 1u)) { ok = false; break; }
-                                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                                k_next = true;
-                            }
-                            const uint32_t other = wg ^ 1u, ho = ((todo >> other) & 1u) ? 0u : 1u;
-                            const bool pair = ((todo >> (ho * 2u + other)) & 1u) != 0u && mbar_test(bar(4u + other * 2u + ho), gi & 1u);
-                            if (pair) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                            for (uint32_t ks = 0; ks < HD / 16; ++ks) {
-                                s_step(wg, b ^ 1u, ks);
-                                if (pair && ks < 4u) pv_step(other, ho, ks);
-                            }
-                            if (pair) {
-                                umma_commit(bar(8u + other * 2u + ho));
-                                todo &= ~(1u << (ho * 2u + other));
-                            }
-                            umma_commit(bar(wg));
-                            if (pair && ho == 1u) {
-#pragma unroll
-                                for (uint32_t ks = 0; ks < HD / 16; ++ks) s_step(other, b ^ 1u, ks);
-                                umma_commit(bar(other));
-                            }
-                        }
-                        if (!did) {
-                            if ((++idle & 1023u) == 0u) {
-                                if (t_idle == 0) t_idle = timer_ns();
-                                else if (timer_ns() - t_idle > 1000000000ull) ok = false;
-                            }
-                        } else {
-                            idle = 0; t_idle = 0;
-                        }
+                        for (uint32_t kk = 0; kk < 4u; ++kk)
+                            umma_f16_ts(tmem + 256u + wg * 128u, tmem + wg * 128u + 64u * h + kk * 8u,
+                                        smem_desc(v_sm + b * TILE + (4u * h + kk) * 2048u, SLAB, 1024), idesc_f16(true),
+                                        (it | h | kk) != 0u ? 1u : 0u);
+                        umma_commit(bar(8u + wg * 2u + h));
+                        if (h == 1u) umma_commit(bar(18u + b));
+                        if (it + 1u < n_tiles) issue_s(gi + 1u, h);
                     }
-                    if (!ok) break;
-                    umma_commit(bar(18u + b));
-                    if (more) umma_commit(bar(16u + (b ^ 1u)));
-                    TC5H_TRACE(12);
                 }
                 if (!ok) *abort_flag = 1u;
             }
         } else {
             // ================= K/V tiles: fetch, widen, place (96 threads) =====================================
-            const uint32_t pt = tid - 288u;
+            const uint32_t pt = tid - 320u;
             constexpr uint32_t ES = DT == VFKV_F8 ? 1u : 2u;
             constexpr uint32_t PIECES = DT == VFKV_F8 ? 1024u : 2048u;          // 16-byte pieces of one K (or V) tile
             constexpr int NP = DT == VFKV_F8 ? 11 : 11;                          // pieces per thread and pass
@@ -1573,7 +1511,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
             p.fail_cta = ctx->debug_fail_split;
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = grid_h;
-            cfg.blockDim = dim3(384);
+            cfg.blockDim = dim3(416);
             cfg.dynamicSmemBytes = kSmemBytes;
             cfg.stream = st;
             cudaLaunchAttribute attr[1];
@@ -1588,7 +1526,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
             (void)cudaGetLastError();          // not all resident: the pieces go to the merge kernel instead
             p.inline_merge = 0u;
         }
-        if (cudaError_t le = launch_dependent(ctx, kern, grid_h, dim3(384), kSmemBytes, st, p, tm_k, tm_v))
+        if (cudaError_t le = launch_dependent(ctx, kern, grid_h, dim3(416), kSmemBytes, st, p, tm_k, tm_v))
             return check_cuda(ctx, le, "tcgen05 prefill attention launch");
         ctx->count_launch();
         if (spread) {

@@ -741,10 +741,16 @@ __device__ __forceinline__ bool flag_wait(const uint32_t *flag, uint32_t want, u
     }
 }
 
+// Threads of the specialised form: 8 softmax warps, 2 that issue MMAs, and the rest for K/V rows.  Registers are
+// handed out per quarter of the SM: 13 warps get as few (128) as 16 do, so FP8 rows, which have to be widened,
+// have six warps; F16 rows come by TMA (the two warps are for drivers without tensor maps) and leave 168.
+template <int DT> constexpr uint32_t kThreadsH = DT == VFKV_F8 ? 512 : 384;
+
 template <int DT, bool CAP>
-__global__ void __launch_bounds__(416, 1) prefill_tc5h_kernel(const Tc5Params p, const __grid_constant__ CUtensorMap tm_k,
+__global__ void __launch_bounds__(kThreadsH<DT>, 1) prefill_tc5h_kernel(const Tc5Params p, const __grid_constant__ CUtensorMap tm_k,
                                                               const __grid_constant__ CUtensorMap tm_v)
 {
+    constexpr uint32_t PT = kThreadsH<DT> - 320u;         // threads that fetch rows
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_bar[22];
     __shared__ uint32_t s_tmem, s_abort, s_seg[7];
@@ -772,7 +778,7 @@ __global__ void __launch_bounds__(416, 1) prefill_tc5h_kernel(const Tc5Params p,
         for (uint32_t i = 0; i < 4; ++i) mbar_init(bar(i), 1);
         for (uint32_t i = 4; i < 8; ++i) mbar_init(bar(i), 128);
         for (uint32_t i = 8; i < 12; ++i) mbar_init(bar(i), 1);
-        for (uint32_t i = 12; i < 16; ++i) mbar_init(bar(i), p.use_tma != 0u ? 1u : 96u);
+        for (uint32_t i = 12; i < 16; ++i) mbar_init(bar(i), p.use_tma != 0u ? 1u : PT);
         for (uint32_t i = 16; i < 20; ++i) mbar_init(bar(i), 2);
         for (uint32_t i = 20; i < 22; ++i) mbar_init(bar(i), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -795,7 +801,7 @@ __global__ void __launch_bounds__(416, 1) prefill_tc5h_kernel(const Tc5Params p,
     if (p.n_cta != 0u) {
         // one thread walking the row blocks with item_extent (divisions, clamps) costs 0.8 us a row
         // block; all threads fill a table once, the walk then only adds
-        for (uint32_t rb = tid; rb < p.n_rb; rb += 416u) {
+        for (uint32_t rb = tid; rb < p.n_rb; rb += kThreadsH<DT>) {
             uint32_t r0, cl, tj;
             item_extent(p, rb, &r0, &cl, &tj);
             s_tj[rb] = tj;
@@ -1124,12 +1130,12 @@ __global__ void __launch_bounds__(416, 1) prefill_tc5h_kernel(const Tc5Params p,
                 if (!ok) *abort_flag = 1u;
             }
         } else {
-            // ================= K/V tiles: fetch, widen, place (96 threads) =====================================
+            // ================= K/V tiles: fetch, widen, place =====================================
             const uint32_t pt = tid - 320u;
             constexpr uint32_t ES = DT == VFKV_F8 ? 1u : 2u;
             constexpr uint32_t PIECES = DT == VFKV_F8 ? 1024u : 2048u;          // 16-byte pieces of one K (or V) tile
-            constexpr int NP = DT == VFKV_F8 ? 11 : 11;                          // pieces per thread and pass
-            constexpr int PASSES = DT == VFKV_F8 ? 1 : 2;
+            constexpr int PASSES = DT == VFKV_F8 ? 1 : 4;
+            constexpr int NP = int((PIECES / PASSES + PT - 1) / PT);             // pieces per thread and pass
             const uint8_t *kg = p.k + uint64_t(kvh) * HD * ES, *vg = p.v + uint64_t(kvh) * HD * ES;
             bool ok = true;
             auto move = [&](const uint8_t *src, uint32_t t0, uint32_t tile_sm, uint32_t free_bar, uint32_t gi) {
@@ -1139,7 +1145,7 @@ __global__ void __launch_bounds__(416, 1) prefill_tc5h_kernel(const Tc5Params p,
                     uint4 raw[NP];
 #pragma unroll
                     for (int i = 0; i < NP; ++i) {
-                        const uint32_t idx = pt + 96u * uint32_t(i) + uint32_t(pass) * (96u * NP);
+                        const uint32_t idx = pt + PT * uint32_t(i) + uint32_t(pass) * (PT * NP);
                         const uint32_t pos = DT == VFKV_F8 ? idx >> 3 : idx >> 4, c = DT == VFKV_F8 ? idx & 7u : idx & 15u;
                         const bool in = idx < PIECES && t0 + pos < p.n_kv;
                         const uint64_t off = uint64_t(in ? t0 + pos : 0u) * p.row_bytes + c * 16;
@@ -1149,7 +1155,7 @@ __global__ void __launch_bounds__(416, 1) prefill_tc5h_kernel(const Tc5Params p,
                     if (pass == 0 && gi >= 2u && !mbar_wait(free_bar, ((gi >> 1) & 1u) ^ 1u)) ok = false;
 #pragma unroll
                     for (int i = 0; i < NP; ++i) {
-                        const uint32_t idx = pt + 96u * uint32_t(i) + uint32_t(pass) * (96u * NP);
+                        const uint32_t idx = pt + PT * uint32_t(i) + uint32_t(pass) * (PT * NP);
                         if (idx >= PIECES) continue;
                         if constexpr (DT == VFKV_F8) {
                             const uint32_t pos = idx >> 3, c16 = idx & 7u;
@@ -1511,7 +1517,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
             p.fail_cta = ctx->debug_fail_split;
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = grid_h;
-            cfg.blockDim = dim3(416);
+            cfg.blockDim = dim3(dtype == VFKV_F8 ? kThreadsH<VFKV_F8> : kThreadsH<VFKV_F16>);
             cfg.dynamicSmemBytes = kSmemBytes;
             cfg.stream = st;
             cudaLaunchAttribute attr[1];
@@ -1526,7 +1532,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
             (void)cudaGetLastError();          // not all resident: the pieces go to the merge kernel instead
             p.inline_merge = 0u;
         }
-        if (cudaError_t le = launch_dependent(ctx, kern, grid_h, dim3(416), kSmemBytes, st, p, tm_k, tm_v))
+        if (cudaError_t le = launch_dependent(ctx, kern, grid_h, dim3(dtype == VFKV_F8 ? kThreadsH<VFKV_F8> : kThreadsH<VFKV_F16>), kSmemBytes, st, p, tm_k, tm_v))
             return check_cuda(ctx, le, "tcgen05 prefill attention launch");
         ctx->count_launch();
         if (spread) {

@@ -532,7 +532,7 @@ extern "C" int32_t vfkv_attend_prefill(vfkv_cache *cache, uint32_t layer, uint32
     if (ctx->attn_impl == 0 && aligned && prefill_one_tile_supported(ctx, dt, D) && (kv.k_scales || mma_ok) &&
         !(two_ok && ctx->tune_stages != 0)) {
         const double one_us = prefill_one_tile_us(ctx, dt, !tc5_accurate, p);
-        const double two_us = two_ok ? prefill_tc5_us(ctx, n_q_heads, hkv, m, q_start, n_kv, kv_start, window) : 1e30;
+        const double two_us = two_ok ? prefill_tc5_us(ctx, dt, n_q_heads, hkv, m, q_start, n_kv, kv_start, window) : 1e30;
         const uint32_t last = q_start + m < n_kv ? q_start + m : n_kv;
         const uint32_t seen = window && window + BM / p.group < last ? window + BM / p.group : last - (kv_start < last ? kv_start : last);
         double mma_us = mma_ok ? 3.0 + 2.2 * (D / 128.0) * ((seen + BN - 1) / BN) : 1e30;

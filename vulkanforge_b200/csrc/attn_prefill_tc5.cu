@@ -1312,33 +1312,37 @@ __global__ void __launch_bounds__(256) prefill_tc5_merge_kernel(const Tc5Params 
     }
 }
 
-// Whether the even shares are allowed for this call and expected to pay; the sum of all items'
-// tiles and the longest item on the way.  p.n_rb is set.
-bool spread_pays(const vfkv_ctx *ctx, const Tc5Params &p, uint64_t *total_out, uint32_t *tj_max_out)
+// The tiles of all items and of the longest one (p.n_rb is set), the time of the call with one CTA an item,
+// and whether even shares are allowed and expected to pay.  The model: an item costs 12 us and 3.0 a tile (FP8
+// rows; 2.6 F16), more items than SMs a quarter over the mean for the last wave; even shares cost 45 us (40)
+// once -- their segments, the pieces and the merge -- and 3.0 (2.55) a tile.
+struct TwoTileCost { uint64_t total; uint32_t longest; double us; bool even; };
+TwoTileCost two_tile_cost(const vfkv_ctx *ctx, uint32_t dtype, const Tc5Params &p)
 {
-    if (!(ctx->tune_stages == 0 || ctx->tune_stages == 3) || ctx->tune_warps == 4 || p.n_rb > kMaxRowBlocks ||
-        p.kv_start >= std::min(p.q_start + 1u, p.n_kv))
-        return false;
-    const uint32_t n_sm = uint32_t(ctx->sm_count);
-    const uint64_t items = uint64_t(p.n_rb) * p.n_kv_heads;
-    uint64_t total = 0;
-    uint32_t tj_max = 0;
+    TwoTileCost c{};
+    const uint64_t items = uint64_t(p.n_rb) * p.n_kv_heads, n_sm = uint64_t(ctx->sm_count);
     for (uint32_t rb = 0; rb < p.n_rb; ++rb) {
         uint32_t r0, cl, tj;
         item_extent(p, rb, &r0, &cl, &tj);
-        total += uint64_t(tj) * p.n_kv_heads;
-        tj_max = std::max(tj_max, tj);
+        c.total += uint64_t(tj) * p.n_kv_heads;
+        c.longest = std::max(c.longest, tj);
     }
-    *total_out = total;
-    *tj_max_out = tj_max;
-    const uint64_t waves = (items + n_sm - 1) / n_sm;
-    // Items for at most half the SMs: shares of two tiles or more, if they shorten the longest CTA
-    // by ten tiles (29 us) -- the shares' segments, the pieces and the merge kernel cost about half of
-    // that (512 queries at 1024, 64 items of 12 tiles: 46 us one CTA an item, 56 us in shares of 5;
-    // 256 queries at 2048, 32 items of 18: 63 against 54; 256 at 8192, 32 of 66: 193 against 85).
-    const bool few = items * 2 <= n_sm && uint64_t(tj_max) >= total / n_sm + 10;
-    const bool worth = ctx->tune_warps == 8 || few || (items * 20 < waves * n_sm * 19 && total >= items * 96);
-    return worth && n_sm >= 2 && total >= uint64_t(n_sm) * (few ? 2 : 8) && total < (1ull << 31);
+    const bool f8 = dtype == VFKV_F8;
+    const double tile = f8 ? 3.0 : 2.6;
+    c.us = 12.0 + tile * c.longest;
+    if (items > n_sm) c.us = std::max(c.us, 1.25 * (12.0 * double(items) + tile * double(c.total)) / double(n_sm));
+    if ((ctx->tune_stages == 0 || ctx->tune_stages == 3) && ctx->tune_warps != 4 && p.n_rb <= kMaxRowBlocks &&
+        p.kv_start < std::min(p.q_start + 1u, p.n_kv) && n_sm >= 2 && c.total >= n_sm * 2 && c.total < (1ull << 31)) {
+        const double even_us = (f8 ? 45.0 : 40.0) + (f8 ? 3.0 : 2.55) * double(c.total) / double(n_sm);
+        // few items: where that is faster by a twentieth; more of them than half the SMs: where the last wave is part
+        // empty and an item has 96 tiles or more (1500 queries at 8000, 192 items of 57: 314 us one CTA an item, 322
+        // in shares; 4096 at 4096, 512 items of 17: several segments a CTA, twice the time)
+        const uint64_t waves = (items + n_sm - 1) / n_sm;
+        c.even = ctx->tune_warps == 8 || (items * 2 <= n_sm && even_us < 0.95 * c.us) ||
+                 (items * 20 < waves * n_sm * 19 && c.total >= items * 96);
+        if (c.even) c.us = even_us;
+    }
+    return c;
 }
 
 }  // namespace
@@ -1393,27 +1397,14 @@ bool prefill_tc5_supported(uint32_t dtype, uint32_t head_dim, uint32_t group, bo
 // Expected time (us): a CTA pays 8 us and 3.5 us a tile of 128 positions, the even shares 45 us (segments,
 // pieces, the merge) and 2.8 us a tile.  Measured: 1000 queries at 3000 (128 items of up to 32 tiles) 121 us;
 // 500 at 7500 (64 of 63, in shares) 131.
-double prefill_tc5_us(const vfkv_ctx *ctx, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m, uint32_t q_start,
-                      uint32_t n_kv, uint32_t kv_start, uint32_t window)
+double prefill_tc5_us(const vfkv_ctx *ctx, uint32_t dtype, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m,
+                      uint32_t q_start, uint32_t n_kv, uint32_t kv_start, uint32_t window)
 {
     Tc5Params p{};
     p.n_q_heads = n_q_heads; p.n_kv_heads = n_kv_heads; p.group = n_q_heads / n_kv_heads;
     p.m = m; p.q_start = q_start; p.n_kv = n_kv; p.kv_start = kv_start; p.window = window;
     p.n_rb = (m * p.group + CTA_ROWS - 1) / CTA_ROWS;
-    uint64_t total = 0;
-    uint32_t tj_max = 0;
-    for (uint32_t rb = 0; rb < p.n_rb; ++rb) {
-        uint32_t r0, cl, tj;
-        item_extent(p, rb, &r0, &cl, &tj);
-        total += uint64_t(tj) * n_kv_heads;
-        tj_max = std::max(tj_max, tj);
-    }
-    const double n_sm = double(ctx->sm_count), items = double(p.n_rb) * n_kv_heads;
-    double us = 8.0 + 3.5 * tj_max;
-    if (items > n_sm) us = std::max(us, 1.25 * (8.0 * items + 3.5 * double(total)) / n_sm);
-    uint64_t t2 = 0;
-    if (spread_pays(ctx, p, &t2, &tj_max)) us = std::min(us, 45.0 + 2.8 * double(total) / n_sm);
-    return us;
+    return two_tile_cost(ctx, dtype, p).us;
 }
 
 int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, const uint8_t *v, const float *q, float *out,
@@ -1458,23 +1449,22 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
     bool spread = false;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     {
-        uint64_t total = 0;
-        uint32_t tj_max = 0;
-        if (spread_pays(ctx, p, &total, &tj_max)) {
+        const TwoTileCost cost = two_tile_cost(ctx, dtype, p);
+        if (cost.even) {
             cudaStreamIsCapturing(st, &capturing);
             uint64_t floats = 0;
             prefill_scratch(ctx, st, &floats);
             if (ctx->d_prefill_scratch != nullptr && ctx->prefill_scratch_ctas >= n_sm) {
                 spread = true;
-                p.total_tiles = uint32_t(total);
+                p.total_tiles = uint32_t(cost.total);
                 p.n_cta = n_sm;
                 p.scratch = ctx->d_prefill_scratch;
                 p.flags = reinterpret_cast<uint32_t *>(p.scratch + size_t(n_sm) * 2 * CTA_ROWS * (HD + 2));
                 // An item is cut into at most ceil(longest item / smallest share) + 1 pieces.  A
                 // captured launch would replay with the flag value of the capture, which the flags
                 // still hold from the replay before: those go through the merge kernel.
-                const uint64_t share = total / n_sm;
-                p.inline_merge = ((tj_max + share - 1) / share <= 3 && capturing == cudaStreamCaptureStatusNone) ? 1u : 0u;
+                const uint64_t share = cost.total / n_sm;
+                p.inline_merge = ((cost.longest + share - 1) / share <= 3 && capturing == cudaStreamCaptureStatusNone) ? 1u : 0u;
             }
         }
     }

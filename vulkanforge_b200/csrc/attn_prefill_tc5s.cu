@@ -540,6 +540,8 @@ __global__ void __launch_bounds__(256) prefill_pieces_kernel(const OneTileParams
 // CTAs that the tiles of a row block are cut over, and the time of the launch (us), by a model of it: a CTA
 // pays t0 once and t1 a tile (measured, in us: 1.07 for FP8 and 0.87 for F16 rows of 128 dims, 1.31 and, with
 // Q in two terms, 1.75 for 256, 1.65 for scaled FP8 of 128), pieces cost a second launch and their traffic.
+// CTAs beyond one an SM share its tensor cores and issue slots: the SMs that got one more set the time (700 queries
+// at 20 000, F16: 176 CTAs take twice one CTA's time).
 struct Cut { uint32_t pieces; double us; };
 Cut best_cut(const vfkv_ctx *ctx, uint32_t dtype, bool split_q, const PrefillParams &p)
 {
@@ -562,7 +564,8 @@ Cut best_cut(const vfkv_ctx *ctx, uint32_t dtype, bool split_q, const PrefillPar
         if (n > 1 && items * n > n_sm * 2) break;
         const double one_cta = t0 + t1 * double((longest + n - 1) / n);
         double us = one_cta;
-        if (items * n > n_sm) us = std::max(us, 1.25 * (t0 * double(items * n) + t1 * double(total)) / double(n_sm));
+        if (items * n > n_sm)
+            us = std::max(us, double((items * n + n_sm - 1) / n_sm) * (t0 + t1 * double(total) / double(items * n)));
         if (n > 1) us += 5.0 + 0.3 * n * D / 128.0;
         if (us < best.us * 0.98) best = {n, us};
     }

@@ -315,7 +315,7 @@ int32_t launch_merge_partials_packed(vfkv_ctx *ctx, const float *packed, uint32_
 // prefill attention on tcgen05 (attn_prefill_tc5.cu); k / v point at the slot's rows of the layer
 bool prefill_tc5_supported(uint32_t dtype, uint32_t head_dim, uint32_t group, bool has_scales);
 // expected time of the call, in us
-double prefill_tc5_us(const vfkv_ctx *ctx, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m, uint32_t q_start,
+double prefill_tc5_us(const vfkv_ctx *ctx, uint32_t dtype, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m, uint32_t q_start,
                       uint32_t n_kv, uint32_t kv_start, uint32_t window);
 int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, const uint8_t *v, const float *q, float *out,
                            uint64_t row_bytes, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m, uint32_t q_start,

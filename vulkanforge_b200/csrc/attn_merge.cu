@@ -142,7 +142,8 @@ uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile)
     // HBM-bound, so a ragged last wave costs little, while every extra split costs a partial
     // write, a ticket and a merge.  Smaller grids are cut until about two CTAs per SM exist, but
     // never below 256 positions per split.
-    const uint64_t base = uint64_t(a.seq.units()) * a.kv.n_kv_heads;
+    const uint32_t parts = tile >= 128 ? attn_mma_parts(a.kv.dtype, a.n_q_heads / a.kv.n_kv_heads) : 1u;
+    const uint64_t base = uint64_t(a.seq.units()) * a.kv.n_kv_heads * parts;
     const uint64_t slots = uint64_t(ctx->sm_count) * 2;
     // (an 8-warp CTA of the tensor-core kernel takes 8 tiles at a time: 256 positions of an FP8
     // cache, 128 of an F16 cache, where 16 splits of 128 measured 6.2 us against 6.6 us with 8 of 256
@@ -223,7 +224,8 @@ int32_t launch_attention(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, c
             return set_error(ctx, VFKV_ERR_INVALID, "workspace too small for this call");
         // the workspace is sized for max_splits of each sequence of one layer; a launch of several layers shares it out
         if (a.seq.n_layers > 1) {
-            const uint64_t g = a.n_q_heads / a.kv.n_kv_heads, groups = uint64_t(a.seq.units()) * a.kv.n_kv_heads;
+            const uint32_t parts = use_mma ? attn_mma_parts(a.kv.dtype, a.n_q_heads / a.kv.n_kv_heads) : 1u;
+            const uint64_t groups = uint64_t(a.seq.units()) * a.kv.n_kv_heads * parts, g = a.n_q_heads / (a.kv.n_kv_heads * parts);
             const uint64_t most = use_mma ? (groups <= ws->n_counters ? ws->tag_words / (groups * (g * (a.kv.head_dim + 2) + 2)) : 1)
                                           : uint64_t(ws->max_seqs) * ws->max_splits / a.seq.units();
             if (n_splits > most) n_splits = most > 1 ? uint32_t(most) : 1u;

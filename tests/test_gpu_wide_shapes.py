@@ -16,6 +16,13 @@ pytestmark = pytest.mark.gpu
     ("F8", True, 32, 2, 128, [129, 31], 0, 0.0, 2),
     ("F16", False, 34, 2, 128, [600], 0, 0.0, 0),
     ("F16", False, 24, 1, 64, [65, 64], 0, 50.0, 1),
+    # 512-dim heads and 64-dim FP8 rows: tiles of 128 positions (64 for F16)
+    ("F8", False, 16, 2, 512, [1, 128, 1029], 0, 0.0, 0),
+    ("F8", True, 10, 1, 512, [300, 129], 0, 0.0, 2),
+    ("F16", False, 16, 2, 512, [64, 65, 700], 100, 50.0, 0),
+    ("F16", False, 2, 2, 512, [2000], 0, 0.0, 1),
+    ("F8", False, 8, 8, 64, [1, 2500, 127], 0, 0.0, 0),
+    ("F8", True, 24, 2, 64, [129, 31], 0, 30.0, 0),
 ])
 def test_wide_shapes_match_the_cuda_core_kernel(ctx, dtype, scaled, hq, hkv, d, lens, window, softcap, n_splits):
     import torch

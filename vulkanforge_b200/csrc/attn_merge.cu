@@ -231,8 +231,9 @@ int32_t launch_attention(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, c
             if (n_splits > most) n_splits = most > 1 ? uint32_t(most) : 1u;
         }
     }
-    int32_t rc = use_mma ? launch_attn_mma(ctx, ws, a, n_splits, st)
-                         : launch_attn_generic(ctx, ws, a, n_splits, st);
+    int32_t rc = use_mma                                              ? launch_attn_mma(ctx, ws, a, n_splits, st)
+                 : ctx->attn_impl == 0 && attn_wide_supported(a) ? launch_attn_wide(ctx, ws, a, n_splits, st)
+                                                                      : launch_attn_generic(ctx, ws, a, n_splits, st);
     if (rc != VFKV_OK) return rc;
     // the tensor-core kernel merges its own partials (last CTA of each kv-head)
     if (n_splits > 1 && !use_mma) rc = launch_merge_ws(ctx, ws, a, n_splits, st);

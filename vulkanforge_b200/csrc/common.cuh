@@ -331,6 +331,9 @@ uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile);
 int32_t launch_attn_generic(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits,
                             cudaStream_t st);
 bool attn_mma_supported(const AttnArgs &a);
+bool attn_wide_supported(const AttnArgs &a);
+int32_t launch_attn_wide(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits,
+                         cudaStream_t st);
 uint32_t attn_mma_parts(uint32_t dtype, uint32_t g);
 bool encode_layer_maps(vfkv_ctx *ctx, const KvView &v, uint32_t n_layers, void *tm_k_out, void *tm_v_out);
 int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits,

@@ -26,13 +26,27 @@ merge_kernel(const float *__restrict__ pm, const float *__restrict__ pl, const f
         orow = uint64_t(lr.layer_ids[i]) * lr.per_layer + (blockIdx.x - i * lr.per_layer);
     }
     pdl_wait();
-    constexpr int kMaxDims = 4;                      // 128 threads x 4 = head_dim 512
-    __shared__ float s_red[4], s_sum[4];
+    __shared__ float s_red[4], s_sum[4], s_acc[4][128];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // The shader walks the partials with a running (max, sum, acc); the same result, up to
     // rounding, comes from taking the maximum first and then one weighted sum, which leaves
     // every load independent of the others.  The launch is a chain of L2 round trips and nothing
-    // else, so it is kept to two: the maxima and sums (one or two parts per thread), then the o rows.
+    // else: a warp takes four parts at a time (its first four are on their way behind the maximum), lane: dims
+    // lane + 32 j of the block's 128, every load unconditional.  (One thread a dim walking all parts, with a
+    // condition on the dim, serialised them: 64 parts of 16 rows of 512, 59 us.)
+    constexpr int U = 4;
+    float pv[U][4], pw[U];
+    auto fetch = [&](uint32_t i0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t i = min(i0 + u, n_parts - 1);
+            pw[u] = pm[uint64_t(i) * ml_part + row * ml_row];
+            const float *const o = po + uint64_t(i) * o_part + row * o_row;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) pv[u][j] = o[min(blockIdx.y * 128 + lane + 32 * j, head_dim - 1)];
+        }
+    };
+    fetch(warp * U);
     float gmax = kMaskedScore;
     float m_own[2] = {kMaskedScore, kMaskedScore}, l_own[2] = {0.f, 0.f};      // parts tid and tid + 128
 #pragma unroll
@@ -59,30 +73,30 @@ merge_kernel(const float *__restrict__ pm, const float *__restrict__ pl, const f
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) gsum += __shfl_xor_sync(0xffffffffu, gsum, o);
     if (lane == 0) s_sum[warp] = gsum;
-    float acc[kMaxDims] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 16
-    for (uint32_t i = 0; i < n_parts; ++i) {
-        const uint64_t oi = uint64_t(i) * o_part + row * o_row;
-        const float kn = __expf(pm[uint64_t(i) * ml_part + row * ml_row] - gmax);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (uint32_t i0 = warp * U; i0 < n_parts; i0 += 4 * U) {
+        if (i0 != warp * U) fetch(i0);
 #pragma unroll
-        for (int j = 0; j < kMaxDims; ++j) {
-            uint32_t d = threadIdx.x + j * 128;
-            float t = d < head_dim ? po[oi + d] : 0.f;
-            acc[j] = fmaf(t, kn, acc[j]);
+        for (int u = 0; u < U; ++u) {
+            if (i0 + u < n_parts) {
+                const float kn = __expf(pw[u] - gmax);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[j] = fmaf(pv[u][j], kn, acc[j]);
+            }
         }
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s_acc[warp][lane + 32 * j] = acc[j];
     __syncthreads();
     gsum = (s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]);
     const float inv = gsum > 0.f ? 1.0f / gsum : 0.f;   // an empty range yields zeros, not NaN
-#pragma unroll
-    for (int j = 0; j < kMaxDims; ++j) {
-        uint32_t d = threadIdx.x + j * 128;
-        if (d < head_dim) {
-            if (out) out[orow * head_dim + d] = acc[j] * inv;
-            if (out_o) out_o[orow * head_dim + d] = acc[j];
-        }
+    const uint32_t t = threadIdx.x, d = blockIdx.y * 128 + t;
+    const float o = (s_acc[0][t] + s_acc[1][t]) + (s_acc[2][t] + s_acc[3][t]);
+    if (d < head_dim) {
+        if (out) out[orow * head_dim + d] = o * inv;
+        if (out_o) out_o[orow * head_dim + d] = o;
     }
-    if (out_o && threadIdx.x == 0) { out_m[orow] = gmax; out_l[orow] = gsum; }
+    if (out_o && d == 0) { out_m[orow] = gmax; out_l[orow] = gsum; }
 }
 
 int32_t launch_merge_ws(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits,
@@ -96,7 +110,7 @@ int32_t launch_merge_ws(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, ui
     }
     ProfScope ps(ctx, VFKV_PROF_FA_REDUCE, st);
     const uint64_t D = a.kv.head_dim;
-    const cudaError_t e = launch_dependent(ctx, merge_kernel, dim3(rows), dim3(128), 0, st, ws->part_m, ws->part_l, ws->part_o,
+    const cudaError_t e = launch_dependent(ctx, merge_kernel, dim3(rows, (a.kv.head_dim + 127) / 128), dim3(128), 0, st, ws->part_m, ws->part_l, ws->part_o,
                                            n_splits, uint64_t(1), uint64_t(n_splits), D, n_splits * D, a.kv.head_dim, a.out,
                                            a.out_m, a.out_l, a.out_o, lr);
     ctx->count_launch(a.seq.n_layers);
@@ -109,7 +123,7 @@ int32_t launch_merge_partials(vfkv_ctx *ctx, const float *m, const float *l, con
 {
     if (n_rows == 0) return VFKV_OK;
     ProfScope ps(ctx, VFKV_PROF_FA_REDUCE, st);
-    merge_kernel<<<n_rows, 128, 0, st>>>(m, l, o, n_parts, n_rows, 1, uint64_t(n_rows) * head_dim, head_dim,
+    merge_kernel<<<dim3(n_rows, (head_dim + 127) / 128), 128, 0, st>>>(m, l, o, n_parts, n_rows, 1, uint64_t(n_rows) * head_dim, head_dim,
                                         head_dim, out, nullptr, nullptr, nullptr, LayerRows{});
     ctx->count_launch();
     return check_cuda(ctx, cudaGetLastError(), "merge_partials launch");
@@ -123,7 +137,7 @@ int32_t launch_merge_partials_packed(vfkv_ctx *ctx, const float *packed, uint32_
     if (n_rows == 0) return VFKV_OK;
     const uint64_t block = uint64_t(n_rows) * (head_dim + 2);
     ProfScope ps(ctx, VFKV_PROF_FA_REDUCE, st);
-    merge_kernel<<<n_rows, 128, 0, st>>>(packed, packed + n_rows, packed + 2 * uint64_t(n_rows), n_parts, block, 1,
+    merge_kernel<<<dim3(n_rows, (head_dim + 127) / 128), 128, 0, st>>>(packed, packed + n_rows, packed + 2 * uint64_t(n_rows), n_parts, block, 1,
                                         block, head_dim, head_dim, out, nullptr, nullptr, nullptr, LayerRows{});
     ctx->count_launch();
     return check_cuda(ctx, cudaGetLastError(), "merge_partials_packed launch");
@@ -156,7 +170,8 @@ uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile)
     // The CTA that merges reads every split's partial: beyond 16 splits that tail costs more than
     // the extra CTAs save (one sequence of 16384 positions, 64 q-heads: 15.9 us with 16 splits,
     // 19.5 us with 37), unless the length rule below asks for more.
-    if (want > 16) want = 16;
+    // (The wide-row kernel -- tile 64 -- leaves the merge to a launch with a CTA for each row.)
+    if (want > 16 && tile != 64) want = 16;
     // Fewer than eight groups (one long sequence whose kv-heads are spread over several GPUs): the
     // merge is then shared by up to sixteen CTAs of the group, each combining its outputs with a
     // team of lanes, and one CTA per SM pays: 148 / groups splits.
@@ -214,9 +229,9 @@ int32_t launch_attention(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, c
     const bool mma_ok = attn_mma_supported(a);
     if (ctx->attn_impl == 2 && !mma_ok)
         return set_error(ctx, VFKV_ERR_UNSUPPORTED, "shape outside the tensor-core attention kernel");
-    const bool use_mma = mma_ok && ctx->attn_impl != 1;
+    const bool use_mma = mma_ok && ctx->attn_impl != 1, use_wide = !mma_ok && ctx->attn_impl == 0 && attn_wide_supported(a);
 
-    uint32_t n_splits = a.n_splits ? a.n_splits : choose_splits(ctx, a, use_mma ? 128 : 32);
+    uint32_t n_splits = a.n_splits ? a.n_splits : choose_splits(ctx, a, use_mma ? 128 : use_wide ? 64 : 32);
     if (n_splits > 1) {
         if (!ws) return set_error(ctx, VFKV_ERR_INVALID, "a workspace is required when n_splits > 1");
         if (n_splits > ws->max_splits) n_splits = ws->max_splits;
@@ -231,9 +246,9 @@ int32_t launch_attention(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, c
             if (n_splits > most) n_splits = most > 1 ? uint32_t(most) : 1u;
         }
     }
-    int32_t rc = use_mma                                              ? launch_attn_mma(ctx, ws, a, n_splits, st)
-                 : ctx->attn_impl == 0 && attn_wide_supported(a) ? launch_attn_wide(ctx, ws, a, n_splits, st)
-                                                                      : launch_attn_generic(ctx, ws, a, n_splits, st);
+    int32_t rc = use_mma    ? launch_attn_mma(ctx, ws, a, n_splits, st)
+                 : use_wide ? launch_attn_wide(ctx, ws, a, n_splits, st)
+                            : launch_attn_generic(ctx, ws, a, n_splits, st);
     if (rc != VFKV_OK) return rc;
     // the tensor-core kernel merges its own partials (last CTA of each kv-head)
     if (n_splits > 1 && !use_mma) rc = launch_merge_ws(ctx, ws, a, n_splits, st);

@@ -15,7 +15,7 @@
 //           dims of a 512-dim head, along the positions of a 64-dim one).  Lane tig takes positions 4 tig .. 4 tig + 3
 //           of a block of 16, lane gid 8 consecutive dims of each; a byte permute pairs positions.
 //   The next tile's K rows are loaded behind the first product, its V rows behind the second, so one of the two is
-//   always in flight; 64 registers a lane each at 512 bytes a row, which leaves one CTA an SM.
+//   always in flight: 32 registers a lane each, two CTAs an SM (short rows: two tiles of each instead).
 #include "attn_params.cuh"
 #include "mma_sync.cuh"
 #include "softcap.cuh"
@@ -29,7 +29,8 @@ constexpr int kWarps = 8;
 template <int DT, int D> struct Wide {
     static constexpr int ES = DT == VFKV_F8 ? 1 : 2;
     static constexpr int ROW = D * ES;                       // bytes of a head's row
-    static constexpr int T = ROW > 512 ? 64 : 128;           // positions of a tile
+    static constexpr int T = ROW > 512 ? 32 : ROW > 256 ? 64 : 128;     // positions of a tile: 32 KB of rows or less
+    static constexpr int NBUF = ROW > 256 ? 1 : 2;           // tiles of K and of V in registers or on their way there
     static constexpr int DP = kWarps / (T / 16);             // warps along the dims in the first product
     static constexpr int E = 16 / ES;                        // dims of a lane's 16 bytes
     static constexpr int NU = ROW / 64 / DP;                 // 64-byte units of a row a warp contracts over
@@ -71,7 +72,7 @@ template <int DT, int VW> __device__ __forceinline__ void v_fragment(const uint3
 }
 
 template <int DT, int D>
-__global__ void __launch_bounds__(kWarps * 32, D == 64 ? 3 : 1)
+__global__ void __launch_bounds__(kWarps * 32, 2)
 attn_wide_kernel(const AttnParams p)
 {
     using W = Wide<DT, D>;
@@ -101,8 +102,8 @@ attn_wide_kernel(const AttnParams p)
     const uint8_t *const vb = p.v + head_at + (dg * 64 + gid * 8) * W::ES;
 
     // rows past the range are read as its last one; their P is zero
-    uint4 kr[W::NU][2];
-    auto load_k = [&](uint32_t t) {
+    uint4 kr[W::NBUF][W::NU][2];
+    auto load_k = [&](uint32_t t, uint4 (&kr)[W::NU][2]) {
         const uint32_t t0 = begin + t * W::T + pg * 16 + gid;
         const uint8_t *const r0 = kb + uint64_t(min(t0, end - 1)) * row_bytes, *const r1 = kb + uint64_t(min(t0 + 8, end - 1)) * row_bytes;
 #pragma unroll
@@ -111,8 +112,8 @@ attn_wide_kernel(const AttnParams p)
             kr[u][1] = *reinterpret_cast<const uint4 *>(r1 + u * 64);
         }
     };
-    uint32_t vr[W::PB][4][W::VW];
-    auto load_v = [&](uint32_t t) {
+    uint32_t vr[W::NBUF][W::PB][4][W::VW];
+    auto load_v = [&](uint32_t t, uint32_t (&vr)[W::PB][4][W::VW]) {
 #pragma unroll
         for (int b = 0; b < W::PB; ++b)
 #pragma unroll
@@ -128,7 +129,23 @@ attn_wide_kernel(const AttnParams p)
                 }
             }
     };
-    if (n_tiles) { load_k(0); load_v(0); }
+    const float *const ksc = p.k_scales ? p.k_scales + uint64_t(slot) * p.slot_stride_scales + kvh : nullptr;
+    const float *const vsc = p.v_scales ? p.v_scales + uint64_t(slot) * p.slot_stride_scales + kvh : nullptr;
+    float ks_next[4], vs_next[4];            // scales of the next tile's positions 4 lane .. 4 lane + 3
+    auto load_scales = [&](uint32_t t) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t pos = begin + t * W::T + 4 * lane + i;
+            const bool ok = lane < uint32_t(W::T / 4) && pos < end;
+            ks_next[i] = ok ? ksc[uint64_t(pos) * p.n_kv_heads] : 1.f;
+            vs_next[i] = ok ? vsc[uint64_t(pos) * p.n_kv_heads] : 0.f;
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < W::NBUF; ++i)
+        if (uint32_t(i) < n_tiles) { load_k(i, kr[i]); load_v(i, vr[i]); }
+    const bool scaled = DT == VFKV_F8 && ksc != nullptr;
+    if (scaled && n_tiles) load_scales(0);
 
     // Q: head `warp`, scaled by a power of two (largest element in [128, 256)), as B fragments
     float mult;
@@ -164,8 +181,6 @@ attn_wide_kernel(const AttnParams p)
     }
     __syncthreads();
 
-    const float *const ksc = p.k_scales ? p.k_scales + uint64_t(slot) * p.slot_stride_scales + kvh : nullptr;
-    const float *const vsc = p.v_scales ? p.v_scales + uint64_t(slot) * p.slot_stride_scales + kvh : nullptr;
     const float inv_cap = p.softcap > 0.f ? 1.0f / p.softcap : 0.f;
     float m = kMaskedScore, l = 0.f;         // head `warp`
     uint32_t vs_ref = 0u;                    // exponent that the V scales of the accumulators are relative to
@@ -173,7 +188,7 @@ attn_wide_kernel(const AttnParams p)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
 
-    for (uint32_t t = 0; t < n_tiles; ++t) {
+    auto tile = [&](uint32_t t, uint4 (&kr)[W::NU][2], uint32_t (&vr)[W::PB][4][W::VW]) {
         const uint32_t t0 = begin + t * W::T;
         // ---- S^T = K Q^T for 16 positions; four chains of products ----
         {
@@ -195,7 +210,7 @@ attn_wide_kernel(const AttnParams p)
 #pragma unroll
             for (int i = 0; i < 4; ++i) out[(i & 1) * W::S_PITCH + (i >> 1) * 8] = (s[0][i] + s[2][i]) + (s[1][i] + s[3][i]);
         }
-        if (t + 1 < n_tiles) load_k(t + 1);
+        if (t + W::NBUF < n_tiles) load_k(t + W::NBUF, kr);
         __syncthreads();
 
         // ---- softmax of head `warp`; lane: positions 4 lane .. 4 lane + 3 ----
@@ -206,23 +221,20 @@ attn_wide_kernel(const AttnParams p)
             if (mine) {
                 const float4 a = *reinterpret_cast<const float4 *>(ss + warp * W::S_PITCH + 4 * lane);
                 x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-                if constexpr (W::DP == 2) {
-                    const float4 b = *reinterpret_cast<const float4 *>(ss + (8 + warp) * W::S_PITCH + 4 * lane);
+#pragma unroll
+                for (int i = 1; i < W::DP; ++i) {
+                    const float4 b = *reinterpret_cast<const float4 *>(ss + (8 * i + warp) * W::S_PITCH + 4 * lane);
                     x[0] += b.x; x[1] += b.y; x[2] += b.z; x[3] += b.w;
                 }
             } else {
                 x[0] = x[1] = x[2] = x[3] = 0.f;
             }
             float vs[4] = {kPScale, kPScale, kPScale, kPScale}, vs_corr = 1.f;
-            if (DT == VFKV_F8 && ksc) {
+            if (scaled) {
                 float top = 0.f;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const bool ok = mine && pos + i < end;
-                    x[i] *= ok ? ksc[uint64_t(pos + i) * p.n_kv_heads] : 1.f;
-                    vs[i] = ok ? vsc[uint64_t(pos + i) * p.n_kv_heads] : 0.f;
-                    top = fmaxf(top, vs[i]);
-                }
+                for (int i = 0; i < 4; ++i) { x[i] *= ks_next[i]; vs[i] = vs_next[i]; top = fmaxf(top, vs[i]); }
+                if (t + 1 < n_tiles) load_scales(t + 1);
                 // powers of two relative to the largest scale so far; scales are at least 1e-12 and at most 2^119
                 const uint32_t top_e = __reduce_max_sync(0xffffffffu, __float_as_uint(top)) & 0x7f800000u;
                 if (top_e > vs_ref) {
@@ -280,7 +292,12 @@ attn_wide_kernel(const AttnParams p)
                 }
             }
         }
-        if (t + 1 < n_tiles) load_v(t + 1);
+        if (t + W::NBUF < n_tiles) load_v(t + W::NBUF, vr);
+    };
+    for (uint32_t t = 0; t < n_tiles; t += W::NBUF) {
+#pragma unroll
+        for (int i = 0; i < W::NBUF; ++i)
+            if (t + i < n_tiles) tile(t + i, kr[i], vr[i]);
     }
 
     // ---- epilogue: maxima and sums by head, then this warp's 64 dims (after a sum over the warps of a 64-dim head) ----

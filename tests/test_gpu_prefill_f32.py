@@ -1,5 +1,5 @@
 """The f32 tiles of chunked prefill (attn_prefill_f32.cu): every cache type at the edges of its tiles
-(64 rows, 64 positions), its clusters (a block's tiles cut over 1, 2, 4 or 8 CTAs) and its masks."""
+(64 rows, 64 positions), its shares (a block's tiles cut over several CTAs, several blocks in one) and its masks."""
 import numpy as np
 import pytest
 
@@ -15,7 +15,7 @@ ODT = {"F32": oracle.F32, "F16": oracle.F16, "F8": oracle.F8, "F8s": oracle.F32}
     ("F32", 32, 8, 128, 1, 0, 0, 0, 0.0),          # one row block of four rows, one position
     ("F32", 32, 8, 128, 16, 47, 0, 0, 0.0),        # exactly one tile of rows and one of positions
     ("F32", 32, 8, 128, 17, 48, 0, 0, 0.0),        # one more of each
-    ("F32", 8, 1, 128, 20, 900, 0, 0, 0.0),        # three blocks: clusters of eight
+    ("F32", 8, 1, 128, 20, 900, 0, 0, 0.0),        # three blocks, a tile a CTA
     ("F32", 8, 8, 64, 70, 300, 0, 100, 30.0),      # g = 1, head_dim 64, window, soft-cap
     ("F32", 10, 2, 256, 33, 500, 7, 0, 0.0),       # g = 5 does not tile 64 rows
     ("F32", 16, 2, 512, 40, 130, 0, 0, 0.0),
@@ -25,7 +25,7 @@ ODT = {"F32": oracle.F32, "F16": oracle.F16, "F8": oracle.F8, "F8s": oracle.F32}
     ("F8", 24, 8, 128, 50, 200, 0, 0, 50.0),
     ("F8s", 32, 8, 128, 100, 333, 0, 0, 0.0),      # a scale for each position and head
     ("F8s", 16, 8, 256, 30, 1000, 0, 256, 50.0),
-    ("F8s", 64, 8, 128, 300, 700, 0, 0, 0.0),      # enough blocks for one CTA each
+    ("F8s", 64, 8, 128, 300, 700, 0, 0, 0.0),      # several blocks a CTA
 ])
 def test_f32_tiles_match_the_oracle(ctx, dtype, hq, hkv, d, m, q_start, kv_start, window, softcap):
     import torch

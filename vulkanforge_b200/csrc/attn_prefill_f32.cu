@@ -11,9 +11,12 @@
 //   PV: thread = 8 rows x 4 dims; 3 16-byte shared loads for 32 FMAs.
 // Both keep the FMA pipe, not shared memory, as the bound (74 TFLOP/s at 1.96 GHz).
 //
-// A chunk of a short prompt has few row blocks (200 queries x 4 heads x 8 kv-heads: 104), so the K/V
-// tiles of a block may be cut over a cluster of 2, 4 or 8 CTAs, which merge their (m, l, O) through
-// distributed shared memory: no scratch, no second launch.
+// Row blocks are few and uneven (200 queries x 4 heads x 8 kv-heads: 104 blocks of 8 to 11 tiles), and an SM is
+// at its rate only with two CTAs on it, so the tiles of all (row block, kv-head) items form one line of which every
+// resident CTA takes an even share.  An item that a share ends in goes to scratch in pieces, which a second kernel
+// puts together.  200 queries at 700 positions, F32: 119 us with a CTA or a cluster of two an item, whose second
+// CTAs sat on 60 of 148 SMs; 85 in even shares.  Sixteen rows a warp, four warps a CTA (fewer shared loads a product)
+// were faster only from about 1000 positions on (200 at 1500: 153 against 160; 368 at 368: 84 against 76).
 #include "fp8_codec.cuh"
 #include "prefill_params.cuh"
 #include "softcap.cuh"
@@ -26,6 +29,7 @@ namespace {
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int BM = 64, BN = 64;           // rows per CTA, positions per tile
 constexpr int kWarps = 8, kThreads = kWarps * 32;
+constexpr int WR = BM / kWarps, HR = WR / 4;      // rows of a warp, and of a thread in S
 constexpr int kPiece = 4096;              // elements of a piece of K ([64 positions][64 dims]) or V ([VP][CW])
 constexpr int kPitchK = 68;               // floats per K row: 16-byte units of consecutive rows fall into different banks
 
@@ -38,8 +42,9 @@ template <int D> struct F32Shape {
     static constexpr int PITCH_Q = D + 4;
     static constexpr int Q_BYTES = BM * PITCH_Q * 4;
     static constexpr int BUF_BYTES = BN * kPitchK * 4;
-    static constexpr int P_BYTES = kWarps * BN * 8 * 4;
+    static constexpr int P_BYTES = BM * BN * 4;
     static constexpr int SMEM = Q_BYTES + 2 * BUF_BYTES + P_BYTES;
+    static constexpr int PIECE = BM * (D + 2);       // floats of a piece: O, then the rows' maxima, then their sums
 };
 
 __device__ __forceinline__ float fast_exp2(float x)
@@ -49,8 +54,8 @@ __device__ __forceinline__ float fast_exp2(float x)
     return y;
 }
 
-// One thread's share of a piece as it lies in the cache: 16 elements.
-template <int DT> struct Raw { uint4 w[DT == VFKV_F32 ? 4 : DT == VFKV_F16 ? 2 : 1]; };
+// One thread's share of a piece as it lies in the cache.
+template <int DT> struct Raw { uint4 w[kPiece / kThreads / (DT == VFKV_F32 ? 4 : DT == VFKV_F16 ? 8 : 16)]; };
 
 // Unit u of a piece with `cols` elements a row: a unit is 16 bytes of one row.
 template <int DT> struct Unit { static constexpr int ELEMS = DT == VFKV_F32 ? 4 : DT == VFKV_F16 ? 8 : 16; };
@@ -77,57 +82,87 @@ __device__ __forceinline__ void widen(const uint4 &w, float scale, float *x)
     }
 }
 
-template <int DT, int D>
-__global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel(const PrefillParams p)
+// The line of tiles: items in the order (row block, kv-head); CTA c takes tiles [share(c), share(c + 1)).
+struct F32Params {
+    PrefillParams a;
+    uint32_t n_rb, n_cta, each, rest;         // CTAs below `rest` take each + 1 tiles, the others `each`
+    float *scratch;                   // [n_cta][2] pieces: an item begun by an earlier CTA, an item left to the next;
+                                      // null: a CTA for each item
+};
+__device__ __forceinline__ uint32_t share(const F32Params &p, uint32_t c) { return c * p.each + min(c, p.rest); }
+__device__ __forceinline__ uint32_t owner(const F32Params &p, uint32_t tile)
 {
+    const uint32_t longer = p.rest * (p.each + 1u);
+    return tile < longer ? tile / (p.each + 1u) : p.rest + (tile - longer) / p.each;
+}
+// Positions row block rb sees, [*lo, *hi), and its tiles: at least one, so that rows without a position are written.
+__host__ __device__ __forceinline__ uint32_t block_tiles(const PrefillParams &p, uint32_t rb, uint32_t *lo, uint32_t *hi)
+{
+    uint32_t qb = (rb * BM + BM - 1) / p.group, lo_b, hi_a;
+    if (qb >= p.m) qb = p.m - 1;
+    query_range(p, rb * BM / p.group, lo, &hi_a);                  // ranges are monotone in the query index
+    query_range(p, qb, &lo_b, hi);
+    return *hi > *lo ? (*hi + BN - 1) / BN - *lo / BN : 1u;
+}
+
+template <int DT, int D>
+__global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel(const F32Params fp)
+{
+    const PrefillParams &p = fp.a;
     using S = F32Shape<D>;
-    constexpr int UE = Unit<DT>::ELEMS, NU = 16 / UE, ES = DT == VFKV_F32 ? 4 : DT == VFKV_F16 ? 2 : 1;
+    constexpr int UE = Unit<DT>::ELEMS, NU = kPiece / kThreads / UE, ES = DT == VFKV_F32 ? 4 : DT == VFKV_F16 ? 2 : 1;
     extern __shared__ __align__(16) float sm[];
     float *const sq = sm;                                          // [64][PITCH_Q]
     float *const sbuf = sq + BM * S::PITCH_Q;                      // [2][64 * 68]
     float *const sp = sbuf + 2 * BN * kPitchK;                     // [warp][position][8 rows]
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t split = blockIdx.x, n_splits = gridDim.x, kvh = blockIdx.z, g = p.group;
-    const uint32_t row0 = (gridDim.y - 1u - blockIdx.y) * BM;      // heaviest row blocks (latest queries) first
-    const uint32_t n_rows = p.m * g;
-
-    // tiles of this row block, and this CTA's share of them
-    uint32_t c_lo, c_hi, t_begin, t_end;
-    {
-        uint32_t qb = (row0 + BM - 1) / g, lo_b, hi_a;
-        if (qb >= p.m) qb = p.m - 1;
-        query_range(p, row0 / g, &c_lo, &hi_a);                    // ranges are monotone in the query index
-        query_range(p, qb, &lo_b, &c_hi);
-        const uint32_t first = c_lo / BN, n = c_hi > c_lo ? (c_hi + BN - 1) / BN - first : 0u;
-        t_begin = first + uint32_t(uint64_t(n) * split / n_splits);
-        t_end = first + uint32_t(uint64_t(n) * (split + 1) / n_splits);
-    }
+    const uint32_t g = p.group, n_rows = p.m * g;
+    const uint32_t rp = (lane >> 3) * HR, cl = lane & 7;           // first of the thread's HR rows of the warp, first position
+    const float q_mult = p.scale * (p.softcap > 0.f ? 1.0f : kLog2e);      // into the log2 domain; after a soft-cap if there is one
+    float *const my_p = sp + warp * BN * WR;
+    uint32_t line = fp.scratch ? share(fp, blockIdx.x) : 0u;
+    const uint32_t line_end = fp.scratch ? share(fp, blockIdx.x + 1u) : 1u;
     pdl_wait();
-    // Q rows, scaled into the log2 domain (with a soft-cap the factor is applied after it)
-    const float q_mult = p.scale * (p.softcap > 0.f ? 1.0f : kLog2e);
-    for (uint32_t i = threadIdx.x; i < uint32_t(BM * D / 4); i += kThreads) {
-        const uint32_t r = i / (D / 4), c = i % (D / 4), row = row0 + r;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (row < n_rows)
-            x = *reinterpret_cast<const float4 *>(p.q + (uint64_t(row / g) * p.n_q_heads + kvh * g + row % g) * D + 4 * c);
-        *reinterpret_cast<float4 *>(sq + r * S::PITCH_Q + 4 * c) = make_float4(x.x * q_mult, x.y * q_mult, x.z * q_mult, x.w * q_mult);
+
+    while (line < line_end) {
+    // ---- the item that tile `line` belongs to, and how much of it is this CTA's ----
+    uint32_t rb = blockIdx.x / p.n_kv_heads, kvh = blockIdx.x % p.n_kv_heads, n_item = 0u, off = 0u, c_lo, c_hi;
+    for (uint32_t base = 0, before = 0; fp.scratch != nullptr; base += 32) {
+        uint32_t lo, hi;
+        const uint32_t n = base + lane < fp.n_rb ? block_tiles(p, base + lane, &lo, &hi) : 0u;
+        uint32_t x = n * p.n_kv_heads;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        const uint32_t here = __ballot_sync(0xffffffffu, before + x > line);
+        if (here != 0u || base + 32 >= fp.n_rb) {
+            const int k = here != 0u ? __ffs(here) - 1 : 0;
+            n_item = __shfl_sync(0xffffffffu, n, k);
+            const uint32_t rel = line - before - (__shfl_sync(0xffffffffu, x, k) - n_item * p.n_kv_heads);
+            rb = base + uint32_t(k); kvh = rel / n_item; off = rel % n_item;
+            break;
+        }
+        before += __shfl_sync(0xffffffffu, x, 31);
     }
-    // this thread's two rows in S
-    const uint32_t rp = (lane >> 3) * 2, cl = lane & 7;            // row pair of the warp's 8 rows, first position
-    uint32_t r_lo[2], r_hi[2], w_lo, w_hi, full_lo, full_hi;
+    const uint32_t n_all = block_tiles(p, rb, &c_lo, &c_hi);
+    if (fp.scratch == nullptr) n_item = n_all;
+    const uint32_t row0 = rb * BM, n_mine = fp.scratch ? min(n_item - off, line_end - line) : n_item;
+    const uint32_t t_begin = c_lo / BN + off, t_end = t_begin + n_mine;
+
+    // this thread's rows in S
+    uint32_t r_lo[HR], r_hi[HR], w_lo, w_hi, full_lo, full_hi;
     {
         uint32_t mx_lo = 0u, mn_hi = 0xffffffffu, mn_lo = 0xffffffffu, mx_hi = 0u;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t row = row0 + warp * 8 + rp + h;
+        for (int h = 0; h < HR; ++h) {
+            const uint32_t row = row0 + warp * WR + rp + h;
             r_lo[h] = r_hi[h] = 0u;
             if (row < n_rows) {
                 query_range(p, row / g, &r_lo[h], &r_hi[h]);
                 mn_lo = min(mn_lo, r_lo[h]); mx_hi = max(mx_hi, r_hi[h]);
                 mx_lo = max(mx_lo, r_lo[h]); mn_hi = min(mn_hi, r_hi[h]);
-            } else {
-                mn_hi = 0u;                                        // rows past the end: always masked
-            }
+            }                                                      // rows past the end: whatever, they are not written
         }
         w_lo = __reduce_min_sync(0xffffffffu, mn_lo); w_hi = __reduce_max_sync(0xffffffffu, mx_hi);
         full_lo = __reduce_max_sync(0xffffffffu, mx_lo); full_hi = __reduce_min_sync(0xffffffffu, mn_hi);
@@ -171,24 +206,33 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
         }
     };
 
-    float acc[S::CB][8][S::LC];
+    float acc[S::CB][WR][S::LC];
 #pragma unroll
     for (int b = 0; b < S::CB; ++b)
 #pragma unroll
-        for (int r = 0; r < 8; ++r)
+        for (int r = 0; r < WR; ++r)
 #pragma unroll
             for (int j = 0; j < S::LC; ++j) acc[b][r][j] = 0.f;
-    float m_run[2] = {kMaskedScore, kMaskedScore}, l_run[2] = {0.f, 0.f};
-    float *const my_p = sp + warp * BN * 8;
-
-    if (t_begin < t_end) fetch(t_begin, 0);
+    float m_run[HR], l_run[HR];
+#pragma unroll
+    for (int h = 0; h < HR; ++h) { m_run[h] = kMaskedScore; l_run[h] = 0.f; }
+    fetch(t_begin, 0);
+    // Q rows, scaled
+    __syncthreads();                                               // the item before is done with its own
+    for (uint32_t i = threadIdx.x; i < uint32_t(BM * D / 4); i += kThreads) {
+        const uint32_t r = i / (D / 4), c = i % (D / 4), row = row0 + r;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < n_rows)
+            x = *reinterpret_cast<const float4 *>(p.q + (uint64_t(row / g) * p.n_q_heads + kvh * g + row % g) * D + 4 * c);
+        *reinterpret_cast<float4 *>(sq + r * S::PITCH_Q + 4 * c) = make_float4(x.x * q_mult, x.y * q_mult, x.z * q_mult, x.w * q_mult);
+    }
     for (uint32_t t = t_begin; t < t_end; ++t) {
         const uint32_t t0 = t * BN;
         const bool live = t0 < w_hi && t0 + BN > w_lo;             // some row of this warp sees some of the tile
         const bool full = t0 >= full_lo && t0 + BN <= full_hi;
-        float s[2][8];
+        float s[HR][8];
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < HR; ++h)
 #pragma unroll
             for (int j = 0; j < 8; ++j) s[h][j] = 0.f;
 #pragma unroll
@@ -197,25 +241,31 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
             __syncthreads();
             fetch(t, c + 1);
             if (live) {
-                const float *const qa = sq + (warp * 8 + rp) * S::PITCH_Q + c * 64, *const ka = sbuf + (c & 1) * BN * kPitchK + cl * kPitchK;
+                const float *const qa = sq + (warp * WR + rp) * S::PITCH_Q + c * 64, *const ka = sbuf + (c & 1) * BN * kPitchK + cl * kPitchK;
 #pragma unroll 4
                 for (int k = 0; k < 64; k += 4) {
-                    const float4 q0 = *reinterpret_cast<const float4 *>(qa + k), q1 = *reinterpret_cast<const float4 *>(qa + S::PITCH_Q + k);
+                    float4 qv[HR];
+#pragma unroll
+                    for (int h = 0; h < HR; ++h) qv[h] = *reinterpret_cast<const float4 *>(qa + h * S::PITCH_Q + k);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const float4 kv = *reinterpret_cast<const float4 *>(ka + j * 8 * kPitchK + k);
-                        s[0][j] = fmaf(q0.x, kv.x, s[0][j]); s[1][j] = fmaf(q1.x, kv.x, s[1][j]);
-                        s[0][j] = fmaf(q0.y, kv.y, s[0][j]); s[1][j] = fmaf(q1.y, kv.y, s[1][j]);
-                        s[0][j] = fmaf(q0.z, kv.z, s[0][j]); s[1][j] = fmaf(q1.z, kv.z, s[1][j]);
-                        s[0][j] = fmaf(q0.w, kv.w, s[0][j]); s[1][j] = fmaf(q1.w, kv.w, s[1][j]);
+#pragma unroll
+                        for (int h = 0; h < HR; ++h) {
+                            s[h][j] = fmaf(qv[h].x, kv.x, s[h][j]);
+                            s[h][j] = fmaf(qv[h].y, kv.y, s[h][j]);
+                            s[h][j] = fmaf(qv[h].z, kv.z, s[h][j]);
+                            s[h][j] = fmaf(qv[h].w, kv.w, s[h][j]);
+                        }
                     }
                 }
             }
         }
         if (live) {                                                // masks, online softmax, P to the warp's buffer
-            float corr[2];
+            float corr[HR];
+            bool moved = false;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int h = 0; h < HR; ++h) {
                 float mx = kMaskedScore;
                 if (p.softcap > 0.f) {
                     softcap_all(s[h], p.softcap, 1.0f / p.softcap);
@@ -234,6 +284,7 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
                 for (int o = 1; o < 8; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
                 const float mn = fmaxf(m_run[h], mx);
                 corr[h] = fast_exp2(m_run[h] - mn);
+                moved |= corr[h] != 1.f;
                 m_run[h] = mn;
                 float sum = 0.f;
 #pragma unroll
@@ -246,11 +297,14 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
                 l_run[h] = l_run[h] * corr[h] + sum;               // this lane's positions; summed over lanes at the end
             }
 #pragma unroll
-            for (int j = 0; j < 8; ++j) *reinterpret_cast<float2 *>(my_p + (cl + 8 * j) * 8 + rp) = make_float2(s[0][j], s[1][j]);
-            if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
+            for (int j = 0; j < 8; ++j) {
+                float *const d = my_p + (cl + 8 * j) * WR + rp;
+                *reinterpret_cast<float2 *>(d) = make_float2(s[0][j], s[1][j]);
+            }
+            if (__any_sync(0xffffffffu, moved)) {
 #pragma unroll
-                for (int r = 0; r < 8; ++r) {
-                    const float f = __shfl_sync(0xffffffffu, corr[r & 1], (r >> 1) << 3);
+                for (int r = 0; r < WR; ++r) {
+                    const float f = __shfl_sync(0xffffffffu, corr[r % HR], (r / HR) << 3);
 #pragma unroll
                     for (int b = 0; b < S::CB; ++b)
 #pragma unroll
@@ -267,7 +321,7 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
             if (vi + 1 < S::NK) fetch(t, c + 1);
             else if (t + 1 < t_end) fetch(t + 1, 0);
             if (live) {
-                const float *const va = sbuf + (c & 1) * BN * kPitchK + lane * S::LC, *const pa = my_p + pb * S::VP * 8;
+                const float *const va = sbuf + (c & 1) * BN * kPitchK + lane * S::LC, *const pa = my_p + pb * S::VP * WR;
                 auto step = [&](int i, bool masked) {
                     float v[S::LC];
                     if constexpr (S::LC == 4) {
@@ -277,21 +331,33 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
                         const float2 x = *reinterpret_cast<const float2 *>(va + i * S::CW);
                         v[0] = x.x; v[1] = x.y;
                     }
-                    const float4 pl = *reinterpret_cast<const float4 *>(pa + i * 8), ph = *reinterpret_cast<const float4 *>(pa + i * 8 + 4);
-                    const float pr[8] = {pl.x, pl.y, pl.z, pl.w, ph.x, ph.y, ph.z, ph.w};
+                    float pr[WR];
 #pragma unroll
-                    for (int r = 0; r < 8; ++r)
+                    for (int r = 0; r < WR; r += 4) {
+                        const float4 x = *reinterpret_cast<const float4 *>(pa + i * WR + r);
+                        pr[r] = x.x; pr[r + 1] = x.y; pr[r + 2] = x.z; pr[r + 3] = x.w;
+                    }
+#pragma unroll
+                    for (int r = 0; r < WR; ++r)
 #pragma unroll
                         for (int j = 0; j < S::LC; ++j)
                             // a row that does not see a position takes nothing from it, not even 0 x infinity
                             acc[cb][r][j] = masked && pr[r] == 0.f ? acc[cb][r][j] : fmaf(pr[r], v[j], acc[cb][r][j]);
                 };
-                if (full) {
+                // the piece's positions that some row of the warp sees, and those that all of them see
+                const int first = int(t0) + pb * S::VP;
+                const int lo = max(int(w_lo) - first, 0), hi = min(int(w_hi) - first, S::VP);
+                const int all_lo = min(max(int(full_lo) - first, lo), hi), all_hi = max(min(int(full_hi) - first, hi), all_lo);
+                if (lo == 0 && all_lo == 0 && all_hi == S::VP) {
 #pragma unroll 8
                     for (int i = 0; i < S::VP; ++i) step(i, false);
                 } else {
-#pragma unroll 2
-                    for (int i = 0; i < S::VP; ++i) step(i, true);
+#pragma unroll 1
+                    for (int i = lo; i < all_lo; ++i) step(i, true);
+#pragma unroll 1
+                    for (int i = all_lo; i < all_hi; ++i) step(i, false);
+#pragma unroll 1
+                    for (int i = all_hi; i < hi; ++i) step(i, true);
                 }
             }
         }
@@ -300,15 +366,15 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
 
     // row sums over the eight lanes that share a row
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int h = 0; h < HR; ++h)
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], o);
 
-    if (n_splits == 1u) {
+    if (n_mine == n_item) {
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const float l = __shfl_sync(0xffffffffu, l_run[r & 1], (r >> 1) << 3);
-            const uint32_t row = row0 + warp * 8 + r;
+        for (int r = 0; r < WR; ++r) {
+            const float l = __shfl_sync(0xffffffffu, l_run[r % HR], (r / HR) << 3);
+            const uint32_t row = row0 + warp * WR + r;
             if (row >= n_rows) continue;
             const float inv = l > 0.f ? 1.0f / l : 0.f;            // an empty range yields zeros
             float *o = p.out + (uint64_t(row / g) * p.n_q_heads + kvh * g + row % g) * D + lane * S::LC;
@@ -320,56 +386,83 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
                     *reinterpret_cast<float2 *>(o + b * S::CW) = make_float2(acc[b][r][0] * inv, acc[b][r][1] * inv);
             }
         }
-        return;
-    }
-
-    // ---- the cluster's CTAs merge: O over Q's place, m and l over P's; CTA r writes the r-th rows ----
-    __syncthreads();                                               // Q, K/V pieces and P are dead
-    float *const so = sq, *const s_m = sp, *const s_l = sp + BM;
+    } else {
+        float *const o = fp.scratch + (uint64_t(blockIdx.x) * 2 + (off == 0u ? 1 : 0)) * S::PIECE;
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
+        for (int r = 0; r < WR; ++r)
 #pragma unroll
-        for (int b = 0; b < S::CB; ++b)
+            for (int b = 0; b < S::CB; ++b) {
+                float *const d = o + (warp * WR + r) * D + b * S::CW + lane * S::LC;
+                if constexpr (S::LC == 4) *reinterpret_cast<float4 *>(d) = make_float4(acc[b][r][0], acc[b][r][1], acc[b][r][2], acc[b][r][3]);
+                else *reinterpret_cast<float2 *>(d) = make_float2(acc[b][r][0], acc[b][r][1]);
+            }
+        if (cl == 0u) {
 #pragma unroll
-            for (int j = 0; j < S::LC; ++j) so[(warp * 8 + r) * D + b * S::CW + lane * S::LC + j] = acc[b][r][j];
-    if (cl == 0u) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) { s_m[warp * 8 + rp + h] = m_run[h]; s_l[warp * 8 + rp + h] = l_run[h]; }
-    }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    const uint32_t rows_each = BM / n_splits;
-    auto peer = [&](const float *a, uint32_t rank) {
-        uint32_t addr;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(uint32_t(__cvta_generic_to_shared(a))), "r"(rank));
-        return addr;
-    };
-    auto peer_f = [&](const float *a, uint32_t rank) {
-        float x;
-        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(peer(a, rank)) : "memory");
-        return x;
-    };
-    for (uint32_t i = threadIdx.x; i < rows_each * (D / 4); i += kThreads) {
-        const uint32_t r = split * rows_each + i / (D / 4), c = 4 * (i % (D / 4)), row = row0 + r;
-        if (row >= n_rows) continue;
-        float M = kMaskedScore, L = 0.f;
-        for (uint32_t k = 0; k < n_splits; ++k) M = fmaxf(M, peer_f(s_m + r, k));
-        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (uint32_t k = 0; k < n_splits; ++k) {
-            const float f = fast_exp2(peer_f(s_m + r, k) - M);
-            L = fmaf(peer_f(s_l + r, k), f, L);
-            float4 x;
-            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(peer(so + r * D + c, k)) : "memory");
-            o.x = fmaf(x.x, f, o.x); o.y = fmaf(x.y, f, o.y); o.z = fmaf(x.z, f, o.z); o.w = fmaf(x.w, f, o.w);
+            for (int h = 0; h < HR; ++h) {
+                o[BM * D + warp * WR + rp + h] = m_run[h];
+                o[BM * D + BM + warp * WR + rp + h] = l_run[h];
+            }
         }
-        const float inv = L > 0.f ? 1.0f / L : 0.f;
-        *reinterpret_cast<float4 *>(p.out + (uint64_t(row / g) * p.n_q_heads + kvh * g + row % g) * D + c) =
-            make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
     }
-    __syncthreads();
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // a peer may still be reading this CTA's memory
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    line += n_mine;
+    }
+}
+
+// The items that were cut, put together: a warp per row, four pieces at a time.  grid = (items, groups of eight rows).
+template <int D>
+__global__ void __launch_bounds__(kThreads) prefill_f32_merge_kernel(const F32Params fp)
+{
+    using S = F32Shape<D>;
+    constexpr int NV = D < 128 ? 1 : D / 128, LANES = D / 4 < 32 ? D / 4 : 32, U = 4;
+    const PrefillParams &p = fp.a;
+    pdl_wait();
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = p.group;
+    const uint32_t rb = blockIdx.x / p.n_kv_heads, kvh = blockIdx.x % p.n_kv_heads;
+    uint32_t before = 0, lo, hi;
+    for (uint32_t r = lane; r < rb; r += 32) before += block_tiles(p, r, &lo, &hi);
+    before = __reduce_add_sync(0xffffffffu, before);
+    const uint32_t n = block_tiles(p, rb, &lo, &hi), begin = before * p.n_kv_heads + kvh * n;
+    const uint32_t c0 = owner(fp, begin), n_pieces = owner(fp, begin + n - 1u) - c0 + 1u;
+    if (n_pieces == 1u) return;                                    // one CTA had all of it
+    auto piece = [&](uint32_t i) {                                 // the first piece lies in its CTA's second place
+        i = min(i, n_pieces - 1u);
+        return fp.scratch + (uint64_t(c0 + i) * 2 + (i == 0u ? 1 : 0)) * S::PIECE;
+    };
+    const uint32_t rl = blockIdx.y * (kThreads / 32) + warp, row = rb * BM + rl;
+    if (row >= p.m * g) return;
+    float M = kMaskedScore;
+    for (uint32_t i = lane; i < n_pieces; i += 32) M = fmaxf(M, __ldcg(piece(i) + BM * D + rl));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+    float L = 0.f;
+    float4 acc[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t i0 = 0; i0 < n_pieces; i0 += U) {
+        float4 x[U][NV];
+        float f[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const float *const o = piece(i0 + u);
+            f[u] = i0 + u < n_pieces ? fast_exp2(__ldcg(o + BM * D + rl) - M) : 0.f;
+            L = fmaf(f[u], __ldcg(o + BM * D + BM + rl), L);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) x[u][v] = __ldcg(reinterpret_cast<const float4 *>(o + rl * D) + lane % LANES + 32 * v);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                acc[v].x = fmaf(f[u], x[u][v].x, acc[v].x); acc[v].y = fmaf(f[u], x[u][v].y, acc[v].y);
+                acc[v].z = fmaf(f[u], x[u][v].z, acc[v].z); acc[v].w = fmaf(f[u], x[u][v].w, acc[v].w);
+            }
+    }
+    const float inv = L > 0.f ? 1.0f / L : 0.f;                // an empty range yields zeros
+    if (lane < uint32_t(LANES)) {
+        float4 *const out = reinterpret_cast<float4 *>(p.out + (uint64_t(row / g) * p.n_q_heads + kvh * g + row % g) * D) + lane;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) out[32 * v] = make_float4(acc[v].x * inv, acc[v].y * inv, acc[v].z * inv, acc[v].w * inv);
+    }
 }
 
 template <int DT, int D>
@@ -383,16 +476,28 @@ int32_t launch_t(vfkv_ctx *ctx, const PrefillParams &p, cudaStream_t st)
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(f32 prefill attention)");
         configured[ctx->device & 63].store(true, std::memory_order_release);
     }
-    const uint32_t row_blocks = uint32_t((uint64_t(p.m) * p.group + BM - 1) / BM);
-    // Cut a block's K/V tiles while that still adds CTAs to idle SMs and leaves each at least two
-    // tiles: 104 blocks of up to 11 tiles take two CTAs per SM of a D <= 128 kernel in clusters of two.
-    const uint64_t blocks = uint64_t(row_blocks) * p.n_kv_heads, slots = uint64_t(ctx->sm_count) * (D <= 128 ? 2 : 1);
-    const uint32_t visible = p.window && p.window < p.n_kv ? p.window + BM / p.group : p.n_kv - (p.kv_start < p.n_kv ? p.kv_start : p.n_kv);
-    const uint32_t tiles = (visible + BN - 1) / BN;
-    uint32_t n_splits = 1;
-    while (n_splits < 8 && blocks * n_splits * 2 <= slots + slots / 4 && tiles >= n_splits * 4) n_splits *= 2;
-    const cudaError_t e = launch_clusters(ctx, kern, dim3(n_splits, row_blocks, p.n_kv_heads), dim3(kThreads), S::SMEM, st, n_splits, p);
+    F32Params fp{};
+    fp.a = p;
+    fp.n_rb = uint32_t((uint64_t(p.m) * p.group + BM - 1) / BM);
+    uint64_t total = 0;
+    for (uint32_t rb = 0; rb < fp.n_rb; ++rb) {
+        uint32_t lo, hi;
+        total += uint64_t(block_tiles(p, rb, &lo, &hi)) * p.n_kv_heads;
+    }
+    if (total >= (1ull << 31)) return set_error(ctx, VFKV_ERR_UNSUPPORTED, "f32 prefill attention: too many tiles in a call");
+    const uint64_t items = uint64_t(fp.n_rb) * p.n_kv_heads, slots = uint64_t(ctx->sm_count) * (D <= 128 ? 2 : 1);
+    fp.n_cta = uint32_t(total < slots ? total : slots);
+    fp.each = uint32_t(total) / fp.n_cta;
+    fp.rest = uint32_t(total) % fp.n_cta;
+    uint64_t floats = 0;
+    fp.scratch = prefill_scratch(ctx, st, &floats);
+    if (floats < uint64_t(fp.n_cta) * 2 * S::PIECE) fp.scratch = nullptr;
+    cudaError_t e = launch_dependent(ctx, kern, dim3(fp.scratch ? fp.n_cta : uint32_t(items)), dim3(kThreads), S::SMEM, st, fp);
     ctx->count_launch();
+    if (e == cudaSuccess && fp.scratch && fp.n_cta > 1) {
+        e = launch_dependent(ctx, prefill_f32_merge_kernel<D>, dim3(uint32_t(items), BM / (kThreads / 32)), dim3(kThreads), 0, st, fp);
+        ctx->count_launch();
+    }
     return check_cuda(ctx, e, "f32 prefill attention launch");
 }
 

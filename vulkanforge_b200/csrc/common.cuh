@@ -235,27 +235,6 @@ inline cudaError_t launch_dependent(const vfkv_ctx *ctx, void (*kern)(P...), dim
     cfg.numAttrs = ctx->pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
-// The same in clusters of `cluster` CTAs along x.
-template <typename... P, typename... A>
-inline cudaError_t launch_clusters(const vfkv_ctx *ctx, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
-                                   cudaStream_t st, uint32_t cluster, A &&...args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    unsigned n = 0;
-    if (ctx->pdl) {
-        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    if (cluster > 1) {
-        attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = cluster; attr[n].val.clusterDim.y = 1; attr[n++].val.clusterDim.z = 1;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
-}
 
 #ifdef __CUDACC__
 // Waits for everything in front of this kernel on its stream, then lets the next kernel be scheduled.

@@ -328,11 +328,12 @@ int32_t vfkv_decode_token(vfkv_cache *cache, vfkv_workspace *ws, const float *d_
  * h_positions / h_slot_ids (NULL = identity) are host arrays of n_seqs.
  * windows: NULL, or n_layers entries (0 = global layer).  This is the
  * forward_token boundary (src/backend/vulkan/forward/decode.rs:567-626) reduced
- * to the hot path.  On a non-default stream the layers run as up to four cached
- * CUDA graphs, and a second stream owned by the workspace copies the next
- * group's inputs and the previous group's outputs while a group computes; the
- * call returns when h_out is complete.  Pinned host buffers make the copies
- * asynchronous. */
+ * to the hot path.  On a non-default stream outside a capture the call is recorded as a CUDA
+ * graph, which the next call with the same buffers replays.  Tokens of some megabytes cross the
+ * bus in up to four groups of layers, on streams owned by the workspace, so that a group computes
+ * while the next one's inputs travel; smaller ones from pinned, 16-byte aligned buffers are read
+ * by one kernel and leave by the attention kernel's own stores.  The call returns when h_out is
+ * complete.  Pinned host buffers make the copies asynchronous. */
 int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const float *h_q,
                                const float *h_k, const float *h_v, float *h_out,
                                uint32_t n_q_heads, const uint32_t *h_slot_ids,
@@ -486,7 +487,7 @@ int32_t vfkv_stream_synchronize(vfkv_ctx *ctx, void *stream);
 /* ---------------------------------------------------------------------- */
 /* Selects the attention implementation for subsequent calls on this context:
  * 0 = automatic, 1 = CUDA-core kernel only, 2 = tensor-core kernel only
- * (VFKV_ERR_UNSUPPORTED from attend when the shape is outside it), 3 = automatic, but
+ * with TMA-fed rows (VFKV_ERR_UNSUPPORTED from attend when the shape is outside it), 3 = automatic, but
  * vfkv_attend_prefill takes its mma.sync kernel where it would take the tcgen05 one. */
 int32_t vfkv_ctx_set_attn_impl(vfkv_ctx *ctx, uint32_t impl);
 /* Shape of the tensor-core attention kernel for subsequent calls: warps per CTA x TMA stages per
@@ -498,25 +499,24 @@ int32_t vfkv_ctx_set_attn_impl(vfkv_ctx *ctx, uint32_t impl);
  * tensor maps).  The specialised form runs either one CTA per
  * (kv-head, block of 256 rows) item -- always with 4x3 -- or one CTA per SM, each taking an even
  * share of all items' K/V tiles -- with 8x3 whenever the call allows it (every query sees at
- * least one position, at most 512 row blocks, at least 8 tiles a share), with 0x0 when in
- * addition one CTA per item would leave a twentieth of the SM time unused and an item averages 96
- * tiles or more, or the items are at most half the SMs and the shares are ten tiles shorter than
- * the longest item.  Items cut between CTAs
- * are put together by the CTA holding the item's head (a cooperative launch, at most four
- * pieces an item, not inside a stream capture) or by a small second kernel.  The shares need
- * 39 MB of device scratch, which the context allocates at the first such call outside a stream
- * capture and frees in vfkv_ctx_destroy; calls that would use it must not run concurrently on
- * two streams of one context. */
+ * least one position, at most 512 row blocks, at least 2 tiles a share), with 0x0 when that is
+ * expected to be faster.  Items cut between CTAs are put together by the CTA holding the item's
+ * head (a cooperative launch, at most four pieces an item, not inside a stream capture) or by a
+ * small second kernel.  With 0x0 shorter calls take a kernel with one tile of 128 rows a CTA, whose
+ * items may be cut the same way.  Pieces need 39 MB of device scratch, which the context allocates
+ * at a stream's first such call outside a capture, for up to four streams, and frees in
+ * vfkv_ctx_destroy; on further streams nothing is cut.  A call captured on a stream without
+ * scratch uses the first stream's: its replays must not overlap other such calls. */
 int32_t vfkv_ctx_set_attn_tuning(vfkv_ctx *ctx, uint32_t warps, uint32_t stages);
-/* Programmatic dependent launch of the tensor-core attention kernel, the CUDA counterpart of
+/* Programmatic dependent launch of the library's kernels, the CUDA counterpart of
  * relaxing the full pipeline barrier the reference records between dispatches
  * (src/backend/vulkan/forward/runs.rs:1541, executor/attention.rs:583-596) to the buffers that
  * really depend on one another.
  *   0  off: a kernel starts when the previous work in the stream has finished (default).
  *   1  the kernel may be scheduled while its predecessor in the stream drains; it waits for the
  *      predecessor before it reads or writes any global memory.  Always safe.
- *   2  as 1, but it reads the position / slot arrays and prefetches this layer's K/V rows before
- *      that wait.  The caller promises that the kernel enqueued immediately before on the stream
+ *   2  as 1, but the decode kernel with TMA-fed rows reads the position / slot arrays and
+ *      prefetches this layer's K/V rows before that wait.  The caller promises that the kernel enqueued immediately before on the stream
  *      writes neither those arrays nor this layer's cache rows (true for consecutive layers of a
  *      decode step, and for a forward pass whose preceding kernel is a projection or RoPE).
  *      Only that one kernel matters: a mode-2 kernel releases its successor after its own wait,

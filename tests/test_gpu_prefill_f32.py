@@ -58,3 +58,31 @@ def test_f32_tiles_match_the_oracle(ctx, dtype, hq, hkv, d, m, q_start, kv_start
     finally:
         fwd.workspace.destroy()
         cache.destroy()
+
+
+def test_pieces_on_several_streams(ctx):
+    """Calls that leave pieces may overlap on different streams of a context; a fifth stream cuts nothing."""
+    import torch
+    hq, hkv, d, m, L = 32, 8, 128, 60, 500
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, L), vf.KvDtype.F32)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    try:
+        kv = torch.randn(2, L, hkv, d, device="cuda", generator=gen)
+        fwd.b_step_kv_write(0, kv[0], kv[1], L, 0)
+        qs = [torch.randn(m, hq, d, device="cuda", generator=gen) for _ in range(6)]
+        want, got = ([torch.zeros_like(q) for q in qs] for _ in range(2))
+        for q, o in zip(qs, want):
+            fwd.run_flash_attn_batch(0, q, o, m, L - m, L, 1, 0)
+        torch.cuda.synchronize()
+        streams = [torch.cuda.Stream() for _ in qs]
+        for _ in range(3):
+            for q, o, s in zip(qs, got, streams):
+                fwd.stream = s.cuda_stream
+                fwd.run_flash_attn_batch(0, q, o, m, L - m, L, 1, 0)
+        torch.cuda.synchronize()
+        assert all(float((a - b).abs().max()) < 1e-5 for a, b in zip(want, got))
+    finally:
+        fwd.stream = None
+        fwd.workspace.destroy()
+        cache.destroy()

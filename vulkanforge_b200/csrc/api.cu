@@ -163,7 +163,7 @@ int32_t vfkv_ctx_destroy(vfkv_ctx *ctx)
     if (!ctx) return VFKV_OK;
     DeviceGuard g(ctx->device);
     cudaFree(ctx->d_status);
-    cudaFree(ctx->d_prefill_scratch);
+    for (auto &s : ctx->prefill_scratch) cudaFree(s.d);
     prof_clear(ctx);
     delete ctx;
     return VFKV_OK;

@@ -1347,29 +1347,39 @@ TwoTileCost two_tile_cost(const vfkv_ctx *ctx, uint32_t dtype, const Tc5Params &
 
 }  // namespace
 
-// Device scratch for pieces of row blocks: allocated at the first call outside a stream capture, owned by
-// the context; null where there is none (the caller then cuts nothing).
+// Device scratch for pieces of row blocks, owned by the context: allocated at a stream's first call outside a
+// capture, for up to four streams, so that calls on several of them may overlap.  A call that is being captured on a
+// stream without one takes the first there is (its replays must not overlap other such calls).  Null where there is
+// none: the caller then cuts nothing.
 float *prefill_scratch(vfkv_ctx *ctx, cudaStream_t st, uint64_t *floats)
 {
     const uint32_t n_sm = uint32_t(ctx->sm_count);
     const uint64_t n = uint64_t(n_sm) * 2 * CTA_ROWS * (HD + 2);
-    if (ctx->d_prefill_scratch == nullptr) {
-        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-        cudaStreamIsCapturing(st, &capturing);
-        if (capturing != cudaStreamCaptureStatusNone) return nullptr;
-        void *d = nullptr;
-        // the pieces, then one flag per CTA
-        if (cudaMalloc(&d, n * sizeof(float) + n_sm * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMemset(static_cast<float *>(d) + n, 0, n_sm * sizeof(uint32_t)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            cudaFree(d);
-            return nullptr;
+    *floats = 0;
+    for (auto &s : ctx->prefill_scratch) {
+        if (s.d != nullptr && s.stream != st) continue;
+        if (s.d == nullptr) {
+            cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+            cudaStreamIsCapturing(st, &capturing);
+            if (capturing != cudaStreamCaptureStatusNone) break;
+            void *d = nullptr;
+            // the pieces, then one flag per CTA
+            if (cudaMalloc(&d, n * sizeof(float) + n_sm * sizeof(uint32_t)) != cudaSuccess ||
+                cudaMemset(static_cast<float *>(d) + n, 0, n_sm * sizeof(uint32_t)) != cudaSuccess) {
+                (void)cudaGetLastError();
+                cudaFree(d);
+                return nullptr;
+            }
+            s = {st, static_cast<float *>(d)};
         }
-        ctx->d_prefill_scratch = static_cast<float *>(d);
-        ctx->prefill_scratch_ctas = n_sm;
+        *floats = n;
+        return s.d;
     }
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(st, &capturing);
+    if (capturing == cudaStreamCaptureStatusNone || ctx->prefill_scratch[0].d == nullptr) return nullptr;
     *floats = n;
-    return ctx->d_prefill_scratch;
+    return ctx->prefill_scratch[0].d;
 }
 
 // A byte-typed map of rows of row_bytes, boxes of 128 bytes x box_rows with the 128-byte swizzle.
@@ -1453,12 +1463,11 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
         if (cost.even) {
             cudaStreamIsCapturing(st, &capturing);
             uint64_t floats = 0;
-            prefill_scratch(ctx, st, &floats);
-            if (ctx->d_prefill_scratch != nullptr && ctx->prefill_scratch_ctas >= n_sm) {
+            p.scratch = prefill_scratch(ctx, st, &floats);
+            if (p.scratch != nullptr) {
                 spread = true;
                 p.total_tiles = uint32_t(cost.total);
                 p.n_cta = n_sm;
-                p.scratch = ctx->d_prefill_scratch;
                 p.flags = reinterpret_cast<uint32_t *>(p.scratch + size_t(n_sm) * 2 * CTA_ROWS * (HD + 2));
                 // An item is cut into at most ceil(longest item / smallest share) + 1 pieces.  A
                 // captured launch would replay with the flag value of the capture, which the flags

@@ -19,8 +19,8 @@ struct vfkv_ctx {
     uint32_t *d_status = nullptr;      // device word written by bounded waits that give up
     uint32_t attn_impl = 0;            // 0 auto, 1 CUDA-core only, 2 tensor-core only, 3 as 0 but mma.sync instead of tcgen05 (prefill)
     uint32_t tune_warps = 0, tune_stages = 0;   // tensor-core kernel shape, 0 = choose
-    float *d_prefill_scratch = nullptr;         // pieces of prefill items cut between CTAs; allocated at first use
-    uint32_t prefill_scratch_ctas = 0;
+    // Pieces of prefill items cut between CTAs: a buffer for each of the first streams that need one
+    struct PrefillScratch { cudaStream_t stream; float *d; } prefill_scratch[4] = {};
     uint32_t prefill_epoch = 0;                 // value the flags of the current spread prefill launch take
     uint32_t pdl = 0;                  // programmatic dependent launch mode (0 / 1 / 2)
     // K addresses that the last launch on this context wrote cache rows into, or an empty range: a

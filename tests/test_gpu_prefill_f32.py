@@ -73,13 +73,13 @@ def test_pieces_on_several_streams(ctx):
         qs = [torch.randn(m, hq, d, device="cuda", generator=gen) for _ in range(6)]
         want, got = ([torch.zeros_like(q) for q in qs] for _ in range(2))
         for q, o in zip(qs, want):
-            fwd.run_flash_attn_batch(0, q, o, m, L - m, L, 1, 0)
+            fwd.run_flash_attn_batch(0, q, o, m, L - m, L, 0, 0)
         torch.cuda.synchronize()
         streams = [torch.cuda.Stream() for _ in qs]
         for _ in range(3):
             for q, o, s in zip(qs, got, streams):
                 fwd.stream = s.cuda_stream
-                fwd.run_flash_attn_batch(0, q, o, m, L - m, L, 1, 0)
+                fwd.run_flash_attn_batch(0, q, o, m, L - m, L, 0, 0)
         torch.cuda.synchronize()
         assert all(float((a - b).abs().max()) < 1e-5 for a, b in zip(want, got))
     finally:

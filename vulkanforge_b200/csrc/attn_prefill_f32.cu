@@ -7,9 +7,11 @@
 // scores to the output: scores, maxima, P and O never leave it, and the only CTA-wide step is the
 // hand-over of the next 16 KB piece of K or V (double-buffered in shared memory, the piece after it
 // in flight in registers).
-//   S: thread = 2 rows x 8 positions; 10 16-byte shared loads for 64 FMAs.
+//   S: thread = 4 rows x 4 positions; 8 16-byte shared loads for 64 FMAs.
 //   PV: thread = 8 rows x 4 dims; 3 16-byte shared loads for 32 FMAs.
-// Both keep the FMA pipe, not shared memory, as the bound (74 TFLOP/s at 1.96 GHz).
+// Shared memory is the bound (a 16-byte load of a warp takes four of its cycles whoever shares an address: 63 % of
+// them used over a launch, the FMA pipe 35 %), so the thread's tile of S is square: 2 x 8, with ten loads for the
+// same FMAs, took 90.5 us where this takes 84.6 (200 queries at 700 positions, F32).
 //
 // Row blocks are few and uneven (200 queries x 4 heads x 8 kv-heads: 104 blocks of 8 to 11 tiles), and an SM is
 // at its rate only with two CTAs on it, so the tiles of all (row block, kv-head) items form one line of which every
@@ -29,7 +31,8 @@ namespace {
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int BM = 64, BN = 64;           // rows per CTA, positions per tile
 constexpr int kWarps = 8, kThreads = kWarps * 32;
-constexpr int WR = BM / kWarps, HR = WR / 4;      // rows of a warp, and of a thread in S
+constexpr int WR = BM / kWarps, HR = 4;           // rows of a warp, and of a thread in S
+constexpr int LR = 32 / (WR / HR), HP = BN / LR;  // lanes that share a row of S, and positions of each
 constexpr int kPiece = 4096;              // elements of a piece of K ([64 positions][64 dims]) or V ([VP][CW])
 constexpr int kPitchK = 68;               // floats per K row: 16-byte units of consecutive rows fall into different banks
 
@@ -117,7 +120,7 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
     float *const sp = sbuf + 2 * BN * kPitchK;                     // [warp][position][8 rows]
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t g = p.group, n_rows = p.m * g;
-    const uint32_t rp = (lane >> 3) * HR, cl = lane & 7;           // first of the thread's HR rows of the warp, first position
+    const uint32_t rp = lane / LR * HR, cl = lane % LR;            // first of the thread's HR rows of the warp, first position
     const float q_mult = p.scale * (p.softcap > 0.f ? 1.0f : kLog2e);      // into the log2 domain; after a soft-cap if there is one
     float *const my_p = sp + warp * BN * WR;
     uint32_t line = fp.scratch ? share(fp, blockIdx.x) : 0u;
@@ -230,11 +233,11 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
         const uint32_t t0 = t * BN;
         const bool live = t0 < w_hi && t0 + BN > w_lo;             // some row of this warp sees some of the tile
         const bool full = t0 >= full_lo && t0 + BN <= full_hi;
-        float s[HR][8];
+        float s[HR][HP];
 #pragma unroll
         for (int h = 0; h < HR; ++h)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) s[h][j] = 0.f;
+            for (int j = 0; j < HP; ++j) s[h][j] = 0.f;
 #pragma unroll
         for (int c = 0; c < S::NK; ++c) {                          // S = Q K^T, 64 dims at a time
             place(c);
@@ -248,8 +251,8 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
 #pragma unroll
                     for (int h = 0; h < HR; ++h) qv[h] = *reinterpret_cast<const float4 *>(qa + h * S::PITCH_Q + k);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float4 kv = *reinterpret_cast<const float4 *>(ka + j * 8 * kPitchK + k);
+                    for (int j = 0; j < HP; ++j) {
+                        const float4 kv = *reinterpret_cast<const float4 *>(ka + j * LR * kPitchK + k);
 #pragma unroll
                         for (int h = 0; h < HR; ++h) {
                             s[h][j] = fmaf(qv[h].x, kv.x, s[h][j]);
@@ -270,25 +273,25 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
                 if (p.softcap > 0.f) {
                     softcap_all(s[h], p.softcap, 1.0f / p.softcap);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) s[h][j] *= kLog2e;
+                    for (int j = 0; j < HP; ++j) s[h][j] *= kLog2e;
                 }
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
+                for (int j = 0; j < HP; ++j) {
                     float x = s[h][j];
-                    const uint32_t pos = t0 + cl + 8 * j;
+                    const uint32_t pos = t0 + cl + LR * j;
                     if (!full && (pos < r_lo[h] || pos >= r_hi[h])) x = kMaskedScore;
                     s[h][j] = x;
                     mx = fmaxf(mx, x);
                 }
 #pragma unroll
-                for (int o = 1; o < 8; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                for (int o = 1; o < LR; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
                 const float mn = fmaxf(m_run[h], mx);
                 corr[h] = fast_exp2(m_run[h] - mn);
                 moved |= corr[h] != 1.f;
                 m_run[h] = mn;
                 float sum = 0.f;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
+                for (int j = 0; j < HP; ++j) {
                     // a masked position contributes nothing, also while the row's maximum is still the sentinel
                     const float e = (full || s[h][j] > 0.5f * kMaskedScore) ? fast_exp2(s[h][j] - mn) : 0.f;
                     s[h][j] = e;
@@ -297,14 +300,14 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
                 l_run[h] = l_run[h] * corr[h] + sum;               // this lane's positions; summed over lanes at the end
             }
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float *const d = my_p + (cl + 8 * j) * WR + rp;
-                *reinterpret_cast<float2 *>(d) = make_float2(s[0][j], s[1][j]);
+            for (int j = 0; j < HP; ++j) {
+                float *const d = my_p + (cl + LR * j) * WR + rp;
+                *reinterpret_cast<float4 *>(d) = make_float4(s[0][j], s[1][j], s[2][j], s[3][j]);
             }
             if (__any_sync(0xffffffffu, moved)) {
 #pragma unroll
                 for (int r = 0; r < WR; ++r) {
-                    const float f = __shfl_sync(0xffffffffu, corr[r % HR], (r / HR) << 3);
+                    const float f = __shfl_sync(0xffffffffu, corr[r % HR], r / HR * LR);
 #pragma unroll
                     for (int b = 0; b < S::CB; ++b)
 #pragma unroll
@@ -368,12 +371,12 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
 #pragma unroll
     for (int h = 0; h < HR; ++h)
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], o);
+        for (int o = 1; o < LR; o <<= 1) l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], o);
 
     if (n_mine == n_item) {
 #pragma unroll
         for (int r = 0; r < WR; ++r) {
-            const float l = __shfl_sync(0xffffffffu, l_run[r % HR], (r / HR) << 3);
+            const float l = __shfl_sync(0xffffffffu, l_run[r % HR], r / HR * LR);
             const uint32_t row = row0 + warp * WR + r;
             if (row >= n_rows) continue;
             const float inv = l > 0.f ? 1.0f / l : 0.f;            // an empty range yields zeros

@@ -69,3 +69,35 @@ def test_one_tile_kernel_matches_the_oracle(ctx, dtype, hq, hkv, d, m, q_start, 
     finally:
         fwd.workspace.destroy()
         cache.destroy()
+
+
+@pytest.mark.parametrize("hq,hkv,d,L", [(16, 8, 256, 200), (8, 8, 64, 1500)])
+def test_rows_that_one_position_dominates(ctx, hq, hkv, d, L):
+    """Position 100 outweighs position 10 by less than the kernel moves a row's maximum for, and all others by far: its
+    p is not 1 but a number that half precision rounds by up to 2^-12, which the row's sum has to follow."""
+    import torch
+    m = 34
+    rng = np.random.default_rng(d)
+    k = np.zeros((L, hkv, d), np.float32)
+    k[10, :, 0], k[100, :, 0] = 10.0, 11.0
+    v = rng.standard_normal((L, hkv, d), dtype=np.float32).astype(np.float16).astype(np.float32)
+    q = np.zeros((m, hq, d), np.float32)
+    q[:, :, 0] = ((4.0 + 0.03 * np.arange(m)) * np.sqrt(d))[:, None]           # scores 40 .. 50 and a tenth more
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, L), vf.KvDtype.F16)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    try:
+        fwd.b_step_kv_write(0, to_dev(k), to_dev(v), L, 0)
+        out = torch.zeros(m, hq, d, device="cuda")
+        fwd.run_flash_attn_batch(0, to_dev(q), out, m, L - m, L, 0, 0)
+        torch.cuda.synchronize()
+        s = (q[:, 0, 0].astype(np.float64) / np.sqrt(np.float64(d)))[:, None] * k[:, 0, 0].astype(np.float64)      # [m][L]
+        s[np.arange(L)[None] > (L - m + np.arange(m))[:, None]] = -np.inf
+        p = np.exp(s - s.max(1, keepdims=True))
+        p /= p.sum(1, keepdims=True)
+        want = np.repeat(np.einsum("ml,lhd->mhd", p, v.astype(np.float64)), hq // hkv, axis=1)
+        # the dominating p off by 2^-12 shifts the mean of the two rows by that share of the other's weight (at most e^-4)
+        tol = 2.0 ** -12 * np.exp(-4.0) * np.abs(v[100] - v[10]).max() + 4e-6 * np.abs(v).max()
+        assert np.abs(out.cpu().numpy() - want).max() < tol
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

@@ -12,7 +12,9 @@
 // 64 positions a tile, because Q of 256 dims in two terms takes 128 KB and leaves room for three stages (two
 // of K, whose products come a tile earlier, and one of V).
 // A row's exponents refer to a maximum that is moved, and O rescaled, only when the true one has outgrown
-// it by a few binary orders.
+// it by a few binary orders.  The largest p is then any number up to 2^8 and not 1, so a row's sum is taken of the
+// p as they go into the product, rounded to half precision: a row that one position dominates is that position's V
+// whatever its p was rounded to (with the sum of the unrounded p: off by up to 2^-12).
 //
 // SPLITQ: Q = high + low half-precision term, scaled per row by a power of two (two products for S).
 // SC: the scales of K multiply the scores, those of V multiply P, in f32; P is then also fed as two terms,
@@ -306,9 +308,8 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
                 float e = fast_exp2(s[j] - mref);
                 if (!warp_full) e = s[j] > 0.5f * kMaskedScore ? e : 0.f;
                 s[j] = e;
-                sum += e;
+                if constexpr (SC) sum += e;
             }
-            lrow += sum;
             if constexpr (SC) {
 #pragma unroll
                 for (int j = 0; j < 64; j += 4) {
@@ -318,7 +319,12 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
             }
             float pk[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) pk[j] = __uint_as_float(pack_half2(s[2 * j], s[2 * j + 1]));
+            for (int j = 0; j < 32; ++j) {
+                const uint32_t w = pack_half2(s[2 * j], s[2 * j + 1]);
+                pk[j] = __uint_as_float(w);
+                if constexpr (!SC) sum = add_halves(sum, w);
+            }
+            lrow += sum;
             tmem_st32(tm_s, pk);
             if constexpr (SC) {
 #pragma unroll

@@ -147,6 +147,13 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi)
     __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t *>(&h);
 }
+// sum + the two halves of a pair
+__device__ __forceinline__ float add_halves(float sum, uint32_t pair)
+{
+    asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %1;\n\t"
+        "add.f32.f16 %0, a, %0;\n\tadd.f32.f16 %0, b, %0;\n\t}" : "+f"(sum) : "r"(pair));
+    return sum;
+}
 // A from tensor memory (half pairs packed into columns).
 __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {

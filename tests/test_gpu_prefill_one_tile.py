@@ -101,3 +101,30 @@ def test_rows_that_one_position_dominates(ctx, hq, hkv, d, L):
     finally:
         fwd.workspace.destroy()
         cache.destroy()
+
+
+@pytest.mark.parametrize("hq,hkv,m,q_start,softcap", [(64, 8, 166, 99, 0.0), (32, 8, 17, 485, 50.0), (32, 8, 60, 1000, 0.0)])
+def test_short_f16_calls_take_q_in_two_terms(ctx, hq, hkv, m, q_start, softcap):
+    """Q of one half-precision term moves a score s by up to 2^-12 |s| and each p by as much again; with two terms what is
+    left is the rounding of p to half precision.  Queries 25 times larger (scores of some 70): 1e-3 or 5e-5."""
+    import torch
+    d, L = 128, q_start + m
+    gen = torch.Generator(device="cuda").manual_seed(L)
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, L), vf.KvDtype.F16)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq, softcap=softcap)
+    try:
+        k, v = (torch.randn(L, hkv, d, device="cuda", generator=gen).half().float() for _ in range(2))
+        q = torch.randn(m, hq, d, device="cuda", generator=gen) * 25
+        fwd.b_step_kv_write(0, k, v, L, 0)
+        out = torch.zeros(m, hq, d, device="cuda")
+        fwd.run_flash_attn_batch(0, q, out, m, q_start, L, 0, 0)
+        s = torch.einsum("mhgd,lhd->hgml", q.double().view(m, hkv, hq // hkv, d), k.double()) / d ** 0.5
+        if softcap:
+            s = softcap * torch.tanh(s / softcap)
+        s = s.masked_fill(torch.arange(L, device="cuda") > q_start + torch.arange(m, device="cuda")[:, None], -float("inf"))
+        want = torch.einsum("hgml,lhd->mhgd", s.softmax(-1), v.double()).reshape(m, hq, d)
+        error = float((out.double() - want).norm() / want.norm())
+        assert error < 2.0 ** -12                              # half an ulp of p at most, in the mean less
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

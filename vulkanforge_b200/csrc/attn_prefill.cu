@@ -515,10 +515,10 @@ extern "C" int32_t vfkv_attend_prefill(vfkv_cache *cache, uint32_t layer, uint32
                         (dt == VFKV_F8 || dt == VFKV_F16) && (D == 64 || D == 128 || D == 256);
     if (ctx->attn_impl == 2 && !mma_ok)
         return set_error(ctx, VFKV_ERR_UNSUPPORTED, "vfkv_attend_prefill: shape outside the tensor-core kernel");
-    // F16 caches carry the error budget of the reference's f32 shader (2e-3 absolute): the tcgen05
+    // F16 caches carry the error budget of the reference's f32 shader (2e-3 absolute): the two-tile
     // kernel feeds Q as one half-precision value, which holds it (1e-4 .. 5e-4 measured) with the usual
-    // 1/sqrt(head_dim) scale but not with scale 1.0 (1e-2: the Gemma-4 rule); those keep the
-    // mma.sync kernel and its hi + lo split of Q.
+    // 1/sqrt(head_dim) scale but not with scale 1.0 (1e-2: the Gemma-4 rule); those take the kernels
+    // that split Q into a high and a low term.
     const bool tc5_accurate = dt == VFKV_F8 || scale * sqrtf(float(D)) <= 1.5f;
     const bool two_ok = mma_ok && ctx->attn_impl != 3 && prefill_tc5_supported(dt, D, p.group, false) && tc5_accurate;
     // Three kernels do the same work in different portions, and the one whose model of the call is the
@@ -529,17 +529,21 @@ extern "C" int32_t vfkv_attend_prefill(vfkv_cache *cache, uint32_t layer, uint32
     //   64 queries at 0: - / 11 / 9 us;  64 at 1936: 24 / 20 / 76;  16 at 30 000: 92 / 50 / -;
     //   333 at 1000: 44 / 38 / -;  1000 at 3000: 133 / 139 / -;  2000 at 0: 94 / 107 / -
     // attn_impl 2 and the tuning knob force the first where it holds the shape.
+    // F16 rows of 128 dims: the short calls keep Q in two terms, the ones whose products bind them take it in one
+    // (166 queries at 99 positions, 64 / 8 heads: error against 64 bits 1.7e-4 in two terms, 2.8e-4 in one; the second
+    // term costs a tile of 64 positions 0.2 us of 0.9).
     if (ctx->attn_impl == 0 && aligned && prefill_one_tile_supported(ctx, dt, D) && (kv.k_scales || mma_ok) &&
         !(two_ok && ctx->tune_stages != 0)) {
-        const double one_us = prefill_one_tile_us(ctx, dt, !tc5_accurate, p);
-        const double two_us = two_ok ? prefill_tc5_us(ctx, dt, n_q_heads, hkv, m, q_start, n_kv, kv_start, window) : 1e30;
+        const bool split_q = !tc5_accurate || (dt == VFKV_F16 && D == 128 && prefill_tc5_short(ctx, n_q_heads, hkv, m, q_start, n_kv, kv_start, window));
+        const double one_us = prefill_one_tile_us(ctx, dt, split_q, p);
+        const double two_us = two_ok && !split_q ? prefill_tc5_us(ctx, dt, n_q_heads, hkv, m, q_start, n_kv, kv_start, window) : 1e30;
         const uint32_t last = q_start + m < n_kv ? q_start + m : n_kv;
         const uint32_t seen = window && window + BM / p.group < last ? window + BM / p.group : last - (kv_start < last ? kv_start : last);
         double mma_us = mma_ok ? 3.0 + 2.2 * (D / 128.0) * ((seen + BN - 1) / BN) : 1e30;
         const double ctas_a_slot = double((uint64_t(m) * p.group + BM - 1) / BM) * hkv / (1.6 * ctx->sm_count);
         if (ctas_a_slot > 1.0) mma_us *= ctas_a_slot;
         if (one_us <= two_us && one_us < mma_us)
-            return launch_prefill_one_tile(ctx, dt, !tc5_accurate, p, st);
+            return launch_prefill_one_tile(ctx, dt, split_q, p, st);
         if (two_us < mma_us)
             return launch_prefill_tc5(ctx, dt, p.k, p.v, d_q, d_out, p.row_bytes, n_q_heads, hkv, m, q_start, n_kv, kv_start,
                                       window, scale, softcap, st);

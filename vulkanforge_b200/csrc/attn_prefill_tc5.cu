@@ -1404,17 +1404,35 @@ bool prefill_tc5_supported(uint32_t dtype, uint32_t head_dim, uint32_t group, bo
     return (dtype == VFKV_F8 || dtype == VFKV_F16) && head_dim == 128 && !has_scales && group != 0 && BM % group == 0;
 }
 
-// Expected time (us): a CTA pays 8 us and 3.5 us a tile of 128 positions, the even shares 45 us (segments,
-// pieces, the merge) and 2.8 us a tile.  Measured: 1000 queries at 3000 (128 items of up to 32 tiles) 121 us;
-// 500 at 7500 (64 of 63, in shares) 131.
-double prefill_tc5_us(const vfkv_ctx *ctx, uint32_t dtype, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m,
-                      uint32_t q_start, uint32_t n_kv, uint32_t kv_start, uint32_t window)
+static Tc5Params call_params(uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m, uint32_t q_start, uint32_t n_kv,
+                             uint32_t kv_start, uint32_t window)
 {
     Tc5Params p{};
     p.n_q_heads = n_q_heads; p.n_kv_heads = n_kv_heads; p.group = n_q_heads / n_kv_heads;
     p.m = m; p.q_start = q_start; p.n_kv = n_kv; p.kv_start = kv_start; p.window = window;
     p.n_rb = (m * p.group + CTA_ROWS - 1) / CTA_ROWS;
-    return two_tile_cost(ctx, dtype, p).us;
+    return p;
+}
+
+// By the model of two_tile_cost.  Measured: 1000 queries at 3000 (128 items of up to 32 tiles) 121 us; 500 at 7500
+// (64 of 63, in shares) 131.
+double prefill_tc5_us(const vfkv_ctx *ctx, uint32_t dtype, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m,
+                      uint32_t q_start, uint32_t n_kv, uint32_t kv_start, uint32_t window)
+{
+    return two_tile_cost(ctx, dtype, call_params(n_q_heads, n_kv_heads, m, q_start, n_kv, kv_start, window)).us;
+}
+
+bool prefill_tc5_short(const vfkv_ctx *ctx, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m, uint32_t q_start,
+                       uint32_t n_kv, uint32_t kv_start, uint32_t window)
+{
+    const Tc5Params p = call_params(n_q_heads, n_kv_heads, m, q_start, n_kv, kv_start, window);
+    if (uint64_t(p.n_rb) * n_kv_heads * 4 >= uint64_t(ctx->sm_count) * 3) return false;
+    for (uint32_t rb = 0; rb < p.n_rb; ++rb) {
+        uint32_t r0, cl, tiles;
+        item_extent(p, rb, &r0, &cl, &tiles);
+        if (tiles >= 10) return false;
+    }
+    return true;
 }
 
 int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, const uint8_t *v, const float *q, float *out,

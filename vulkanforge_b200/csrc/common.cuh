@@ -296,6 +296,9 @@ bool prefill_tc5_supported(uint32_t dtype, uint32_t head_dim, uint32_t group, bo
 // expected time of the call, in us
 double prefill_tc5_us(const vfkv_ctx *ctx, uint32_t dtype, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m, uint32_t q_start,
                       uint32_t n_kv, uint32_t kv_start, uint32_t window);
+// at most three quarters of the SMs have a block of 256 rows, and none of them ten tiles of 128 positions
+bool prefill_tc5_short(const vfkv_ctx *ctx, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m, uint32_t q_start,
+                       uint32_t n_kv, uint32_t kv_start, uint32_t window);
 int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, const uint8_t *v, const float *q, float *out,
                            uint64_t row_bytes, uint32_t n_q_heads, uint32_t n_kv_heads, uint32_t m, uint32_t q_start,
                            uint32_t n_kv, uint32_t kv_start, uint32_t window, float scale, float softcap,

@@ -117,3 +117,37 @@ def test_host_token_pinned_buffers_and_replays(ctx, n_layers, n, pinned):
         fwd.workspace.destroy()
         ref.workspace.destroy()
         cache.destroy()
+
+
+@pytest.mark.parametrize("dtype,hq,hkv,d,layers,L", [
+    ("F8", 32, 8, 128, 20, 8192),          # heads on the N side: one CTA for each of 160 groups
+    ("F16", 64, 8, 128, 20, 8192),         # heads on the M side
+    ("F16", 32, 4, 256, 12, 16384),
+    ("F16", 16, 2, 512, 4, 20000),         # attn_wide.cu
+])
+def test_long_sums_keep_their_accuracy(ctx, dtype, hq, hkv, d, layers, L):
+    """Layers that share a launch leave a warp a long line of positions.  What its sums lose there (to the tensor cores'
+    cutting off: 2^-24 of the sum for each product) must not exceed what f32 sums lose: results within 2^-20."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(layers, hkv, d, L), vf.KvDtype[dtype])
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    try:
+        rows = torch.randn(layers, 2, L, hkv, d, device="cuda", generator=gen)
+        rows = rows.to(torch.float8_e4m3fn).float() if dtype == "F8" else rows.half().float()
+        for i in range(layers):
+            fwd.b_step_kv_write(i, rows[i, 0, :L - 1], rows[i, 1, :L - 1], L - 1, 0)
+        q, out = torch.randn(layers, 1, hq, d, device="cuda", generator=gen), torch.zeros(layers, 1, hq, d, device="cuda")
+        new = rows[:, :, L - 1].contiguous()
+        fwd.decode_token(q, new[:, 0].contiguous(), new[:, 1].contiguous(), out, None,
+                         torch.tensor([L - 1], dtype=torch.int32, device="cuda"), 1, L)
+        worst = 0.0
+        for i in range(layers):
+            k, v = rows[i, 0].double(), rows[i, 1].double()
+            s = torch.einsum("hgd,lhd->hgl", q[i, 0].double().view(hkv, hq // hkv, d), k) / d ** 0.5
+            want = torch.einsum("hgl,lhd->hgd", s.softmax(-1), v).reshape(hq, d)
+            worst = max(worst, float((out[i, 0].double() - want).norm() / want.norm()))
+        assert worst < 2.0 ** -20
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

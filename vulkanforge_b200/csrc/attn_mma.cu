@@ -686,8 +686,37 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     float acc[NACC][4];
 #pragma unroll
     for (int nb = 0; nb < NACC; ++nb) { acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.f; }
+    // A long sum loses what its terms have below its own last bit: a row's sum of p to rounding, the accumulators to the
+    // tensor cores' cutting off towards zero (one sequence of 8192 FP8 positions, 64 tiles a warp: results 1.8e-6 off,
+    // 6e-7 in chains).  So a chain of products is some tiles long, and the chains of the high terms (the low ones are
+    // 2^11 smaller) and of l add up in f32 registers of their own.  The shape with two stages and three CTAs an SM is
+    // chosen for eight tiles or less.
+    constexpr bool CHAINS = !ROWS2 && !(W == 4 && NS == 2 && S::STAGE_BYTES <= 8192);
+    constexpr uint32_t kChain = 8;
+    float tot[CHAINS ? NACC : 1][2], l_tot = 0.f, m_tot = kMaskedScore;      // relative to the maximum (and the scale) they were left at
+    uint32_t vs_tot = 0u;
+#pragma unroll
+    for (int nb = 0; nb < (CHAINS ? NACC : 1); ++nb) { tot[nb][0] = tot[nb][1] = 0.f; }
     bool timed_out = false;
     uint32_t vs_ref = 0u;                // SC: exponent bits of the largest V scale so far; acc is relative to it
+    // the high terms of a chain (columns 0 and 2 of the transposed form, rows 0 and 1 of the other) onto those before
+    constexpr int HI1 = TR ? 2 : 1;
+    auto end_chain = [&]() {
+        if constexpr (CHAINS) {
+            float f = fast_exp2(m_tot - m[0]);
+            l_tot = fmaf(l_tot, f, l[0]);
+            l[0] = 0.f;
+            if constexpr (SC) f *= vs_tot != 0u && vs_ref - vs_tot < (127u << 23) ? __uint_as_float((127u << 23) - (vs_ref - vs_tot)) : 0.f;
+#pragma unroll
+            for (int nb = 0; nb < NACC; ++nb) {
+                tot[nb][0] = fmaf(tot[nb][0], f, acc[nb][0]);
+                tot[nb][1] = fmaf(tot[nb][1], f, acc[nb][HI1]);
+                acc[nb][0] = acc[nb][HI1] = 0.f;
+            }
+            m_tot = m[0];
+            vs_tot = vs_ref;
+        }
+    };
     // ---- split ticket -----------------------------------------------------------------------------
     // Every CTA of a (sequence, kv-head) draws one ticket from a 64-bit word that only ever counts
     // up; there is one word per split count, so ticket / n_splits is the number of the launch among
@@ -957,6 +986,9 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         }
         }
 
+        if constexpr (CHAINS)
+            if (n % kChain == kChain - 1u) end_chain();
+
         // ---- refill this stage -----------------------------------------------------------------
         // The stage was only read (ldmatrix / ld.shared) since its barrier completed, except in a
         // split's last tile, which is never refilled; __syncwarp orders those reads before the issue.
@@ -994,6 +1026,13 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     VFKV_TRACE(6);
     const bool gave_up = s_flag != 0u;
     if (gave_up && mp.cluster == 0u) return;      // in a cluster every CTA has to reach the cluster barriers
+
+    if constexpr (CHAINS) {
+        end_chain();
+        l[0] = l_tot;
+#pragma unroll
+        for (int nb = 0; nb < NACC; ++nb) { acc[nb][0] = tot[nb][0]; acc[nb][HI1] = tot[nb][1]; }
+    }
 
     // ---- merge the warps' partials in shared memory ---------------------------------------------
     constexpr int NH = (FP8 || !ROWS2) ? 8 : 16;              // head rows this CTA can hold

@@ -1,0 +1,51 @@
+"""Memory that the library shares between calls, when the calls come on several streams."""
+import numpy as np
+import pytest
+
+import vulkanforge_b200 as vf
+
+pytestmark = pytest.mark.gpu
+
+
+def _attention(q, k, v, first):
+    """float64 attention of queries at positions first.. over k and v."""
+    import torch
+    m, hq, d = q.shape
+    L, hkv = k.shape[:2]
+    s = torch.einsum("mhgd,lhd->hgml", q.double().view(m, hkv, hq // hkv, d), k.double()) / d ** 0.5
+    s = s.masked_fill(torch.arange(L, device="cuda") > first + torch.arange(m, device="cuda")[:, None], -float("inf"))
+    return torch.einsum("hgml,lhd->mhgd", s.softmax(-1), v.double()).reshape(m, hq, d)
+
+
+def test_new_memory_is_clear_before_its_first_use(ctx):
+    """A workspace and a stream's scratch, made while the default stream is busy and used on another one at once."""
+    import torch
+    hq, hkv, d, L, m = 32, 8, 128, 16384, 256                    # pieces put together by the launch itself, by flags
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    k, v = (torch.randn(L, hkv, d, device="cuda", generator=gen).half().float() for _ in range(2))
+    q = torch.randn(m, hq, d, device="cuda", generator=gen)
+    own = vf.Context(0)
+    own.set_attn_tuning(8, 3)
+    cache = vf.KvCache(own, vf.KvCacheConfig(1, hkv, d, L), vf.KvDtype.F16)
+    stream = torch.cuda.Stream()
+    fwd = None
+    try:
+        out, row = torch.zeros_like(q), torch.zeros(1, hq, d, device="cuda")
+        torch.cuda.synchronize()
+        torch.cuda._sleep(200_000_000)                           # some 0.1 s on the default stream
+        fwd = vf.CudaForward(own, cache, n_heads=hq)
+        fwd.stream = stream.cuda_stream
+        fwd.b_step_kv_write(0, k, v, L, 0)
+        torch.cuda._sleep(200_000_000)
+        fwd.run_flash_attn_batch(0, q, out, m, L - m, L, 0, 0)
+        fwd.step_attention(0, q[-1:], row, L - 1)
+        torch.cuda.synchronize()
+        own.poll()
+        want = _attention(q, k, v, L - m)
+        assert float((out - want).norm() / want.norm()) < 2e-3
+        assert float((row - want[-1:]).norm() / want[-1:].norm()) < 1e-5
+    finally:
+        if fwd:
+            fwd.workspace.destroy()
+        cache.destroy()
+        own.destroy()

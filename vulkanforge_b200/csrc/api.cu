@@ -506,6 +506,8 @@ int32_t vfkv_workspace_create(vfkv_ctx *ctx, uint32_t max_seqs, uint32_t n_q_hea
     uint8_t *base = nullptr;
     cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&base), ws->bytes);
     if (e == cudaSuccess) e = cudaMemset(base, 0, zeroed);
+    // the first call may come on a stream that nothing orders behind this one
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
         cudaFree(base);
         cudaGetLastError();

@@ -1363,9 +1363,9 @@ float *prefill_scratch(vfkv_ctx *ctx, cudaStream_t st, uint64_t *floats)
             cudaStreamIsCapturing(st, &capturing);
             if (capturing != cudaStreamCaptureStatusNone) break;
             void *d = nullptr;
-            // the pieces, then one flag per CTA
+            // the pieces, then one flag per CTA, cleared in the order of the stream that will use them
             if (cudaMalloc(&d, n * sizeof(float) + n_sm * sizeof(uint32_t)) != cudaSuccess ||
-                cudaMemset(static_cast<float *>(d) + n, 0, n_sm * sizeof(uint32_t)) != cudaSuccess) {
+                cudaMemsetAsync(static_cast<float *>(d) + n, 0, n_sm * sizeof(uint32_t), st) != cudaSuccess) {
                 (void)cudaGetLastError();
                 cudaFree(d);
                 return nullptr;

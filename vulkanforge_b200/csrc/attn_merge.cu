@@ -26,6 +26,15 @@ merge_kernel(const float *__restrict__ pm, const float *__restrict__ pl, const f
         orow = uint64_t(lr.layer_ids[i]) * lr.per_layer + (blockIdx.x - i * lr.per_layer);
     }
     pdl_wait();
+    if (n_parts == 0u) {                                // nothing to merge: an empty range
+        const uint32_t d = blockIdx.y * 128 + threadIdx.x;
+        if (d < head_dim) {
+            if (out) out[orow * head_dim + d] = 0.f;
+            if (out_o) out_o[orow * head_dim + d] = 0.f;
+        }
+        if (out_o && d == 0) { out_m[orow] = kMaskedScore; out_l[orow] = 0.f; }
+        return;
+    }
     __shared__ float s_red[4], s_sum[4], s_acc[4][128];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // The shader walks the partials with a running (max, sum, acc); the same result, up to

@@ -151,3 +151,29 @@ def test_long_sums_keep_their_accuracy(ctx, dtype, hq, hkv, d, layers, L):
     finally:
         fwd.workspace.destroy()
         cache.destroy()
+
+
+def test_phase_trace_stays_in_its_buffer(ctx):
+    """A ring of one block for each layer's launch (16 x 8 bytes a CTA): decode_token fills it and writes nothing behind it."""
+    import torch
+    hq, hkv, d, layers, L, splits = 32, 8, 128, 6, 4096, 4
+    own = vf.Context(0)
+    cache = vf.KvCache(own, vf.KvCacheConfig(layers, hkv, d, L), vf.KvDtype.F8)
+    fwd = vf.CudaForward(own, cache, n_heads=hq, n_splits=splits)
+    try:
+        cache.zero_fill()
+        words = layers * hkv * splits * 16
+        ring = torch.zeros(words + 65536, dtype=torch.int64, device="cuda")
+        q, out = (torch.zeros(layers, 1, hq, d, device="cuda") for _ in range(2))
+        kv = torch.zeros(2, layers, 1, hkv, d, device="cuda")
+        own.check(own._lib.vfkv_ctx_set_trace_buffer(own.handle, ring.data_ptr()))
+        own.check(own._lib.vfkv_ctx_set_trace_ring(own.handle, layers))
+        for _ in range(3):
+            fwd.decode_token(q, kv[0], kv[1], out, None, torch.tensor([L - 1], dtype=torch.int32, device="cuda"), 1, L)
+        torch.cuda.synchronize()
+        assert (ring[:words].view(-1, 16)[:, 0] != 0).all() and not ring[words:].any()
+    finally:
+        own.check(own._lib.vfkv_ctx_set_trace_buffer(own.handle, None))
+        fwd.workspace.destroy()
+        cache.destroy()
+        own.destroy()

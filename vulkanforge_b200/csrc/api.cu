@@ -781,7 +781,8 @@ static int32_t decode_layers(vfkv_cache *cache, vfkv_workspace *ws, uint32_t l0,
     // a grid holds at most 65535 units, and the row coordinate of a tensor map is a signed 32-bit number
     uint32_t most = 65535u / n_seqs;
     if (most > kMaxLaunchLayers) most = kMaxLaunchLayers;
-    if (most < 2 || (fused && cache->tm_all_state != 1)) {
+    // the phase trace has room for the grids of single layers
+    if (most < 2 || ctx->d_trace || (fused && cache->tm_all_state != 1)) {
         const uint64_t q_stride = uint64_t(n_seqs) * n_q_heads * D, kv_stride = uint64_t(n_seqs) * Hkv * D;
         for (uint32_t l = l0; l < l1; ++l) {
             rc = vfkv_decode_step(cache, ws, l, d_q + l * q_stride, d_k + l * kv_stride, d_v + l * kv_stride,

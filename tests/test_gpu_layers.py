@@ -177,3 +177,45 @@ def test_phase_trace_stays_in_its_buffer(ctx):
         fwd.workspace.destroy()
         cache.destroy()
         own.destroy()
+
+
+def test_recorded_token_follows_the_scale_planes(ctx):
+    """A cache made anew where another one's K and V lay, with its scales elsewhere: the token recorded for the old one
+    (same buffers, same sizes) is not the new one's."""
+    import ctypes as C
+    import torch
+    hq, hkv, d, layers, L = 16, 8, 128, 2, 4096
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    rows = torch.randn(layers, 2, L, hkv, d, device="cuda", generator=gen)
+    q, out = (torch.zeros(layers, 1, hq, d).pin_memory() for _ in range(2))
+    q.copy_(torch.randn(layers, 1, hq, d))
+    new = rows[:, :, L - 1].cpu()
+    k, v = new[:, 0].contiguous().pin_memory(), new[:, 1].contiguous().pin_memory()
+    pos = np.array([L - 1], np.uint32)
+    ws, fillers, planes = None, [], layers * L * hkv * 4
+    stream = torch.cuda.Stream()
+    try:
+        for again in range(2):
+            cache = vf.KvCache(ctx, vf.KvCacheConfig(layers, hkv, d, L, scale_mode=1), vf.KvDtype.F8)
+            fwd = vf.CudaForward(ctx, cache, n_heads=hq, workspace=ws)
+            ws, fwd.stream = fwd.workspace, stream.cuda_stream
+            scale = 1.0 + 3.0 * again
+            for i in range(layers):
+                fwd.b_step_kv_write(i, rows[i, 0, :L - 1] * scale, rows[i, 1, :L - 1] * scale, L - 1, 0)
+            for _ in range(3):                             # remembered, recorded, replayed
+                fwd.decode_token_host(q, k, v, out, pos, 1)
+            want = torch.zeros(layers, 1, hq, d, device="cuda")
+            dq, dk, dv = q.cuda(), k.cuda(), v.cuda()
+            for i in range(layers):
+                fwd.decode_step(i, dq[i], dk[i], dv[i], want[i], None, to_dev(pos), 1, L)
+            torch.cuda.synchronize()
+            assert float((out - want.cpu()).abs().max()) < 1e-5 * max(1.0, float(want.abs().max()))
+            cache.destroy()
+            for _ in range(2):                             # where the scales lay
+                p = C.c_void_p()
+                ctx.check(ctx._lib.vfkv_malloc(ctx.handle, planes, C.byref(p)))
+                fillers.append(p)
+    finally:
+        for p in fillers:
+            ctx.check(ctx._lib.vfkv_free(ctx.handle, p))
+        ws.destroy()

@@ -1006,6 +1006,7 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
     for (uint32_t l = 0; windows && l < L; ++l) mix(windows[l]);
     // a cache object re-created at the same address must not find the old graphs
     mix(reinterpret_cast<uint64_t>(kv.k_buffer)); mix(reinterpret_cast<uint64_t>(kv.v_buffer));
+    mix(reinterpret_cast<uint64_t>(kv.k_scales)); mix(reinterpret_cast<uint64_t>(kv.v_scales));
     mix(L); mix(D); mix(Hkv); mix(uint64_t(kv.kv_dtype)); mix(kv.config.max_seq_len); mix(kv.config.n_slots);
     mix(kv.config.scale_mode); mix(ctx->merge_wait_ns); mix(ctx->debug_fail_split);
     uint32_t fs, fc;
@@ -1134,6 +1135,7 @@ int32_t vfkv_decode_token_host_submit(vfkv_cache *cache, vfkv_workspace *ws, con
     auto mix = [&](uint64_t x) { wh = (wh ^ x) * 1099511628211ull; };
     for (uint32_t l = 0; windows && l < L; ++l) mix(windows[l]);
     mix(reinterpret_cast<uint64_t>(kv.k_buffer)); mix(reinterpret_cast<uint64_t>(kv.v_buffer));
+    mix(reinterpret_cast<uint64_t>(kv.k_scales)); mix(reinterpret_cast<uint64_t>(kv.v_scales));
     mix(L); mix(D); mix(Hkv); mix(uint64_t(kv.kv_dtype)); mix(kv.config.max_seq_len); mix(kv.config.n_slots);
     mix(reinterpret_cast<uint64_t>(ws->tag_part));
     uint32_t fs, fc;

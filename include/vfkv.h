@@ -566,7 +566,8 @@ int32_t vfkv_ctx_set_trace_buffer(vfkv_ctx *ctx, void *d_buffer);
 int32_t vfkv_ctx_set_trace_ring(vfkv_ctx *ctx, uint32_t n_blocks);
 /* Kernels this context has launched since creation (for launch accounting); one that carries several
  * layers of a token (vfkv_decode_token) counts once for each layer, so that the count of a step does
- * not depend on how its layers are grouped.  vfkv_ctx_kernel_count counts it once. */
+ * not depend on how its layers are grouped.  vfkv_ctx_kernel_count counts it once, and the kernel that
+ * fetches the inputs of a small vfkv_decode_token_host from pinned memory, which belongs to no layer. */
 uint64_t vfkv_ctx_launch_count(const vfkv_ctx *ctx);
 uint64_t vfkv_ctx_kernel_count(const vfkv_ctx *ctx);
 

@@ -219,3 +219,23 @@ def test_recorded_token_follows_the_scale_planes(ctx):
         for p in fillers:
             ctx.check(ctx._lib.vfkv_free(ctx.handle, p))
         ws.destroy()
+
+
+def test_kernel_count_of_a_host_token(ctx):
+    """From pinned buffers: one kernel fetches the inputs, one does all layers, recorded or not."""
+    import torch
+    hq, hkv, d, layers = 16, 8, 128, 3
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(layers, hkv, d, 64), vf.KvDtype.F8)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    stream = torch.cuda.Stream()
+    try:
+        fwd.stream = stream.cuda_stream
+        q, out = (torch.zeros(layers, 1, hq, d).pin_memory() for _ in range(2))
+        k, v = (torch.zeros(layers, 1, hkv, d).pin_memory() for _ in range(2))
+        for p in range(4):
+            kernels, launches = ctx.kernel_count(), ctx.launch_count()
+            fwd.decode_token_host(q, k, v, out, np.array([p], np.uint32), 1)
+            assert (ctx.kernel_count() - kernels, ctx.launch_count() - launches) == (2, layers)
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

@@ -325,6 +325,7 @@ int32_t launch_stage_in(vfkv_ctx *ctx, const StageArgs &a, cudaStream_t st)
     uint64_t blocks = (units + 255) / 256, cap = uint64_t(ctx->sm_count) * 4;
     if (blocks > cap) blocks = cap;
     const cudaError_t e = launch_dependent(ctx, stage_in_kernel, dim3(unsigned(blocks)), dim3(256), 0, st, a);
+    ++ctx->kernels;                // belongs to no layer: not in `launches`
     ctx->set_written_any();        // what follows reads its positions from here: no reading ahead
     return check_cuda(ctx, e, "stage_in launch");
 }

@@ -40,7 +40,8 @@ struct vfkv_ctx {
     uint32_t debug_fail_split = 0xFFFFFFFFu;  // failure injection for tests (vfkv_ctx_debug_fail_split)
     uint32_t cluster_merge = 0;        // 1: merge the splits inside a thread-block cluster where the device allows it
     // kernels enqueued, and the same count with a kernel that carries several layers of a token
-    // counted once for each of them (so that it does not depend on how layers are grouped)
+    // counted once for each of them (so that it does not depend on how layers are grouped) and the
+    // one that fetches a host token's inputs not at all
     uint64_t kernels = 0, launches = 0;
     void count_launch(uint32_t layers = 1) { ++kernels; launches += layers; }
     unsigned long long *d_trace = nullptr;   // caller-owned device buffer for kernel phase timestamps, or null

@@ -60,3 +60,26 @@ def test_wide_shapes_match_the_cuda_core_kernel(ctx, dtype, scaled, hq, hkv, d, 
         ctx.set_attn_impl(0)
         fwd.workspace.destroy()
         cache.destroy()
+
+
+def test_impl_3_decodes_as_0(ctx):
+    """attn_impl 3 differs from 0 in prefill only: the same kernel, so the same bits (the CUDA-core kernel's are others)."""
+    import torch
+    hq, hkv, d, L = 16, 2, 512, 700
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, L), vf.KvDtype.F16)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    try:
+        kv = torch.randn(2, L, hkv, d, device="cuda", generator=gen)
+        fwd.b_step_kv_write(0, kv[0], kv[1], L, 0)
+        q, got = torch.randn(hq, d, device="cuda", generator=gen), {}
+        for impl in (0, 1, 3):
+            ctx.set_attn_impl(impl)
+            got[impl] = torch.zeros_like(q)
+            fwd.step_attention(0, q, got[impl], L - 1)
+        torch.cuda.synchronize()
+        assert torch.equal(got[3], got[0]) and not torch.equal(got[1], got[0])
+    finally:
+        ctx.set_attn_impl(0)
+        fwd.workspace.destroy()
+        cache.destroy()

@@ -238,7 +238,7 @@ int32_t launch_attention(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, c
     const bool mma_ok = attn_mma_supported(a);
     if (ctx->attn_impl == 2 && !mma_ok)
         return set_error(ctx, VFKV_ERR_UNSUPPORTED, "shape outside the tensor-core attention kernel");
-    const bool use_mma = mma_ok && ctx->attn_impl != 1, use_wide = !mma_ok && ctx->attn_impl == 0 && attn_wide_supported(a);
+    const bool use_mma = mma_ok && ctx->attn_impl != 1, use_wide = !mma_ok && ctx->attn_impl != 1 && attn_wide_supported(a);
 
     uint32_t n_splits = a.n_splits ? a.n_splits : choose_splits(ctx, a, use_mma ? 128 : use_wide ? 64 : 32);
     if (n_splits > 1) {

@@ -48,8 +48,7 @@ template <> struct Enc<VFKV_F32> {  // 4 elements -> 16 bytes
 
 // ---- raw store: n f32 -> dst, 16-byte vector body + word-sized tail -------
 template <int DT>
-__global__ void __launch_bounds__(256) store_vec_kernel(const float *__restrict__ src,
-                                                        uint8_t *__restrict__ dst, uint64_t n)
+__global__ void __launch_bounds__(256) store_vec_kernel(const float *src, uint8_t *dst, uint64_t n)
 {
     constexpr int E = Enc<DT>::kElems;
     const uint64_t n_vec = n / E;
@@ -64,8 +63,7 @@ __global__ void __launch_bounds__(256) store_vec_kernel(const float *__restrict_
 // One 32-bit word per thread, exactly the reference's granularity, with its
 // zero padding of a ragged tail (kv_store_fp8.comp:58-66, kv_copy_fp16.comp:46-50).
 template <int DT>
-__global__ void __launch_bounds__(256) store_word_kernel(const float *__restrict__ src,
-                                                         uint32_t *__restrict__ dst,
+__global__ void __launch_bounds__(256) store_word_kernel(const float *src, uint32_t *dst,
                                                          uint64_t first, uint64_t n)
 {
     constexpr int W = DT == VFKV_F8 ? 4 : DT == VFKV_F16 ? 2 : 1;
@@ -334,8 +332,7 @@ int32_t launch_stage_in(vfkv_ctx *ctx, const StageArgs &a, cudaStream_t st)
 // HBM-bound: 3 bytes an element.  A thread has four 16-byte loads in flight, and stores 32 bytes, a
 // whole sector, at a time (two 16-byte stores 32 bytes apart write every sector twice by halves).
 constexpr int kCvtUnroll = 4;
-__global__ void __launch_bounds__(256) fp8_to_f16_vec_kernel(const uint4 *__restrict__ src,
-                                                             uint4 *__restrict__ dst, uint64_t n_vec, bool wide)
+__global__ void __launch_bounds__(256) fp8_to_f16_vec_kernel(const uint4 *src, uint4 *dst, uint64_t n_vec, bool wide)
 {
     pdl_wait();
     const uint64_t first = blockIdx.x * uint64_t(256 * kCvtUnroll) + threadIdx.x;
@@ -365,8 +362,7 @@ __global__ void __launch_bounds__(256) fp8_to_f16_vec_kernel(const uint4 *__rest
     }
 }
 
-__global__ void __launch_bounds__(256) fp8_to_f16_scalar_kernel(const uint8_t *__restrict__ src,
-                                                                __half *__restrict__ dst,
+__global__ void __launch_bounds__(256) fp8_to_f16_scalar_kernel(const uint8_t *src, __half *dst,
                                                                 uint64_t first, uint64_t n)
 {
     pdl_wait();

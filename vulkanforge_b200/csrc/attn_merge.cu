@@ -14,10 +14,9 @@ namespace vfkv {
 struct LayerRows { uint32_t per_layer; uint16_t layer_ids[kMaxLaunchLayers]; };
 
 __global__ void __launch_bounds__(128)
-merge_kernel(const float *__restrict__ pm, const float *__restrict__ pl, const float *__restrict__ po,
+merge_kernel(const float *pm, const float *pl, const float *po,
              uint32_t n_parts, uint64_t ml_part, uint64_t ml_row, uint64_t o_part, uint64_t o_row, uint32_t head_dim,
-             float *__restrict__ out, float *__restrict__ out_m, float *__restrict__ out_l,
-             float *__restrict__ out_o, const LayerRows lr)
+             float *out, float *out_m, float *out_l, float *out_o, const LayerRows lr)
 {
     const uint64_t row = blockIdx.x;
     uint64_t orow = row;

@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(256) prefill_tc5_kernel(const Tc5Params p)
                     const uint32_t idx = tid + 256 * (i & 3), pos = idx >> 3, c16 = idx & 7u;
                     const bool ok = t0 + pos < p.n_kv;
                     const uint64_t off = uint64_t(ok ? t0 + pos : 0u) * p.row_bytes + c16 * 16;
-                    raw[i] = ok ? __ldg(reinterpret_cast<const uint4 *>((i < 4 ? kg : vg) + off)) : make_uint4(0u, 0u, 0u, 0u);
+                    raw[i] = ok ? *reinterpret_cast<const uint4 *>((i < 4 ? kg : vg) + off) : make_uint4(0u, 0u, 0u, 0u);
                 }
                 auto widen = [&](int i) {
                     const uint32_t idx = tid + 256 * (i & 3), pos = idx >> 3, c16 = idx & 7u;
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(256) prefill_tc5_kernel(const Tc5Params p)
                     const uint32_t idx = tid + 256 * i, pos = idx >> 4, c = idx & 15u;
                     const bool ok = t0 + pos < p.n_kv;
                     const uint64_t off = uint64_t(ok ? t0 + pos : 0u) * p.row_bytes + c * 16;
-                    raw[i] = ok ? __ldg(reinterpret_cast<const uint4 *>(src + off)) : make_uint4(0u, 0u, 0u, 0u);
+                    raw[i] = ok ? *reinterpret_cast<const uint4 *>(src + off) : make_uint4(0u, 0u, 0u, 0u);
                 }
             };
             auto place = [&](uint32_t tile_sm) {
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(256, 1) prefill_tc5p_kernel(const Tc5Params p)
             const uint32_t pos = DT == VFKV_F8 ? idx >> 3 : idx >> 4, c = DT == VFKV_F8 ? idx & 7u : idx & 15u;
             const bool ok = t0 + pos < p.n_kv;
             const uint64_t off = uint64_t(ok ? t0 + pos : 0u) * p.row_bytes + c * 16;
-            raw[i] = ok ? __ldg(reinterpret_cast<const uint4 *>(src + off)) : make_uint4(0u, 0u, 0u, 0u);
+            raw[i] = ok ? *reinterpret_cast<const uint4 *>(src + off) : make_uint4(0u, 0u, 0u, 0u);
         }
     };
     auto place = [&](const uint4 (&raw)[NP], uint32_t tile_sm) {
@@ -871,8 +871,8 @@ __global__ void __launch_bounds__(kThreadsH<DT>, 1) prefill_tc5h_kernel(const Tc
                     const uint32_t i = i0 + QT * u, row = i >> 4, c = i & 15u, rr = row0 + row;
                     const bool in = i < uint32_t(CTA_ROWS * 16) && rr < n_rows;
                     const float *qp = p.q + (uint64_t(in ? rr >> g_shift : 0u) * p.n_q_heads + kvh * g + (in ? rr & (g - 1u) : 0u)) * HD + 8 * c;
-                    qa[u] = in ? __ldg(reinterpret_cast<const float4 *>(qp)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    qb[u] = in ? __ldg(reinterpret_cast<const float4 *>(qp + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    qa[u] = in ? *reinterpret_cast<const float4 *>(qp) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    qb[u] = in ? *reinterpret_cast<const float4 *>(qp + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
                 for (uint32_t u = 0; u < QB; ++u) {
@@ -1149,7 +1149,7 @@ __global__ void __launch_bounds__(kThreadsH<DT>, 1) prefill_tc5h_kernel(const Tc
                         const uint32_t pos = DT == VFKV_F8 ? idx >> 3 : idx >> 4, c = DT == VFKV_F8 ? idx & 7u : idx & 15u;
                         const bool in = idx < PIECES && t0 + pos < p.n_kv;
                         const uint64_t off = uint64_t(in ? t0 + pos : 0u) * p.row_bytes + c * 16;
-                        raw[i] = in ? __ldg(reinterpret_cast<const uint4 *>(src + off)) : make_uint4(0u, 0u, 0u, 0u);
+                        raw[i] = in ? *reinterpret_cast<const uint4 *>(src + off) : make_uint4(0u, 0u, 0u, 0u);
                     }
                     // the buffer is free once the products of the tile that used it two tiles ago are complete
                     if (pass == 0 && gi >= 2u && !mbar_wait(free_bar, ((gi >> 1) & 1u) ^ 1u)) ok = false;

@@ -145,7 +145,7 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
         for (uint32_t i = 0; i < NP; ++i) {
             const uint32_t idx = pt + 96u * i, pos = t0 + idx / (D / 16), c = idx % (D / 16);
             const bool in = idx < PIECES && pos < p.n_kv;
-            raw[i] = in ? __ldg(reinterpret_cast<const uint4 *>(src + uint64_t(pos) * p.row_bytes + c * 16)) : make_uint4(0u, 0u, 0u, 0u);
+            raw[i] = in ? *reinterpret_cast<const uint4 *>(src + uint64_t(pos) * p.row_bytes + c * 16) : make_uint4(0u, 0u, 0u, 0u);
         }
     };
     if constexpr (FP8)
@@ -162,8 +162,8 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
                 const uint32_t idx = (c0 + 11u * u) * 32u + lane, r = row0 + idx / (D / 8), c = idx % (D / 8);
                 const bool in = c0 + 11u * u < CHUNKS && r < n_rows;
                 const float4 *src = reinterpret_cast<const float4 *>(p.q + (uint64_t(r / g) * p.n_q_heads + kvh * g + r % g) * D + 8 * c);
-                a[u] = in ? __ldg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
-                b[u] = in ? __ldg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+                a[u] = in ? *src : make_float4(0.f, 0.f, 0.f, 0.f);
+                b[u] = in ? src[1] : make_float4(0.f, 0.f, 0.f, 0.f);
             }
 #pragma unroll
             for (uint32_t u = 0; u < QB; ++u) {
@@ -220,8 +220,8 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
             for (uint32_t i = 0; i < 2; ++i) {
                 const uint32_t pos = c_lo + it * BN + lane + 32u * i;
                 const bool in = it < n_tiles && pos < p.n_kv;
-                ks_next[i] = in ? __ldg(p.k_scales + uint64_t(pos) * p.n_kv_heads + kvh) : 1.f;
-                vs_next[i] = in ? __ldg(p.v_scales + uint64_t(pos) * p.n_kv_heads + kvh) : 0.f;
+                ks_next[i] = in ? p.k_scales[uint64_t(pos) * p.n_kv_heads + kvh] : 1.f;
+                vs_next[i] = in ? p.v_scales[uint64_t(pos) * p.n_kv_heads + kvh] : 0.f;
             }
         };
         if constexpr (SC) load_scales(0);

@@ -239,6 +239,9 @@ inline cudaError_t launch_dependent(const vfkv_ctx *ctx, void (*kern)(P...), dim
 
 #ifdef __CUDACC__
 // Waits for everything in front of this kernel on its stream, then lets the next kernel be scheduled.
+// A kernel that begins with it may be resident while its inputs are still being written.  So it reads them with plain
+// loads, which stay behind the wait: __ldg, the L1's read-only path and what const __restrict__ allows a compiler
+// are for memory that nobody writes while the kernel lives.
 // Nothing that the predecessor may have written, and nothing that it may still read, is touched before.
 // (The release comes after the wait, so a kernel that reads ahead of its own wait only ever overlaps
 // its direct predecessor.)  Both do nothing in a launch without the attribute.

@@ -60,8 +60,8 @@ __device__ __forceinline__ bool await_word(const uint64_t *p, uint64_t &w, uint3
 // requested at once; only those whose tag is not there yet are polled.  A wait that runs out sets
 // bit 8 of the status word and the row is written as zeros.
 __global__ void __launch_bounds__(128)
-exchange_merge_kernel(PeerFanout fan, const uint64_t *__restrict__ local, uint32_t *__restrict__ ctl,
-                      uint32_t head_dim, uint64_t wait_ns, float *__restrict__ out, uint32_t *__restrict__ status)
+exchange_merge_kernel(PeerFanout fan, const uint64_t *local, uint32_t *ctl, uint32_t head_dim, uint64_t wait_ns,
+                      float *out, uint32_t *status)
 {
     constexpr int kMaxDims = 4, kMaxWorld = 8;
     __shared__ float s_m[kMaxWorld], s_l[kMaxWorld];

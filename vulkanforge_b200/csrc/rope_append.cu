@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kRopeThreads) rope_append_kernel(const RopeApp
         auto load = [&](const float *src) {
 #pragma unroll
             for (int j = 0; j < E; j += 4) {
-                const float4 f = __ldg(reinterpret_cast<const float4 *>(src + j));
+                const float4 f = *reinterpret_cast<const float4 *>(src + j);
                 x[j] = f.x; x[j + 1] = f.y; x[j + 2] = f.z; x[j + 3] = f.w;
             }
         };
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(kRopeThreads) rope_append_kernel(const RopeApp
             const float2 *const cs = table + r * half + d0;
 #pragma unroll
             for (int j = 0; j < E; j += 4) {
-                const float4 f = __ldg(reinterpret_cast<const float4 *>(src + half + d0 + j));
+                const float4 f = *reinterpret_cast<const float4 *>(src + half + d0 + j);
                 const float b[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kRopeThreads) rope_append_kernel(const RopeApp
 // or not.  grid.y cuts the heads of a few rows over several blocks.
 __global__ void __launch_bounds__(kRopeThreads)
 rope_rows_kernel(const float *x, float *out, uint32_t n_rows, uint32_t n_heads, uint32_t head_dim, uint32_t heads_per_block,
-                 const uint32_t *__restrict__ positions, uint32_t base_pos, uint32_t n_dims, float theta_scale,
+                 const uint32_t *positions, uint32_t base_pos, uint32_t n_dims, float theta_scale,
                  float freq_scale, uint32_t rows_per_block)
 {
     extern __shared__ float2 table[];
@@ -190,7 +190,7 @@ rope_rows_kernel(const float *x, float *out, uint32_t n_rows, uint32_t n_heads, 
 // The same for shapes or buffers that do not come in 16-byte pieces: one thread per pair.
 __global__ void __launch_bounds__(256)
 rope_neox_kernel(const float *x, float *out, uint64_t n_rows, uint32_t n_heads, uint32_t head_dim,
-                 const uint32_t *__restrict__ positions, uint32_t base_pos, uint32_t n_dims, float theta_scale, float freq_scale)
+                 const uint32_t *positions, uint32_t base_pos, uint32_t n_dims, float theta_scale, float freq_scale)
 {
     const uint32_t half = n_dims / 2, tail = head_dim - n_dims;
     const uint32_t per_head = half + tail;              // work items per head: pairs, then pass-through dims

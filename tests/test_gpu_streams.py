@@ -49,3 +49,33 @@ def test_new_memory_is_clear_before_its_first_use(ctx):
             fwd.workspace.destroy()
         cache.destroy()
         own.destroy()
+
+
+def test_decode_behind_a_raw_read_out_into_its_rows(ctx):
+    """Mode-2 attention reads ahead of its predecessor, but not when that is a read-out that fills the rows it reads."""
+    import torch
+    hq, hkv, d, L = 32, 8, 128, 65536
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    src = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, L), vf.KvDtype.F8)
+    dst = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, L), vf.KvDtype.F16)
+    fill, read = vf.CudaForward(ctx, src, n_heads=hq), vf.CudaForward(ctx, dst, n_heads=hq)
+    try:
+        k, v = (torch.randn(L, hkv, d, device="cuda", generator=gen).to(torch.float8_e4m3fn).float() for _ in range(2))
+        q = torch.randn(1, hq, d, device="cuda", generator=gen)
+        fill.b_step_kv_write(0, k, v, L, 0)
+        want = _attention(q, k, v, L - 1)
+        for mode in (0, 2, 2):
+            ctx.set_dependent_launch(mode)
+            dst.zero_fill()
+            out = torch.zeros_like(q)
+            torch.cuda.synchronize()
+            fill.run_kv_fp8_to_f16(src.k_buffer, dst.k_buffer, L * hkv * d)
+            fill.run_kv_fp8_to_f16(src.v_buffer, dst.v_buffer, L * hkv * d)
+            read.step_attention(0, q, out, L - 1)
+            torch.cuda.synchronize()
+            assert float((out - want).norm() / want.norm()) < 2e-6
+    finally:
+        ctx.set_dependent_launch(0)
+        for f, c in ((fill, src), (read, dst)):
+            f.workspace.destroy()
+            c.destroy()

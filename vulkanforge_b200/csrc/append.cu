@@ -395,6 +395,7 @@ int32_t launch_fp8_to_f16(vfkv_ctx *ctx, const void *src, void *dst, uint64_t n,
             return check_cuda(ctx, e, "fp8_to_f16 launch");
         ctx->count_launch();
     }
+    ctx->set_written_any();        // a raw destination, as in launch_store_t
     return check_cuda(ctx, cudaGetLastError(), "fp8_to_f16 launch");
 }
 

@@ -128,3 +128,27 @@ def test_short_f16_calls_take_q_in_two_terms(ctx, hq, hkv, m, q_start, softcap):
     finally:
         fwd.workspace.destroy()
         cache.destroy()
+
+
+def test_more_row_blocks_than_a_grid_axis_holds(ctx):
+    """65 541 blocks of 128 rows (one kv-head, 64 q-heads of 64): every query sees a window of 1024."""
+    import torch
+    hq, hkv, d, m = 64, 1, 64, 131080
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, m), vf.KvDtype.F8)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(2)
+        k, v = (torch.randn(m, hkv, d, device="cuda", generator=gen).to(torch.float8_e4m3fn).float() for _ in range(2))
+        fwd.b_step_kv_write(0, k, v, m, 0)
+        q = torch.randn(m, hq, d, device="cuda", generator=gen)
+        out = torch.full((m, hq, d), 7.0, device="cuda")
+        fwd.run_flash_attn_batch(0, q, out, m, 0, m, 0, 0, window=1024)      # long enough a window for this kernel
+        for i in (0, 1, 127, 70000, 131070, m - 1):
+            lo = max(0, i + 1 - 1024)
+            s = q[i].double() @ k[lo:i + 1, 0].double().T / d ** 0.5
+            want = s.softmax(-1) @ v[lo:i + 1, 0].double()
+            assert float((out[i] - want).norm() / want.norm()) < 5e-3
+        assert bool(torch.isfinite(out).all()) and not bool((out == 7.0).all(2).any())
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

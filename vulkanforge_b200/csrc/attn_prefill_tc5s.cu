@@ -122,9 +122,11 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(small + 240u), "n"(T::TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    const uint32_t kvh = blockIdx.x / op.n_split, split = blockIdx.x - kvh * op.n_split;
+    // blocks in the order (row block, kv-head, piece), on the one grid axis that holds any number of them
+    const uint32_t line = blockIdx.x / op.n_split, split = blockIdx.x - line * op.n_split;
+    const uint32_t rb = line / p.n_kv_heads, kvh = line - rb * p.n_kv_heads;
     uint32_t row0, c_lo, n_tiles;
-    block_extent(p, op.n_rb, blockIdx.y, &row0, &c_lo, &n_tiles);
+    block_extent(p, op.n_rb, rb, &row0, &c_lo, &n_tiles);
     if (op.n_split > 1u) {
         const uint32_t first = uint32_t(uint64_t(n_tiles) * split / op.n_split), last = uint32_t(uint64_t(n_tiles) * (split + 1u) / op.n_split);
         c_lo += first * BN;
@@ -350,7 +352,7 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
         float row_scale;
         float *row_dst;
         if (op.n_split > 1u) {
-            float *const piece = op.scratch + (uint64_t(blockIdx.y) * gridDim.x + blockIdx.x) * T::PIECE;
+            float *const piece = op.scratch + uint64_t(blockIdx.x) * T::PIECE;
             piece[BM * D + tid] = ran ? mref : kMaskedScore;
             piece[BM * D + BM + tid] = ran ? lrow : 0.f;
             row_scale = unit;
@@ -490,7 +492,8 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
     if (warp == 4u) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "n"(T::TMEM) : "memory");
 }
 
-// The pieces of every row block put together: a warp per row.  grid = (kv-head x 16 row groups, row blocks).
+// The pieces of every row block put together: a warp per row.  grid = (kv-head x 16 row groups, row blocks: at most
+// two CTAs an SM are cut).
 template <int D>
 __global__ void __launch_bounds__(256) prefill_pieces_kernel(const OneTileParams op)
 {
@@ -605,7 +608,7 @@ int32_t launch_one_tile_t(vfkv_ctx *ctx, OneTileParams op, cudaStream_t st)
         if (op.n_split > most) op.n_split = most > 1 ? uint32_t(most) : 1u;
     }
     op.status = ctx->d_status;
-    cudaError_t e = launch_dependent(ctx, kern, dim3(op.n_split * p.n_kv_heads, op.n_rb), dim3(kThreads), T::SMEM, st, op, tm_k, tm_v);
+    cudaError_t e = launch_dependent(ctx, kern, dim3(op.n_split * p.n_kv_heads * op.n_rb), dim3(kThreads), T::SMEM, st, op, tm_k, tm_v);
     ctx->count_launch();
     if (e == cudaSuccess && op.n_split > 1) {
         e = launch_dependent(ctx, prefill_pieces_kernel<D>, dim3(p.n_kv_heads * 16, op.n_rb), dim3(256), 0, st, op);

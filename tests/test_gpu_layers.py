@@ -239,3 +239,37 @@ def test_kernel_count_of_a_host_token(ctx):
     finally:
         fwd.workspace.destroy()
         cache.destroy()
+
+
+def test_host_buffer_with_an_unregistered_page_is_not_pinned(ctx):
+    """Four pages of Q, the third not registered: no kernel reads that buffer, whatever its two ends are."""
+    import mmap
+    import torch
+    hq, hkv, d, layers, page = 16, 8, 128, 2, mmap.PAGESIZE
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(layers, hkv, d, 64), vf.KvDtype.F8)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    stream, cudart = torch.cuda.Stream(), torch.cuda.cudart()
+    memory = mmap.mmap(-1, layers * hq * d * 4)
+    q = np.frombuffer(memory, np.float32).reshape(layers, 1, hq, d)
+    at = q.ctypes.data
+    parts = [(at, 2 * page), (at + 3 * page, q.nbytes - 3 * page)]
+    q[:] = np.random.default_rng(1).standard_normal(q.shape, dtype=np.float32)
+    out = torch.zeros(layers, 1, hq, d).pin_memory()
+    k, v = (torch.randn(layers, 1, hkv, d).pin_memory() for _ in range(2))
+    try:
+        for p, n in parts:
+            assert int(cudart.cudaHostRegister(p, n, 0)) == 0
+        fwd.stream = stream.cuda_stream
+        kernels = ctx.kernel_count()
+        try:
+            fwd.decode_token_host(q, k, v, out, np.array([0], np.uint32), 1)
+        except vf.VfkvError:                               # the runtime may refuse to copy such a range
+            return
+        assert ctx.kernel_count() - kernels == 1
+        want = v.to(torch.float8_e4m3fn).float().repeat_interleave(hq // hkv, 2)     # one position: its V
+        assert float((out - want).abs().max()) < 1e-5 * float(want.abs().max())
+    finally:
+        for p, _ in parts:
+            cudart.cudaHostUnregister(p)
+        fwd.workspace.destroy()
+        cache.destroy()

@@ -154,6 +154,10 @@ int32_t vfkv_ctx_create(int32_t device_ordinal, vfkv_ctx **out)
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) == cudaSuccess &&
         qres == cudaDriverEntryPointSuccess)
         ctx->encode_tiled = fn;
+    fn = nullptr;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &qres) == cudaSuccess &&
+        qres == cudaDriverEntryPointSuccess)
+        ctx->pointer_attributes = fn;
     *out = ctx;
     return VFKV_OK;
 }
@@ -840,6 +844,22 @@ int32_t vfkv_decode_token(vfkv_cache *cache, vfkv_workspace *ws, const float *d_
                          n_seqs, max_seq_len_hint, windows, scale, softcap, n_splits, stream);
 }
 
+// Whether [p, p + bytes) lies in one pinned host allocation or registration that the device addresses as the host does.
+// (Both ends of it being pinned says nothing about what lies between two registrations.)
+static bool pinned_range(const vfkv_ctx *ctx, uintptr_t p, uint64_t bytes)
+{
+    if (!ctx->pointer_attributes) return false;
+    typedef CUresult (*Fn)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    unsigned type = 0;
+    CUdeviceptr device = 0, start = 0;
+    size_t size = 0;
+    void *to[4] = {&type, &device, &start, &size};
+    return reinterpret_cast<Fn>(ctx->pointer_attributes)(4, what, to, CUdeviceptr(p)) == CUDA_SUCCESS && type == CU_MEMORYTYPE_HOST &&
+           device == p && start <= p && p - start <= size && bytes <= size - (p - start);
+}
+
 int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const float *h_q, const float *h_k,
                                const float *h_v, float *h_out, uint32_t n_q_heads, const uint32_t *h_slot_ids,
                                const uint32_t *h_positions, uint32_t n_seqs, const uint32_t *windows, float scale,
@@ -886,16 +906,9 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
     cudaError_t e = cudaSuccess;
     // Buffers in pinned memory are on the device's own bus: the attention kernel writes its rows straight
     // into h_out, and the inputs of a small token come by one kernel.
-    auto pinned_at = [](uintptr_t p) {
-        cudaPointerAttributes at;
-        const bool ok = cudaPointerGetAttributes(&at, reinterpret_cast<void *>(p)) == cudaSuccess &&
-                        at.type == cudaMemoryTypeHost && reinterpret_cast<uintptr_t>(at.devicePointer) == p;
-        cudaGetLastError();
-        return ok;
-    };
     auto pinned = [&](const float *p, uint64_t n) {
         const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-        return a % 16 == 0 && pinned_at(a) && pinned_at(a + n * 4 - 4);
+        return a % 16 == 0 && pinned_range(ctx, a, n * 4);
     };
     const bool out_direct = pipelined && pinned(h_out, q_elems);
     const bool in_pinned = pinned(h_q, q_elems) && pinned(h_k, kv_elems) && pinned(h_v, kv_elems);

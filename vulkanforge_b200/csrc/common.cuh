@@ -47,7 +47,7 @@ struct vfkv_ctx {
     unsigned long long *d_trace = nullptr;   // caller-owned device buffer for kernel phase timestamps, or null
     uint32_t trace_ring = 1;                 // blocks in d_trace; launch k of the decode kernel writes block k % trace_ring
     uint64_t trace_seq = 0;
-    void *encode_tiled = nullptr;      // cuTensorMapEncodeTiled, resolved at run time
+    void *encode_tiled = nullptr, *pointer_attributes = nullptr;     // cuTensorMapEncodeTiled, cuPointerGetAttributes, resolved at run time
     // per-kernel GPU timing, the analogue of the reference's ShaderProfiler
     // (src/backend/vulkan/profiler.rs:28-187); off unless vfkv_profile_enable(ctx, 1)
     bool profiling = false;

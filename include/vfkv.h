@@ -505,8 +505,10 @@ int32_t vfkv_ctx_set_attn_impl(vfkv_ctx *ctx, uint32_t impl);
  * small second kernel.  With 0x0 shorter calls take a kernel with one tile of 128 rows a CTA, whose
  * items may be cut the same way.  Pieces need 39 MB of device scratch, which the context allocates
  * at a stream's first such call outside a capture, for up to four streams, and frees in
- * vfkv_ctx_destroy; on further streams nothing is cut.  A call captured on a stream without
- * scratch uses the first stream's: its replays must not overlap other such calls. */
+ * vfkv_ctx_destroy; a further stream takes over the one that was used longest ago, behind its last
+ * use.  In a capture only the even shares of the form above leave pieces: such a call uses its
+ * stream's scratch, or else the first there is, and its replays must not overlap other calls that
+ * leave pieces. */
 int32_t vfkv_ctx_set_attn_tuning(vfkv_ctx *ctx, uint32_t warps, uint32_t stages);
 /* Programmatic dependent launch of the library's kernels, the CUDA counterpart of
  * relaxing the full pipeline barrier the reference records between dispatches

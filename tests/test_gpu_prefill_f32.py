@@ -61,7 +61,8 @@ def test_f32_tiles_match_the_oracle(ctx, dtype, hq, hkv, d, m, q_start, kv_start
 
 
 def test_pieces_on_several_streams(ctx):
-    """Calls that leave pieces may overlap on different streams of a context; a fifth stream cuts nothing."""
+    """Calls that leave pieces may overlap on different streams of a context; a fifth stream takes over the
+    scratch that was used longest ago."""
     import torch
     hq, hkv, d, m, L = 32, 8, 128, 60, 500
     gen = torch.Generator(device="cuda").manual_seed(1)

@@ -79,3 +79,75 @@ def test_decode_behind_a_raw_read_out_into_its_rows(ctx):
         for f, c in ((fill, src), (read, dst)):
             f.workspace.destroy()
             c.destroy()
+
+
+def _short_prompt(ctx, n, seed):
+    """A full-precision cache with 500 positions, n query chunks of 60 (two launches: tiles in shares, then the pieces)."""
+    import torch
+    hq, hkv, d, m, L = 32, 8, 128, 60, 500
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, L), vf.KvDtype.F32)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    kv = torch.randn(2, L, hkv, d, device="cuda", generator=gen)
+    fwd.b_step_kv_write(0, kv[0], kv[1], L, 0)
+    qs = [torch.randn(m, hq, d, device="cuda", generator=gen) for _ in range(n)]
+    want = [_attention(q, kv[0], kv[1], L - m) for q in qs]
+    torch.cuda.synchronize()
+    return cache, fwd, qs, want, lambda q, o: fwd.run_flash_attn_batch(0, q, o, m, L - m, L, 0, 0)
+
+
+def test_every_stream_gets_scratch(ctx):
+    """Streams that come and go, more than there are buffers: each call leaves its pieces and no two use one buffer at once."""
+    import torch
+    own = vf.Context(0)
+    cache, fwd, qs, want, run = _short_prompt(own, 7, 5)
+    try:
+        for _ in range(3):
+            got = [torch.zeros_like(q) for q in qs]
+            streams = [torch.cuda.Stream() for _ in qs]
+            for _ in range(4):
+                for q, o, s in zip(qs, got, streams):
+                    fwd.stream, before = s.cuda_stream, own.launch_count()
+                    run(q, o)
+                    assert own.launch_count() - before == 2
+            torch.cuda.synchronize()
+            assert all(float((a - b).abs().max()) < 1e-5 for a, b in zip(got, want))
+    finally:
+        fwd.stream = None
+        fwd.workspace.destroy()
+        cache.destroy()
+        own.destroy()
+
+
+def test_captured_calls_share_no_scratch(ctx):
+    """Two recordings of a short prompt, replayed beside each other and beside a call that leaves pieces."""
+    import torch
+    cache, fwd, qs, want, run = _short_prompt(ctx, 3, 6)
+    try:
+        got = [torch.zeros_like(q) for q in qs]
+        streams, graphs = [torch.cuda.Stream() for _ in qs], []
+        fwd.stream = streams[0].cuda_stream
+        run(qs[0], got[0])                                       # the context has scratch
+        torch.cuda.synchronize()
+        for q, o, s in zip(qs[1:], got[1:], streams[1:]):
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                fwd.stream, before = s.cuda_stream, ctx.launch_count()
+                run(q, o)
+                assert ctx.launch_count() - before == 1          # in one piece
+            graphs.append(g)
+        for o in got:
+            o.zero_()
+        torch.cuda.synchronize()
+        for _ in range(20):
+            for g, s in zip(graphs, streams[1:]):
+                with torch.cuda.stream(s):
+                    g.replay()
+            fwd.stream = streams[0].cuda_stream
+            run(qs[0], got[0])
+        torch.cuda.synchronize()
+        assert all(float((a - b).abs().max()) < 1e-5 for a, b in zip(got, want))
+    finally:
+        fwd.stream = None
+        fwd.workspace.destroy()
+        cache.destroy()

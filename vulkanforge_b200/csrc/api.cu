@@ -167,7 +167,10 @@ int32_t vfkv_ctx_destroy(vfkv_ctx *ctx)
     if (!ctx) return VFKV_OK;
     DeviceGuard g(ctx->device);
     cudaFree(ctx->d_status);
-    for (auto &s : ctx->prefill_scratch) cudaFree(s.d);
+    for (auto &s : ctx->prefill_scratch) {
+        cudaFree(s.d);
+        if (s.last) cudaEventDestroy(s.last);
+    }
     prof_clear(ctx);
     delete ctx;
     return VFKV_OK;

@@ -508,6 +508,7 @@ extern "C" int32_t vfkv_attend_prefill(vfkv_cache *cache, uint32_t layer, uint32
     p.m = m; p.q_start = q_start; p.n_kv = n_kv; p.kv_start = kv_start; p.window = window;
     p.scale = scale; p.softcap = softcap;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    p.whole = stream_is_capturing(st);
     Guard g(ctx->device);
     const bool aligned = (reinterpret_cast<uintptr_t>(d_q) | reinterpret_cast<uintptr_t>(d_out) |
                           reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) % 16 == 0;

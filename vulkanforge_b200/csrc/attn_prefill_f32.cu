@@ -501,6 +501,7 @@ int32_t launch_t(vfkv_ctx *ctx, const PrefillParams &p, cudaStream_t st)
         e = launch_dependent(ctx, prefill_f32_merge_kernel<D>, dim3(uint32_t(items), BM / (kThreads / 32)), dim3(kThreads), 0, st, fp);
         ctx->count_launch();
     }
+    prefill_scratch_used(ctx, st, fp.scratch);
     return check_cuda(ctx, e, "f32 prefill attention launch");
 }
 

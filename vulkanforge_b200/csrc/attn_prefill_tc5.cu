@@ -1347,39 +1347,75 @@ TwoTileCost two_tile_cost(const vfkv_ctx *ctx, uint32_t dtype, const Tc5Params &
 
 }  // namespace
 
-// Device scratch for pieces of row blocks, owned by the context: allocated at a stream's first call outside a
-// capture, for up to four streams, so that calls on several of them may overlap.  A call that is being captured on a
-// stream without one takes the first there is (its replays must not overlap other such calls).  Null where there is
-// none: the caller then cuts nothing.
+// Device scratch for pieces of row blocks, owned by the context: a buffer for each of up to four streams, allocated
+// at a stream's first such call, so that calls on several of them may overlap.  A fifth stream takes over the buffer
+// that was used longest ago, behind the event of its last use; the events are recorded only once all buffers have
+// an owner (before that a take-over waits for the device).  Not for calls that are being captured: a recording may be
+// replayed whenever the host likes, beside anything.  Null where there is none: the caller then cuts nothing.
 float *prefill_scratch(vfkv_ctx *ctx, cudaStream_t st, uint64_t *floats)
 {
     const uint32_t n_sm = uint32_t(ctx->sm_count);
     const uint64_t n = uint64_t(n_sm) * 2 * CTA_ROWS * (HD + 2);
     *floats = 0;
+    unsigned long long id = 0;
+    if (stream_is_capturing(st) || cudaStreamGetId(st, &id) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    vfkv_ctx::PrefillScratch *mine = nullptr, *oldest = nullptr;
     for (auto &s : ctx->prefill_scratch) {
-        if (s.d != nullptr && s.stream != st) continue;
         if (s.d == nullptr) {
-            cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-            cudaStreamIsCapturing(st, &capturing);
-            if (capturing != cudaStreamCaptureStatusNone) break;
             void *d = nullptr;
             // the pieces, then one flag per CTA, cleared in the order of the stream that will use them
             if (cudaMalloc(&d, n * sizeof(float) + n_sm * sizeof(uint32_t)) != cudaSuccess ||
-                cudaMemsetAsync(static_cast<float *>(d) + n, 0, n_sm * sizeof(uint32_t), st) != cudaSuccess) {
+                cudaMemsetAsync(static_cast<float *>(d) + n, 0, n_sm * sizeof(uint32_t), st) != cudaSuccess ||
+                cudaEventCreateWithFlags(&s.last, cudaEventDisableTiming) != cudaSuccess) {
                 (void)cudaGetLastError();
                 cudaFree(d);
                 return nullptr;
             }
-            s = {st, static_cast<float *>(d)};
+            s.stream = id;
+            s.d = static_cast<float *>(d);
+            mine = &s;
+            break;
         }
-        *floats = n;
-        return s.d;
+        if (s.stream == id) { mine = &s; break; }
+        if (!s.captured && (!oldest || s.used < oldest->used)) oldest = &s;
     }
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(st, &capturing);
-    if (capturing == cudaStreamCaptureStatusNone || ctx->prefill_scratch[0].d == nullptr) return nullptr;
+    if (mine == nullptr) {
+        if (oldest == nullptr) return nullptr;
+        if ((oldest->recorded ? cudaStreamWaitEvent(st, oldest->last, 0) : cudaDeviceSynchronize()) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        mine = oldest;
+        mine->stream = id;
+    }
+    mine->used = ++ctx->prefill_uses;
     *floats = n;
-    return ctx->prefill_scratch[0].d;
+    return mine->d;
+}
+
+// After the last launch that reads what prefill_scratch() returned on this stream.
+void prefill_scratch_used(vfkv_ctx *ctx, cudaStream_t st, const float *scratch)
+{
+    const uint32_t last = sizeof(ctx->prefill_scratch) / sizeof(ctx->prefill_scratch[0]) - 1;
+    if (scratch == nullptr || ctx->prefill_scratch[last].d == nullptr) return;
+    for (auto &s : ctx->prefill_scratch)
+        if (s.d == scratch && !s.captured) s.recorded = cudaEventRecord(s.last, st) == cudaSuccess;
+}
+
+// Of a captured call of the two-tile kernel: the stream's own buffer, or else the first, which then stays where it is
+// (the caller's replays must not overlap other calls that leave pieces).
+static float *captured_scratch(vfkv_ctx *ctx, cudaStream_t st)
+{
+    unsigned long long id = 0;
+    if (cudaStreamGetId(st, &id) != cudaSuccess) (void)cudaGetLastError();
+    auto *found = &ctx->prefill_scratch[0];
+    for (auto &s : ctx->prefill_scratch)
+        if (s.d != nullptr && s.stream == id) found = &s;
+    found->captured = found->captured || found->d != nullptr;
+    return found->d;
 }
 
 // A byte-typed map of rows of row_bytes, boxes of 128 bytes x box_rows with the 128-byte swizzle.
@@ -1475,13 +1511,12 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
     const uint32_t n_sm = uint32_t(ctx->sm_count);
     const uint64_t items = uint64_t(p.n_rb) * n_kv_heads;
     bool spread = false;
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    const bool capturing = stream_is_capturing(st);
     {
         const TwoTileCost cost = two_tile_cost(ctx, dtype, p);
         if (cost.even) {
-            cudaStreamIsCapturing(st, &capturing);
             uint64_t floats = 0;
-            p.scratch = prefill_scratch(ctx, st, &floats);
+            p.scratch = capturing ? captured_scratch(ctx, st) : prefill_scratch(ctx, st, &floats);
             if (p.scratch != nullptr) {
                 spread = true;
                 p.total_tiles = uint32_t(cost.total);
@@ -1491,7 +1526,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
                 // captured launch would replay with the flag value of the capture, which the flags
                 // still hold from the replay before: those go through the merge kernel.
                 const uint64_t share = cost.total / n_sm;
-                p.inline_merge = ((cost.longest + share - 1) / share <= 3 && capturing == cudaStreamCaptureStatusNone) ? 1u : 0u;
+                p.inline_merge = ((cost.longest + share - 1) / share <= 3 && !capturing) ? 1u : 0u;
             }
         }
     }
@@ -1544,6 +1579,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
             cfg.numAttrs = 1;
             if (cudaLaunchKernelEx(&cfg, kern, p, tm_k, tm_v) == cudaSuccess) {
                 ctx->count_launch();
+                prefill_scratch_used(ctx, st, p.scratch);
                 return check_cuda(ctx, cudaGetLastError(), "tcgen05 prefill attention launch");
             }
             (void)cudaGetLastError();          // not all resident: the pieces go to the merge kernel instead
@@ -1565,6 +1601,7 @@ int32_t launch_prefill_tc5(vfkv_ctx *ctx, uint32_t dtype, const uint8_t *k, cons
             cfg.attrs = attr;
             cfg.numAttrs = 1;
             cudaError_t e = cudaLaunchKernelEx(&cfg, prefill_tc5_merge_kernel, p);
+            if (!capturing) prefill_scratch_used(ctx, st, p.scratch);
             if (e != cudaSuccess) return check_cuda(ctx, e, "tcgen05 prefill merge launch");
             ctx->count_launch();
         }

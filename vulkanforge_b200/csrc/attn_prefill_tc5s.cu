@@ -570,7 +570,7 @@ Cut best_cut(const vfkv_ctx *ctx, uint32_t dtype, bool split_q, const PrefillPar
     const uint64_t items = uint64_t(n_rb) * p.n_kv_heads, n_sm = uint64_t(ctx->sm_count);
     Cut best{1, 1e30};
     for (uint32_t n = 1; n <= 64 && n <= std::max(longest, 1u); ++n) {
-        if (n > 1 && items * n > n_sm * 2) break;
+        if (n > 1 && (p.whole || items * n > n_sm * 2)) break;
         const double one_cta = t0 + t1 * double((longest + n - 1) / n);
         double us = one_cta;
         if (items * n > n_sm)
@@ -614,6 +614,7 @@ int32_t launch_one_tile_t(vfkv_ctx *ctx, OneTileParams op, cudaStream_t st)
         e = launch_dependent(ctx, prefill_pieces_kernel<D>, dim3(p.n_kv_heads * 16, op.n_rb), dim3(256), 0, st, op);
         ctx->count_launch();
     }
+    prefill_scratch_used(ctx, st, op.scratch);
     return check_cuda(ctx, e, "one-tile prefill attention launch");
 }
 

@@ -19,8 +19,15 @@ struct vfkv_ctx {
     uint32_t *d_status = nullptr;      // device word written by bounded waits that give up
     uint32_t attn_impl = 0;            // 0 auto, 1 CUDA-core only, 2 tensor-core only, 3 as 0 but mma.sync instead of tcgen05 (prefill)
     uint32_t tune_warps = 0, tune_stages = 0;   // tensor-core kernel shape, 0 = choose
-    // Pieces of prefill items cut between CTAs: a buffer for each of the first streams that need one
-    struct PrefillScratch { cudaStream_t stream; float *d; } prefill_scratch[4] = {};
+    // Pieces of prefill items cut between CTAs: a buffer for each of up to four streams (prefill_scratch())
+    struct PrefillScratch {
+        unsigned long long stream = 0;     // id of its stream: handles are given out again
+        float *d = nullptr;
+        cudaEvent_t last = nullptr;        // behind its last use, once every buffer has an owner
+        bool recorded = false, captured = false;
+        uint64_t used = 0;                 // of prefill_uses
+    } prefill_scratch[4];
+    uint64_t prefill_uses = 0;
     uint32_t prefill_epoch = 0;                 // value the flags of the current spread prefill launch take
     uint32_t pdl = 0;                  // programmatic dependent launch mode (0 / 1 / 2)
     // K addresses that the last launch on this context wrote cache rows into, or an empty range: a
@@ -235,6 +242,12 @@ inline cudaError_t launch_dependent(const vfkv_ctx *ctx, void (*kern)(P...), dim
     cfg.attrs = attr;
     cfg.numAttrs = ctx->pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
+inline bool stream_is_capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
 }
 
 #ifdef __CUDACC__

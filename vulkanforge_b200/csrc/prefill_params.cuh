@@ -13,6 +13,7 @@ struct PrefillParams {
     uint64_t row_bytes;
     uint32_t n_q_heads, n_kv_heads, group, head_dim, m, q_start, n_kv, kv_start, window;
     float scale, softcap;
+    bool whole;                        // host side only: leave no pieces (the call is being captured)
 };
 
 // f32-accurate tiled kernel on CUDA cores (attn_prefill_f32.cu): every dtype, scales, any group size
@@ -29,6 +30,7 @@ double prefill_one_tile_us(const vfkv_ctx *ctx, uint32_t dtype, bool split_q, co
 
 // shared by the tcgen05 kernels (attn_prefill_tc5.cu)
 float *prefill_scratch(vfkv_ctx *ctx, cudaStream_t st, uint64_t *floats);
+void prefill_scratch_used(vfkv_ctx *ctx, cudaStream_t st, const float *scratch);
 bool encode_rows_map(vfkv_ctx *ctx, CUtensorMap *out, const void *base, uint64_t row_bytes, uint32_t rows, uint32_t box_rows);
 
 #ifdef __CUDACC__

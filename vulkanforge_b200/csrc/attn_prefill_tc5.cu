@@ -1391,6 +1391,7 @@ float *prefill_scratch(vfkv_ctx *ctx, cudaStream_t st, uint64_t *floats)
         mine = oldest;
         mine->stream = id;
     }
+    mine->handle = st;
     mine->used = ++ctx->prefill_uses;
     *floats = n;
     return mine->d;
@@ -1409,11 +1410,10 @@ void prefill_scratch_used(vfkv_ctx *ctx, cudaStream_t st, const float *scratch)
 // (the caller's replays must not overlap other calls that leave pieces).
 static float *captured_scratch(vfkv_ctx *ctx, cudaStream_t st)
 {
-    unsigned long long id = 0;
-    if (cudaStreamGetId(st, &id) != cudaSuccess) (void)cudaGetLastError();
+    // (a stream's id cannot be asked for while it is being captured)
     auto *found = &ctx->prefill_scratch[0];
     for (auto &s : ctx->prefill_scratch)
-        if (s.d != nullptr && s.stream == id) found = &s;
+        if (s.d != nullptr && s.handle == st) found = &s;
     found->captured = found->captured || found->d != nullptr;
     return found->d;
 }

@@ -21,7 +21,8 @@ struct vfkv_ctx {
     uint32_t tune_warps = 0, tune_stages = 0;   // tensor-core kernel shape, 0 = choose
     // Pieces of prefill items cut between CTAs: a buffer for each of up to four streams (prefill_scratch())
     struct PrefillScratch {
-        unsigned long long stream = 0;     // id of its stream: handles are given out again
+        unsigned long long stream = 0;     // id of its stream: handles are given out again (a capture knows only those)
+        cudaStream_t handle = nullptr;
         float *d = nullptr;
         cudaEvent_t last = nullptr;        // behind its last use, once every buffer has an owner
         bool recorded = false, captured = false;

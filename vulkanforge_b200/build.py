@@ -61,10 +61,16 @@ def build(force: bool = False, verbose: bool = False) -> str:
         failed |= p.returncode != 0
     if failed:
         raise RuntimeError("nvcc failed; see messages above")
-    link = [_nvcc(), "-shared", "-o", OUT] + objs + ARCH + ["-ccbin", "/usr/bin/g++"]
-    subprocess.run(link, check=True)
+    link(objs)
     build_calls()
     return OUT
+
+
+def link(objs) -> None:
+    # the soname is what the bindings ask for, and find beside themselves wherever the package lies; without one they
+    # would ask for the path that it was built at
+    subprocess.run([_nvcc(), "-shared", "-o", OUT] + objs + ARCH + ["-ccbin", "/usr/bin/g++", "-Xlinker",
+                    "-soname=" + os.path.basename(OUT)], check=True)
 
 
 def build_calls() -> str:

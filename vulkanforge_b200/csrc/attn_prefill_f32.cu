@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
                 float sum = 0.f;
 #pragma unroll
                 for (int j = 0; j < HP; ++j) {
-                    // a masked position contributes nothing, also while the row's maximum is still the sentinel
-                    const float e = (full || s[h][j] > 0.5f * kMaskedScore) ? fast_exp2(s[h][j] - mn) : 0.f;
+                    // a masked position contributes nothing, also while the row's maximum is still the sentinel; a NaN stays one
+                    const float e = (full || !(s[h][j] <= 0.5f * kMaskedScore)) ? fast_exp2(s[h][j] - mn) : 0.f;
                     s[h][j] = e;
                     sum += e;
                 }

@@ -84,9 +84,49 @@ __device__ __forceinline__ uint32_t chunk_off(uint32_t r, uint32_t c, uint32_t s
     return (c >> 3) * slab + r * 128u + (((c & 7u) ^ (r & 7u)) << 4);
 }
 
+// One row by one warp over positions [lo, hi), each read only if the row sees it; to dst as the rows of the kernel below,
+// final or (m != null) as a piece.  For rows that came out of the products as infinities or NaN: 0 x V of a position that
+// a row does not see is not 0 when that V is not finite, and the tiles multiply all rows with all positions.
+template <int DT, int D>
+__device__ __noinline__ void row_alone(const PrefillParams *params, uint32_t r, uint32_t kvh, uint32_t lo, uint32_t hi, float *dst, float *m_out, float *l_out)
+{
+    const PrefillParams &p = *params;
+    constexpr int N = D / 32;
+    const uint32_t lane = threadIdx.x & 31u, g = p.group;
+    const float *const q = p.q + (uint64_t(r / g) * p.n_q_heads + kvh * g + r % g) * D + lane;
+    auto element = [&](const uint8_t *row, int j) {
+        if constexpr (DT == VFKV_F16) return __half2float(reinterpret_cast<const __half *>(row)[lane + 32 * j]);
+        else return e4m3x2_to_float2(row[lane + 32 * j]).x;
+    };
+    float m = kMaskedScore, l = 0.f, o[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) o[j] = 0.f;
+    for (uint32_t pos = lo; pos < hi; ++pos) {
+        const uint64_t at = uint64_t(pos) * p.row_bytes + uint64_t(kvh) * D * (DT == VFKV_F16 ? 2 : 1);
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < N; ++j) s = fmaf(q[32 * j], element(p.k + at, j), s);
+#pragma unroll
+        for (int x = 16; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+        if (p.k_scales) s *= p.k_scales[uint64_t(pos) * p.n_kv_heads + kvh];
+        s *= p.scale;
+        if (p.softcap > 0.f) s = softcap_any(s, p.softcap, 1.0f / p.softcap);
+        const float mn = fmaxf(m, s), corr = __expf(m - mn), e = __expf(s - mn);
+        const float pv = p.v_scales ? e * p.v_scales[uint64_t(pos) * p.n_kv_heads + kvh] : e;
+        l = l * corr + e;
+#pragma unroll
+        for (int j = 0; j < N; ++j) o[j] = o[j] * corr + pv * element(p.v + at, j);
+        m = mn;
+    }
+    const float f = m_out ? 1.0f : l > 0.f ? 1.0f / l : 0.f;
+#pragma unroll
+    for (int j = 0; j < N; ++j) dst[lane + 32 * j] = o[j] * f;
+    if (m_out && lane == 0u) { *m_out = m * kLog2e; *l_out = l; }
+}
+
 template <int DT, int D, bool SPLITQ, bool SC, bool CAP>
 __global__ void __launch_bounds__(kThreads, 1)
-prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v)
+prefill_one_tile_kernel(const __grid_constant__ OneTileParams op, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v)
 {
     using T = OneTile<D, SPLITQ>;
     static_assert(!SC || (SPLITQ && DT == VFKV_F8), "scales belong to FP8 caches and keep f32 accuracy");
@@ -308,7 +348,7 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
 #pragma unroll
             for (int j = 0; j < 64; ++j) {
                 float e = fast_exp2(s[j] - mref);
-                if (!warp_full) e = s[j] > 0.5f * kMaskedScore ? e : 0.f;
+                if (!warp_full) e = s[j] <= 0.5f * kMaskedScore ? 0.f : e;      // a NaN stays one
                 s[j] = e;
                 if constexpr (SC) sum += e;
             }
@@ -349,10 +389,10 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
         // ---- rows out: each warp stages its 32 rows where Q and the ring were (every product has been
         // through with them), so that a store covers whole rows
         const float unit = SC ? __uint_as_float(vs_ref) * (1.0f / kPUnit) : 1.0f;
-        float row_scale;
-        float *row_dst;
+        float row_scale, finite = 0.f;             // finite: 0, or NaN if an element is not
+        float *row_dst, *piece = nullptr;
         if (op.n_split > 1u) {
-            float *const piece = op.scratch + uint64_t(blockIdx.x) * T::PIECE;
+            piece = op.scratch + uint64_t(blockIdx.x) * T::PIECE;
             piece[BM * D + tid] = ran ? mref : kMaskedScore;
             piece[BM * D + BM + tid] = ran ? lrow : 0.f;
             row_scale = unit;
@@ -373,9 +413,11 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
                 for (int j = 0; j < 32; ++j) v[j] = 0.f;
             }
 #pragma unroll
+            for (int j = 0; j < 32; ++j) { v[j] *= row_scale; finite = fmaf(v[j], 0.f, finite); }
+#pragma unroll
             for (uint32_t j = 0; j < 8; ++j)
                 *reinterpret_cast<float4 *>(stage + lane * ROWB + (((8u * c + j) ^ (lane & SW)) << 4)) =
-                    make_float4(v[4 * j] * row_scale, v[4 * j + 1] * row_scale, v[4 * j + 2] * row_scale, v[4 * j + 3] * row_scale);
+                    make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         }
         __syncwarp();
         const unsigned long long mine = reinterpret_cast<unsigned long long>(row_dst);
@@ -385,6 +427,15 @@ prefill_one_tile_kernel(const OneTileParams op, const __grid_constant__ CUtensor
             const unsigned long long dst = __shfl_sync(0xffffffffu, mine, int(rr));
             const float4 x = *reinterpret_cast<const float4 *>(stage + rr * ROWB + ((u ^ (rr & SW)) << 4));
             if (dst != 0ull) *reinterpret_cast<float4 *>(reinterpret_cast<float *>(dst) + 4u * u) = x;
+        }
+        const uint32_t cta_end = c_lo + n_tiles * BN;
+        for (uint32_t again = __ballot_sync(0xffffffffu, finite != 0.f && r_ok); again != 0u; again &= again - 1u) {
+            const int rr = __ffs(int(again)) - 1;
+            const uint32_t lo = max(__shfl_sync(0xffffffffu, r_lo, rr), c_lo), hi = min(__shfl_sync(0xffffffffu, r_hi, rr), cta_end);
+            float *const dst = reinterpret_cast<float *>(__shfl_sync(0xffffffffu, mine, rr));
+            float *const m_out = piece ? piece + BM * D + warp * 32u + uint32_t(rr) : nullptr;
+            __syncwarp();
+            row_alone<DT, D>(&op.a, row0 + warp * 32u + uint32_t(rr), kvh, lo, hi, dst, m_out, m_out ? m_out + BM : nullptr);
         }
     } else if (warp == 4u) {
         // ================= the MMA thread ===================================================================

@@ -87,3 +87,26 @@ def test_pieces_on_several_streams(ctx):
         fwd.stream = None
         fwd.workspace.destroy()
         cache.destroy()
+
+
+@pytest.mark.parametrize("hq,hkv,d,m,L", [(32, 8, 128, 200, 700), (16, 8, 256, 60, 1500), (8, 8, 64, 200, 3000)])
+def test_scores_of_a_hundred_keep_their_accuracy(ctx, hq, hkv, d, m, L):
+    """A score of 100 in 32 bits is 4e-6 (half an ulp) off at best, and its p by as much; results average that over the
+    positions and cancel what the p have in common.  Sums of sixteen products stay below 2^-19.5, one of all d does not."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(L)
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, L), vf.KvDtype.F32)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    try:
+        k, v = (torch.randn(L, hkv, d, device="cuda", generator=gen) for _ in range(2))
+        q = torch.randn(m, hq, d, device="cuda", generator=gen) * 25
+        fwd.b_step_kv_write(0, k, v, L, 0)
+        out = torch.zeros_like(q)
+        fwd.run_flash_attn_batch(0, q, out, m, L - m, L, 0, 0)
+        s = torch.einsum("mhgd,lhd->hgml", q.double().view(m, hkv, hq // hkv, d), k.double()) / d ** 0.5
+        s = s.masked_fill(torch.arange(L, device="cuda") > L - m + torch.arange(m, device="cuda")[:, None], -float("inf"))
+        want = torch.einsum("hgml,lhd->mhgd", s.softmax(-1), v.double()).reshape(m, hq, d)
+        assert float((out.double() - want).norm() / want.norm()) < 2.0 ** -19.5
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

@@ -11,13 +11,16 @@
 //   PV: thread = 8 rows x 4 dims; 3 16-byte shared loads for 32 FMAs.
 // Shared memory is the bound (a 16-byte load of a warp takes four of its cycles whoever shares an address: 63 % of
 // them used over a launch, the FMA pipe 35 %), so the thread's tile of S is square: 2 x 8, with ten loads for the
-// same FMAs, took 90.5 us where this takes 84.6 (200 queries at 700 positions, F32).
+// same FMAs, took 90.5 us where this took 84.6 (200 queries at 700 positions, F32).
+//
+// A score's products are summed sixteen at a time.  In one chain of head_dim products (85.5 us) a result was 4.8e-7 off
+// against 64 bits, and 2.4e-6 with scores of 100; now 3.1e-7 and 8.4e-7 (88.4 us), in chains of four 3.5e-7 and 1.3e-6 (91.7).
 //
 // Row blocks are few and uneven (200 queries x 4 heads x 8 kv-heads: 104 blocks of 8 to 11 tiles), and an SM is
 // at its rate only with two CTAs on it, so the tiles of all (row block, kv-head) items form one line of which every
 // resident CTA takes an even share.  An item that a share ends in goes to scratch in pieces, which a second kernel
 // puts together.  200 queries at 700 positions, F32: 119 us with a CTA or a cluster of two an item, whose second
-// CTAs sat on 60 of 148 SMs; 85 in even shares.  Sixteen rows a warp, four warps a CTA (fewer shared loads a product)
+// CTAs sat on 60 of 148 SMs; 85 in even shares (88 with the shorter sums above).  Sixteen rows a warp, four warps a CTA (fewer shared loads a product)
 // were faster only from about 1000 positions on (200 at 1500: 153 against 160; 368 at 368: 84 against 76).
 #include "fp8_codec.cuh"
 #include "prefill_params.cuh"
@@ -245,22 +248,30 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
             fetch(t, c + 1);
             if (live) {
                 const float *const qa = sq + (warp * WR + rp) * S::PITCH_Q + c * 64, *const ka = sbuf + (c & 1) * BN * kPitchK + cl * kPitchK;
-#pragma unroll 4
-                for (int k = 0; k < 64; k += 4) {
-                    float4 qv[HR];
+#pragma unroll 1
+                for (int k16 = 0; k16 < 64; k16 += 16) {           // chains of sixteen products: a shorter one loses less
+                    float part[HR][HP];
 #pragma unroll
-                    for (int h = 0; h < HR; ++h) qv[h] = *reinterpret_cast<const float4 *>(qa + h * S::PITCH_Q + k);
+                    for (int k = k16; k < k16 + 16; k += 4) {
+                        float4 qv[HR];
 #pragma unroll
-                    for (int j = 0; j < HP; ++j) {
-                        const float4 kv = *reinterpret_cast<const float4 *>(ka + j * LR * kPitchK + k);
+                        for (int h = 0; h < HR; ++h) qv[h] = *reinterpret_cast<const float4 *>(qa + h * S::PITCH_Q + k);
 #pragma unroll
-                        for (int h = 0; h < HR; ++h) {
-                            s[h][j] = fmaf(qv[h].x, kv.x, s[h][j]);
-                            s[h][j] = fmaf(qv[h].y, kv.y, s[h][j]);
-                            s[h][j] = fmaf(qv[h].z, kv.z, s[h][j]);
-                            s[h][j] = fmaf(qv[h].w, kv.w, s[h][j]);
+                        for (int j = 0; j < HP; ++j) {
+                            const float4 kv = *reinterpret_cast<const float4 *>(ka + j * LR * kPitchK + k);
+#pragma unroll
+                            for (int h = 0; h < HR; ++h) {
+                                part[h][j] = k == k16 ? qv[h].x * kv.x : fmaf(qv[h].x, kv.x, part[h][j]);
+                                part[h][j] = fmaf(qv[h].y, kv.y, part[h][j]);
+                                part[h][j] = fmaf(qv[h].z, kv.z, part[h][j]);
+                                part[h][j] = fmaf(qv[h].w, kv.w, part[h][j]);
+                            }
                         }
                     }
+#pragma unroll
+                    for (int h = 0; h < HR; ++h)
+#pragma unroll
+                        for (int j = 0; j < HP; ++j) s[h][j] += part[h][j];
                 }
             }
         }

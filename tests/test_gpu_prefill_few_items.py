@@ -1,5 +1,5 @@
-"""The tcgen05 prefill kernel with an item's K/V tiles cut over a cluster: few items, pieces of unequal
-size and pieces without a tile, every mask; and the soft-cap on either side of its polynomial's range."""
+"""The kernel that the prefill dispatch takes for few items of 128-dim rows against the mma.sync kernel and the oracle:
+pieces of unequal size, every mask, and the soft-cap on either side of its polynomial's range."""
 import numpy as np
 import pytest
 
@@ -13,14 +13,14 @@ ODT = {"F16": oracle.F16, "F8": oracle.F8}
 
 @pytest.mark.parametrize("dtype,hq,hkv,m,q_start,kv_start,window,softcap,q_gain", [
     ("F8", 32, 8, 64, 1500, 0, 0, 0.0, 1.0),       # 8 items of 13 tiles
-    ("F16", 32, 8, 333, 1000, 0, 0, 0.0, 1.0),     # 48 items of up to 11 tiles: clusters of three
+    ("F16", 32, 8, 333, 1000, 0, 0, 0.0, 1.0),     # 48 items of up to 11 tiles
     ("F8", 32, 8, 100, 3000, 0, 700, 0.0, 1.0),    # window
     ("F8", 64, 8, 40, 2000, 300, 0, 0.0, 1.0),     # kv_start; g = 8
-    ("F16", 8, 1, 300, 600, 0, 0, 30.0, 1.0),      # one kv-head; early row blocks have fewer tiles than CTAs
+    ("F16", 8, 1, 300, 600, 0, 0, 30.0, 1.0),      # one kv-head; early row blocks have fewer tiles
     ("F8", 32, 8, 64, 2500, 0, 0, 50.0, 12.0),     # scores beyond the cap
     ("F16", 32, 8, 70, 1300, 1310, 0, 0.0, 1.0),   # early queries see nothing -> zeros
 ])
-def test_items_cut_over_clusters(ctx, dtype, hq, hkv, m, q_start, kv_start, window, softcap, q_gain):
+def test_few_items_match_mma_sync_and_the_oracle(ctx, dtype, hq, hkv, m, q_start, kv_start, window, softcap, q_gain):
     import torch
     d, L = 128, q_start + m
     rng = np.random.default_rng(m + q_start)

@@ -1,7 +1,9 @@
 // Chunked-prefill causal attention over the cache on the 5th-generation tensor cores
 // (tcgen05.mma with accumulators in tensor memory).  Same function as prefill_mma_kernel in
 // attn_prefill.cu (flash_attn_batch.comp:105-208); used for head_dim 128, FP8 caches and, with the
-// usual attention scale, F16 caches.
+// usual attention scale, F16 caches.  Three forms: the specialised one further down is what the dispatch takes; the
+// pipelined one stands in for F16 rows where the driver makes no tensor maps; the simple one is reached by
+// vfkv_ctx_set_attn_tuning alone, as the plain statement of the algorithm that the others are tested against:
 //
 // One CTA = two Q tiles of 128 rows (256 / g consecutive queries x the g q-heads of one kv-head),
 // one warpgroup per Q tile, x K/V tiles of 128 positions shared by both.  While one warpgroup does
@@ -712,20 +714,19 @@ __global__ void __launch_bounds__(256, 1) prefill_tc5p_kernel(const Tc5Params p)
 // the two forms above: 0.5-0.7 us per group of 8), and in those forms that thread also owns a row
 // of the softmax, so 127 threads wait for it at every barrier.  Here the roles are separate warps:
 //   warps 0-3 / 4-7   softmax of Q tile 0 / 1 (thread t = row t), in halves of 64 positions;
-//   warp 8            one thread issues every MMA;
-//   warps 9-11        fetch, widen and place the K/V tiles (two buffers each); F16 rows: one thread
-//                     of them issues TMA copies instead.
-// Twelve warps leave 168 registers a thread, which is why a row is handled 64 columns at a time;
-// per Q tile and K/V tile: S = Q K^T (N = 128, one piece: two N = 64 products measured twice the
-// time) -> softmax of columns 0-63 -> P half a (tensor memory) -> O += P V (K = 64) while the
-// softmax of columns 64-127 runs -> P half b -> O += P V, and right behind that the S of the next
-// K/V tile.  MMAs issued by the one thread execute in issue order, which is what lets the next S be
-// issued behind the P V that reads P from the same tensor-memory columns; with two Q tiles the
-// tensor pipe has the other tile's products to run while one is in its softmax.
-// mbarriers (count): S ready [tile] (1, commit)   P ready [tile][half] (128)   P V done
-// [tile][half] (1, commit)   K / V ready [buffer] (96)   K / V free [buffer] (1, commit).  Each
-// completes once per K/V tile (or once per two), so a wait on a phase parity is never more than
-// one phase away from the barrier's state.
+//   warps 8 and 9     one thread each issues the MMAs of Q tile 0 / 1;
+//   the rest          K/V tiles (two buffers each): FP8 rows fetched, widened and placed by six warps, F16 rows copied by
+//                     TMA from one thread of two warps.
+// Registers are handed out to quarters of the SM, 128 a thread with FP8 rows and 168 with F16, which is why a row is
+// handled 64 columns at a time.  Per Q tile and K/V tile, for each half of 64 positions: S = Q K^T (N = 64) -> softmax ->
+// P over the half's own S columns (tensor memory) -> O += P V (K = 64) while the softmax of the other half runs; S of the
+// same half of the next K/V tile goes right behind the P V that reads P from its columns (MMAs of one thread execute in
+// order).  With two Q tiles and a thread for each the tensor pipe has the other tile's products to run while one is in
+// its softmax.  (One thread for both, S in one product of N = 128: 727 us for 2048 queries at 14 336 where this takes 638.)
+// mbarriers (count): S ready [half][tile] (1, commit)   P ready [tile][half] (128)   P V done [tile][half] (1, commit)
+// K / V ready [buffer] (its row threads, or 1 and the bytes of the TMA copies)   K / V free [buffer] (2, a commit of each
+// MMA thread).  Each completes once per K/V tile (or once per two), so a wait on a phase parity is never more than one
+// phase away from the barrier's state.
 // Bounded wait for a flag that another CTA of this (cooperative) launch sets; false after limit_ns.
 __device__ __forceinline__ bool flag_wait(const uint32_t *flag, uint32_t want, uint64_t limit_ns)
 {

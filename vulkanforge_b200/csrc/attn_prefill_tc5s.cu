@@ -14,7 +14,8 @@
 // A row's exponents refer to a maximum that is moved, and O rescaled, only when the true one has outgrown
 // it by a few binary orders.  The largest p is then any number up to 2^8 and not 1, so a row's sum is taken of the
 // p as they go into the product, rounded to half precision: a row that one position dominates is that position's V
-// whatever its p was rounded to (with the sum of the unrounded p: off by up to 2^-12).
+// whatever its p was rounded to (with the sum of the unrounded p: off by up to 2^-12; 32.3 -> 33.0 us for 333 queries at
+// 1000 positions, F16).
 //
 // SPLITQ: Q = high + low half-precision term, scaled per row by a power of two (two products for S).
 // SC: the scales of K multiply the scores, those of V multiply P, in f32; P is then also fed as two terms,

@@ -278,8 +278,8 @@ attn_wide_kernel(const AttnParams p)
         // ---- O^T += V^T P^T ----
         {
             // The tensor cores cut off towards zero what an accumulator does not hold, so a tile's products start
-            // from zero and are added to the others in f32 (F16, 20 000
-            // positions x 4 layers: results 3.1e-6 off in one chain, 3.1e-7 so; 95.6 -> 100.2 us).
+            // from zero and are added to the others in f32 (F16, 20 000 positions x 4 layers: results 3.1e-6 off in one
+            // chain, 3.1e-7 so; 95.6 -> 100.2 us).
             const float2 c = *reinterpret_cast<const float2 *>(sc_corr + 2 * tig);
             float o[4][4];
 #pragma unroll

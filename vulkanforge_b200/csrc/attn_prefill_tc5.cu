@@ -922,26 +922,16 @@ __global__ void __launch_bounds__(kThreadsH<DT>, 1) prefill_tc5h_kernel(const Tc
                     const bool full = t0 >= r_lo && t0 + 64u <= r_hi;
                     const bool warp_full = __all_sync(0xffffffffu, full);
                     if constexpr (CAP) softcap_all(s, p.softcap, inv_cap);
-                    float mx = kMaskedScore;
-                    if (warp_full && !CAP) {
+                    if constexpr (CAP) {
 #pragma unroll
-                        for (int j = 0; j < 64; j += 2) mx = fmaxf(mx, fmaxf(s[j], s[j + 1]));
-                    } else if (warp_full) {
-#pragma unroll
-                        for (int j = 0; j < 64; ++j) { s[j] *= kLog2e; mx = fmaxf(mx, s[j]); }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 64; ++j) {
-                            float x = s[j];
-                            if constexpr (CAP) x *= kLog2e;
-                            if (!full) {
-                                const uint32_t pos = t0 + j;
-                                if (pos < r_lo || pos >= r_hi) x = kMaskedScore;
-                            }
-                            s[j] = x;
-                            mx = fmaxf(mx, x);
-                        }
+                        for (int j = 0; j < 64; ++j) s[j] *= kLog2e;
                     }
+                    if (!warp_full) {
+#pragma unroll
+                        for (int j = 0; j < 64; ++j)
+                            if (t0 + j < r_lo || t0 + j >= r_hi) s[j] = kMaskedScore;
+                    }
+                    const float mx = max_of(s);
                     const bool grow = mx > mref + 8.0f;
                     if (__any_sync(0xffffffffu, grow)) {
                         const float mnew = grow ? mx : mref;
@@ -967,16 +957,13 @@ __global__ void __launch_bounds__(kThreadsH<DT>, 1) prefill_tc5h_kernel(const Tc
                     if (tid == 0) TC5H_TRACE(18 + 4 * h);
                     // (the offsets and the row sum as packed add.f32x2, two columns an instruction:
                     // 653 -> 696 us on 2048 queries at 14 336, not kept)
+                    // a row that has seen nothing yet refers to half the masked score, from where exp2 gives 0
+                    const float from = fmaxf(mref, 0.5f * kMaskedScore);
                     float sum = 0.f;
                     float pk[32];
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
-                        const float x0 = s[2 * j], x1 = s[2 * j + 1];
-                        float p0 = fast_exp2(x0 - mref), p1 = fast_exp2(x1 - mref);
-                        if (!warp_full) {
-                            p0 = x0 > 0.5f * kMaskedScore ? p0 : 0.f;
-                            p1 = x1 > 0.5f * kMaskedScore ? p1 : 0.f;
-                        }
+                        const float p0 = fast_exp2(s[2 * j] - from), p1 = fast_exp2(s[2 * j + 1] - from);
                         sum += p0 + p1;
                         pk[j] = __uint_as_float(pack_half2(p0, p1));   // position 2j in the low half
                     }

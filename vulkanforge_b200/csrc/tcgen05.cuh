@@ -142,6 +142,26 @@ __device__ __forceinline__ float fast_exp2(float x)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// The largest of 64: eight chains of three-input maxima.
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+    float y;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
+__device__ __forceinline__ float max_of(const float (&s)[64])
+{
+    float m[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = max3(s[i], s[i + 4], s[i + 8]);
+#pragma unroll
+    for (int j = 12; j < 60; j += 8)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) m[i] = max3(m[i], s[j + i], s[j + 4 + i]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = fmaxf(m[i], s[60 + i]);
+    return fmaxf(max3(m[0], m[1], m[2]), m[3]);
+}
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi)
 {
     __half2 h = __floats2half2_rn(lo, hi);

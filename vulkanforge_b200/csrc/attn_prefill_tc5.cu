@@ -710,11 +710,13 @@ __global__ void __launch_bounds__(256, 1) prefill_tc5p_kernel(const Tc5Params p)
 
 
 // ---- specialised form ----------------------------------------------------------------------------------
-// tcgen05.mma holds the thread that issues it for as long as the tensor pipe is busy (measured in
-// the two forms above: 0.5-0.7 us per group of 8), and in those forms that thread also owns a row
-// of the softmax, so 127 threads wait for it at every barrier.  Here the roles are separate warps:
+// Issuing the products takes the thread that does it 0.5-0.7 us per group of 8 in the two forms above, and there that
+// thread also owns a row of the softmax, so 127 threads wait for it at every barrier.  Here the roles are separate warps:
 //   warps 0-3 / 4-7   softmax of Q tile 0 / 1 (thread t = row t), in halves of 64 positions;
-//   warps 8 and 9     one thread each issues the MMAs of Q tile 0 / 1;
+//   warps 8 and 9     issue the MMAs of Q tile 0 / 1, all lanes running through so that the operands stay in uniform registers
+//                     (one thread in a branch of its own took 100 cycles a product of 32 or 64, which made the issue of a
+//                     half tile's products as long as its softmax: 567 -> 521 us for 2048 queries at 14 336, FP8; 418 ->
+//                     312 for 675 of 12 750, F16, 64 / 8 heads);
 //   the rest          K/V tiles (two buffers each): FP8 rows fetched, widened and placed by six warps, F16 rows copied by
 //                     TMA from one thread of two warps.
 // Registers are handed out to quarters of the SM, 128 a thread with FP8 rows and 168 with F16, which is why a row is
@@ -722,7 +724,7 @@ __global__ void __launch_bounds__(256, 1) prefill_tc5p_kernel(const Tc5Params p)
 // P over the half's own S columns (tensor memory) -> O += P V (K = 64) while the softmax of the other half runs; S of the
 // same half of the next K/V tile goes right behind the P V that reads P from its columns (MMAs of one thread execute in
 // order).  With two Q tiles and a thread for each the tensor pipe has the other tile's products to run while one is in
-// its softmax.  (One thread for both, S in one product of N = 128: 727 us for 2048 queries at 14 336 where this takes 638.)
+// its softmax.  (One thread for both, S in one product of N = 128: 727 us for 2048 queries at 14 336 where this took 638.)
 // mbarriers (count): S ready [half][tile] (1, commit)   P ready [tile][half] (128)   P V done [tile][half] (1, commit)
 // K / V ready [buffer] (its row threads, or 1 and the bytes of the TMA copies)   K / V free [buffer] (2, a commit of each
 // MMA thread).  Each completes once per K/V tile (or once per two), so a wait on a phase parity is never more than one
@@ -759,7 +761,7 @@ __global__ void __launch_bounds__(kThreadsH<DT>, 1) prefill_tc5h_kernel(const Tc
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
     uint8_t *sm = smem_raw + (base - smem_addr(smem_raw));
     const uint32_t q_sm = base, k_sm = base + 2 * TILE, v_sm = base + 4 * TILE;
-    const uint32_t tid = threadIdx.x, warp = tid >> 5;
+    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     // One CTA per item (n_cta == 0): grid = (kv-heads, row blocks), the heaviest row blocks (latest
     // queries) of every kv-head start first.  Work spread evenly (n_cta != 0): grid = n_cta, this CTA
     // takes its share of the line of all items' tiles as a sequence of segments, each a run of
@@ -902,7 +904,7 @@ __global__ void __launch_bounds__(kThreadsH<DT>, 1) prefill_tc5h_kernel(const Tc
             const uint32_t q_idx = r_ok ? r / g : 0u, hj = r_ok ? r % g : 0u;
             uint32_t r_lo, r_hi;
             query_range(p, q_idx, &r_lo, &r_hi);
-            if (!r_ok) { r_lo = 0u; r_hi = 0u; }
+            if (!r_ok) { r_lo = 0u; r_hi = 0xffffffffu; }        // nothing to mask in rows past the end: they are not written
             const uint32_t t_lane = ((warp & 3u) * 32u) << 16;
             const uint32_t tm_s = tmem + wg * 128u, tm_o = tmem + 256u + wg * 128u;
             float mref = kMaskedScore, lrow = 0.f;
@@ -1075,44 +1077,47 @@ __global__ void __launch_bounds__(kThreadsH<DT>, 1) prefill_tc5h_kernel(const Tc
                 __syncwarp();
             }
         } else if (warp < 10) {
-            // ================= the MMA threads, one per Q tile ==================================================
-            if ((tid & 31u) == 0u && n_tiles > 0u) {
-                const uint32_t wg = warp - 8u;
+            // ================= the MMA warps, one per Q tile ====================================================
+            // (all lanes run through, one issues: see mma_leader())
+            const uint32_t nt = __shfl_sync(0xffffffffu, n_tiles, 0);
+            if (nt > 0u) {
+                const uint32_t leader = mma_leader(), wg = warp - 8u, tm = __shfl_sync(0xffffffffu, tmem, 0), g0 = __shfl_sync(0xffffffffu, gt, 0);
                 bool ok = true;
                 // S of half h of a K/V tile (64 positions): its columns hold P of the tile before until the P V of
                 // that half, which is issued first (the MMAs of a thread run in order)
                 auto issue_s = [&](uint32_t gi, uint32_t h) {
                     const uint32_t b = gi & 1u;
                     if (h == 0u) {
-                        if (!mbar_wait(bar(12u + b), (gi >> 1) & 1u)) { ok = false; return; }
+                        if (!__all_sync(0xffffffffu, mbar_wait(bar(12u + b), (gi >> 1) & 1u))) { ok = false; return; }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     }
 #pragma unroll
                     for (uint32_t ks = 0; ks < HD / 16; ++ks) {
                         const uint32_t o = (ks >> 2) * SLAB + (ks & 3u) * 32;
-                        umma_f16(tmem + wg * 128u + 64u * h, smem_desc(q_sm + wg * TILE + o, 16, 1024),
-                                 smem_desc(k_sm + b * TILE + h * 8192u + o, 16, 1024), idesc_f16(false, 64), ks);
+                        umma_f16_by(leader, tm + wg * 128u + 64u * h, smem_desc(q_sm + wg * TILE + o, 16, 1024),
+                                    smem_desc(k_sm + b * TILE + h * 8192u + o, 16, 1024), idesc_f16(false, 64), ks);
                     }
-                    umma_commit(bar(h * 20u + wg));
-                    if (h == 1u) umma_commit(bar(16u + b));
+                    umma_commit_by(leader, bar(h * 20u + wg));
+                    if (h == 1u) umma_commit_by(leader, bar(16u + b));
                 };
-                issue_s(gt, 0u);
-                if (ok) issue_s(gt, 1u);
-                for (uint32_t it = 0; it < n_tiles && ok; ++it) {
-                    const uint32_t gi = gt + it, b = gi & 1u;
-                    if (!mbar_wait(bar(14u + b), (gi >> 1) & 1u)) { ok = false; break; }
-#pragma unroll 1
-                    for (uint32_t h = 0; h < 2u && ok; ++h) {
-                        if (!mbar_wait(bar(4u + wg * 2u + h), gi & 1u)) { ok = false; break; }
+                issue_s(g0, 0u);
+                if (ok) issue_s(g0, 1u);
+                for (uint32_t it = 0; it < nt && ok; ++it) {
+                    const uint32_t gi = g0 + it, b = gi & 1u;
+                    if (!__all_sync(0xffffffffu, mbar_wait(bar(14u + b), (gi >> 1) & 1u))) { ok = false; break; }
+#pragma unroll
+                    for (uint32_t h = 0; h < 2u; ++h) {
+                        if (!__all_sync(0xffffffffu, mbar_wait(bar(4u + wg * 2u + h), gi & 1u))) { ok = false; break; }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                         for (uint32_t kk = 0; kk < 4u; ++kk)
-                            umma_f16_ts(tmem + 256u + wg * 128u, tmem + wg * 128u + 64u * h + kk * 8u,
-                                        smem_desc(v_sm + b * TILE + (4u * h + kk) * 2048u, SLAB, 1024), idesc_f16(true),
-                                        (it | h | kk) != 0u ? 1u : 0u);
-                        umma_commit(bar(8u + wg * 2u + h));
-                        if (h == 1u) umma_commit(bar(18u + b));
-                        if (it + 1u < n_tiles) issue_s(gi + 1u, h);
+                            umma_f16_ts_by(leader, tm + 256u + wg * 128u, tm + wg * 128u + 64u * h + kk * 8u,
+                                           smem_desc(v_sm + b * TILE + (4u * h + kk) * 2048u, SLAB, 1024), idesc_f16(true),
+                                           (it | h | kk) != 0u ? 1u : 0u);
+                        umma_commit_by(leader, bar(8u + wg * 2u + h));
+                        if (h == 1u) umma_commit_by(leader, bar(18u + b));
+                        if (it + 1u < nt) issue_s(gi + 1u, h);
+                        if (!ok) break;
                     }
                 }
                 if (!ok) *abort_flag = 1u;

@@ -45,19 +45,19 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar) : "memory");
 }
-// Bounded wait for the phase with the given parity; false after one second.  The hint lets the
-// hardware park the thread for up to that long instead of returning for another look (a waiting
-// warp that spins takes issue slots from the warps of its scheduler that work).
-constexpr uint32_t kSuspendNs = 20000u;
+// Bounded wait for the phase with the given parity; false after one second.  try_wait parks the thread for a time that the
+// hardware chooses instead of returning for another look at once: a warp that spins takes issue slots from the warps of
+// its scheduler that work (looking 64 times first: 523 -> 529 us for 2048 FP8 queries at 14 336, 53 -> 65 for 30 at 35 666),
+// one that is parked for 20 us by a hint wakes later (524 against 515).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
 {
     uint64_t t0 = 0;
     for (uint32_t it = 0;; ++it) {
         uint32_t done;
         asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
                      "selp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done) : "r"(bar), "r"(parity), "r"(kSuspendNs) : "memory");
+                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
         if (done) return true;
         // the timer is slow to read: look at it only now and then
         if ((it & 255u) == 255u) {
@@ -136,6 +136,16 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float *v)
                     "r"(__float_as_uint(v[28])), "r"(__float_as_uint(v[29])), "r"(__float_as_uint(v[30])), "r"(__float_as_uint(v[31]))
                  : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float *v)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 :: "r"(taddr),
+                    "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
+                    "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
+                    "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
+                    "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
+                 : "memory");
+}
 __device__ __forceinline__ float fast_exp2(float x)
 {
     float y;
@@ -173,6 +183,32 @@ __device__ __forceinline__ float add_halves(float sum, uint32_t pair)
     asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %1;\n\t"
         "add.f32.f16 %0, a, %0;\n\tadd.f32.f16 %0, b, %0;\n\t}" : "+f"(sum) : "r"(pair));
     return sum;
+}
+// The same issued by a warp: all of its lanes run through the code, so that addresses and descriptors stay in uniform
+// registers, and the one that `leader` (mma_leader()) names issues.  A thread by itself, in a branch of its own, moves every
+// operand over for every product, and takes 40 to 110 cycles each for products of 32 or 64.
+__device__ __forceinline__ uint32_t mma_leader()
+{
+    uint32_t yes;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(yes));
+    return yes;
+}
+__device__ __forceinline__ void umma_f16_by(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
+__device__ __forceinline__ void umma_f16_ts_by(uint32_t leader, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 :: "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
+__device__ __forceinline__ void umma_commit_by(uint32_t leader, uint32_t bar)
+{
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" :: "r"(bar), "r"(leader) : "memory");
 }
 // A from tensor memory (half pairs packed into columns).
 __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)

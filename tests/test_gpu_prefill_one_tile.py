@@ -152,3 +152,47 @@ def test_more_row_blocks_than_a_grid_axis_holds(ctx):
     finally:
         fwd.workspace.destroy()
         cache.destroy()
+
+
+@pytest.mark.parametrize("dtype,hq,hkv,d,tiles", [(dt, hq, hkv, d, n) for dt, hq, hkv, d in
+                                                  (("F8s", 32, 8, 128), ("F16", 16, 8, 256), ("F8", 16, 8, 256), ("F16", 8, 8, 64))
+                                                  for n in ((1, 2, 3) if dt == "F8s" else (3,)) + (4, 5, 6, 9, 10)])
+def test_a_reference_that_moves_in_every_tile(ctx, dtype, hq, hkv, d, tiles):
+    """Scores that rise by 20 (29 binary orders) a tile of 64 positions for one query in three, fall for the next and stay for
+    the third: the two groups of softmax warps, which take the even and the odd tiles, hand the reference maximum to and fro
+    at every number of tiles around that of the score buffers (two and four).  P is rounded to half precision, its sum
+    too (scales: neither), which moves a weighted mean of V by at most 2^-11 of the largest V on either side."""
+    import torch
+    scaled, name = dtype == "F8s", "F16" if dtype == "F16" else "F8"
+    m, L = 35, tiles * 64 - 5
+    rng = np.random.default_rng(tiles * d)
+    k = np.zeros((L, hkv, d), np.float32)
+    k[:, :, 0] = (np.arange(L) // 16)[:, None] * 0.25                          # exact in E4M3 up to 4, in F16 throughout
+    if name == "F8":
+        k[:, :, 0] = torch.from_numpy(k[:, :, 0].copy()).to(torch.float8_e4m3fn).float().numpy()
+    v = torch.from_numpy(rng.standard_normal((L, hkv, d), dtype=np.float32)).to(torch.float8_e4m3fn).float().numpy()
+    if scaled:                                                                  # scales are a power of two: nothing is rounded
+        k[:, :, 1], v[:, :, 0] = 7.0, 448.0
+        k *= 64.0
+    slope = np.array([20.0, -20.0, 0.0], np.float32)[np.arange(m) % 3] * np.sqrt(np.float32(d)) / (64.0 if scaled else 1.0)
+    q = np.zeros((m, hq, d), np.float32)
+    q[:, :, 0] = slope[:, None]
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, L, scale_mode=int(scaled)), vf.KvDtype[name])
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    try:
+        fwd.b_step_kv_write(0, to_dev(k), to_dev(v), L, 0)
+        out = torch.full((m, hq, d), float("nan"), device="cuda")
+        fwd.run_flash_attn_batch(0, to_dev(q), out, m, L - m, L, 0, 0)
+        torch.cuda.synchronize()
+        ctx.poll()
+        s = (q[:, 0, 0].astype(np.float64) / np.sqrt(np.float64(d)))[:, None] * k[:, 0, 0].astype(np.float64)      # [m][L]
+        s[np.arange(L)[None] > (L - m + np.arange(m))[:, None]] = -np.inf
+        p = np.exp(s - s.max(1, keepdims=True))
+        p /= p.sum(1, keepdims=True)
+        want = np.repeat(np.einsum("ml,lhd->mhd", p, v.astype(np.float64)), hq // hkv, axis=1)
+        top = np.abs(v).max(axis=(0, 1))
+        tol = (2e-5 if scaled else 2.0 ** -10) * top + (1e-5 if scaled else 0.0)
+        assert (np.abs(out.cpu().numpy() - want) <= tol).all()
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

@@ -525,14 +525,14 @@ extern "C" int32_t vfkv_attend_prefill(vfkv_cache *cache, uint32_t layer, uint32
     // Three kernels do the same work in different portions, and the one whose model of the call is the
     // shortest takes it: two Q tiles of 128 rows a CTA (attn_prefill_tc5.cu: large chunks; most work per K/V
     // byte), one tile (attn_prefill_tc5s.cu: fewer rows, tiles cut over idle SMs, and the shapes the first
-    // does not hold), and 64 rows on mma.sync (a few positions: no tensor memory to set up).  Measured with
-    // the RoPE and append launches in front, 32 / 8 / 128 FP8, two tiles / one / mma.sync:
-    //   64 queries at 0: - / 11 / 9 us;  64 at 1936: 24 / 20 / 76;  16 at 30 000: 92 / 50 / -;
-    //   333 at 1000: 44 / 38 / -;  1000 at 3000: 133 / 139 / -;  2000 at 0: 94 / 107 / -
+    // does not hold), and 64 rows on mma.sync (a few positions: no tensor memory to set up).  Measured on
+    // 32 / 8 / 128, FP8, two tiles / one / mma.sync:
+    //   (attention alone) 64 queries at 0: 12 / - / 6 us;  64 at 2000: 49 / 19 / 71;  16 at 30 000: 66 / 39 / -;
+    //   400 at 1000: 46 / 27 / 63;  800 at 4000: 90 / 96 / 372;  200 at 30 000: 151 / - / -
     // attn_impl 2 and the tuning knob force the first where it holds the shape.
     // F16 rows of 128 dims: the short calls keep Q in two terms, the ones whose products bind them take it in one
     // (166 queries at 99 positions, 64 / 8 heads: error against 64 bits 1.7e-4 in two terms, 2.8e-4 in one; the second
-    // term costs a tile of 64 positions 0.2 us of 0.9).
+    // term costs a tile of 64 positions 0.06 us of 0.55).
     if (ctx->attn_impl == 0 && aligned && prefill_one_tile_supported(ctx, dt, D) && (kv.k_scales || mma_ok) &&
         !(two_ok && ctx->tune_stages != 0)) {
         const bool split_q = !tc5_accurate || (dt == VFKV_F16 && D == 128 && prefill_tc5_short(ctx, n_q_heads, hkv, m, q_start, n_kv, kv_start, window));
@@ -540,9 +540,9 @@ extern "C" int32_t vfkv_attend_prefill(vfkv_cache *cache, uint32_t layer, uint32
         const double two_us = two_ok && !split_q ? prefill_tc5_us(ctx, dt, n_q_heads, hkv, m, q_start, n_kv, kv_start, window) : 1e30;
         const uint32_t last = q_start + m < n_kv ? q_start + m : n_kv;
         const uint32_t seen = window && window + BM / p.group < last ? window + BM / p.group : last - (kv_start < last ? kv_start : last);
-        // mma.sync: 3 us, 2.2 a tile of 64 positions of 128 dims (64 queries at 1936: 32 tiles, 76 us with the launches in
-        // front; at 0: 9), 1.6 CTAs an SM at a time
-        double mma_us = mma_ok ? 3.0 + 2.2 * (D / 128.0) * ((seen + BN - 1) / BN) : 1e30;
+        // mma.sync: 3 us, and 1.5 / 2.05 / 3 a tile of 64 positions of 64 / 128 / 256 dims (16 queries at 2000: 51 / 68 / 98 us,
+        // at 0: 4 / 5 / 7), 1.6 CTAs an SM at a time
+        double mma_us = mma_ok ? 3.0 + (D == 64 ? 1.5 : D == 128 ? 2.05 : 3.0) * ((seen + BN - 1) / BN) : 1e30;
         const double ctas_a_slot = double((uint64_t(m) * p.group + BM - 1) / BM) * hkv / (1.6 * ctx->sm_count);
         if (ctas_a_slot > 1.0) mma_us *= ctas_a_slot;
         if (one_us <= two_us && one_us < mma_us)

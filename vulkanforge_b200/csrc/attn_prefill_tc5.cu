@@ -1306,9 +1306,9 @@ __global__ void __launch_bounds__(256) prefill_tc5_merge_kernel(const Tc5Params 
 }
 
 // The tiles of all items and of the longest one (p.n_rb is set), the time of the call with one CTA an item,
-// and whether even shares are allowed and expected to pay.  The model: an item costs 12 us and 3.0 a tile (FP8
-// rows; 2.6 F16), more items than SMs a quarter over the mean for the last wave; even shares cost 45 us (40)
-// once -- their segments, the pieces and the merge -- and 3.0 (2.55) a tile.
+// and whether even shares are allowed and expected to pay.  The model: an item costs 12 us and 2.5 a tile (FP8
+// rows; 2.4 F16), more items than SMs a quarter over the mean for the last wave; even shares cost 30 us
+// once -- their segments, the pieces and the merge -- and 2.5 (2.4) a tile.
 struct TwoTileCost { uint64_t total; uint32_t longest; double us; bool even; };
 TwoTileCost two_tile_cost(const vfkv_ctx *ctx, uint32_t dtype, const Tc5Params &p)
 {
@@ -1321,12 +1321,12 @@ TwoTileCost two_tile_cost(const vfkv_ctx *ctx, uint32_t dtype, const Tc5Params &
         c.longest = std::max(c.longest, tj);
     }
     const bool f8 = dtype == VFKV_F8;
-    const double tile = f8 ? 3.0 : 2.6;
+    const double tile = f8 ? 2.5 : 2.4;
     c.us = 12.0 + tile * c.longest;
     if (items > n_sm) c.us = std::max(c.us, 1.25 * (12.0 * double(items) + tile * double(c.total)) / double(n_sm));
     if ((ctx->tune_stages == 0 || ctx->tune_stages == 3) && ctx->tune_warps != 4 && p.n_rb <= kMaxRowBlocks &&
         p.kv_start < std::min(p.q_start + 1u, p.n_kv) && n_sm >= 2 && c.total >= n_sm * 2 && c.total < (1ull << 31)) {
-        const double even_us = (f8 ? 45.0 : 40.0) + (f8 ? 3.0 : 2.55) * double(c.total) / double(n_sm);
+        const double even_us = 30.0 + tile * double(c.total) / double(n_sm);
         // few items: where that is faster by a twentieth; more of them than half the SMs: where the last wave is part
         // empty and an item has 96 tiles or more (1500 queries at 8000, 192 items of 57: 314 us one CTA an item, 322
         // in shares; 4096 at 4096, 512 items of 17: several segments a CTA, twice the time)

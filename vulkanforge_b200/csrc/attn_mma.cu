@@ -37,6 +37,7 @@
 // context's status word and returns without touching the output.
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "attn_params.cuh"
@@ -370,6 +371,8 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 {
     using S = Shape<DT, D, W, NS>;
     constexpr int kWarps = W;
+    constexpr bool SOLO = W == 1;                        // a warp by itself: one split, no exchange
+    constexpr uint32_t kDrawer = SOLO ? 0u : 32u;        // the thread that draws the ticket
     constexpr int kStages = NS;
     constexpr int TP = S::TP, NB = S::NB, NC = S::NC, KSTEPS = S::KSTEPS, NDB = S::NDB;
     constexpr bool FP8 = DT == VFKV_F8;
@@ -463,7 +466,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // number at once: every CTA reads the number before it draws (the ticket's operand depends on
     // the value read), so the last drawer knows that all of them hold the old number.
     auto load_epoch = [&]() {
-        if (threadIdx.x == 32 && p.fan != nullptr) {
+        if (!SOLO && threadIdx.x == kDrawer && p.fan != nullptr) {
             s_fan = *p.fan;
             const uint32_t e = *reinterpret_cast<const volatile uint32_t *>(s_fan.epoch);
             s_epoch = e;
@@ -693,7 +696,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // pay 2 to 4 % (131 072 positions x 8 layers: 366 -> 373 us).  The shape with two stages and three CTAs an SM is
     // chosen for eight tiles or less.
     constexpr bool CHAINS = !ROWS2 && !(W == 4 && NS == 2 && S::STAGE_BYTES <= 8192);
-    constexpr uint32_t kChain = 8;
+    constexpr uint32_t kChain = SOLO ? 1 : 8;         // by itself a warp has the tiles that four had before: no longer sums than theirs
     float tot[CHAINS ? NACC : 1][2], l_tot = 0.f, m_tot = kMaskedScore;      // relative to the maximum (and the scale) they were left at
     uint32_t vs_tot = 0u;
 #pragma unroll
@@ -730,7 +733,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // tiles, so the words stay consistent.
     unsigned long long ticket = 0ull;
     bool drawn = false;
-    const bool draws = threadIdx.x == 32 && p.n_splits > 1u && mp.cluster == 0u;
+    const bool draws = !SOLO && threadIdx.x == kDrawer && p.n_splits > 1u && mp.cluster == 0u;
     auto draw_ticket = [&]() {
         ticket = atomicAdd(mp.tickets + (uint64_t(s) * p.n_kv_heads + kvh) * 256u + p.n_splits, 1ull);
         drawn = true;
@@ -1004,7 +1007,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     if (timed_out) {
         if (lane == 0) { atomicOr(p.status, 1u); s_flag = 1; }
     }
-    if (threadIdx.x == 32) {
+    if (!SOLO && threadIdx.x == kDrawer) {
         uint32_t tag = 0u, merger = 0u;
         if (draws) {
             if (!drawn) draw_ticket();            // a wait that ran out before the last tile
@@ -1095,8 +1098,8 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     }
     __syncthreads();
 
-    const bool direct = p.n_splits == 1;
-    const bool fan = p.fan != nullptr;
+    const bool direct = SOLO || p.n_splits == 1;
+    const bool fan = !SOLO && p.fan != nullptr;
     FanoutSlot fs{};
     if (fan) fs = fanout_slot(s_fan, D, s_fan.rank, s_epoch + 1u);
 
@@ -1106,7 +1109,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // outputs across all CTAs through distributed shared memory (flash_attn_reduce.comp:51-80).
     // No partial goes to global memory, no ticket is drawn.  The closing barrier keeps every CTA's
     // shared memory alive until its peers have read it.
-    if (mp.cluster != 0u) {
+    if (!SOLO && mp.cluster != 0u) {
         float *cx_o = sm_l + kWarps * NH;                      // [g][D]
         float *cx_m = cx_o + NH * D;                           // [g]
         float *cx_l = cx_m + NH;                               // [g]
@@ -1267,7 +1270,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         VFKV_TRACE(8);
     }
     const bool xrank = fan && mp.fan_merge != 0u;
-    if (direct && !xrank) { VFKV_TRACE(9); return; }
+    if (SOLO || (direct && !xrank)) { VFKV_TRACE(9); return; }
 
     // ---- the last drawers merge the splits ---------------------------------------------------------------
     // Everything from here on runs once per launch on a few CTAs per (sequence, kv-head), straight
@@ -1565,7 +1568,6 @@ int32_t launch_c(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
     constexpr bool kWide = Shape<DT, D, 8, 3>::SMEM_BYTES <= 200 * 1024;
     const uint64_t ctas = uint64_t(mp.a.n_splits) * mp.a.n_kv_heads * mp.a.n_seqs * mp.a.n_layers;
     uint32_t w = ctx->tune_warps, ns = ctx->tune_stages;
-    if (w == 0) w = (kWide && ctas <= uint64_t(ctx->sm_count)) ? 8 : 4;
     // 4 warps: as many stages (up to 3) as still let two CTAs share an SM.  At head_dim 256 a stage
     // is 16 KB, so that is one stage (64 KB per CTA): measured 5.5 TB/s against 3.9 TB/s with three
     // stages and a single CTA of 4 warps per SM (F16, 8 sequences x 32768, windows 1024 / none).
@@ -1575,9 +1577,29 @@ int32_t launch_c(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
     constexpr bool kOk2 = Shape<DT, D, 4, 2>::SMEM_BYTES <= kTwoPerSm && kMergeBytes <= Shape<DT, D, 4, 2>::RING_BYTES;
     constexpr bool kOk1 = Shape<DT, D, 4, 1>::SMEM_BYTES <= kTwoPerSm && kMergeBytes <= Shape<DT, D, 4, 1>::RING_BYTES;
     const uint32_t longest = mp.a.window && mp.a.window < mp.longest ? mp.a.window : mp.longest;
+    // Sequences of a few tiles, more of them than 4-warp CTAs are resident at a time: a warp each.  A CTA of four warps is then
+    // setting up, joining its warps and writing for most of its life, and two or three of them share an SM; of these
+    // there are up to twelve, which share nothing.  32 layers x 32 sequences, 32 q / 8 kv / 128, FP8: 24 positions 84.6 ->
+    // 29.9 us, 128 92 -> 55, 256 123 -> 94, 400 163 -> 146, 600 208 -> 207; F16, 16 q / 8 kv / 256: 64 164 -> 103, 256 358 -> 320;
+    // 16 layers x 4 sequences, FP8: 64 8.7 -> 5.8, 256 11.7 -> 10.0 (where the 4-warp CTAs run side by side, at most 2 tiles
+    // are as fast).  Three stages a warp where they cost no further wave (2048 sequences of 400: 50 us with two, 42 with three).
+    if (w == 0 && mp.a.n_splits == 1u && mp.a.fan == nullptr && ctas > uint64_t(ctx->sm_count) * (D == 64 ? 4u : 3u)) {
+        const uint32_t tiles = ((mp.a.window && mp.a.window < mp.longest ? mp.a.window : mp.longest) + Shape<DT, D, 1, 2>::TP - 1) / Shape<DT, D, 1, 2>::TP;
+        if (tiles <= 16u) {
+            auto waves = [&](uint64_t smem) {
+                const uint64_t slots = uint64_t(ctx->sm_count) * std::min<uint64_t>(12u, 227u * 1024u / (smem + 1024u));
+                return (ctas + slots - 1) / slots;
+            };
+            w = 1;
+            ns = tiles > 2u && waves(Shape<DT, D, 1, 3>::SMEM_BYTES) <= waves(Shape<DT, D, 1, 2>::SMEM_BYTES) ? 3u : 2u;
+        }
+    }
+    if (w == 0) w = (kWide && ctas <= uint64_t(ctx->sm_count)) ? 8 : 4;
     const bool few_tiles = (longest + mp.a.n_splits - 1) / mp.a.n_splits <= 8u * 4u * uint32_t(Shape<DT, D, 4, 2>::TP);
     if (ns == 0 && w == 4 && kOk2 && Shape<DT, D, 4, 2>::STAGE_BYTES <= 8192 && few_tiles && ctas > uint64_t(ctx->sm_count) * 2) ns = 2;
     if (ns == 0) ns = (w == 8 || Shape<DT, D, 4, 3>::SMEM_BYTES <= kTwoPerSm) ? 3 : kOk2 ? 2 : kOk1 ? 1 : 3;
+    if (w == 1 && ns == 2) return launch_k<DT, D, ROWS2, 1, 2, CAP, TR, SC>(ctx, tk, tv, mp, st);
+    if (w == 1 && ns == 3) return launch_k<DT, D, ROWS2, 1, 3, CAP, TR, SC>(ctx, tk, tv, mp, st);
     if (w == 8 && ns == 3) return launch_k<DT, D, ROWS2, 8, 3, CAP, TR, SC>(ctx, tk, tv, mp, st);
     if (w == 4 && ns == 3) return launch_k<DT, D, ROWS2, 4, 3, CAP, TR, SC>(ctx, tk, tv, mp, st);
     if (w == 4 && ns == 2) return launch_k<DT, D, ROWS2, 4, 2, CAP, TR, SC>(ctx, tk, tv, mp, st);

@@ -16,7 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libvfkv.so")
 CALLS = os.path.join(HERE, "_native.so")        # Python bindings of the per-layer calls (csrc/py_calls.cpp), linked to OUT
-SOURCES = ["api.cu", "append.cu", "attn_generic.cu", "attn_mma.cu", "attn_wide.cu", "attn_merge.cu", "exchange.cu", "attn_prefill.cu", "attn_prefill_f32.cu", "attn_prefill_tc5.cu", "attn_prefill_tc5s.cu", "rope_append.cu", "routes.cpp", "noalloc.cu", "kv_cache.cpp"]
+SOURCES = ["api.cu", "append.cu", "attn_generic.cu", "attn_mma.cu", "attn_mma_host.cu", "attn_wide.cu", "attn_merge.cu", "exchange.cu", "attn_prefill.cu", "attn_prefill_f32.cu", "attn_prefill_tc5.cu", "attn_prefill_tc5s.cu", "rope_append.cu", "routes.cpp", "noalloc.cu", "kv_cache.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

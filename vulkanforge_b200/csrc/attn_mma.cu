@@ -45,9 +45,16 @@
 #include "mma_sync.cuh"
 #include "softcap.cuh"
 
+// attn_mma_host.cu compiles this file again, for the launches that read a token's inputs out of pinned host memory (one split).
+#ifndef VFKV_HOST_INPUTS
+#define VFKV_HOST_INPUTS 0
+#endif
+
 namespace vfkv {
 
 namespace {
+
+constexpr bool kHostInputs = VFKV_HOST_INPUTS != 0;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
@@ -371,7 +378,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 {
     using S = Shape<DT, D, W, NS>;
     constexpr int kWarps = W;
-    constexpr bool SOLO = W == 1;                        // a warp by itself: one split, no exchange
+    constexpr bool SOLO = W == 1, ONE = SOLO || kHostInputs;     // a warp by itself; one split, no exchange
     constexpr uint32_t kDrawer = SOLO ? 0u : 32u;        // the thread that draws the ticket
     constexpr int kStages = NS;
     constexpr int TP = S::TP, NB = S::NB, NC = S::NC, KSTEPS = S::KSTEPS, NDB = S::NDB;
@@ -390,7 +397,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *ring_ptr = smem_raw + (ring - smem_u32(smem_raw));
     const uint32_t bars = ring + S::RING_BYTES;           // kWarps*kStages mbarriers, 8 bytes each
-    __shared__ uint32_t s_flag, s_epoch, s_tag, s_merger, s_late;
+    __shared__ uint32_t s_flag, s_epoch, s_tag, s_merger, s_late, s_pos_slot[2];
     __shared__ PeerFanout s_fan;          // the group's fan-out table (position-sharded calls only)
 
     const uint32_t split = blockIdx.x, kvh = blockIdx.y, s = blockIdx.z;     // s: unit of the launch (tickets, partials)
@@ -421,11 +428,12 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // grid's own wait, the early prefetch can only ever overlap the direct predecessor.
     // Both instructions do nothing in a launch without the attribute.
     if (mp.pdl != 2u) asm volatile("griddepcontrol.wait;" ::: "memory");
-    auto load_q = [&]() {
+    const float *const q_rows = p.q + (uint64_t(sr) * p.n_q_heads + kvh * g) * D;      // the group's
+    auto load_q = [&](const float *q0) {
     if constexpr (TR) {
         const uint32_t hcol = gid >> 1;
         const bool hv = hcol < g;
-        const float *qp = p.q + (uint64_t(sr) * p.n_q_heads + kvh * g + (hv ? hcol : 0)) * D;
+        const float *qp = q0 + (hv ? hcol : 0) * D;
 #pragma unroll
         for (int u = 0; u < NQB; ++u) {
             if constexpr (FP8) {
@@ -442,7 +450,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     for (int r = 0; r < RS; ++r) {
         const uint32_t hrow = gid + 8 * r;
         const bool hv = hrow < g;
-        const float *qp = p.q + (uint64_t(sr) * p.n_q_heads + kvh * g + (hv ? hrow : 0)) * D;
+        const float *qp = q0 + (hv ? hrow : 0) * D;
 #pragma unroll
         for (int ks = 0; ks < KSTEPS; ++ks) {
             if constexpr (FP8) {
@@ -466,7 +474,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // number at once: every CTA reads the number before it draws (the ticket's operand depends on
     // the value read), so the last drawer knows that all of them hold the old number.
     auto load_epoch = [&]() {
-        if (!SOLO && threadIdx.x == kDrawer && p.fan != nullptr) {
+        if (!ONE && threadIdx.x == kDrawer && p.fan != nullptr) {
             s_fan = *p.fan;
             const uint32_t e = *reinterpret_cast<const volatile uint32_t *>(s_fan.epoch);
             s_epoch = e;
@@ -481,11 +489,22 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             }
         }
     };
-    if (mp.pdl != 2u) { load_q(); load_epoch(); }
+    // From host memory Q comes once for all warps, through shared memory, and behind the first K/V tiles: the bus takes
+    // longer than HBM.
+    if (!kHostInputs && mp.pdl != 2u) { load_q(q_rows); load_epoch(); }
 
     VFKV_TRACE(0);
     uint32_t slot, start, len, begin, end;
-    seq_range(p, unit, &slot, &start, &len);
+    if constexpr (kHostInputs) {
+        if (threadIdx.x == 0) {
+            s_pos_slot[0] = p.positions[unit.seq];
+            s_pos_slot[1] = p.slot_ids ? p.slot_ids[unit.seq] : p.slot0 + unit.seq;
+        }
+        __syncthreads();
+        seq_range(p, unit, &slot, &start, &len, s_pos_slot);
+    } else {
+        seq_range(p, unit, &slot, &start, &len);
+    }
     split_range(start, len, p.n_splits, split, 32, &begin, &end);
     const uint32_t n_tiles = (end - begin + TP - 1) / TP;
     VFKV_TRACE(1);
@@ -536,11 +555,18 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     };
     if constexpr (SC) load_scales(0);
 
-    if (mp.pdl == 2u) {       // the prefetch is in flight; now wait for the predecessor, then read Q
+    if (!kHostInputs && mp.pdl == 2u) {       // the prefetch is in flight; now wait for the predecessor, then read Q
         asm volatile("griddepcontrol.wait;" ::: "memory");
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-        load_q();
+        load_q(q_rows);
         load_epoch();
+    }
+    if constexpr (kHostInputs) {
+        float *const staged = reinterpret_cast<float *>(ring_ptr + S::RING_BYTES + 256);       // behind the barriers
+        for (uint32_t i = threadIdx.x; i < g * (D / 4); i += W * 32)
+            reinterpret_cast<float4 *>(staged)[i] = reinterpret_cast<const float4 *>(q_rows)[i];
+        __syncthreads();
+        load_q(staged);
     }
 
     // ---- fused append (KvWrite of the decode step): the CTA whose range ends at the sequence's
@@ -733,7 +759,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // tiles, so the words stay consistent.
     unsigned long long ticket = 0ull;
     bool drawn = false;
-    const bool draws = !SOLO && threadIdx.x == kDrawer && p.n_splits > 1u && mp.cluster == 0u;
+    const bool draws = !ONE && threadIdx.x == kDrawer && p.n_splits > 1u && mp.cluster == 0u;
     auto draw_ticket = [&]() {
         ticket = atomicAdd(mp.tickets + (uint64_t(s) * p.n_kv_heads + kvh) * 256u + p.n_splits, 1ull);
         drawn = true;
@@ -1007,7 +1033,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     if (timed_out) {
         if (lane == 0) { atomicOr(p.status, 1u); s_flag = 1; }
     }
-    if (!SOLO && threadIdx.x == kDrawer) {
+    if (!ONE && threadIdx.x == kDrawer) {
         uint32_t tag = 0u, merger = 0u;
         if (draws) {
             if (!drawn) draw_ticket();            // a wait that ran out before the last tile
@@ -1098,8 +1124,8 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     }
     __syncthreads();
 
-    const bool direct = SOLO || p.n_splits == 1;
-    const bool fan = !SOLO && p.fan != nullptr;
+    const bool direct = ONE || p.n_splits == 1;
+    const bool fan = !ONE && p.fan != nullptr;
     FanoutSlot fs{};
     if (fan) fs = fanout_slot(s_fan, D, s_fan.rank, s_epoch + 1u);
 
@@ -1109,7 +1135,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // outputs across all CTAs through distributed shared memory (flash_attn_reduce.comp:51-80).
     // No partial goes to global memory, no ticket is drawn.  The closing barrier keeps every CTA's
     // shared memory alive until its peers have read it.
-    if (!SOLO && mp.cluster != 0u) {
+    if (!ONE && mp.cluster != 0u) {
         float *cx_o = sm_l + kWarps * NH;                      // [g][D]
         float *cx_m = cx_o + NH * D;                           // [g]
         float *cx_l = cx_m + NH;                               // [g]
@@ -1270,7 +1296,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         VFKV_TRACE(8);
     }
     const bool xrank = fan && mp.fan_merge != 0u;
-    if (SOLO || (direct && !xrank)) { VFKV_TRACE(9); return; }
+    if (ONE || (direct && !xrank)) { VFKV_TRACE(9); return; }
 
     // ---- the last drawers merge the splits ---------------------------------------------------------------
     // Everything from here on runs once per launch on a few CTAs per (sequence, kv-head), straight
@@ -1466,7 +1492,8 @@ int32_t launch_k(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
         // the flag only saves the call
         static std::atomic<bool> configured[64];
         if (!configured[ctx->device & 63].load(std::memory_order_acquire)) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES);
+            constexpr int kMost = !kHostInputs ? S::SMEM_BYTES : S::SMEM_BYTES + 16 * D * 4 < 227 * 1024 ? S::SMEM_BYTES + 16 * D * 4 : 227 * 1024;
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
             if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(tensor-core attention)");
             configured[ctx->device & 63].store(true, std::memory_order_release);
         }
@@ -1510,7 +1537,8 @@ int32_t launch_k(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = grid;
             cfg.blockDim = dim3(W * 32);
-            cfg.dynamicSmemBytes = S::SMEM_BYTES;
+            cfg.dynamicSmemBytes = S::SMEM_BYTES + (kHostInputs ? mp.a.group * D * 4 : 0);         // Q behind the barriers
+            if (kHostInputs && cfg.dynamicSmemBytes > 227 * 1024) return set_error(ctx, VFKV_ERR_UNSUPPORTED, "no room for Q in shared memory");
             cfg.stream = st;
             cudaLaunchAttribute attr[2];
             unsigned n_attr = 0;
@@ -1600,11 +1628,13 @@ int32_t launch_c(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
     if (ns == 0) ns = (w == 8 || Shape<DT, D, 4, 3>::SMEM_BYTES <= kTwoPerSm) ? 3 : kOk2 ? 2 : kOk1 ? 1 : 3;
     if (w == 1 && ns == 2) return launch_k<DT, D, ROWS2, 1, 2, CAP, TR, SC>(ctx, tk, tv, mp, st);
     if (w == 1 && ns == 3) return launch_k<DT, D, ROWS2, 1, 3, CAP, TR, SC>(ctx, tk, tv, mp, st);
-    if (w == 8 && ns == 3) return launch_k<DT, D, ROWS2, 8, 3, CAP, TR, SC>(ctx, tk, tv, mp, st);
+    if constexpr (!kHostInputs) {
+        if (w == 8 && ns == 3) return launch_k<DT, D, ROWS2, 8, 3, CAP, TR, SC>(ctx, tk, tv, mp, st);
+        if (w == 8 && ns == 1) return launch_k<DT, D, ROWS2, 8, 1, CAP, TR, SC>(ctx, tk, tv, mp, st);
+    }
     if (w == 4 && ns == 3) return launch_k<DT, D, ROWS2, 4, 3, CAP, TR, SC>(ctx, tk, tv, mp, st);
     if (w == 4 && ns == 2) return launch_k<DT, D, ROWS2, 4, 2, CAP, TR, SC>(ctx, tk, tv, mp, st);
     if (w == 4 && ns == 1) return launch_k<DT, D, ROWS2, 4, 1, CAP, TR, SC>(ctx, tk, tv, mp, st);
-    if (w == 8 && ns == 1) return launch_k<DT, D, ROWS2, 8, 1, CAP, TR, SC>(ctx, tk, tv, mp, st);
     return set_error(ctx, VFKV_ERR_INVALID, "attention tuning must be 4x1, 4x2, 4x3, 8x1 or 8x3 (warps x stages)");
 }
 
@@ -1623,6 +1653,7 @@ int32_t launch_t(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
 
 }  // namespace
 
+#if !VFKV_HOST_INPUTS
 // Parts a group of q-heads is cut into, each of as many heads as the kernel's tiles take: eight, or the sixteen of
 // the F16 form with two rows of heads where the group is one part.  The parts run side by side and find each
 // other's K/V rows in L2 (32 q-heads on 2 kv-heads, FP8, 3 x 20 000 positions x 4 layers: 518 us on CUDA cores).
@@ -1648,8 +1679,17 @@ bool attn_mma_supported(const AttnArgs &a)
     return false;
 }
 
+#endif
+
+#if VFKV_HOST_INPUTS
+int32_t launch_attn_mma_host(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits, cudaStream_t st)
+{
+    if (n_splits != 1 || a.fan) return set_error(ctx, VFKV_ERR_UNSUPPORTED, "inputs in host memory are read with one split only");
+#else
 int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits, cudaStream_t st)
 {
+    if (a.host_in) return launch_attn_mma_host(ctx, ws, a, n_splits, st);
+#endif
     if (!ctx->encode_tiled) return set_error(ctx, VFKV_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable in this driver");
     const uint32_t D = a.kv.head_dim, es = a.kv.dtype == VFKV_F8 ? 1 : 2;
     const uint64_t row_bytes = uint64_t(a.kv.n_kv_heads) * D * es;
@@ -1701,7 +1741,7 @@ int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, ui
     // append), the prefetch has to wait as well.
     const uint64_t last_layer = a.seq.layer_ids ? a.seq.layer_ids[a.seq.n_layers - 1] : 0u;      // the list ascends
     const uint64_t slab_bytes = (last_layer + 1) * rows * row_bytes;
-    mp.pdl = (ctx->pdl == 2u && ctx->reads_written(a.kv.k, slab_bytes)) ? 1u : ctx->pdl;
+    mp.pdl = (ctx->pdl == 2u && (a.host_in || ctx->reads_written(a.kv.k, slab_bytes))) ? 1u : ctx->pdl;
     mp.cluster = 0;
     mp.fan_merge = (a.fan && a.fan_merge) ? 1u : 0u;
     mp.fail_split = ctx->debug_fail_split;
@@ -1734,6 +1774,7 @@ int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, ui
     return rc;
 }
 
+#if !VFKV_HOST_INPUTS
 // Pre-encodes the two tensor maps of n_layers layers of a cache from the one that v views on (host
 // memory; reused by every call).
 bool encode_layer_maps(vfkv_ctx *ctx, const KvView &v, uint32_t n_layers, void *tm_k_out, void *tm_v_out)
@@ -1748,12 +1789,15 @@ bool encode_layer_maps(vfkv_ctx *ctx, const KvView &v, uint32_t n_layers, void *
     return encode_map(ctx, static_cast<CUtensorMap *>(tm_k_out), v.k, row_bytes, rows, box_rows) &&
            encode_map(ctx, static_cast<CUtensorMap *>(tm_v_out), v.v, row_bytes, rows, box_rows);
 }
+#endif
 
 }  // namespace vfkv
 
+#if !VFKV_HOST_INPUTS
 extern "C" int32_t vfkv_ctx_set_cluster_merge(vfkv_ctx *ctx, uint32_t on)
 {
     if (!ctx || on > 1) return VFKV_ERR_INVALID;
     ctx->cluster_merge = on;
     return VFKV_OK;
 }
+#endif

@@ -70,14 +70,15 @@ __device__ __forceinline__ UnitOf unit_of(const AttnParams &p, uint32_t u)
 // Visible range [start, len) of a unit's sequence and its slot.  Out-of-range
 // arguments from device arrays are clamped and reported through the status
 // word instead of being dereferenced.
+// pos_slot: the sequence's position and slot where the caller has them already.
 __device__ __forceinline__ void seq_range(const AttnParams &p, const UnitOf &unit, uint32_t *slot,
-                                          uint32_t *start, uint32_t *len)
+                                          uint32_t *start, uint32_t *len, const uint32_t *pos_slot = nullptr)
 {
     const uint32_t s = unit.seq;
-    uint32_t sl = p.slot_ids ? p.slot_ids[s] : p.slot0 + s;
+    uint32_t sl = pos_slot ? pos_slot[1] : p.slot_ids ? p.slot_ids[s] : p.slot0 + s;
     uint32_t n, st;
     if (p.positions) {
-        n = p.positions[s] + 1u;
+        n = (pos_slot ? pos_slot[0] : p.positions[s]) + 1u;
         st = p.window ? (n > p.window ? n - p.window : 0u)
                       : (p.kv_starts ? p.kv_starts[s] : p.kv_start_scalar);
     } else {

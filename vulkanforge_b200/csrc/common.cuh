@@ -208,6 +208,7 @@ struct AttnArgs {
     // only the tensor-core kernel consumes these (it writes the cache rows itself)
     const float *k_new = nullptr;
     const float *v_new = nullptr;
+    bool host_in = false;         // q, k_new, v_new, positions and slots are pinned host memory (tensor-core kernel, one split)
     const PeerFanout *fan = nullptr;   // device copy of the group's fan-out table, or null (tensor-core kernel only)
     // with fan: the attention kernel also waits for the other ranks' blocks in its own buffer, merges
     // them and writes the final rows to `out` (one launch per layer); otherwise vfkv_exchange_merge does
@@ -338,6 +339,7 @@ uint32_t attn_mma_parts(uint32_t dtype, uint32_t g);
 bool encode_layer_maps(vfkv_ctx *ctx, const KvView &v, uint32_t n_layers, void *tm_k_out, void *tm_v_out);
 int32_t launch_attn_mma(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits,
                         cudaStream_t st);
+int32_t launch_attn_mma_host(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits, cudaStream_t st);
 // merges ws partials [seq][head][split] into a.out (normalised) or a.out_{m,l,o}
 int32_t launch_merge_ws(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits,
                         cudaStream_t st);

@@ -4,6 +4,8 @@
 // Forward::run_flash_attn_split_reduce (src/backend/vulkan/forward/runs.rs:1463-1571).
 #include "attn_params.cuh"
 
+#include <algorithm>
+
 namespace vfkv {
 
 // flash_attn_reduce.comp:51-80: out = sum_i o_i e^(m_i - M) / sum_i l_i e^(m_i - M) with M the
@@ -155,6 +157,28 @@ int32_t launch_merge_partials_packed(vfkv_ctx *ctx, const float *packed, uint32_
 // positions (runs.rs:766-769); here the count only has to fill the GPU: aim
 // for about two CTAs per SM, never cut below 256 positions per split (128 on the tensor cores
 // with an F16 cache).
+// Expected time (us) of a tensor-core decode launch with n splits of sequences of len positions, base (sequence, kv-head)
+// pairs: a wave of CTAs costs 8 us and its stream, splits cost their merge.  An SM streams 39 KB a us with one CTA of 8 warps, 27
+// with two of 4 and 17 with one of those (HBM, shared, is in that); a CTA works through its positions in rounds of a tile for
+// each warp.  The numbers are a fit to 280 grids of 9 to 295 pairs (23 to 130 000 positions, all dtypes and groups), each
+// timed with 1 to 64 splits.
+static double split_us(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t len, uint64_t base, uint32_t n)
+{
+    const uint32_t es = a.kv.dtype == VFKV_F8 ? 1 : 2, tp = a.kv.dtype == VFKV_F8 ? 32 : 16, per = (len + n - 1) / n;
+    const double row = 2.0 * a.kv.head_dim * es;
+    const uint64_t ctas = base * n, n_sm = uint64_t(ctx->sm_count);
+    auto wave = [&](uint32_t warps, double rate) {
+        const uint32_t round = warps * tp;
+        return 8.0 + double((per + round - 1) / round * round) * row / rate;
+    };
+    double us = n > 1 ? 4.0 + 0.11 * n : 0.0;
+    if (a.kv.head_dim < 256 && ctas <= n_sm) return us + wave(8, 39400.0);
+    const uint64_t full = ctas / (2 * n_sm), last = ctas % (2 * n_sm);
+    us += double(full) * wave(4, 27000.0 / 2);
+    if (last) us += wave(4, last <= n_sm ? 17000.0 : 27000.0 / 2);
+    return us;
+}
+
 uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile)
 {
     uint32_t max_len = a.seq.max_len_hint ? a.seq.max_len_hint : a.kv.max_seq;
@@ -225,6 +249,21 @@ uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile)
             if (score > best) { best = score; pick = n; }
         }
         want = pick;
+    }
+    // Between nine pairs (fewer are a layer at a time, whose calls the host bounds) and two CTAs an SM the count of the rules
+    // above gives way to the one that the model of the launch finds, if it promises a tenth or more (64 q / 8 kv heads over FP8, 8
+    // layers x 131 072 positions: 9 splits 363 to 372 us, 2 329 to 370 by the SM clock; 128 pairs of 3000 28.0 -> 18.4; scaled, 256 pairs of 2001 to 4099 57 -> 49; F16,
+    // 192 pairs of at most 319, sixteen q-heads each 24 -> 11; over the 280 grids a tenth on average, one of them 6 % slower, one 2).
+    // Not for 64-dim rows, of which four CTAs share an SM, nor for more than a GB with at most four q-heads a kv-head, where only
+    // HBM counts and every SM (64 pairs of 41 443, F16: 9 splits 208 us, 2 216).
+    const bool hbm_bound = a.n_q_heads / (a.kv.n_kv_heads * parts) <= 4 &&
+                           double(max_len) * double(base) * 2.0 * a.kv.head_dim * (a.kv.dtype == VFKV_F8 ? 1 : 2) > 1e9;
+    if (tile >= 128 && base > 8 && base < slots && a.kv.head_dim != 64 && !hbm_bound) {
+        double best = 0.9 * split_us(ctx, a, max_len, base, uint32_t(want));
+        for (uint32_t n = 1; n == 1 || (n <= 64 && base * n <= 3 * uint64_t(ctx->sm_count) && uint64_t(n) * 128 <= max_len); ++n) {
+            const double us = split_us(ctx, a, max_len, base, n);
+            if (us < best) { best = us; want = n; }
+        }
     }
     return uint32_t(want);
 }

@@ -9,18 +9,20 @@
 // in flight in registers).
 //   S: thread = 4 rows x 4 positions; 8 16-byte shared loads for 64 FMAs.
 //   PV: thread = 8 rows x 4 dims; 3 16-byte shared loads for 32 FMAs.
-// Shared memory is the bound (a 16-byte load of a warp takes four of its cycles whoever shares an address: 63 % of
-// them used over a launch, the FMA pipe 35 %), so the thread's tile of S is square: 2 x 8, with ten loads for the
+// No pipe is full (shared-memory wavefronts 48 %, FMA pipe 46 %, issue slots 61 %); a 16-byte load of a warp takes four
+// shared-memory cycles whoever shares an address, so the thread's tile of S is square: 2 x 8, with ten loads for the
 // same FMAs, took 90.5 us where this took 84.6 (200 queries at 700 positions, F32).
 //
-// A score's products are summed sixteen at a time.  In one chain of head_dim products (85.5 us) a result was 4.8e-7 off
-// against 64 bits, and 2.4e-6 with scores of 100; now 3.1e-7 and 8.4e-7 (88.4 us), in chains of four 3.5e-7 and 1.3e-6 (91.7).
+// A score's products are summed two at a time (fma.rn.f32x2: the even and the odd dims) in chains of sixteen.  In one chain
+// of head_dim products (85.5 us) a result was 4.8e-7 off against 64 bits, and 2.4e-6 with scores of 100; in chains of sixteen 3.1e-7
+// and 8.4e-7 (88.4 us, one product an instruction; 84.2 with two), in chains of four 3.5e-7 and 1.3e-6 (91.7).  The same for P V,
+// which has to pair values up first, gained nothing (84.6).
 //
 // Row blocks are few and uneven (200 queries x 4 heads x 8 kv-heads: 104 blocks of 8 to 11 tiles), and an SM is
 // at its rate only with two CTAs on it, so the tiles of all (row block, kv-head) items form one line of which every
 // resident CTA takes an even share.  An item that a share ends in goes to scratch in pieces, which a second kernel
 // puts together.  200 queries at 700 positions, F32: 119 us with a CTA or a cluster of two an item, whose second
-// CTAs sat on 60 of 148 SMs; 85 in even shares (88 with the shorter sums above).  Sixteen rows a warp, four warps a CTA (fewer shared loads a product)
+// CTAs sat on 60 of 148 SMs; 85 in even shares (in one chain a score).  Sixteen rows a warp, four warps a CTA (fewer shared loads a product)
 // were faster only from about 1000 positions on (200 at 1500: 153 against 160; 368 at 368: 84 against 76).
 #include "fp8_codec.cuh"
 #include "prefill_params.cuh"
@@ -36,6 +38,7 @@ constexpr int BM = 64, BN = 64;           // rows per CTA, positions per tile
 constexpr int kWarps = 8, kThreads = kWarps * 32;
 constexpr int WR = BM / kWarps, HR = 4;           // rows of a warp, and of a thread in S
 constexpr int LR = 32 / (WR / HR), HP = BN / LR;  // lanes that share a row of S, and positions of each
+constexpr int CHAIN = 32;                 // products of a score in two chains before they go onto its sum
 constexpr int kPiece = 4096;              // elements of a piece of K ([64 positions][64 dims]) or V ([VP][CW])
 constexpr int kPitchK = 68;               // floats per K row: 16-byte units of consecutive rows fall into different banks
 
@@ -59,6 +62,22 @@ __device__ __forceinline__ float fast_exp2(float x)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+
+// Two f32 in one register pair, an operation on both at a time.
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ float lo2(uint64_t a) { return __uint_as_float(uint32_t(a)); }
+__device__ __forceinline__ float hi2(uint64_t a) { return __uint_as_float(uint32_t(a >> 32)); }
 
 // One thread's share of a piece as it lies in the cache.
 template <int DT> struct Raw { uint4 w[kPiece / kThreads / (DT == VFKV_F32 ? 4 : DT == VFKV_F16 ? 8 : 16)]; };
@@ -249,29 +268,27 @@ __global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1) prefill_f32_kernel
             if (live) {
                 const float *const qa = sq + (warp * WR + rp) * S::PITCH_Q + c * 64, *const ka = sbuf + (c & 1) * BN * kPitchK + cl * kPitchK;
 #pragma unroll 1
-                for (int k16 = 0; k16 < 64; k16 += 16) {           // chains of sixteen products: a shorter one loses less
-                    float part[HR][HP];
+                for (int k0 = 0; k0 < 64; k0 += CHAIN) {           // two chains of CHAIN / 2 products each: a shorter one loses less
+                    uint64_t part[HR][HP];
 #pragma unroll
-                    for (int k = k16; k < k16 + 16; k += 4) {
-                        float4 qv[HR];
+                    for (int k = k0; k < k0 + CHAIN; k += 4) {
+                        ulonglong2 qv[HR];
 #pragma unroll
-                        for (int h = 0; h < HR; ++h) qv[h] = *reinterpret_cast<const float4 *>(qa + h * S::PITCH_Q + k);
+                        for (int h = 0; h < HR; ++h) qv[h] = *reinterpret_cast<const ulonglong2 *>(qa + h * S::PITCH_Q + k);
 #pragma unroll
                         for (int j = 0; j < HP; ++j) {
-                            const float4 kv = *reinterpret_cast<const float4 *>(ka + j * LR * kPitchK + k);
+                            const ulonglong2 kv = *reinterpret_cast<const ulonglong2 *>(ka + j * LR * kPitchK + k);
 #pragma unroll
                             for (int h = 0; h < HR; ++h) {
-                                part[h][j] = k == k16 ? qv[h].x * kv.x : fmaf(qv[h].x, kv.x, part[h][j]);
-                                part[h][j] = fmaf(qv[h].y, kv.y, part[h][j]);
-                                part[h][j] = fmaf(qv[h].z, kv.z, part[h][j]);
-                                part[h][j] = fmaf(qv[h].w, kv.w, part[h][j]);
+                                part[h][j] = k == k0 ? mul2(qv[h].x, kv.x) : fma2(qv[h].x, kv.x, part[h][j]);
+                                part[h][j] = fma2(qv[h].y, kv.y, part[h][j]);
                             }
                         }
                     }
 #pragma unroll
                     for (int h = 0; h < HR; ++h)
 #pragma unroll
-                        for (int j = 0; j < HP; ++j) s[h][j] += part[h][j];
+                        for (int j = 0; j < HP; ++j) s[h][j] += lo2(part[h][j]) + hi2(part[h][j]);
                 }
             }
         }

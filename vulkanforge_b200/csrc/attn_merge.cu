@@ -251,13 +251,14 @@ uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile)
         want = pick;
     }
     // Between nine pairs (fewer are a layer at a time, whose calls the host bounds) and two CTAs an SM the count of the rules
-    // above gives way to the one that the model of the launch finds, if it promises a tenth or more (64 q / 8 kv heads over FP8, 8
-    // layers x 131 072 positions: 9 splits 363 to 372 us, 2 329 to 370 by the SM clock; 128 pairs of 3000 28.0 -> 18.4; scaled, 256 pairs of 2001 to 4099 57 -> 49; F16,
-    // 192 pairs of at most 319, sixteen q-heads each 24 -> 11; over the 280 grids a tenth on average, one of them 6 % slower, one 2).
-    // Not for 64-dim rows, of which four CTAs share an SM, nor for more than a GB with at most four q-heads a kv-head, where only
-    // HBM counts and every SM (64 pairs of 41 443, F16: 9 splits 208 us, 2 216).
-    const bool hbm_bound = a.n_q_heads / (a.kv.n_kv_heads * parts) <= 4 &&
-                           double(max_len) * double(base) * 2.0 * a.kv.head_dim * (a.kv.dtype == VFKV_F8 ? 1 : 2) > 1e9;
+    // above gives way to the one that the model of the launch finds, if it promises a tenth or more (128 pairs of 3000 28.0 -> 18.4;
+    // scaled, 256 pairs of 2001 to 4099 57 -> 49; F16, 192 pairs of at most 319, sixteen q-heads each 24 -> 11; over the 280 grids a
+    // tenth on average, one of them 6 % slower, one 2).
+    // Not for 64-dim rows, of which four CTAs share an SM, nor for more than 700 MB, where only HBM and every SM count (64 pairs of
+    // 41 443, F16: 9 splits 208 us, 2 216; at 820 to 980 MB 0.95 to 1.05 of the time with the model's count, one case 0.90) and the
+    // clock that the GPU keeps up decides (64 q / 8 kv heads over FP8, 8 layers x 131 072 positions: 9 splits 363 to 383 us, 2 329
+    // for the first milliseconds, 399 where the power limit then holds).  At 300 to 660 MB it gains 2 to 16 %.
+    const bool hbm_bound = double(max_len) * double(base) * 2.0 * a.kv.head_dim * (a.kv.dtype == VFKV_F8 ? 1 : 2) > 7e8;
     if (tile >= 128 && base > 8 && base < slots && a.kv.head_dim != 64 && !hbm_bound) {
         double best = 0.9 * split_us(ctx, a, max_len, base, uint32_t(want));
         for (uint32_t n = 1; n == 1 || (n <= 64 && base * n <= 3 * uint64_t(ctx->sm_count) && uint64_t(n) * 128 <= max_len); ++n) {

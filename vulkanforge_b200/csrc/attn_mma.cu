@@ -716,13 +716,15 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 #pragma unroll
     for (int nb = 0; nb < NACC; ++nb) { acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.f; }
     // A long sum loses what its terms have below its own last bit: a row's sum of p to rounding, the accumulators to the
-    // tensor cores' cutting off towards zero.  So a chain of products is eight tiles long, and the chains of the high
+    // tensor cores' cutting off towards zero.  So a chain of products is four or eight tiles long, and the chains of the high
     // terms (the low ones are 2^11 smaller) and of l add up in f32 registers of their own.  36 layers of 8192 FP8
     // positions, 64 tiles a warp: results 1.8e-6 off in one chain, 6.7e-7 so, at the same 102 us; groups of eight heads
-    // pay 2 to 4 % (131 072 positions x 8 layers: 366 -> 373 us).  The shape with two stages and three CTAs an SM is
+    // pay 2 to 4 % (131 072 positions x 8 layers: 366 -> 373 us).  Four, where it costs nothing (up to four heads a kv-head) or
+    // where few splits leave a warp many tiles (eight warps: 21 grids against 64 bits, 0.95 of the error that the counts of the
+    // rules had with chains of eight, 1.04 with eight here too); four warps with eight heads of 256-dim FP8 rows would pay 2 %.  The shape with two stages and three CTAs an SM is
     // chosen for eight tiles or less.
     constexpr bool CHAINS = !ROWS2 && !(W == 4 && NS == 2 && S::STAGE_BYTES <= 8192);
-    constexpr uint32_t kChain = SOLO ? 1 : 8;         // by itself a warp has the tiles that four had before: no longer sums than theirs
+    constexpr uint32_t kChain = SOLO ? 1 : TR || W == 8 ? 4 : 8;         // by itself a warp has the tiles that four had before: no longer sums than theirs
     float tot[CHAINS ? NACC : 1][2], l_tot = 0.f, m_tot = kMaskedScore;      // relative to the maximum (and the scale) they were left at
     uint32_t vs_tot = 0u;
 #pragma unroll

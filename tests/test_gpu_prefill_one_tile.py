@@ -196,3 +196,43 @@ def test_a_reference_that_moves_in_every_tile(ctx, dtype, hq, hkv, d, tiles):
     finally:
         fwd.workspace.destroy()
         cache.destroy()
+
+
+@pytest.mark.parametrize("dtype,hq,hkv,d,lens", [("F16", 8, 8, 64, 1500), ("F16", 32, 8, 128, 700), ("F16", 16, 8, 256, 300), ("F8s", 32, 8, 128, 200),
+                                                 ("F8s", 16, 8, 256, 130)])
+def test_scores_beyond_what_f32_counts_in_units(ctx, dtype, hq, hkv, d, lens):
+    """Scores of 2^8 to 2^31, most of them below zero, one position's far above the others': its row of V, whatever a unit in the
+    maximum's last place is (2 from 2^24 on; half precision has nothing below 2^-24).  Only the calls whose Q is in two terms,
+    scaled, hold such queries."""
+    import torch
+    scaled, name = dtype == "F8s", "F16" if dtype == "F16" else "F8"
+    m = 48
+    L = lens + m
+    rng = np.random.default_rng(d + lens)
+    k = np.zeros((L, hkv, d), np.float32)
+    k[:, :, 0] = 128.0                                     # with q[0]: where all scores lie
+    pick = lens // 2
+    k[pick, :, 2] = 64.0
+    v = torch.from_numpy(rng.standard_normal((L, hkv, d), dtype=np.float32)).to(torch.float8_e4m3fn).float().numpy()
+    if scaled:
+        v[:, :, 0] = 448.0                                 # scales of V are 1
+        k *= 3.5                                           # of K too: 448 in every row
+    q = np.zeros((m, hq, d), np.float32)
+    size = np.exp2(np.linspace(8, 31, m))[:, None] * np.sqrt(d) * (1.0 + 0.4 * rng.random((m, hq)))
+    sign = np.where(np.arange(m) % 5 == 4, 1.0, -1.0)[:, None]
+    q[:, :, 0] = size * sign / k[0, 0, 0]
+    q[:, :, 2] = size / 4 / 64.0
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, L, scale_mode=int(scaled)), vf.KvDtype[name])
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    try:
+        fwd.b_step_kv_write(0, to_dev(k), to_dev(v), L, 0)
+        out = torch.full((m, hq, d), float("nan"), device="cuda")
+        fwd.run_flash_attn_batch(0, to_dev(q), out, m, lens, L, 0, 0)
+        torch.cuda.synchronize()
+        ctx.poll()
+        want = np.broadcast_to(np.repeat(v[pick], hq // hkv, axis=0), (m, hq, d))
+        # the other positions are e^-64 and further below
+        assert float(np.abs(out.cpu().numpy() - want).max()) <= 1e-5 * float(np.abs(v).max())
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

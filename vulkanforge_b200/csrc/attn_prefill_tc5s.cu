@@ -98,27 +98,57 @@ __device__ __forceinline__ uint32_t chunk_off(uint32_t r, uint32_t c, uint32_t s
     return (c >> 3) * slab + r * 128u + (((c & 7u) ^ (r & 7u)) << 4);
 }
 
-// A value in shared memory that carries in its low bits the number of the group's tile that left it: who finds the tile that
-// it waits for, or a later one (at most a second), has the value.  A group is at most three of its tiles ahead of the other's
-// question.  With four bits the value is as good as exact: 2^(maximum - reference) still rounds to 1 in half precision.
-constexpr uint32_t kCountBits = 0xfu;
-__device__ __forceinline__ void word_set(uint32_t at, uint32_t value, uint32_t count)
+// What a group tells the other of a row: the reference, and the number of its tiles that it is of.  Who finds the tile that it
+// waits for, or a later one (at most a second), has the reference of that tile or a later one: they only rise.  One word of
+// 64 bits, stored and loaded whole; with scales, where shared memory has no room for those and the exponent goes along, the
+// references and a count behind them for each warp (28 against 29.5 us a call of 98 queries at 2616, but 25.0 against 24.2 for
+// 333 of 1333, F16).  The count in the reference's own low bits would move it by up to 15 units in its last place, which from
+// scores of 2^24 on is more binary orders than half precision has.
+__device__ __forceinline__ void word_set(uint32_t at, uint32_t value)
 {
-    asm volatile("st.volatile.shared::cta.u32 [%0], %1;" :: "r"(at), "r"((value & ~kCountBits) | (count & kCountBits)) : "memory");
+    asm volatile("st.volatile.shared::cta.u32 [%0], %1;" :: "r"(at), "r"(value) : "memory");
 }
-__device__ __forceinline__ bool word_wait(uint32_t at, uint32_t count, uint32_t *value)
+__device__ __forceinline__ uint32_t word_get(uint32_t at)
+{
+    uint32_t value;
+    asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(value) : "r"(at) : "memory");
+    return value;
+}
+__device__ __forceinline__ void pair_set(uint32_t at, float value, uint32_t count)
+{
+    asm volatile("st.volatile.shared::cta.u64 [%0], %1;" :: "r"(at), "l"(uint64_t(count) << 32 | __float_as_uint(value)) : "memory");
+}
+__device__ __forceinline__ void count_set(uint32_t at, uint32_t count)      // by one lane, behind __syncwarp()
+{
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" :: "r"(at), "r"(count) : "memory");
+}
+template <typename Look> __device__ __forceinline__ bool wait_until(Look look)
 {
     uint64_t t0 = 0;
     for (uint32_t it = 0;; ++it) {
-        uint32_t w;
-        asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(w) : "r"(at) : "memory");
-        *value = w & ~kCountBits;
-        if (((w - count) & kCountBits) <= kCountBits / 2) return true;
+        if (look()) return true;
         if ((it & 1023u) == 1023u) {
             if (t0 == 0) t0 = timer_ns();
             else if (timer_ns() - t0 > 1000000000ull) return false;
         }
     }
+}
+__device__ __forceinline__ bool pair_wait(uint32_t at, uint32_t count, float *value)
+{
+    return wait_until([&]() {
+        uint64_t w;
+        asm volatile("ld.volatile.shared::cta.u64 %0, [%1];" : "=l"(w) : "r"(at) : "memory");
+        *value = __uint_as_float(uint32_t(w));
+        return uint32_t(w >> 32) >= count;
+    });
+}
+__device__ __forceinline__ bool count_wait(uint32_t at, uint32_t count)
+{
+    return wait_until([&]() {
+        uint32_t n;
+        asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(n) : "r"(at) : "memory");
+        return n >= count;
+    });
 }
 
 // One row by one warp over positions [lo, hi), each read only if the row sees it; to dst as the rows of the kernel below,
@@ -174,12 +204,12 @@ prefill_one_tile_kernel(const __grid_constant__ OneTileParams op, const __grid_c
     const uint32_t base = smem_addr(sm), q_sm = base, ring = base + T::Q, small = ring + NST * T::STAGE;
     uint8_t *const sm_small = sm + T::Q + NST * T::STAGE;
     // 0: barriers   352: tensor memory address, abort flag   384: row multipliers [128]
-    // 896: the reference maximum of a row as a group knows it, with the number of its tiles in the low bits [group][128]
-    // 1920: SC: the same of the exponent of the largest V scale [group][quarter of the rows]   2048: SC: a tile's scales
-    // [group][64 of K, 64 of V]
+    // 896: the reference maximum of a row as a group knows it and the number of the group's tiles that it is of [group][128]
+    // SC: 896: the reference [group][128]   1920: the exponent of the largest V scale [group][quarter of the rows]   1952: the
+    // number of tiles that these are of [group][quarter]   2048: a tile's scales [group][64 of K, 64 of V]
     volatile uint32_t *const s_ctl = reinterpret_cast<uint32_t *>(sm_small + 352);
     float *const s_mult = reinterpret_cast<float *>(sm_small + 384);
-    const uint32_t refs = small + 896u, vrefs = small + 1920u;
+    const uint32_t refs = small + 896u, vrefs = small + 1920u, counts = small + 1952u;
     float *const s_scales = reinterpret_cast<float *>(sm_small + 2048);
     const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31u;
     const uint32_t g = p.group, n_rows = p.m * g;
@@ -201,7 +231,11 @@ prefill_one_tile_kernel(const __grid_constant__ OneTileParams op, const __grid_c
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_ctl[1] = 0u;
     }
-    if (tid < 264u) word_set(tid < 256u ? refs + 4u * tid : vrefs + 4u * (tid - 256u), 0u, 0u);
+    if constexpr (SC) {
+        if (tid < 16u) word_set(vrefs + 4u * tid, 0u);     // the counts as well
+    } else {
+        if (tid < 256u) pair_set(refs + 8u * tid, 0.f, 0u);
+    }
     if (warp == 8) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(small + 352u), "n"(T::TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -343,7 +377,7 @@ prefill_one_tile_kernel(const __grid_constant__ OneTileParams op, const __grid_c
         // what is left to multiply the scores by when they are exponentiated
         const float late = CAP ? kLog2e : SC ? 1.0f : mult;
         constexpr float GROW = SC ? 9.0f : 14.0f;            // half precision holds p up to 2^16
-        float mref = __uint_as_float(__float_as_uint(kMaskedScore) & ~kCountBits), lrow = 0.f;      // the row's reference as this group knows it, and its sum of p in terms of it
+        float mref = kMaskedScore, lrow = 0.f;      // the row's reference as this group knows it, and its sum of p in terms of it
         uint32_t vs_ref = 0u;                      // SC: exponent bits of the largest V scale so far
         float *const my_scales = s_scales + grp * 128u;
         float sc_next = 0.f;                       // SC: this thread's one of the next tile's 64 + 64 scales
@@ -368,10 +402,16 @@ prefill_one_tile_kernel(const __grid_constant__ OneTileParams op, const __grid_c
             // tile that leaves the reference alone is settled as soon as its maximum is known, whatever the tile before did.)
             bool moved = false;
             auto their_ref = [&]() -> bool {
-                uint32_t w, v = 0u;
-                const bool there = word_wait(refs + 4u * ((grp ^ 1u) * 128u + rt), (it + 1u) / 2u, &w) &&
-                                   (!SC || word_wait(vrefs + 4u * ((grp ^ 1u) * 4u + quarter), (it + 1u) / 2u, &v));
-                const float theirs = __uint_as_float(w);         // references only rise: the later one is the larger
+                bool there;
+                float theirs;                                    // references only rise: the later one is the larger
+                uint32_t v = 0u;
+                if constexpr (SC) {
+                    there = count_wait(counts + 4u * ((grp ^ 1u) * 4u + quarter), (it + 1u) / 2u);
+                    theirs = __uint_as_float(word_get(refs + 4u * ((grp ^ 1u) * 128u + rt)));
+                    v = word_get(vrefs + 4u * ((grp ^ 1u) * 4u + quarter));
+                } else {
+                    there = pair_wait(refs + 8u * ((grp ^ 1u) * 128u + rt), (it + 1u) / 2u, &theirs);
+                }
                 moved = theirs > mref;
                 if (moved) {
                     lrow *= fast_exp2(mref - theirs);
@@ -427,7 +467,7 @@ prefill_one_tile_kernel(const __grid_constant__ OneTileParams op, const __grid_c
                         if (!their_ref()) { ok = false; break; }
                     }
                     asked = true;
-                    const float mnew = mx > mref + GROW ? __uint_as_float(__float_as_uint(mx) & ~kCountBits) : mref;
+                    const float mnew = mx > mref + GROW ? mx : mref;
                     float f = fast_exp2(mref - mnew);
                     lrow *= f;
                     mref = mnew;
@@ -449,8 +489,14 @@ prefill_one_tile_kernel(const __grid_constant__ OneTileParams op, const __grid_c
                     }
                 }
                 if (pass == 0u) {                  // what this tile does to the reference is done, or nothing
-                    word_set(refs + 4u * (grp * 128u + rt), __float_as_uint(mref), it / 2u + 1u);
-                    if (SC && lane == 0u) word_set(vrefs + 4u * (grp * 4u + quarter), vs_ref, it / 2u + 1u);
+                    if constexpr (SC) {
+                        word_set(refs + 4u * (grp * 128u + rt), __float_as_uint(mref));
+                        if (lane == 0u) word_set(vrefs + 4u * (grp * 4u + quarter), vs_ref);
+                        __syncwarp();
+                        if (lane == 0u) count_set(counts + 4u * (grp * 4u + quarter), it / 2u + 1u);
+                    } else {
+                        pair_set(refs + 8u * (grp * 128u + rt), mref, it / 2u + 1u);
+                    }
                 }
                 // a row that has seen nothing yet refers to a finite value, from where exp2 gives 0 for it
                 const float from = fmaxf(mref, 0.5f * kMaskedScore);
@@ -517,11 +563,7 @@ prefill_one_tile_kernel(const __grid_constant__ OneTileParams op, const __grid_c
         // the later reference is the one that O is at, the sums of before are brought to it
         mref = fmaxf(s_end[BM + rt], s_end[3u * BM + rt]);
         lrow = s_end[rt] * fast_exp2(s_end[BM + rt] - mref) + s_end[2u * BM + rt] * fast_exp2(s_end[3u * BM + rt] - mref);
-        if constexpr (SC) {
-            uint32_t v;
-            word_wait(vrefs + 4u * ((grp ^ 1u) * 4u + quarter), n_tiles > grp ? (n_tiles + grp) / 2u : 0u, &v);
-            vs_ref = max(vs_ref, v);
-        }
+        if constexpr (SC) vs_ref = max(vs_ref, word_get(vrefs + 4u * ((grp ^ 1u) * 4u + quarter)));        // both groups are through
         const float unit = SC ? __uint_as_float(vs_ref) * (1.0f / kPUnit) : 1.0f;
         float row_scale, finite = 0.f;             // finite: 0, or NaN if an element is not
         float *row_dst, *piece = nullptr;

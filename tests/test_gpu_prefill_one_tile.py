@@ -236,3 +236,49 @@ def test_scores_beyond_what_f32_counts_in_units(ctx, dtype, hq, hkv, d, lens):
     finally:
         fwd.workspace.destroy()
         cache.destroy()
+
+
+@pytest.mark.parametrize("hq,hkv,d,L,gain", [(32, 8, 128, 300, 1.0), (32, 8, 128, 4000, 3.0), (16, 8, 256, 500, 2.0), (8, 8, 64, 300, 1.0)])
+def test_v_scales_far_apart(ctx, hq, hkv, d, L, gain):
+    """Eight positions whose V is 2^12 larger than the others' and whose p is e^-14 of theirs.  P times its V scale is fed as two
+    half-precision terms, 2^-22 of it or the last bit of the second, which is 2^-34 of (the row's largest p x the largest V scale)."""
+    import torch
+    m = 35
+    gen = torch.Generator(device="cuda").manual_seed(L)
+    k, v = (torch.randn(L, hkv, d, device="cuda", generator=gen) for _ in range(2))
+    k[:, :, 0] = 14.0
+    sinks = torch.arange(8, device="cuda") * (L // 9) + 3
+    k[sinks, :, 0] = 0.0
+    v[sinks] *= 4096.0
+    q = torch.randn(m, hq, d, device="cuda", generator=gen) * gain
+    q[:, :, 0] = d ** 0.5
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(1, hkv, d, L, scale_mode=1), vf.KvDtype.F8)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq)
+    try:
+        fwd.b_step_kv_write(0, k, v, L, 0)
+        out = torch.zeros(m, hq, d, device="cuda")
+        fwd.run_flash_attn_batch(0, q, out, m, L - m, L, 0, 0)
+        torch.cuda.synchronize()
+        ctx.poll()
+
+        def rows(buf, scales):                             # the codes and scales that the append stored
+            codes = torch.from_numpy(dev_view_bytes(buf, L * hkv * d)).view(torch.float8_e4m3fn).view(L, hkv, d).cuda().double()
+            return codes, torch.from_numpy(dev_view_bytes(scales, L * hkv * 4).view(np.float32).copy()).view(L, hkv, 1).cuda().double()
+
+        (kc, ks), (vc, vs) = rows(cache.k_buffer, cache.k_scales), rows(cache.v_buffer, cache.v_scales)
+        s = torch.einsum("mhgd,lhd->hgml", q.double().view(m, hkv, hq // hkv, d), kc * ks) / d ** 0.5
+        s = s.masked_fill(torch.arange(L, device="cuda") > L - m + torch.arange(m, device="cuda")[:, None], -float("inf"))
+        p = torch.exp(s - s.amax(-1, keepdim=True))
+        total = p.sum(-1)[..., None]
+        mean = lambda x: (torch.einsum("hgml,lhd->hgmd", p, x) / total).permute(2, 0, 1, 3).reshape(m, hq, d)
+        want = mean(vc * vs)
+        # two terms of every product, and 4e-6 of the sum for scores and exponentials in f32 (scores up to some 20)
+        fed = torch.einsum("hgml,lhd->hgmd", (s > -1e30).double(), vc.abs()) * 2.0 ** -35 * vs.max() / total
+        tol = fed.permute(2, 0, 1, 3).reshape(m, hq, d) + (2.0 ** -22 + 4e-6) * mean((vc * vs).abs())
+        worst = float(((out.double() - want).abs() / tol).max())
+        error = float((out.double() - want).norm() / want.norm())
+        print("V scales far apart: %.2e of 64 bits, %.2f of the bound" % (error, worst))
+        assert worst <= 1.0
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

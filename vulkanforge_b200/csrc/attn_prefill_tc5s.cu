@@ -27,8 +27,10 @@
 //
 // SPLITQ: Q = high + low half-precision term, scaled per row by a power of two (two products for S).
 // SC: the scales of K multiply the scores, those of V multiply P, in f32; P is then also fed as two terms,
-// relative to the largest power of two among the V scales so far (all of it exact but the terms' own
-// 2^-22), which makes the result as accurate as f32 tiles on the CUDA cores.
+// relative to the largest power of two among the V scales so far (exact but for 2^-22 of it, or for the last bit of the second
+// term: 2^-34 of the row's largest p x the largest V scale), which makes the result as accurate as f32 tiles on the CUDA cores.
+// So the reference lags by 2^4 at most here: room for a lag of 2^9 in the first term would take five bits from the second
+// (V scales 2^12 apart, 256 dims x 500 positions: 1.2e-5 off against 64 bits where this is 2.3e-6; no faster).
 //
 // The tiles of a row block are cut over n_split CTAs when the blocks leave SMs idle; the pieces go to
 // scratch and prefill_pieces_kernel puts them together (flash_attn_reduce.comp:51-80, maximum first).
@@ -52,7 +54,7 @@ constexpr int BM = 128, BN = 64;
 template <int DT> constexpr uint32_t kThreads = DT == VFKV_F8 ? 480 : 352;
 constexpr uint32_t SLAB_Q = 128 * 128, SLAB_KV = 64 * 128;      // [rows][64 halves], 128-byte swizzle
 constexpr uint32_t kSmall = 3072;                               // barriers, row multipliers, tile scales
-constexpr float kPUnit = 32.0f;                                 // SC: P terms are fed as p * v_scale / reference * 2^5 <= 2^15
+constexpr float kPUnit = 1024.0f;                               // SC: P terms are fed as p * v_scale / reference * 2^10 <= 2^15
 
 struct OneTileParams {
     PrefillParams a;
@@ -376,7 +378,7 @@ prefill_one_tile_kernel(const __grid_constant__ OneTileParams op, const __grid_c
         const float mult = SPLITQ ? s_mult[rt] : 1.0f, inv_cap = CAP ? 1.0f / p.softcap : 0.f;
         // what is left to multiply the scores by when they are exponentiated
         const float late = CAP ? kLog2e : SC ? 1.0f : mult;
-        constexpr float GROW = SC ? 9.0f : 14.0f;            // half precision holds p up to 2^16
+        constexpr float GROW = SC ? 4.0f : 14.0f;            // half precision holds p up to 2^16
         float mref = kMaskedScore, lrow = 0.f;      // the row's reference as this group knows it, and its sum of p in terms of it
         uint32_t vs_ref = 0u;                      // SC: exponent bits of the largest V scale so far
         float *const my_scales = s_scales + grp * 128u;

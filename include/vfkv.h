@@ -333,8 +333,9 @@ int32_t vfkv_decode_token(vfkv_cache *cache, vfkv_workspace *ws, const float *d_
  * bus in up to four groups of layers, on streams owned by the workspace, so that a group computes
  * while the next one's inputs travel; smaller ones from pinned, 16-byte aligned buffers are read
  * by one kernel and leave by the attention kernel's own stores.  From such buffers, where there are
- * more (layer, sequence, kv-head) triples than SMs and none is split, the attention kernel itself
- * reads the inputs, and nothing is recorded.  The call returns when h_out is complete.  Pinned host buffers make the copies asynchronous. */
+ * many (layer, sequence, kv-head) triples and none is split, the attention kernel itself reads the
+ * inputs, and nothing is recorded.  The call returns when h_out is complete.  Pinned host buffers make
+ * the copies asynchronous. */
 int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const float *h_q,
                                const float *h_k, const float *h_v, float *h_out,
                                uint32_t n_q_heads, const uint32_t *h_slot_ids,

@@ -849,10 +849,16 @@ int32_t vfkv_decode_token(vfkv_cache *cache, vfkv_workspace *ws, const float *d_
 }
 
 // Whether the launches of decode_layers() for a whole token are all of the tensor-core kernel with one split, and each with
-// more CTAs than SMs: then that kernel may read the token's inputs where they are, in pinned host memory.  Each is read once, and
-// the K/V streams of other CTAs hide the bus.
+// enough pairs: then that kernel may read the token's inputs where they are, in pinned host memory.  Each is read once, and the
+// K/V streams of other CTAs hide the bus.  In one wave all CTAs wait for the bus at once, and what a kernel fetches in front of
+// the launch is there sooner.  `fetched`: a kernel would (and not copies, which any such launch beats: 64 q / 8 kv, 336 pairs
+// of 60, 3.1 MB 98 -> 85 us).  `longest`: of the sequences.  Against that kernel, in us fetched / read by the attention kernel:
+//   up to two CTAs an SM: 288 pairs of 8192, FP8 132 / 140 (142 and 143 on two more hosts, 125 on a fourth); 288 of 100 48 / 55
+//   up to three, unless rows of 300 KB to 2 MB hide it: F16, 320 of 209 54 / 59, of 1577 92 / 87; 400 of 600 73 / 70; FP8, 320 of
+//   1577 73 / 73, of 4000 113 / 110, of 8192 180 / 184 (and not for groups of more than four heads: 336 of 3000 111 / 117)
+//   up to four, where a pair has less than 150 KB: FP8, 464 of 60 65 / 71, 576 81 / 83; 464 of 600 71 / 72, 576 84 / 82
 static bool reads_host_inputs(vfkv_cache *cache, const float *q, float *out, uint32_t n_q_heads, uint32_t n_seqs, uint32_t hint,
-                              const uint32_t *windows, uint32_t n_splits)
+                              uint32_t longest, bool fetched, const uint32_t *windows, uint32_t n_splits)
 {
     vfkv_ctx *ctx = cache->ctx;
     KvCache &kv = cache->kv;
@@ -873,7 +879,9 @@ static bool reads_host_inputs(vfkv_cache *cache, const float *q, float *out, uin
         a.seq.window = w;
         a.seq.n_layers = 0;
         for (uint32_t l = first; l < L; ++l) a.seq.n_layers += (windows ? windows[l] : 0u) == w;
-        if (uint64_t(a.seq.units()) * a.kv.n_kv_heads <= uint64_t(ctx->sm_count) || (n_splits == 0u && choose_splits(ctx, a, 128) != 1u))
+        const double bytes = 2.0 * (w && w < longest ? w : longest) * a.kv.head_dim * (a.kv.dtype == VFKV_F8 ? 1 : 2);
+        const uint32_t ctas = !fetched ? 1u : bytes >= 3e5 && bytes < 2e6 && n_q_heads / a.kv.n_kv_heads <= 4u ? 2u : bytes >= 1.5e5 ? 3u : 4u;
+        if (uint64_t(a.seq.units()) * a.kv.n_kv_heads <= uint64_t(ctx->sm_count) * ctas || (n_splits == 0u && choose_splits(ctx, a, 128) != 1u))
             return false;
     }
     return true;
@@ -990,16 +998,16 @@ int32_t vfkv_decode_token_host(vfkv_cache *cache, vfkv_workspace *ws, const floa
             return set_error(ctx, VFKV_ERR_CUDA, "vfkv_decode_token_host: streams and events");
         }
     }
-    // the length hint steers the split count only; it is rounded up so that recordings stay valid for long
+    // the length hint steers the split count and the kernel's shape; it is rounded up so that recordings stay valid for long
     uint32_t hint = (max_pos + 1 + 1023u) / 1024u * 1024u;
     if (hint > kv.config.max_seq_len) hint = kv.config.max_seq_len;
     memcpy(ws->tok_u32, h_positions, n_seqs * 4);
     if (h_slot_ids) memcpy(ws->tok_u32 + ws->max_seqs, h_slot_ids, n_seqs * 4);
-    // A token that fills the GPU with whole sequences is one launch for each window, which takes its inputs straight from the
-    // host's buffers and leaves its outputs there: the bus works while HBM streams, and nothing is fetched first (36 layers of
-    // one sequence at 8192, FP8, 0.9 MB in, 0.6 MB out: 133 -> 127 us; 32 layers of 5
-    // sequences of 65 to 250, 32 q / 2 kv, F16 214 -> 122; 51 of 39 to 59, scaled FP8, 42 MB in 1254 -> 1194).
-    if (in_pinned && out_direct && reads_host_inputs(cache, h_q, h_out, n_q_heads, n_seqs, hint, windows, n_splits)) {
+    // A token of more whole sequences than the GPU holds at a time is one launch for each window, which takes its inputs straight
+    // from the host's buffers and leaves its outputs there: the bus works while HBM streams, and nothing is fetched first (32
+    // layers of 5 sequences of 101 to 2025, F16 254 -> 180 us; 16 of 12, 40 q / 8 kv, FP8 234 -> 189; 51 of 39 to 59, scaled FP8,
+    // 42 MB in 1254 -> 1194).
+    if (in_pinned && out_direct && reads_host_inputs(cache, h_q, h_out, n_q_heads, n_seqs, hint, max_pos + 1, one_kernel_in, windows, n_splits)) {
         const int32_t drc = decode_layers(cache, ws, 0, L, h_q, h_k, h_v, h_out, n_q_heads, h_slot_ids ? ws->tok_u32 + ws->max_seqs : nullptr,
                                           ws->tok_u32, n_seqs, hint, windows, scale, softcap, n_splits, stream, true);
         const cudaError_t de = cudaStreamSynchronize(st);

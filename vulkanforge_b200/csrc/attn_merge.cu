@@ -179,6 +179,16 @@ static double split_us(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t len, uin
     return us;
 }
 
+// The same where one sequence is that long and the others are short: its CTAs, few to an SM, stream 80 KB a us each with 8 warps
+// and 42 with 4, and the others' cost 2.4 us for every three an SM, whatever they find to do.
+static double split_us_alone(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t len, uint64_t base, uint32_t n)
+{
+    const double row = 2.0 * a.kv.head_dim * (a.kv.dtype == VFKV_F8 ? 1 : 2);
+    const double rate = a.kv.head_dim < 256 && base * n <= uint64_t(ctx->sm_count) ? 80000.0 : 42000.0;
+    return (n > 1 ? 4.0 + 0.11 * n : 0.0) + 8.0 + double((len + n - 1) / n) * row / rate +
+           2.4 * double(base * n) / double(3 * uint64_t(ctx->sm_count));
+}
+
 uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile)
 {
     uint32_t max_len = a.seq.max_len_hint ? a.seq.max_len_hint : a.kv.max_seq;
@@ -259,10 +269,19 @@ uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile)
     // clock that the GPU keeps up decides (64 q / 8 kv heads over FP8, 8 layers x 131 072 positions: 9 splits 363 to 383 us, 2 329
     // for the first milliseconds, 399 where the power limit then holds).  At 300 to 660 MB it gains 2 to 16 %.
     const bool hbm_bound = double(max_len) * double(base) * 2.0 * a.kv.head_dim * (a.kv.dtype == VFKV_F8 ? 1 : 2) > 7e8;
+    // The model knows of one length, the longest.  In a batch whose other sequences are short, fewer splits leave the longest to
+    // a few CTAs while the other SMs stand idle (4 layers x 4 sequences, FP8, one of 16 384 and three of 600: 1 split 70 us, 9 42),
+    // so what it promises if all are as long has to be 2.4 times what that would cost.  53 grids of 2 to 32 sequences, each with
+    // all as long / down to half of it / down to a 32nd / half of them a 16th / all but one, in times of the rules' counts:
+    // always the model's 1.14 / 1.10 / 1.05 / 1.06 / 0.88 as fast (at worst 0.99 / 0.92 / 0.76 / 0.80 / 0.38), so
+    // 1.11 / 1.09 / 1.07 / 1.07 / 1.01 (1.00 / 0.97 / 0.86 / 0.83 / 0.70).
     if (tile >= 128 && base > 8 && base < slots && a.kv.head_dim != 64 && !hbm_bound) {
-        double best = 0.9 * split_us(ctx, a, max_len, base, uint32_t(want));
+        const uint32_t rules = uint32_t(want);
+        const double rules_us = split_us(ctx, a, max_len, base, rules), rules_alone = split_us_alone(ctx, a, max_len, base, rules);
+        double best = 0.9 * rules_us;
         for (uint32_t n = 1; n == 1 || (n <= 64 && base * n <= 3 * uint64_t(ctx->sm_count) && uint64_t(n) * 128 <= max_len); ++n) {
             const double us = split_us(ctx, a, max_len, base, n);
+            if (a.seq.n_seqs > 1u && n < rules && rules_us - us < 2.4 * (split_us_alone(ctx, a, max_len, base, n) - rules_alone)) continue;
             if (us < best) { best = us; want = n; }
         }
     }

@@ -67,3 +67,33 @@ def test_a_warp_a_sequence(ctx, dtype, scaled, hq, hkv, d, lens, window, softcap
     finally:
         fwd.workspace.destroy()
         cache.destroy()
+
+
+@pytest.mark.parametrize("hq,hkv,d,lens", [(16, 1, 128, [30] * 63 + [1]), (24, 2, 256, [1, 16, 33, 100] * 8), (32, 2, 64, [17, 128, 250, 5] * 8)])
+def test_groups_of_nine_to_sixteen_feed_p_in_two_terms(ctx, hq, hkv, d, lens):
+    """Against attention in 64 bits of the Q that half precision holds: what is left is sums in f32 (P rounded to half precision as
+    well: 1.5e-4)."""
+    import torch
+    n, longest = len(lens), max(lens)
+    n_layers = -(-700 // (n * hkv))                        # above four CTAs an SM
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    cache = vf.KvCache(ctx, vf.KvCacheConfig(n_layers, hkv, d, longest, n_slots=n), vf.KvDtype.F16)
+    fwd = vf.CudaForward(ctx, cache, n_heads=hq, max_batch=n)
+    try:
+        k, v = (torch.randn(n_layers, n, longest, hkv, d, device="cuda", generator=gen).half().float() for _ in range(2))
+        for layer in range(n_layers):
+            for i, length in enumerate(lens):
+                fwd.b_step_kv_write(layer, k[layer, i, :length].contiguous(), v[layer, i, :length].contiguous(), length, 0, i)
+        at = torch.tensor([x - 1 for x in lens], device="cuda")
+        new_k, new_v = (torch.stack([x[:, i, length - 1] for i, length in enumerate(lens)], 1).contiguous() for x in (k, v))
+        q = torch.randn(n_layers, n, hq, d, device="cuda", generator=gen)
+        out = torch.zeros_like(q)
+        fwd.decode_token(q, new_k, new_v, out, None, at.int(), n, longest)
+        torch.cuda.synchronize()
+        s = torch.einsum("lnhgd,lnphd->lnhgp", q.half().double().view(n_layers, n, hkv, hq // hkv, d), k.double()) / d ** 0.5
+        s = s.masked_fill(torch.arange(longest, device="cuda") > at.view(1, n, 1, 1, 1), -float("inf"))
+        want = torch.einsum("lnhgp,lnphd->lnhgd", s.softmax(-1), v.double()).reshape(out.shape)
+        assert float((out.double() - want).norm() / want.norm()) < 4e-6
+    finally:
+        fwd.workspace.destroy()
+        cache.destroy()

@@ -266,6 +266,21 @@ __device__ __forceinline__ void pv_f16(const uint32_t (&vb)[4], const uint32_t (
     }
 }
 
+// The same with a second term of P.
+template <int TP, int D, int NBK = 0>
+__device__ __forceinline__ void pv_f16_two(const uint32_t (&vb)[4], const uint32_t (&pa)[4], const uint32_t (&pl)[4], float (&acc)[D / 8][4])
+{
+    if constexpr (NBK < D / 8) {
+        uint32_t r0, r1, r2, r3;
+        ldmatrix_x4_trans<(NBK / 8) * TP * 128>(vb[(NBK % 8) / 2], r0, r1, r2, r3);
+        mma_f16(acc[NBK], pa, r0, r1);
+        mma_f16(acc[NBK + 1], pa, r2, r3);
+        mma_f16(acc[NBK], pl, r0, r1);
+        mma_f16(acc[NBK + 1], pl, r2, r3);
+        pv_f16_two<TP, D, NBK + 2>(vb, pa, pl, acc);
+    }
+}
+
 // ---- transposed products (at most 4 q-heads per kv-head) ------------------------------------------
 // With few q-heads the M = 16 rows of an MMA are mostly padding when the heads sit on M.  The
 // transposed products put the positions (S^T = K Q^T) and the output dims (O^T = V^T P^T) on M and
@@ -391,6 +406,10 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // With at most 8 q-heads per kv-head the M tile has room for a second term: rows 0-7 carry the
     // high part of Q (and of P), rows 8-15 the low part, and their products are summed in f32.
     constexpr bool SPLIT = FP8 || !ROWS2;
+    // Nine to sixteen heads fill the M tile: Q and P in one term.  A p that is its warp's maximum is 1 and needs no second one; a
+    // warp by itself has one of these where four had one each, so it feeds P twice instead (24 sequences of 60, 16 layers, 32 q /
+    // 2 kv: error against 64 bits 2.35e-4 with four warps, 2.46e-4 with one, 1.95e-4 so; 17.0, 12.4 and 13.0 us).
+    constexpr bool P_TWO = !SPLIT && SOLO;
     const AttnParams &p = mp.a;
 
     extern __shared__ uint8_t smem_raw[];
@@ -1004,17 +1023,25 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             pv_fp8<TP, D>(vb, pa, acc);
         } else {
             uint32_t pa[4];
+            const uint32_t vb[4] = {vt + v_sw[0], vt + v_sw[1], vt + v_sw[2], vt + v_sw[3]};
             if constexpr (SPLIT) {
                 split_f16x2(x[0][0][0], x[0][0][1], pa[0], pa[1]);
                 split_f16x2(x[0][1][0], x[0][1][1], pa[2], pa[3]);
+                pv_f16<TP, D>(vb, pa, acc);
+            } else if constexpr (P_TWO) {
+                uint32_t pl[4];
+                split_f16x2(x[0][0][0], x[0][0][1], pa[0], pl[0]);
+                split_f16x2(x[0][1][0], x[0][1][1], pa[2], pl[2]);
+                split_f16x2(x[RS - 1][0][0], x[RS - 1][0][1], pa[1], pl[1]);
+                split_f16x2(x[RS - 1][1][0], x[RS - 1][1][1], pa[3], pl[3]);
+                pv_f16_two<TP, D>(vb, pa, pl, acc);
             } else {
                 pa[0] = f32x2_to_f16x2(x[0][0][0], x[0][0][1]);
                 pa[2] = f32x2_to_f16x2(x[0][1][0], x[0][1][1]);
                 pa[1] = f32x2_to_f16x2(x[RS - 1][0][0], x[RS - 1][0][1]);
                 pa[3] = f32x2_to_f16x2(x[RS - 1][1][0], x[RS - 1][1][1]);
+                pv_f16<TP, D>(vb, pa, acc);
             }
-            const uint32_t vb[4] = {vt + v_sw[0], vt + v_sw[1], vt + v_sw[2], vt + v_sw[3]};
-            pv_f16<TP, D>(vb, pa, acc);
         }
         }
 

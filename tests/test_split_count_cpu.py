@@ -48,11 +48,16 @@ def splits(tmp_path_factory):
     # one sequence, many layers: all units are as long as the hint says
     ("F8", 32, 8, 128, 16, 1, 2500, 1, 1),
     ("F8", 32, 8, 128, 36, 1, 8192, 1, 1),
+    ("F16", 16, 8, 256, 16, 1, 2500, 2, 2),
+    ("F8", 16, 8, 256, 2, 1, 9000, 18, 18),                # two more than the rules allow
     # several sequences: fewer splits than by the rules where that costs a long one among short ones little ...
     ("F8", 32, 8, 128, 4, 8, 4099, 1, 1),
     ("F16", 16, 8, 256, 4, 8, 1000, 1, 1),
     ("F8", 32, 8, 128, 2, 7, 3564, 1, 1),
     ("F8", 32, 8, 128, 1, 8, 9906, 2, 2),
+    ("F8", 32, 8, 128, 1, 3, 9000, 6, 6),
+    ("F8", 64, 8, 128, 5, 3, 5000, 1, 1),
+    ("F16", 64, 8, 128, 5, 3, 5000, 1, 1),
     # ... and the rules' count where it would keep a few CTAs busy alone
     ("F8", 32, 8, 128, 4, 4, 16384, 8, 9),
     ("F8", 32, 8, 128, 1, 16, 16384, 8, 9),

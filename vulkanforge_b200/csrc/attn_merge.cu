@@ -153,10 +153,6 @@ int32_t launch_merge_partials_packed(vfkv_ctx *ctx, const float *packed, uint32_
     return check_cuda(ctx, cudaGetLastError(), "merge_partials_packed launch");
 }
 
-// Split count when the caller passes 0.  The reference always cuts at 64
-// positions (runs.rs:766-769); here the count only has to fill the GPU: aim
-// for about two CTAs per SM, never cut below 256 positions per split (128 on the tensor cores
-// with an F16 cache).
 // Expected time (us) of a tensor-core decode launch with n splits of sequences of len positions, base (sequence, kv-head)
 // pairs: a wave of CTAs costs 8 us and its stream, splits cost their merge.  An SM streams 39 KB a us with one CTA of 8 warps, 27
 // with two of 4 and 17 with one of those (HBM, shared, is in that); a CTA works through its positions in rounds of a tile for
@@ -189,6 +185,10 @@ static double split_us_alone(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t le
            2.4 * double(base * n) / double(3 * uint64_t(ctx->sm_count));
 }
 
+// Split count when the caller passes 0.  The reference always cuts at 64
+// positions (runs.rs:766-769); here the count only has to fill the GPU: aim
+// for about two CTAs per SM, never cut below 256 positions per split (128 on the tensor cores
+// with an F16 cache).
 uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile)
 {
     uint32_t max_len = a.seq.max_len_hint ? a.seq.max_len_hint : a.kv.max_seq;

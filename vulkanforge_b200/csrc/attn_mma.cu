@@ -394,7 +394,7 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     using S = Shape<DT, D, W, NS>;
     constexpr int kWarps = W;
     constexpr bool SOLO = W == 1, ONE = SOLO || kHostInputs;     // a warp by itself; one split, no exchange
-    constexpr uint32_t kDrawer = SOLO ? 0u : 32u;        // the thread that draws the ticket
+    constexpr uint32_t kDrawer = 32;                     // the thread that draws the ticket
     constexpr int kStages = NS;
     constexpr int TP = S::TP, NB = S::NB, NC = S::NC, KSTEPS = S::KSTEPS, NDB = S::NDB;
     constexpr bool FP8 = DT == VFKV_F8;
@@ -740,10 +740,12 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // positions, 64 tiles a warp: results 1.8e-6 off in one chain, 6.7e-7 so, at the same 102 us; groups of eight heads
     // pay 2 to 4 % (131 072 positions x 8 layers: 366 -> 373 us).  Four, where it costs nothing (up to four heads a kv-head) or
     // where few splits leave a warp many tiles (eight warps: 21 grids against 64 bits, 0.95 of the error that the counts of the
-    // rules had with chains of eight, 1.04 with eight here too); four warps with eight heads of 256-dim FP8 rows would pay 2 %.  The shape with two stages and three CTAs an SM is
-    // chosen for eight tiles or less.
+    // rules had with chains of eight, 1.04 with eight here too); four warps with eight heads of 256-dim FP8 rows would pay 2 %.
+    // A warp by itself has the tiles that four had before: a chain each.  The shape with two stages and three CTAs an SM is
+    // chosen for eight tiles or less.  Groups of nine to sixteen heads have one sum, however long: their Q in one half-precision
+    // term is off by 2^-12.
     constexpr bool CHAINS = !ROWS2 && !(W == 4 && NS == 2 && S::STAGE_BYTES <= 8192);
-    constexpr uint32_t kChain = SOLO ? 1 : TR || W == 8 ? 4 : 8;         // by itself a warp has the tiles that four had before: no longer sums than theirs
+    constexpr uint32_t kChain = SOLO ? 1 : TR || W == 8 ? 4 : 8;
     float tot[CHAINS ? NACC : 1][2], l_tot = 0.f, m_tot = kMaskedScore;      // relative to the maximum (and the scale) they were left at
     uint32_t vs_tot = 0u;
 #pragma unroll
@@ -1636,12 +1638,14 @@ int32_t launch_c(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
     const uint32_t longest = mp.a.window && mp.a.window < mp.longest ? mp.a.window : mp.longest;
     // Sequences of a few tiles, more of them than 4-warp CTAs are resident at a time: a warp each.  A CTA of four warps is then
     // setting up, joining its warps and writing for most of its life, and two or three of them share an SM; of these
-    // there are up to twelve, which share nothing.  32 layers x 32 sequences, 32 q / 8 kv / 128, FP8: 24 positions 84.6 ->
+    // there are up to twelve (256 dims: six; five to eight heads a kv-head: nine, by registers), which share nothing.  32 layers x 32 sequences, 32 q / 8 kv / 128, FP8: 24 positions 84.6 ->
     // 29.9 us, 128 92 -> 55, 256 123 -> 94, 400 163 -> 146, 600 208 -> 207; F16, 16 q / 8 kv / 256: 64 164 -> 103, 256 358 -> 320;
     // 16 layers x 4 sequences, FP8: 64 8.7 -> 5.8, 256 11.7 -> 10.0 (where the 4-warp CTAs run side by side, at most 2 tiles
-    // are as fast).  Three stages a warp where they cost no further wave (2048 sequences of 400: 50 us with two, 42 with three).
+    // are as fast); 4 layers x 32 sequences, 64 q / 8 kv / 256, FP8, where it spills 0.3 KB a thread: 30 33 -> 18, 250 52 -> 48.
+    // Three stages a warp where they cost no further wave, counted by shared memory (2048 sequences of 400: 50 us with two, 42
+    // with three).
     if (w == 0 && mp.a.n_splits == 1u && mp.a.fan == nullptr && ctas > uint64_t(ctx->sm_count) * (D == 64 ? 4u : 3u)) {
-        const uint32_t tiles = ((mp.a.window && mp.a.window < mp.longest ? mp.a.window : mp.longest) + Shape<DT, D, 1, 2>::TP - 1) / Shape<DT, D, 1, 2>::TP;
+        const uint32_t tiles = (longest + Shape<DT, D, 1, 2>::TP - 1) / Shape<DT, D, 1, 2>::TP;
         if (tiles <= 16u) {
             auto waves = [&](uint64_t smem) {
                 const uint64_t slots = uint64_t(ctx->sm_count) * std::min<uint64_t>(12u, 227u * 1024u / (smem + 1024u));

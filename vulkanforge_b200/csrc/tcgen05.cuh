@@ -152,7 +152,7 @@ __device__ __forceinline__ float fast_exp2(float x)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// The largest of 64: eight chains of three-input maxima.
+// The largest of 64: four chains of three-input maxima.
 __device__ __forceinline__ float max3(float a, float b, float c)
 {
     float y;

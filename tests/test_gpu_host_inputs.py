@@ -14,9 +14,9 @@ pytestmark = pytest.mark.gpu
     ("F8", False, 32, 8, 128, 19, [600, 70, 33], 1024, 0, 0.0, True, 1),          # 456 pairs, four warps a CTA
     ("F8", False, 64, 8, 128, 7, [1, 200, 64, 90, 5, 33, 7], 1024, 0, 30.0, False, 1),       # 3.5 MB; eight q-heads: 4 KB of Q
     ("F8", True, 32, 8, 128, 56, [600], 1024, 0, 0.0, False, 1),
-    ("F8", False, 32, 8, 128, 26, [60, 31, 5], 512, 0, 0.0, False, 1),            # at most sixteen tiles: a warp a sequence
+    ("F8", False, 32, 8, 128, 26, [60, 31, 5], 256, 0, 0.0, False, 1),            # at most eight tiles: a warp a sequence
     ("F16", False, 16, 8, 256, 38, [40, 17, 100], 1024, 50, 0.0, True, 2),        # a window in half of the layers: a launch each
-    ("F16", False, 16, 1, 128, 48, [90, 20, 1, 64, 33, 17, 16, 250, 5, 128], 256, 0, 0.0, False, 1),      # sixteen q-heads: 8 KB of Q
+    ("F16", False, 16, 1, 128, 48, [90, 20, 1, 64, 33, 17, 16, 100, 5, 128], 128, 0, 0.0, False, 1),      # the same; sixteen q-heads: 8 KB of Q
     ("F16", False, 8, 8, 64, 38, [128, 100], 256, 0, 50.0, False, 1),             # 608 pairs, however short
     ("F16", False, 32, 8, 128, 38, [600], 1024, 0, 0.0, False, 1),                # 304 of 300 KB
     ("F8", False, 32, 8, 128, 36, [70], 1024, 0, 0.0, False, 2),                  # 288 pairs: the inputs are fetched first

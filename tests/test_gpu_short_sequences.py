@@ -1,5 +1,6 @@
 """Tokens of many short sequences: a warp each, without splits or a merge, against a decode step per layer (whose grids are
-small enough for CTAs of several warps), at the edges of the kernel's tiles and at the most tiles that this is done for."""
+small enough for CTAs of several warps), at the edges of the kernel's tiles and at the most tiles that this is done for
+(test_split_count_cpu.py has the lines)."""
 import numpy as np
 import pytest
 
@@ -24,7 +25,7 @@ pytestmark = pytest.mark.gpu
 def test_a_warp_a_sequence(ctx, dtype, scaled, hq, hkv, d, lens, window, softcap):
     import torch
     n, longest = len(lens), max(lens)
-    n_layers = -(-700 // (n * hkv))                        # above four CTAs an SM
+    n_layers = -(-1500 // (n * hkv))                       # above ten CTAs an SM: up to sixteen tiles
     rng = np.random.default_rng(longest + d)
     gen = torch.Generator(device="cuda").manual_seed(longest)
     cache = vf.KvCache(ctx, vf.KvCacheConfig(n_layers, hkv, d, longest + 3, n_slots=n, scale_mode=int(scaled)), vf.KvDtype[dtype])
@@ -75,7 +76,7 @@ def test_groups_of_nine_to_sixteen_feed_p_in_two_terms(ctx, hq, hkv, d, lens):
     well: 1.5e-4)."""
     import torch
     n, longest = len(lens), max(lens)
-    n_layers = -(-700 // (n * hkv))                        # above four CTAs an SM
+    n_layers = -(-1500 // (n * hkv))                       # above ten CTAs an SM: up to sixteen tiles
     gen = torch.Generator(device="cuda").manual_seed(d)
     cache = vf.KvCache(ctx, vf.KvCacheConfig(n_layers, hkv, d, longest, n_slots=n), vf.KvDtype.F16)
     fwd = vf.CudaForward(ctx, cache, n_heads=hq, max_batch=n)

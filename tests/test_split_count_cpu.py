@@ -1,4 +1,5 @@
-"""The split count that the decode kernel chooses by itself, asked of the library's own function: no GPU needed."""
+"""The split count that the decode kernel chooses by itself, and the sequences that it gives to a warp each, asked of the library's
+own functions: no GPU needed."""
 import os
 import shutil
 import subprocess
@@ -12,7 +13,6 @@ NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
 DRIVER = r"""
 #include <cstdio>
 #include "common.cuh"
-namespace vfkv { uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile); }
 int main()
 {
     vfkv_ctx ctx;
@@ -23,7 +23,7 @@ int main()
         vfkv::AttnArgs a;
         a.kv.dtype = decltype(a.kv.dtype)(dtype); a.kv.n_kv_heads = hkv; a.kv.head_dim = d; a.kv.max_seq = hint;
         a.n_q_heads = hq; a.seq.n_seqs = seqs; a.seq.n_layers = layers; a.seq.positions = &positions; a.seq.max_len_hint = hint;
-        printf("%u\n", vfkv::choose_splits(&ctx, a, 128));
+        printf("%u %u\n", vfkv::choose_splits(&ctx, a, 128), vfkv::one_warp_tiles(&ctx, dtype, d, uint64_t(layers) * seqs * hkv));
     }
 }
 """
@@ -40,7 +40,8 @@ def splits(tmp_path_factory):
 
     def ask(dtype, hq, hkv, d, layers, seqs, hint):
         line = "%d %d %d %d %d %d %d\n" % (int(vf.KvDtype[dtype]), hq, hkv, d, layers, seqs, hint)
-        return int(subprocess.run([str(where / "main")], input=line, capture_output=True, text=True, check=True, timeout=60).stdout)
+        out = subprocess.run([str(where / "main")], input=line, capture_output=True, text=True, check=True, timeout=60).stdout
+        return [int(x) for x in out.split()]
     return ask
 
 
@@ -68,4 +69,15 @@ def splits(tmp_path_factory):
     ("F8", 32, 8, 128, 10, 4, 4096, 1, 1),
 ])
 def test_count(splits, dtype, hq, hkv, d, layers, seqs, hint, least, most):
-    assert least <= splits(dtype, hq, hkv, d, layers, seqs, hint) <= most
+    assert least <= splits(dtype, hq, hkv, d, layers, seqs, hint)[0] <= most
+
+
+@pytest.mark.parametrize("dtype,d,pairs,tiles", [
+    ("F8", 128, 444, 0), ("F8", 128, 445, 8), ("F8", 128, 888, 8), ("F8", 128, 889, 12), ("F8", 128, 1110, 12), ("F8", 128, 1111, 16),
+    ("F16", 128, 444, 0), ("F16", 128, 445, 10), ("F16", 128, 888, 10), ("F16", 128, 889, 16), ("F16", 128, 65535, 16),
+    ("F8", 256, 444, 0), ("F8", 256, 445, 8), ("F8", 256, 592, 8), ("F8", 256, 593, 12), ("F8", 256, 740, 12), ("F8", 256, 741, 16),
+    ("F16", 256, 592, 8), ("F16", 256, 593, 16), ("F16", 64, 592, 0), ("F16", 64, 593, 8), ("F16", 64, 1184, 8), ("F16", 64, 1185, 12),
+    ("F16", 64, 1480, 12), ("F16", 64, 1481, 16),
+])
+def test_tiles_of_a_sequence_for_a_warp(splits, dtype, d, pairs, tiles):
+    assert splits(dtype, 1, 1, d, 1, pairs, 100)[1] == tiles

@@ -153,6 +153,25 @@ int32_t launch_merge_partials_packed(vfkv_ctx *ctx, const float *packed, uint32_
     return check_cuda(ctx, cudaGetLastError(), "merge_partials_packed launch");
 }
 
+// The most tiles of a sequence that the tensor-core kernel gives to a warp by itself (attn_mma.cu, launch_c), by the CTAs of
+// the launch.  0 up to as many as are resident with 4 warps.  Up to twice that, a warp with more than eight tiles (ten of F16)
+// pays only if all sequences are equally long, and the longest, which the caller names, says nothing of the others; from two and a
+// half times on sixteen pay either way.  Times of four warps / of one, all as long and spread from a 32nd to that, of 128 dims:
+//   520 CTAs, FP8   8 tiles 1.14 0.97   10 1.15 0.87   16 0.97 0.72        F16   10 1.23 0.99   12 1.11 0.91   16 1.03 0.81
+//   896             12 1.16 1.06   14 1.23 0.98   16 1.12 0.93             F16   16 1.13 1.09
+//   1184            16 1.09 1.06                                           F16   16 1.11 1.22
+// 64 dims, four CTAs an SM: 720 8 0.97 0.98, 10 0.95 0.95; 1184 12 1.04 1.04, 16 0.97 0.94.  256 dims, two CTAs an SM: 520, FP8, 8
+// 1.12 0.98, 10 1.22 0.92; 600 12 1.19 0.94; 720 12 1.18 1.02, 16 1.15 0.99; F16, 600 16 1.26 1.06; at three an SM, where it begins, 8 1.11 0.96.
+uint32_t one_warp_tiles(const vfkv_ctx *ctx, uint32_t dtype, uint32_t head_dim, uint64_t ctas)
+{
+    const uint64_t n_sm = uint64_t(ctx->sm_count), resident = n_sm * (head_dim == 64 ? 4u : head_dim == 128 ? 3u : 2u);
+    const bool f16 = dtype == VFKV_F16;
+    if (ctas <= (head_dim == 64 ? resident : 3 * n_sm)) return 0u;
+    if (2 * ctas > 5 * resident) return 16u;
+    if (ctas > 2 * resident) return f16 && head_dim != 64 ? 16u : 12u;
+    return f16 && head_dim == 128 ? 10u : 8u;
+}
+
 // Expected time (us) of a tensor-core decode launch with n splits of sequences of len positions, base (sequence, kv-head)
 // pairs: a wave of CTAs costs 8 us and its stream, splits cost their merge.  An SM streams 39 KB a us with one CTA of 8 warps, 27
 // with two of 4 and 17 with one of those (HBM, shared, is in that); a CTA works through its positions in rounds of a tile for

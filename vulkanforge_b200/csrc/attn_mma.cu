@@ -1636,17 +1636,18 @@ int32_t launch_c(vfkv_ctx *ctx, const CUtensorMap &tk, const CUtensorMap &tv, co
     constexpr bool kOk2 = Shape<DT, D, 4, 2>::SMEM_BYTES <= kTwoPerSm && kMergeBytes <= Shape<DT, D, 4, 2>::RING_BYTES;
     constexpr bool kOk1 = Shape<DT, D, 4, 1>::SMEM_BYTES <= kTwoPerSm && kMergeBytes <= Shape<DT, D, 4, 1>::RING_BYTES;
     const uint32_t longest = mp.a.window && mp.a.window < mp.longest ? mp.a.window : mp.longest;
-    // Sequences of a few tiles, more of them than 4-warp CTAs are resident at a time: a warp each.  A CTA of four warps is then
-    // setting up, joining its warps and writing for most of its life, and two or three of them share an SM; of these
-    // there are up to twelve (256 dims: six; five to eight heads a kv-head: nine, by registers), which share nothing.  32 layers x 32 sequences, 32 q / 8 kv / 128, FP8: 24 positions 84.6 ->
+    // Sequences of a few tiles, more of them than 4-warp CTAs are resident at a time: a warp each (one_warp_tiles() has the lines).
+    // A CTA of four warps is then setting up, joining its warps and writing for most of its life, and two or three of them share
+    // an SM; of these there are up to twelve (256 dims: six; five to eight heads a kv-head: nine, by registers), which share
+    // nothing.  32 layers x 32 sequences, 32 q / 8 kv / 128, FP8: 24 positions 84.6 ->
     // 29.9 us, 128 92 -> 55, 256 123 -> 94, 400 163 -> 146, 600 208 -> 207; F16, 16 q / 8 kv / 256: 64 164 -> 103, 256 358 -> 320;
     // 16 layers x 4 sequences, FP8: 64 8.7 -> 5.8, 256 11.7 -> 10.0 (where the 4-warp CTAs run side by side, at most 2 tiles
     // are as fast); 4 layers x 32 sequences, 64 q / 8 kv / 256, FP8, where it spills 0.3 KB a thread: 30 33 -> 18, 250 52 -> 48.
     // Three stages a warp where they cost no further wave, counted by shared memory (2048 sequences of 400: 50 us with two, 42
     // with three).
-    if (w == 0 && mp.a.n_splits == 1u && mp.a.fan == nullptr && ctas > uint64_t(ctx->sm_count) * (D == 64 ? 4u : 3u)) {
+    if (w == 0 && mp.a.n_splits == 1u && mp.a.fan == nullptr) {
         const uint32_t tiles = (longest + Shape<DT, D, 1, 2>::TP - 1) / Shape<DT, D, 1, 2>::TP;
-        if (tiles <= 16u) {
+        if (tiles <= one_warp_tiles(ctx, DT, D, ctas)) {
             auto waves = [&](uint64_t smem) {
                 const uint64_t slots = uint64_t(ctx->sm_count) * std::min<uint64_t>(12u, 227u * 1024u / (smem + 1024u));
                 return (ctas + slots - 1) / slots;

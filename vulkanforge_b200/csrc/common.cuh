@@ -329,6 +329,7 @@ int32_t launch_fanout_push(vfkv_ctx *ctx, const PeerFanout &fan, const float *st
 
 // attention implementations
 uint32_t choose_splits(const vfkv_ctx *ctx, const AttnArgs &a, uint32_t tile);
+uint32_t one_warp_tiles(const vfkv_ctx *ctx, uint32_t dtype, uint32_t head_dim, uint64_t ctas);
 int32_t launch_attn_generic(vfkv_ctx *ctx, vfkv_workspace *ws, const AttnArgs &a, uint32_t n_splits,
                             cudaStream_t st);
 bool attn_mma_supported(const AttnArgs &a);

@@ -853,7 +853,7 @@ int32_t vfkv_decode_token(vfkv_cache *cache, vfkv_workspace *ws, const float *d_
 // K/V streams of other CTAs hide the bus.  In one wave all CTAs wait for the bus at once, and what a kernel fetches in front of
 // the launch is there sooner.  `fetched`: a kernel would (and not copies, which any such launch beats: 64 q / 8 kv, 336 pairs
 // of 60, 3.1 MB 98 -> 85 us).  `longest`: of the sequences.  Against that kernel, in us fetched / read by the attention kernel:
-//   up to two CTAs an SM: 288 pairs of 8192, FP8 132 / 140 (142 and 143 on two more hosts, 125 on a fourth); 288 of 100 48 / 55
+//   up to two CTAs an SM: 288 pairs of 8192, FP8 132 / 140 (142 and 143 on two more hosts, 124 and 125 on two others); 288 of 100 48 / 55
 //   up to three, unless rows of 300 KB to 2 MB hide it: F16, 320 of 209 54 / 59, of 1577 92 / 87; 400 of 600 73 / 70; FP8, 320 of
 //   1577 73 / 73, of 4000 113 / 110, of 8192 180 / 184 (and not for groups of more than four heads: 336 of 3000 111 / 117)
 //   up to four, where a pair has less than 150 KB: FP8, 464 of 60 65 / 71, 576 81 / 83; 464 of 600 71 / 72, 576 84 / 82
